@@ -2,7 +2,7 @@
 // trees in one persistent launch per phase.  The reference has no batched
 // form; every request has the semantics of its per-call search (search.cuh).
 //
-// Work is cut into chunks of one warp (BATCH_CHUNK threads); each warp takes
+// Work is cut into chunks of up to BATCH_CHUNK queries; each warp takes
 // the next chunk index from a device counter, finds the request it belongs to
 // by a binary search over the requests' first chunks, and runs that request's
 // search body on it.  So small requests of many trees fill the GPU together,
@@ -17,7 +17,7 @@
 namespace ikdg {
 namespace {
 
-constexpr int WARPS_PER_CTA = BATCH_THREADS / BATCH_CHUNK;
+constexpr int WARPS_PER_CTA = BATCH_THREADS / 32;
 
 // Last r in [lo, hi) with starts[r] <= c (starts ascending, starts[lo] <= c).
 __device__ __forceinline__ int find_req(const long long* __restrict__ starts, int lo, int hi, long long c) {
@@ -31,19 +31,21 @@ __device__ __forceinline__ int find_req(const long long* __restrict__ starts, in
     return lo;
 }
 
-// Phase 1 for one class: KC 0..3 are kNN requests with k <= 1, 2, 4, 8 (lists
-// in registers), KC = BATCH_SMEM_CLASS kNN with k <= 16 (lists in shared
-// memory), all producing their final rows; KC = BATCH_RANGE_CLASS box and
-// radius requests (per-query hit counts in counts[cbase + qi]).  One kernel
-// per class keeps each at its own register count.
-template <int KC, int G>
+// Phase 1 for one class: KC 0..2 are kNN requests with k <= 4, 8, 16 (four lanes
+// per query, the list in 1, 2 or 4 registers a lane), producing their final rows;
+// KC = BATCH_RANGE_CLASS box and radius requests (per-query hit counts in
+// counts[cbase + qi]).  One kernel per class keeps each at its own register
+// count.  entries: kNN stack entries per thread (dynamic shared memory).
+template <int KC>
 __global__ void __launch_bounds__(BATCH_THREADS) batch_search_kernel(const DevTree* __restrict__ trees,
                                                                      const BatchReq* __restrict__ reqs,
                                                                      const long long* __restrict__ req_c1, int r0,
                                                                      int r1, long long c_begin, long long c_end,
                                                                      long long* __restrict__ counts,
-                                                                     unsigned long long* __restrict__ ctr) {
-    constexpr int KM = KC == 0 ? 1 : KC == 1 ? 2 : KC == 2 ? 4 : 8;
+                                                                     unsigned long long* __restrict__ ctr,
+                                                                     int entries) {
+    constexpr int G = search::KNN_G, R = KC == 0 ? 1 : KC == 1 ? 2 : 4;
+    extern __shared__ int2 batch_sm[];
     const int lane = threadIdx.x & 31;
     for (;;) {
         // Each warp takes its own chunk: no warp waits for another.
@@ -56,37 +58,38 @@ __global__ void __launch_bounds__(BATCH_THREADS) batch_search_kernel(const DevTr
         c = __shfl_sync(0xffffffffu, c, 0);
         r = __shfl_sync(0xffffffffu, r, 0);
         if (c >= c_end) break;
-        const BatchReq& R = reqs[r];
-        const DevTree t = trees[R.tree];
-        if constexpr (KC == BATCH_SMEM_CLASS) {
-            // 8 < k <= 16: each group's sorted list in shared memory, entry j
-            // of group g at [j * groups + g] (as the per-call kernel does)
-            extern __shared__ float batch_sm[];
-            constexpr int groups = BATCH_THREADS / G;
-            float* sd = batch_sm;
-            int* si = reinterpret_cast<int*>(sd + groups * BATCH_KMAX);
-            int* ss = si + groups * BATCH_KMAX;
-            const int g = threadIdx.x / G;
-            const long long tid = (c - R.c1) * (BATCH_CHUNK / G) + lane / G;
-            search::knn_body<0, G>(t, tid, R.q, R.q_stride, R.nq, R.k, R.max_sq, R.ids, R.d2, R.xyz, R.cnt, nullptr,
-                                   R.perm, sd + g, si + g, ss + g, groups);
-        } else if constexpr (KC < BATCH_RANGE_CLASS) {
-            const long long tid = (c - R.c1) * (BATCH_CHUNK / G) + lane / G;
-            search::knn_body<KM, G>(t, tid, R.q, R.q_stride, R.nq, R.k, R.max_sq, R.ids, R.d2, R.xyz, R.cnt, nullptr,
-                                    R.perm);
+        const BatchReq& Rq = reqs[r];
+        const DevTree t = trees[Rq.tree];
+        if constexpr (KC < BATCH_RANGE_CLASS) {
+            static_assert(G * BATCH_KNN_STEP == 32 && BATCH_THREADS == search::KNN_CTA, "a warp's queries, the stack columns");
+            const search::KnnLane g;
+            int2* stk = batch_sm + threadIdx.x;
+            const search::KnnOut o{Rq.ids, Rq.d2, Rq.xyz, Rq.cnt};
+            const long long q0 = (c - Rq.c1) * Rq.per;
+            for (int i = 0; i < Rq.per && q0 + i < Rq.nq; i += BATCH_KNN_STEP) {
+                long long qi = q0 + i + lane / G;
+                const bool valid = qi < Rq.nq;
+                if (valid && Rq.perm != nullptr) qi = __ldg(Rq.perm + qi);
+                if (!valid) qi = 0;
+                const float* q = Rq.q + qi * Rq.q_stride;
+                const float qx = valid ? q[0] : 0.f, qy = valid ? q[1] : 0.f, qz = valid ? q[2] : 0.f;
+                float ld[R];
+                int ls[R];
+                search::knn_group<R>(t, g, valid, qx, qy, qz, Rq.k, Rq.max_sq, stk, entries, 16, ld, ls);
+                search::knn_write_rows<R>(t, g, valid, ld, ls, Rq.k, qi, o);
+            }
         } else {
             // warp-collective body: every lane calls it
-            long long qi = (c - R.c1) * BATCH_CHUNK + lane;
-            const bool valid = qi < R.nq;
-            if (valid && R.perm != nullptr) qi = __ldg(R.perm + qi);
+            long long qi = (c - Rq.c1) * BATCH_CHUNK + lane;
+            const bool valid = qi < Rq.nq;
+            if (valid && Rq.perm != nullptr) qi = __ldg(Rq.perm + qi);
             const long long n =
-                R.kind == BATCH_BOX
-                    ? search::range_body<0, search::RANGE_COUNT>(t, R.q, R.q_stride, nullptr, 0, qi, valid, 0, 0,
+                Rq.kind == BATCH_BOX
+                    ? search::range_body<0, search::RANGE_COUNT>(t, Rq.q, Rq.q_stride, nullptr, 0, qi, valid, 0, 0,
                                                                  nullptr, nullptr)
-                    : search::range_body<1, search::RANGE_COUNT>(t, R.q, R.q_stride, R.radius, R.r_stride, qi, valid,
-                                                                 0, 0,
-                                                   nullptr, nullptr);
-            if (valid) counts[R.cbase + qi] = n;
+                    : search::range_body<1, search::RANGE_COUNT>(t, Rq.q, Rq.q_stride, Rq.radius, Rq.r_stride, qi,
+                                                                 valid, 0, 0, nullptr, nullptr);
+            if (valid) counts[Rq.cbase + qi] = n;
         }
     }
 }
@@ -181,9 +184,11 @@ __global__ void batch_key_kernel(const DevTree* __restrict__ trees, const BatchR
 
 std::mutex g_grid_mu;
 
-// Dynamic shared memory of a search kernel class (the k <= 16 lists).
-size_t class_smem(int kc, int lanes) {
-    return kc == BATCH_SMEM_CLASS ? (size_t)(BATCH_THREADS / lanes) * BATCH_KMAX * 12 : 0;
+// Dynamic shared memory of a search kernel class: the kNN stacks.
+size_t class_smem(int kc, int height) {
+    return kc < BATCH_RANGE_CLASS
+               ? sizeof(int2) * search::knn_stack_entries(height) * BATCH_THREADS
+               : 0;
 }
 
 int resident_grid(const void* fn, size_t smem = 0) {
@@ -197,62 +202,20 @@ int resident_grid(const void* fn, size_t smem = 0) {
     return (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
 }
 
-}  // namespace
-
-int batch_kclass(int k) { return k <= 1 ? 0 : k <= 2 ? 1 : k <= 4 ? 2 : k <= 8 ? 3 : 4; }
-
-namespace {
-
-template <int KC, int G>
-void search_variant(bool launch, int* grid, const DevTree* trees, const BatchReq* reqs, const long long* req_c1,
-                    int r0, int r1, long long c_begin, long long c_end, long long* counts, unsigned long long* ctr,
-                    unsigned g, cudaStream_t s) {
-    const size_t smem = class_smem(KC, G);
-    if (!launch) {
-        *grid = resident_grid((const void*)batch_search_kernel<KC, G>, smem);
-        return;
-    }
-    batch_search_kernel<KC, G><<<g, BATCH_THREADS, smem, s>>>(trees, reqs, req_c1, r0, r1, c_begin, c_end, counts,
-                                                              ctr);
-}
-
-template <int KC>
-void search_lanes(int lanes, bool launch, int* grid, const DevTree* trees, const BatchReq* reqs,
-                  const long long* req_c1, int r0, int r1, long long c_begin, long long c_end, long long* counts,
-                  unsigned long long* ctr, unsigned g, cudaStream_t s) {
-    if (lanes >= 4)
-        search_variant<KC, 4>(launch, grid, trees, reqs, req_c1, r0, r1, c_begin, c_end, counts, ctr, g, s);
-    else if (lanes == 2)
-        search_variant<KC, 2>(launch, grid, trees, reqs, req_c1, r0, r1, c_begin, c_end, counts, ctr, g, s);
-    else
-        search_variant<KC, 1>(launch, grid, trees, reqs, req_c1, r0, r1, c_begin, c_end, counts, ctr, g, s);
-}
-
-void search_dispatch(int kc, int lanes, bool launch, int* grid, const DevTree* trees, const BatchReq* reqs,
-                     const long long* req_c1, int r0, int r1, long long c_begin, long long c_end, long long* counts,
-                     unsigned long long* ctr, unsigned g, cudaStream_t s) {
-#define IKDG_BKC(KC) search_lanes<KC>(lanes, launch, grid, trees, reqs, req_c1, r0, r1, c_begin, c_end, counts, ctr, g, s)
-    switch (kc) {
-        case 0: IKDG_BKC(0); break;
-        case 1: IKDG_BKC(1); break;
-        case 2: IKDG_BKC(2); break;
-        case 3: IKDG_BKC(3); break;
-        case 4: IKDG_BKC(4); break;
-        default:
-            search_variant<BATCH_RANGE_CLASS, 1>(launch, grid, trees, reqs, req_c1, r0, r1, c_begin, c_end, counts,
-                                                 ctr, g, s);
-            break;
-    }
-#undef IKDG_BKC
+typedef void (*SearchKernel)(const DevTree*, const BatchReq*, const long long*, int, int, long long, long long,
+                             long long*, unsigned long long*, int);
+SearchKernel search_kernel(int kc) {
+    return kc == 0 ? batch_search_kernel<0> : kc == 1 ? batch_search_kernel<1> : kc == 2 ? batch_search_kernel<2>
+                                                                              : batch_search_kernel<BATCH_RANGE_CLASS>;
 }
 
 }  // namespace
 
-int batch_search_grid(int kclass, int lanes) {
+int batch_kclass(int k) { return k <= 4 ? 0 : k <= 8 ? 1 : 2; }
+
+int batch_search_grid(int kclass, int height) {
     std::lock_guard<std::mutex> lock(g_grid_mu);
-    int grid = 0;
-    search_dispatch(kclass, lanes, false, &grid, nullptr, nullptr, nullptr, 0, 0, 0, 0, nullptr, nullptr, 0, nullptr);
-    return grid;
+    return resident_grid((const void*)search_kernel(kclass), class_smem(kclass, height));
 }
 
 int batch_write_grid() {
@@ -261,12 +224,13 @@ int batch_write_grid() {
 }
 
 void launch_batch_search(const DevTree* trees, const BatchReq* reqs, const long long* req_c1, int r0, int r1,
-                         long long c_begin, long long c_end, int kclass, int lanes, long long* counts,
+                         long long c_begin, long long c_end, int kclass, int height, long long* counts,
                          unsigned long long* ctr, int grid, cudaStream_t s) {
     if (c_end <= c_begin || r1 <= r0) return;
     const long long ctas = (c_end - c_begin + WARPS_PER_CTA - 1) / WARPS_PER_CTA;
     const unsigned g = (unsigned)(ctas < grid ? ctas : grid);
-    search_dispatch(kclass, lanes, true, nullptr, trees, reqs, req_c1, r0, r1, c_begin, c_end, counts, ctr, g, s);
+    search_kernel(kclass)<<<g, BATCH_THREADS, class_smem(kclass, height), s>>>(
+        trees, reqs, req_c1, r0, r1, c_begin, c_end, counts, ctr, search::knn_stack_entries(height));
 }
 
 void launch_batch_keys(const DevTree* trees, const BatchReq* reqs, const long long* qstart, int n, long long total,

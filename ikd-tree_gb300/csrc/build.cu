@@ -125,6 +125,7 @@ __global__ void level_seg_kernel(DevTree t, const float4* __restrict__ pts, cons
         write_child_box(t.node, parent, side, b);
         write_child_code(t.node, parent, side, leaf_code(L));
         write_child_cnt(t.ncnt, parent, side, cnt, 0);
+        wide_link(t, t.winfo[parent], side, leaf_code(L), b, cnt);
         seginfo[i] = make_int4(KIND_LEAF, L, s, 0);
         return;
     }
@@ -149,6 +150,9 @@ __global__ void level_seg_kernel(DevTree t, const float4* __restrict__ pts, cons
     write_child_box(t.node, parent, side, b);
     write_child_code(t.node, parent, side, X);
     write_child_cnt(t.ncnt, parent, side, cnt, 0);
+    const int2 wi = t.winfo[parent];
+    wide_link(t, wi, side, X, b, cnt);
+    t.winfo[X] = wide_below(wi, side, X);
     int r = atomicAdd(nseg_next, 2);
     if (r + 1 >= max_next) {  // cannot happen with the host's bound; guard anyway
         atomicOr(&t.st->err, ERR_SEG);
@@ -258,6 +262,8 @@ struct LbShared {
     } u;
     uint16_t ss[2][SEGS], se[2][SEGS];
     int slink[2][SEGS];
+    int swide[2][SEGS];        // wide record above the segment's parent, its position there
+    uint8_t swpos[2][SEGS];
     int snode[SEGS];           // node or leaf index, -1 when allocation failed
     uint16_t snext[SEGS];      // first child segment of a node
     int8_t saxis[SEGS];        // split axis, -1 for leaves
@@ -402,6 +408,9 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 4) local_build_
             sm.ss[0][0] = 0;
             sm.se[0][0] = (uint16_t)n;
             sm.slink[0][0] = jb.z;
+            const int2 wi = t.winfo[jb.z >> 1];
+            sm.swide[0][0] = wi.x;
+            sm.swpos[0][0] = (uint8_t)wi.y;
             // The whole subtree's nodes and leaves from the pools at once
             // (its shape follows from n and the fill); level l takes the
             // indices after those of levels 0 .. l-1.
@@ -455,6 +464,7 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 4) local_build_
                 const uint32_t wb = sm.wsum[warp];
                 const unsigned below = (1u << lane) - 1u;
                 const int parent = link >> 1, side = link & 1;
+                const int2 wi = make_int2(sm.swide[cb][sg], sm.swpos[cb][sg]);
                 Box3 b = empty_box();
                 if (cnt > 0)
                     for (int a = 0; a < 3; ++a) {
@@ -474,6 +484,7 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 4) local_build_
                         write_child_box(t.node, parent, side, b);
                         write_child_code(t.node, parent, side, leaf_code(L));
                         write_child_cnt(t.ncnt, parent, side, cnt, 0);
+                        wide_link(t, wi, side, leaf_code(L), b, cnt);
                     }
                 } else {
                     const int X = pool_pick(sm.run_node, t.free_node, sm.free_node_n, t.node_cap,
@@ -501,6 +512,11 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 4) local_build_
                         write_child_box(t.node, parent, side, b);
                         write_child_code(t.node, parent, side, X);
                         write_child_cnt(t.ncnt, parent, side, cnt, 0);
+                        wide_link(t, wi, side, X, b, cnt);
+                        const int2 wx = wide_below(wi, side, X);
+                        t.winfo[X] = wx;
+                        sm.swide[cb ^ 1][r] = sm.swide[cb ^ 1][r + 1] = wx.x;
+                        sm.swpos[cb ^ 1][r] = sm.swpos[cb ^ 1][r + 1] = (uint8_t)wx.y;
                         sm.ss[cb ^ 1][r] = (uint16_t)s;
                         sm.se[cb ^ 1][r] = (uint16_t)mid;
                         sm.slink[cb ^ 1][r] = X * 2;
@@ -751,6 +767,9 @@ __global__ void __launch_bounds__(MID_THREADS, 1) mid_level_kernel(DevTree t, co
                 write_child_box(t.node, parent, side, b);
                 write_child_code(t.node, parent, side, X);
                 write_child_cnt(t.ncnt, parent, side, cnt, 0);
+                const int2 wi = t.winfo[parent];
+                wide_link(t, wi, side, X, b, cnt);
+                t.winfo[X] = wide_below(wi, side, X);
             }
         }
         __syncthreads();

@@ -171,15 +171,14 @@ struct Tree {
     float del_param = 0.5f, bal_param = 0.6f, ds_size = 0.2f;
     int fill = 16;
     int min_size = 2 * LEAF_CAP;
-    int knn_lanes = 1;     // threads per kNN query (1, 2 or 4)
     // Tree levels used to order a kNN batch before the search: -1 (default)
-    // = QBIN_BITS for batches of at least QBIN_AUTO_QUERIES queries, none
-    // below (measured on the 1M-point map: -12 % at 1M queries, +16 % at
-    // 100k); 0 = never; 1..16 = always (batches of QBIN_MIN_QUERIES or more).
+    // = QBIN_AUTO_BITS for large batches and lists on trees larger than the L2
+    // cache, none otherwise; 0 = never; 1..16 = always (batches of
+    // QBIN_MIN_QUERIES or more).
     int knn_bin_bits = -1;
-    int bin_bits_for(long long nq) const {
+    int bin_bits_for(long long nq, int k) const {
         if (knn_bin_bits >= 0) return knn_bin_bits;
-        return nq >= QBIN_AUTO_QUERIES ? QBIN_BITS : 0;
+        return nq >= QBIN_AUTO_QUERIES && k >= QBIN_AUTO_K && st->root_slots >= QBIN_AUTO_SLOTS ? QBIN_AUTO_BITS : 0;
     }
     // On Grace-Blackwell the GPU reads and writes pageable host memory through
     // NVLink-C2C with the CPU's page tables (cudaDevAttrPageableMemoryAccess).
@@ -241,6 +240,8 @@ struct Tree {
         free_array(dt.ncnt);
         free_array(dt.nparent);
         free_array(dt.nheight);
+        free_array(dt.wide);
+        free_array(dt.winfo);
         free_array(dt.pts);
         free_array(dt.leaf_n);
         free_array(dt.lparent);
@@ -285,6 +286,8 @@ struct Tree {
             grow_array(dt.ncnt, old_n, new_n, 0, stream);
             grow_array(dt.nparent, old_n, new_n, 0xff, stream);
             grow_array(dt.nheight, old_n, new_n, 0, stream);
+            grow_array(dt.wide, (size_t)old_n * 16, (size_t)new_n * 16, -1, stream);
+            grow_array(dt.winfo, old_n, new_n, -1, stream);
             grow_array(dt.free_node, old_n, new_n, -1, stream);
             grow_array(aux.pend, old_n, new_n, 0, stream);
             grow_array(aux.arrive, old_n, new_n, 0, stream);
@@ -337,10 +340,24 @@ struct Tree {
         removed_cap = nc;
     }
 
+    // The root's position in the top wide record (see common.cuh), and what
+    // the searches need to know of the tree's shape.
+    int top_pos = 2;
+    void set_top(long long points) {
+        const int below = build_levels(std::max<long long>(points, 1), fill) - 1;  // levels below the root
+        top_pos = below % 3 == 2 ? 2 : below % 3 == 1 ? 4 : 8;
+        launch_set_top(dt, top_pos, stream);
+    }
+    void set_search_start() {
+        dt.height = st->root_height;
+        dt.start = top_pos == 8 && st->root_code > 0 ? st->root_code : 0;
+    }
+
     // ---- status ------------------------------------------------------------------
     void read_status() {
         CK(cudaMemcpyAsync(st, st_dev, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream));
         CK(cudaStreamSynchronize(stream));
+        set_search_start();
         if (st->err & ERR_ANY_INTERNAL) {
             int e = st->err;
             std::string m = "device error:";
@@ -389,12 +406,22 @@ struct Tree {
         CK(cudaMemcpyAsync(dt.ncnt, &zc, sizeof(zc), cudaMemcpyHostToDevice, stream));
         CK(cudaMemcpyAsync(dt.nparent, &minus1, sizeof(int), cudaMemcpyHostToDevice, stream));
         CK(cudaMemcpyAsync(dt.nheight, &h0, sizeof(int), cudaMemcpyHostToDevice, stream));
+        // the top wide record: owned by the sentinel, every slot empty
+        const int2 top = make_int2(0, 1);
+        CK(cudaMemcpyAsync(dt.winfo, &top, sizeof(top), cudaMemcpyHostToDevice, stream));
+        float slots[8 * WIDE];
+        for (int i = 0; i < WIDE; ++i)
+            for (int f = 0; f < 8; ++f) slots[wide_at(i, f)] = f < 3 ? inf : f < 6 ? -inf : 0.f;
+        CK(cudaMemcpyAsync(dt.wide, slots, sizeof(slots), cudaMemcpyHostToDevice, stream));
         CK(cudaStreamSynchronize(stream));  // the sources above live on this stack frame
         st->node_top = 1;
         st->leaf_top = 0;
         st->free_node_n = st->free_leaf_n = 0;
         st->root_code = 0;
         st->root_slots = st->root_deleted = 0;
+        st->root_height = 0;
+        top_pos = 2;
+        set_search_start();
     }
 
     // ---- rebuild jobs ---------------------------------------------------------------
@@ -539,6 +566,7 @@ struct Tree {
         bld.ensure(build_scratch_bytes(nn, 1, fill) + 4096, stream);
         BuildScratch bs;
         carve_build_scratch(bld.p, nn, 1, fill, &bs);
+        set_top(n);
         build_subtrees(dt, pts, n, job, job + 2, 1, nn, fill, bs, stream);
         launch_snapshot_root(dt, stream);
         read_status();
@@ -821,7 +849,7 @@ struct Tree {
             }
             launch_knn(t, qsrc, stride, nq, k, max_sq_threshold(max_dist), (int*)(c->d + o_ids),
                        (float*)(c->d + o_d2), xyz ? (float*)(c->d + o_xyz) : nullptr,
-                       cnt ? (int*)(c->d + o_cnt) : nullptr, c->d + o_tmp, knn_lanes, bin_bits_for(nq), c->s);
+                       cnt ? (int*)(c->d + o_cnt) : nullptr, c->d + o_tmp, bin_bits_for(nq, k), c->s);
             CK(cudaGetLastError());
             CK(cudaMemcpyAsync(c->h, c->d, o_end, cudaMemcpyDeviceToHost, c->s));
             CK(cudaStreamSynchronize(c->s));
@@ -849,7 +877,7 @@ struct Tree {
         size_t nk = (size_t)nq * k;
         if (device_ptrs) {
             small.ensure(knn_temp_bytes(nq, k) + 256, stream);
-            launch_knn(dt, q, stride, nq, k, lim, ids, d2, xyz, cnt, small.p, knn_lanes, bin_bits_for(nq), stream);
+            launch_knn(dt, q, stride, nq, k, lim, ids, d2, xyz, cnt, small.p, bin_bits_for(nq, k), stream);
             CK(cudaGetLastError());
             return;
         }
@@ -861,7 +889,7 @@ struct Tree {
             // transfer over the chip link overlaps the search instead of
             // following it as one copy.
             small.ensure(knn_temp_bytes(nq, k) + 256, stream);
-            launch_knn(dt, q, stride, nq, k, lim, ids, d2, xyz, cnt, small.p, knn_lanes, bin_bits_for(nq), stream,
+            launch_knn(dt, q, stride, nq, k, lim, ids, d2, xyz, cnt, small.p, bin_bits_for(nq, k), stream,
                        /*host_out=*/true);
             read_status();
             if (st->err & ERR_STACK) throw Internal{"knn: traversal stack overflow"};
@@ -884,7 +912,7 @@ struct Tree {
             CK(cudaMemcpyAsync(dq, q, sizeof(float) * nq * stride, cudaMemcpyHostToDevice, stream));
             qsrc = dq;
         }
-        launch_knn(dt, qsrc, stride, nq, k, lim, dids, dd2, dxyz, dcnt, temp, knn_lanes, bin_bits_for(nq), stream);
+        launch_knn(dt, qsrc, stride, nq, k, lim, dids, dd2, dxyz, dcnt, temp, bin_bits_for(nq, k), stream);
         CK(cudaMemcpyAsync(ids, dids, sizeof(int) * nk, cudaMemcpyDeviceToHost, stream));
         CK(cudaMemcpyAsync(d2, dd2, sizeof(float) * nk, cudaMemcpyDeviceToHost, stream));
         if (xyz) CK(cudaMemcpyAsync(xyz, dxyz, sizeof(float) * nk * 3, cudaMemcpyDeviceToHost, stream));
@@ -987,7 +1015,7 @@ struct Tree {
     void p2p_forward(const float* scan, long long n, const double* pose, int k, double max_dist, float thresh,
                      float* planes, float* res, int* valid, double* loss) {
         if (n < 0 || scan == nullptr || pose == nullptr || planes == nullptr || res == nullptr || valid == nullptr ||
-            k < 3 || k > KNN_SMEM_MAX)
+            k < 3 || k > KNN_GROUP_MAX)
             throw BadArg{"p2p_forward: bad arguments"};
         if (loss) *loss = 0;
         if (n == 0) return;
@@ -1008,7 +1036,7 @@ struct Tree {
         char* temp = c.take<char>(knn_temp_bytes(n, k));
         upload_pose(pose, Rt);
         launch_transform(scan, n, Rt, w, stream);
-        launch_knn(dt, w, 3, n, k, max_sq_threshold(max_dist), ids, d2, nbr, cnt, temp, knn_lanes, bin_bits_for(n),
+        launch_knn(dt, w, 3, n, k, max_sq_threshold(max_dist), ids, d2, nbr, cnt, temp, bin_bits_for(n, k),
                    stream);
         launch_plane_residual(scan, Rt, n, k, nbr, cnt, thresh, (float4*)planes, res, valid, part, stream);
         std::vector<double> h(nb);
@@ -1133,6 +1161,7 @@ struct Tree {
         if (st->root_code == 0) return;
         reset_counters();
         launch_select_root_job(dt, aux, stream);
+        set_top((long long)st->root_slots - st->root_deleted);
         run_jobs(1, nullptr, nullptr, 0);
         // run_jobs already refit the root's parent (the sentinel: nothing to do)
         finish_update(nullptr, nullptr, 0, /*refit_first=*/false);
@@ -1189,10 +1218,9 @@ struct Batch {
         BatchReq d{};
         Tree* tree = nullptr;
         double max_dist = 0;
-        int lanes = 0;  // 0: the tree's kNN lanes setting
     };
     struct Group {
-        int kclass, lanes, r0, r1;
+        int kclass, r0, r1;
         long long c_begin, c_end;
         int grid;
     };
@@ -1214,6 +1242,7 @@ struct Batch {
 
     // plan (rebuilt when requests change)
     bool planned = false;
+    int plan_height = 0;             // the kNN stacks of the plan hold trees this tall
     std::vector<Tree*> trees;
     std::vector<int> order;          // sorted position -> request
     std::vector<int> range_reqs;     // request indices of range requests, in order added
@@ -1302,14 +1331,11 @@ struct Batch {
     }
 
     int req_class(const Req& r) const { return r.d.kind == BATCH_KNN ? batch_kclass(r.d.k) : BATCH_RANGE_CLASS; }
-    int req_lanes(const Req& r) const {
-        if (r.d.kind != BATCH_KNN) return 1;
-        int l = r.lanes > 0 ? r.lanes : r.tree->knn_lanes;
-        return l >= 4 ? 4 : l >= 2 ? 2 : 1;
-    }
-
-    void plan() {
+    // height: room for trees this tall (and a few levels more, so that a tree
+    // that grows a little needs no new plan).
+    void plan(int height) {
         drop_plan();
+        plan_height = std::min(height + 3, MAX_STACK);
         const int n = (int)reqs.size();
         trees.clear();
         range_reqs.clear();
@@ -1323,31 +1349,39 @@ struct Batch {
         order.resize(n);
         for (int i = 0; i < n; ++i) order[i] = i;
         std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-            int ka = req_class(reqs[a]) * 8 + req_lanes(reqs[a]), kb = req_class(reqs[b]) * 8 + req_lanes(reqs[b]);
-            return ka < kb;
+            return req_class(reqs[a]) < req_class(reqs[b]);
         });
         // device descriptors, sorted order
         std::vector<BatchReq> d(n);
         std::vector<long long> c1(n);
         groups.clear();
         long long chunk = 0, cbase = 0;
+        // kNN queries per chunk, by class: as many as leave every resident warp
+        // four chunks (fewer trips to the shared counter), at least one step's.
+        int per[BATCH_RANGE_CLASS];
+        for (int kc = 0; kc < BATCH_RANGE_CLASS; ++kc) {
+            long long total = 0;
+            for (auto& r : reqs)
+                if (req_class(r) == kc) total += r.d.nq;
+            const long long warps = 4ll * batch_search_grid(kc, plan_height);
+            per[kc] = BATCH_CHUNK;
+            while (per[kc] > BATCH_KNN_STEP && total / per[kc] < 4 * warps) per[kc] /= 2;
+        }
         for (int p = 0; p < n; ++p) {
             Req& r = reqs[order[p]];
             BatchReq b = r.d;
             b.tree = tree_of[order[p]];
-            const int kc = req_class(r), lanes = req_lanes(r);
-            b.kclass = kc < BATCH_RANGE_CLASS ? kc : 0;
-            b.lanes = lanes;
-            const long long per = kc < BATCH_RANGE_CLASS ? BATCH_CHUNK / lanes : BATCH_CHUNK;
+            const int kc = req_class(r);
+            b.per = kc < BATCH_RANGE_CLASS ? per[kc] : BATCH_CHUNK;
             b.c1 = chunk;
-            b.n1 = (b.nq + per - 1) / per;
+            b.n1 = (b.nq + b.per - 1) / b.per;
             chunk += b.n1;
             if (b.kind != BATCH_KNN) {
                 b.cbase = cbase;
                 cbase += b.nq;
             }
-            if (groups.empty() || groups.back().kclass != kc || groups.back().lanes != lanes)
-                groups.push_back(Group{kc, lanes, p, p + 1, b.c1, chunk, 0});
+            if (groups.empty() || groups.back().kclass != kc)
+                groups.push_back(Group{kc, p, p + 1, b.c1, chunk, 0});
             else {
                 groups.back().r1 = p + 1;
                 groups.back().c_end = chunk;
@@ -1379,7 +1413,7 @@ struct Batch {
             chunk2 += b.n2;
         }
         c2_end = chunk2;
-        for (auto& g : groups) g.grid = batch_search_grid(g.kclass, g.lanes);
+        for (auto& g : groups) g.grid = batch_search_grid(g.kclass, plan_height);
         write_grid = batch_write_grid();
         // one allocation for the plan
         const size_t nt = trees.size(), nr = range_reqs.size();
@@ -1474,7 +1508,7 @@ struct Batch {
             const Group& G = groups[g];
             cudaStream_t s = g == 0 ? stream : branch[g - 1];
             if (g > 0) CK(cudaStreamWaitEvent(s, ev_fork, 0));
-            launch_batch_search(d_trees, d_reqs, d_c1, G.r0, G.r1, G.c_begin, G.c_end, G.kclass, G.lanes, d_counts,
+            launch_batch_search(d_trees, d_reqs, d_c1, G.r0, G.r1, G.c_begin, G.c_end, G.kclass, plan_height, d_counts,
                                 d_ctr + g, G.grid, s);
             if (g > 0) CK(cudaEventRecord(ev_join[g - 1], s));
         }
@@ -1489,18 +1523,33 @@ struct Batch {
         CK(cudaGetLastError());
     }
 
+    int tallest() {
+        int h = 0;
+        for (auto& r : reqs) {
+            std::unique_lock<std::shared_mutex> lock(r.tree->mu);
+            h = std::max(h, r.tree->dt.height);
+        }
+        return h;
+    }
+
     void run() {
         if (reqs.empty()) return;
-        if (!planned) plan();
+        if (!planned) plan(tallest());
         // the previous run's copy of h_trees must be done before it changes
         if (launched) CK(cudaEventSynchronize(ev_done));
-        for (size_t i = 0; i < trees.size(); ++i) {
-            Tree* t = trees[i];
-            std::unique_lock<std::shared_mutex> lock(t->mu);
-            h_trees[i] = t->dt;
-            h_trees[i].st = d_st;
-            CK(cudaEventRecord(ev_tree[i], t->stream));
-            CK(cudaStreamWaitEvent(stream, ev_tree[i], 0));
+        for (;;) {
+            int height = 0;
+            for (size_t i = 0; i < trees.size(); ++i) {
+                Tree* t = trees[i];
+                std::unique_lock<std::shared_mutex> lock(t->mu);
+                h_trees[i] = t->dt;
+                h_trees[i].st = d_st;
+                height = std::max(height, t->dt.height);
+                CK(cudaEventRecord(ev_tree[i], t->stream));
+                CK(cudaStreamWaitEvent(stream, ev_tree[i], 0));
+            }
+            if (height <= plan_height) break;
+            plan(height);  // a tree outgrew the plan's stacks
         }
         if (use_graph)
             CK(cudaGraphLaunch(exec, stream));
@@ -1555,11 +1604,9 @@ struct Batch {
 };
 
 // Per tree of the batch: the leaf fill (points per leaf when the tree is
-// rebuilt, 8..32) and the lanes per kNN query (1, 2, 4) with the fastest
-// median run of that tree's requests alone.  Leaves the tree rebuilt at the
-// chosen fill and the requests at the chosen lanes.
-void autotune_batch(Batch& b, int reps, const std::vector<int>& fills, const std::vector<int>& lanes_set,
-                    int* chosen) {
+// rebuilt, 8..32) with the fastest median run of that tree's requests alone.
+// Leaves the tree rebuilt at the chosen fill.
+void autotune_batch(Batch& b, int reps, const std::vector<int>& fills, int* chosen) {
     std::vector<Tree*> ts;
     for (auto& r : b.reqs)
         if (std::find(ts.begin(), ts.end(), r.tree) == ts.end()) ts.push_back(r.tree);
@@ -1567,16 +1614,10 @@ void autotune_batch(Batch& b, int reps, const std::vector<int>& fills, const std
         Tree* t = ts[ti];
         Batch sub;
         sub.init(b.device);
-        std::vector<int> map;
         for (size_t i = 0; i < b.reqs.size(); ++i)
-            if (b.reqs[i].tree == t) {
-                sub.reqs.push_back(b.reqs[i]);
-                map.push_back((int)i);
-            }
-        bool has_knn = false;
-        for (auto& r : sub.reqs) has_knn |= r.d.kind == BATCH_KNN;
+            if (b.reqs[i].tree == t) sub.reqs.push_back(b.reqs[i]);
         float best = 1e30f;
-        int best_fill = t->fill, best_lanes = 1;
+        int best_fill = t->fill;
         try {
             for (int f : fills) {
                 {
@@ -1584,16 +1625,10 @@ void autotune_batch(Batch& b, int reps, const std::vector<int>& fills, const std
                     t->fill = f;
                     t->rebuild_all();
                 }
-                for (int l : lanes_set) {
-                    if (!has_knn && l != lanes_set.front()) continue;
-                    for (auto& r : sub.reqs) r.lanes = l;
-                    sub.drop_plan();
-                    float ms = sub.time_runs(reps);
-                    if (ms < best) {
-                        best = ms;
-                        best_fill = f;
-                        best_lanes = l;
-                    }
+                const float ms = sub.time_runs(reps);
+                if (ms < best) {
+                    best = ms;
+                    best_fill = f;
                 }
             }
             {
@@ -1606,14 +1641,11 @@ void autotune_batch(Batch& b, int reps, const std::vector<int>& fills, const std
             throw;
         }
         sub.destroy();
-        for (int i : map)
-            if (b.reqs[i].d.kind == BATCH_KNN) b.reqs[i].lanes = best_lanes;
         if (chosen != nullptr) {
             chosen[2 * ti] = best_fill;
-            chosen[2 * ti + 1] = best_lanes;
+            chosen[2 * ti + 1] = 1;  // the lanes setting has no effect
         }
     }
-    b.drop_plan();
 }
 
 }  // namespace ikdg
@@ -1767,8 +1799,9 @@ int ikdg_set_leaf_fill(ikdg_tree* h, int fill) {
 
 int ikdg_set_knn_lanes(ikdg_tree* h, int lanes) {
     return guarded(h, [&](ikdg::Tree& t) {
+        (void)t;
+        // the searches choose the lanes of a query by the batch's size
         if (lanes != 1 && lanes != 2 && lanes != 4) throw ikdg::BadArg{"kNN lanes must be 1, 2 or 4"};
-        t.knn_lanes = lanes;
     });
 }
 
@@ -1810,7 +1843,7 @@ int ikdg_knn(ikdg_tree* h, const float* q, int64_t nq, int32_t stride, int32_t k
              float* d2, float* xyz, int32_t* cnt) {
     // A few queries with a small k (the per-point Nearest_Search of a mapping
     // front end): concurrent callers search at the same time.
-    if (nq <= ikdg::SMALL_KNN_QUERIES && k <= ikdg::KNN_SMEM_MAX)
+    if (nq <= ikdg::SMALL_KNN_QUERIES && k <= ikdg::KNN_GROUP_MAX)
         return guarded<true>(h, [&](ikdg::Tree& t) { t.knn_small(q, nq, stride, k, max_dist, ids, d2, xyz, cnt); });
     return guarded(h, [&](ikdg::Tree& t) { t.knn(q, nq, stride, k, max_dist, ids, d2, xyz, cnt, false); });
 }
@@ -1825,7 +1858,7 @@ int ikdg_knn_device_noalloc(ikdg_tree* h, const float* q, int64_t nq, int32_t st
     return guarded(h, [&](ikdg::Tree& t) {
         if (nq < 0 || stride < 3 || k < 1 || (nq > 0 && (q == nullptr || ids == nullptr || d2 == nullptr)))
             throw ikdg::BadArg{"knn_device_noalloc: bad arguments"};
-        if (k > ikdg::KNN_SMEM_MAX) throw ikdg::BadArg{"knn_device_noalloc: k must be <= 64"};
+        if (k > ikdg::KNN_GROUP_MAX) throw ikdg::BadArg{"knn_device_noalloc: k must be <= 64"};
         if (nq > ikdg::NOALLOC_MAX_QUERIES)
             throw ikdg::BadArg{"knn_device_noalloc: at most " + std::to_string(ikdg::NOALLOC_MAX_QUERIES) +
                                " queries per call (size of the static scratch array)"};
@@ -1838,7 +1871,7 @@ int ikdg_knn_device_noalloc(ikdg_tree* h, const float* q, int64_t nq, int32_t st
         // levels): the sort is the part that needs scratch.  Smaller batches
         // run unsorted and touch no scratch.  Nothing here allocates.
         ikdg::launch_knn(t.dt, q, stride, nq, k, ikdg::max_sq_threshold(max_dist), ids, d2, xyz, cnt, scratch,
-                         t.knn_lanes, ikdg::QBIN_BITS, t.stream);
+                         ikdg::QBIN_BITS, t.stream);
         CK(cudaGetLastError());
     });
 }
@@ -2117,8 +2150,7 @@ int ikdg_batch_set_knn_lanes(ikdg_batch* h, int32_t request, int32_t lanes) {
     return batch_guarded(h, [&](ikdg::Batch& b) {
         if (request < 0 || request >= (int)b.reqs.size() || !(lanes == 0 || lanes == 1 || lanes == 2 || lanes == 4))
             throw ikdg::BadArg{"batch_set_knn_lanes: bad arguments"};
-        b.reqs[request].lanes = lanes;
-        b.drop_plan();
+        // the batch's kernels choose the lanes of a query
     });
 }
 
@@ -2151,7 +2183,7 @@ int ikdg_batch_synchronize(ikdg_batch* h, int64_t* range_totals) {
 int ikdg_batch_autotune(ikdg_batch* h, int32_t reps, int32_t* chosen) {
     return batch_guarded(h, [&](ikdg::Batch& b) {
         if (reps < 1) throw ikdg::BadArg{"batch_autotune: reps must be >= 1"};
-        ikdg::autotune_batch(b, reps, {8, 12, 16, 24, 32}, {1, 2, 4}, chosen);
+        ikdg::autotune_batch(b, reps, {8, 12, 16, 24, 32}, chosen);
     });
 }
 

@@ -10,6 +10,10 @@
 //     Beside it: per-child slot / deleted counts (int4) and the parent link.
 //   * leaf buckets: LEAF_CAP float4 slots per leaf, {x, y, z, id | flags}.
 //
+//   * wide records: for every third level of internal nodes, the up to eight
+//     descendants three levels down side by side (32 bytes each: AABB, code,
+//     valid points), which the searches test with one lane per child.
+//
 // Child code: > 0 internal node, < 0 leaf (-(leaf + 1)), 0 none.  Node 0 is a
 // sentinel whose left child is the root (the role of STATIC_ROOT_NODE,
 // ikd_Tree.cpp:358-363), so the root's AABB and counts live in node 0's record
@@ -90,6 +94,8 @@ struct DevTree {
     int4* ncnt;          // [node_cap] {slots L, deleted L, slots R, deleted R}
     int* nparent;        // [node_cap] parent * 2 + side, -1 when free
     int* nheight;        // [node_cap] height of the subtree (leaves: 0)
+    float4* wide;        // [node_cap * 16] wide records (see below)
+    int2* winfo;         // [node_cap] {wide record above the node, its path position there}
     float4* pts;         // [leaf_cap * LEAF_CAP]
     int* leaf_n;         // [leaf_cap] slots used
     int* lparent;        // [leaf_cap] parent * 2 + side, -1 when free
@@ -97,6 +103,8 @@ struct DevTree {
     int* free_leaf;      // [leaf_cap]
     int node_cap;
     int leaf_cap;
+    int height;          // levels below the root (set by the host after every mutation)
+    int start;           // wide record every search starts at (host): 0 or the root's own
     DevStatus* st;
 };
 
@@ -225,6 +233,69 @@ __device__ __forceinline__ Box3 empty_box() {
         b.hi[a] = __int_as_float(0xff800000);   // -inf
     }
     return b;
+}
+
+// ---------------------------------------------------------------------------
+// Wide records.  A search that steps through binary nodes pays one dependent
+// L2 round trip per level; a wide record holds three levels at once, so a
+// group of lanes descends a 1M-point tree in 6 round trips instead of 16.
+//
+// A node X that owns a record (a wide root) has winfo[X] = {X, 1}.  Below it, a
+// child's position is its parent's position * 2 + side: positions 2..3 and
+// 4..7 are inside the record, 8..15 are its children (slot = position - 8),
+// which own the next records.  A leaf met at a position below 8 is a child
+// too: it takes the first slot of its range and the rest of the range is
+// empty (code 0, an empty box).  The slots are in left-to-right order.  Node 0
+// (the sentinel) owns the top record; the root's position there, 2, 4 or 8, is
+// chosen when the whole tree is built, so that the records above the leaves come
+// out full: a tree whose leaves lie D levels below the root has 2, 1 or 0 levels
+// in the top record for D = 2, 1, 0 mod 3.
+// The record of node X is the 64 floats at wide[16 X]: for each pair of slots
+// {2 p, 2 p + 1} the 16 floats from 16 p on, {lo x, lo y, lo z, hi x, hi y,
+// hi z, code, valid points}, each for both slots side by side, so that a lane
+// tests its two children with packed arithmetic.
+constexpr int WIDE = 8;
+
+__host__ __device__ constexpr int wide_at(int slot, int field) { return (slot >> 1) * 16 + field * 2 + (slot & 1); }
+
+__device__ __forceinline__ int2 wide_below(int2 parent, int side, int X) {
+    const int pos = parent.y * 2 + side;
+    return pos >= WIDE ? make_int2(X, 1) : make_int2(parent.x, pos);
+}
+
+__device__ __forceinline__ int wide_slot(int pos) {
+    // first slot of position pos (2..15): pos shifted up to the last level
+    return (pos << (3 - (31 - __clz(pos)))) - WIDE;
+}
+
+__device__ __forceinline__ void wide_store(float4* wide, int W, int slot, const Box3& b, int code, int valid) {
+    float* f = reinterpret_cast<float*>(wide + (long long)W * 16) + wide_at(slot, 0);
+    for (int a = 0; a < 3; ++a) {
+        f[2 * a] = b.lo[a];
+        f[2 * (3 + a)] = b.hi[a];
+    }
+    f[12] = __int_as_float(code);
+    f[14] = __int_as_float(valid);
+}
+
+// The child `code` at `side` of a node whose winfo is wi changed its box or
+// counts: its slot, if it has one.
+__device__ __forceinline__ void wide_update(const DevTree& t, int2 wi, int side, int code, const Box3& b, int valid) {
+    const int pos = wi.y * 2 + side;
+    if (pos >= WIDE || code < 0) wide_store(t.wide, wi.x, wide_slot(pos), b, code, valid);
+}
+
+// The same when the child is new there: a leaf above the last level also
+// empties the rest of its slots (a node's descendants cover all of theirs).
+__device__ __forceinline__ void wide_link(const DevTree& t, int2 wi, int side, int code, const Box3& b, int valid) {
+    const int pos = wi.y * 2 + side;
+    if (pos < WIDE && code > 0) return;
+    const int s0 = wide_slot(pos);
+    wide_store(t.wide, wi.x, s0, b, code, valid);
+    if (pos < WIDE) {
+        const int n = 8 >> (31 - __clz(pos));
+        for (int s = 1; s < n; ++s) wide_store(t.wide, wi.x, s0 + s, empty_box(), 0, 0);
+    }
 }
 
 __device__ __forceinline__ void box_grow(Box3& b, float x, float y, float z) {

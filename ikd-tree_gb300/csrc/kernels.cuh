@@ -54,20 +54,26 @@ void build_subtrees(const DevTree& t, const float4* pts, long long n, const int*
 // Batched kNN.  `temp` must hold knn_temp_bytes(nq, k) bytes of device
 // scratch: the query binning (QBIN_BINS counters, a key and a permutation
 // entry per query, for batches of at least QBIN_MIN_QUERIES) and, for
-// k > KNN_SMEM_MAX, k slot indices per query.  The candidate lists live in
-// registers for k <= KNN_REG_MAX, in shared memory for k <= KNN_SMEM_MAX and
-// in the output rows beyond.
-#ifndef IKDG_KNN_REG_MAX
-#define IKDG_KNN_REG_MAX 8
-#endif
-constexpr int KNN_REG_MAX = IKDG_KNN_REG_MAX;
-constexpr int KNN_SMEM_MAX = 64;
+// k > KNN_GROUP_MAX, k slot indices per query.  A group of lanes searches each
+// query, with the candidate list in registers, for k <= KNN_GROUP_MAX; beyond,
+// a thread does, with the list in the output rows.
+constexpr int KNN_GROUP_MAX = 64;
 constexpr int QBIN_BITS = 16;
 constexpr int QBIN_BINS = 1 << QBIN_BITS;
 constexpr long long QBIN_MIN_QUERIES = 2048;
-constexpr long long QBIN_AUTO_QUERIES = 262144;  // default: sort batches from this size
+// By default a batch is sorted when it and its lists are large and the tree does
+// not fit the L2 cache: neighbouring queries then share what they fetch from
+// HBM.  20M-point slab, 1M queries, unsorted / sorted by 14 levels (us, calls on
+// three trees in turn): k = 32 1676 / 1515, k = 16 1151 / 1067, k = 5 829 / 804,
+// k = 1 445 / 481; 20M uniform points k = 5 974 / 979; 10M points, 500k queries
+// k = 5 484 / 498; 3M points, 250k queries 233 / 243; 1M points, 1M queries
+// 770 / 802.
+constexpr long long QBIN_AUTO_QUERIES = 1 << 19;
+constexpr long long QBIN_AUTO_SLOTS = 12000000;
+constexpr int QBIN_AUTO_K = 8;
+constexpr int QBIN_AUTO_BITS = 14;
 size_t knn_temp_bytes(long long nq, int k);
-// Host-pointer kNN calls of at most this many queries (and k <= KNN_SMEM_MAX)
+// Host-pointer kNN calls of at most this many queries (and k <= KNN_GROUP_MAX)
 // run on pooled per-call streams with the tree's lock held shared, so
 // concurrent callers search at the same time.
 constexpr long long SMALL_KNN_QUERIES = 4096;
@@ -76,12 +82,12 @@ constexpr long long SMALL_KNN_QUERIES = 4096;
 constexpr long long NOALLOC_MAX_QUERIES = 1 << 18;
 cudaError_t noalloc_scratch(int device, void** ptr);
 size_t noalloc_scratch_bytes();
-// `lanes` (1, 2 or 4) threads cooperate on each query; `bin_bits` (0 = off,
-// at most QBIN_BITS) levels of the tree order the queries before the search.
+// `bin_bits` (0 = off, at most QBIN_BITS) levels of the tree order the queries
+// before the search.
 // host_out: the outputs are host memory the GPU writes directly (each warp's
 // rows then leave as coalesced 16-byte spans through shared memory).
 void launch_knn(const DevTree& t, const float* q, int q_stride, long long nq, int k, float max_sq,
-                int* out_id, float* out_d2, float* out_xyz, int* out_cnt, void* temp, int lanes, int bin_bits,
+                int* out_id, float* out_d2, float* out_xyz, int* out_cnt, void* temp, int bin_bits,
                 cudaStream_t s, bool host_out = false);
 // Box (mode 0) and radius (mode 1) search.  Pass 1 (ids == nullptr) writes
 // per-query hit counts into `counts`; pass 2 writes ids / xyz starting at
@@ -97,13 +103,12 @@ void launch_range(const DevTree& t, int mode, const float* q, int q_stride, cons
 // One request of a multi-tree batch: a kNN, box or radius search of nq queries
 // on trees[tree].  Phase 1 (search) covers chunks [c1, c1 + n1) of the
 // phase's chunk numbering; range requests also take phase-2 (write) chunks
-// [c2, c2 + n2).  A chunk is one warp, BATCH_CHUNK threads: 32 / lanes kNN
-// queries, or 32 range queries.
+// [c2, c2 + n2).  A chunk is the work a warp takes at once: `per` queries.
 constexpr int BATCH_THREADS = 128;
-constexpr int BATCH_CHUNK = 32;
+constexpr int BATCH_CHUNK = 32;       // queries per chunk, at most
+constexpr int BATCH_KNN_STEP = 8;     // kNN queries a warp searches side by side
 constexpr int BATCH_KMAX = 16;
-constexpr int BATCH_SMEM_CLASS = 4;   // kNN with 8 < k <= 16: lists in shared memory
-constexpr int BATCH_RANGE_CLASS = 5;  // box / radius requests
+constexpr int BATCH_RANGE_CLASS = 3;  // box / radius requests; 0..2: kNN, k <= 4, 8, 16
 enum BatchKind : int { BATCH_KNN = 0, BATCH_BOX = 1, BATCH_RADIUS = 2 };
 
 struct BatchReq {
@@ -112,7 +117,7 @@ struct BatchReq {
     const float* radius;
     long long nq;
     int kind, tree, q_stride, r_stride;
-    int k, kclass, lanes;
+    int k, per;
     float max_sq;
     int* ids;
     float* d2;
@@ -125,17 +130,17 @@ struct BatchReq {
     const int* perm;     // query at position i of the request's run order (nullptr: in order)
 };
 
-// Register class of a kNN request with this k (k <= BATCH_KMAX): 0..4;
+// Register class of a kNN request with this k (k <= BATCH_KMAX): 0..2;
 // range requests are class BATCH_RANGE_CLASS.
 int batch_kclass(int k);
-// Resident CTAs (whole GPU) of the persistent search kernel of a class.
-int batch_search_grid(int kclass, int lanes);
+// Resident CTAs (whole GPU) of the persistent search kernel of a class;
+// `height`: the tallest tree of the batch (sizes the kNN stacks).
+int batch_search_grid(int kclass, int height);
 int batch_write_grid();
-// Phase 1 over requests [r0, r1), all of register class kclass and `lanes`
-// lanes per query, whose chunks are [c_begin, c_end); ctr: a zeroed device
-// counter.
+// Phase 1 over requests [r0, r1), all of register class kclass, whose chunks
+// are [c_begin, c_end); ctr: a zeroed device counter.
 void launch_batch_search(const DevTree* trees, const BatchReq* reqs, const long long* req_c1, int r0, int r1,
-                         long long c_begin, long long c_end, int kclass, int lanes, long long* counts,
+                         long long c_begin, long long c_end, int kclass, int height, long long* counts,
                          unsigned long long* ctr, int grid, cudaStream_t s);
 // Spatial order of every request's queries: key = request position in the
 // high bits, Morton code of the query (kNN / radius: the point; box: its

@@ -11,31 +11,89 @@ namespace {
 
 using search::FINF;
 
-// Threads per CTA of the per-call kNN kernel.
-#ifndef IKDG_KNN_THREADS
-#define IKDG_KNN_THREADS 128
-#endif
-constexpr int KNN_THREADS = IKDG_KNN_THREADS;
+constexpr int KNN_THREADS = search::KNN_CTA;
+inline unsigned blocks_for(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
+// Stores n floats (or int bits) from shared memory to dst with the whole CTA:
+// 16-byte stores where dst is 16-byte aligned, 4-byte stores otherwise.  src is
+// 16-byte aligned.
+__device__ __forceinline__ void block_store(float* dst, const float* src, int n) {
+    int done = 0;
+    if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+        const int n4 = n >> 2;
+        for (int i = threadIdx.x; i < n4; i += KNN_THREADS)
+            reinterpret_cast<float4*>(dst)[i] = reinterpret_cast<const float4*>(src)[i];
+        done = n4 << 2;
+    }
+    for (int i = done + threadIdx.x; i < n; i += KNN_THREADS) dst[i] = src[i];
+}
 
-// STAGED: the outputs are host memory (rows leave through shared memory as
-// coalesced 16-byte stores; see knn_body).
-template <int KMAX, int G, bool STAGED = false, int PAIRS = search::knn_leaf_pairs<KMAX>()>
-__global__ void __launch_bounds__(KNN_THREADS) knn_kernel(DevTree t, const float* __restrict__ q, int q_stride,
-                                                  long long nq, int k, float max_sq, int* __restrict__ out_id,
-                                                  float* __restrict__ out_d2, float* __restrict__ out_xyz,
-                                                  int* __restrict__ out_cnt, int* __restrict__ slots,
-                                                  const int* __restrict__ perm) {
-    const long long gtid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if constexpr (KMAX > 0 && G == 1 && STAGED) {
-        // rows of a warp's consecutive queries leave through shared memory
-        __shared__ __align__(16) float stage[KNN_THREADS / 32][search::knn_stage_floats(KMAX)];
-        search::knn_body<KMAX, G, PAIRS>(t, gtid, q, q_stride, nq, k, max_sq, out_id, out_d2, out_xyz, out_cnt, slots,
-                                         perm, nullptr, nullptr, nullptr, 1,
-                                         perm == nullptr ? stage[threadIdx.x >> 5] : nullptr);
+// kNN, k <= 64: KNN_THREADS / KNN_G queries per CTA.  Dynamic shared memory: the
+// threads' stack columns (`entries` each).  STAGED: the outputs are host memory;
+// the CTA's rows are one span of every array (no permutation), are staged over
+// the stacks once its queries are done and leave as 16-byte stores.
+template <int R, bool STAGED>
+__global__ void __launch_bounds__(KNN_THREADS) knn_group_kernel(DevTree t, const float* __restrict__ q, int q_stride,
+                                                                long long nq, int k, float max_sq, search::KnnOut o,
+                                                                const int* __restrict__ perm, int entries, int per_warp) {
+    extern __shared__ __align__(16) unsigned char knn_sm[];
+    const search::KnnLane g;
+    // query of this group among the CTA's; groups past per_warp idle
+    const int gw = (threadIdx.x & 31) / search::KNN_G, gi = (threadIdx.x >> 5) * per_warp + gw;
+    const int queries = KNN_THREADS / 32 * per_warp;
+    const long long tid = (long long)blockIdx.x * queries + gi;
+    const bool valid = gw < per_warp && tid < nq;
+    long long qi = valid ? tid : 0;
+    if (!STAGED && valid && perm != nullptr) qi = __ldg(perm + tid);
+    const float qx = valid ? q[qi * q_stride + 0] : 0.f;
+    const float qy = valid ? q[qi * q_stride + 1] : 0.f;
+    const float qz = valid ? q[qi * q_stride + 2] : 0.f;
+    float ld[R];
+    int ls[R];
+    search::knn_group<R>(t, g, valid, qx, qy, qz, k, max_sq, reinterpret_cast<int2*>(knn_sm) + threadIdx.x, entries,
+                         per_warp * search::KNN_G / 2, ld, ls);
+    if (!STAGED) {
+        search::knn_write_rows<R>(t, g, valid, ld, ls, k, qi, o);
+        return;
+    }
+    __syncthreads();  // the stacks are dead: stage the rows over them
+    float* st = reinterpret_cast<float*>(knn_sm);
+    search::KnnOut so;
+    so.id = reinterpret_cast<int*>(st);
+    so.d2 = st + queries * k;
+    so.xyz = o.xyz != nullptr ? st + 2 * queries * k : nullptr;
+    so.cnt = reinterpret_cast<int*>(st + 5 * queries * k);
+    search::knn_write_rows<R>(t, g, valid, ld, ls, k, gi, so);
+    __syncthreads();
+    const long long q0 = (long long)blockIdx.x * queries;
+    const int rows = (int)min((long long)queries, nq - q0);
+    block_store(reinterpret_cast<float*>(o.id + q0 * k), reinterpret_cast<const float*>(so.id), rows * k);
+    block_store(o.d2 + q0 * k, so.d2, rows * k);
+    if (o.xyz != nullptr) block_store(o.xyz + q0 * k * 3, so.xyz, rows * k * 3);
+    if (o.cnt != nullptr) block_store(reinterpret_cast<float*>(o.cnt + q0), reinterpret_cast<const float*>(so.cnt), rows);
+}
+
+// Batches of at most this many queries get a warp per query (its other groups
+// idle): no query waits for another one's steps.  1M-point map, k = 5, host
+// clock around one call: 1,000 queries 36.3 us a warp each, 46.8 us eight a
+// warp; 4,000 queries 42.9 / 47.6 us, but 14.1 / 12.3 us a call when calls on
+// several trees overlap; 15,000 queries 79.7 / 51.5 us.
+constexpr long long KNN_SPREAD_QUERIES = 2048;
+
+template <int R>
+void knn_group_launch(const DevTree& t, const float* q, int q_stride, long long nq, int k, float max_sq,
+                      const search::KnnOut& o, const int* perm, bool staged, cudaStream_t s) {
+    const int per_warp = nq <= KNN_SPREAD_QUERIES ? 1 : 32 / search::KNN_G;
+    const int queries = KNN_THREADS / 32 * per_warp;
+    const unsigned grid = blocks_for(nq, queries);
+    const int entries = search::knn_stack_entries(t.height);
+    const size_t stacks = (size_t)KNN_THREADS * entries * sizeof(int2);
+    if (staged) {
+        const size_t rows = (size_t)queries * (5 * k + 1) * sizeof(float);
+        knn_group_kernel<R, true><<<grid, KNN_THREADS, rows > stacks ? rows : stacks, s>>>(t, q, q_stride, nq, k, max_sq,
+                                                                                          o, perm, entries, per_warp);
     } else {
-        search::knn_body<KMAX, G, PAIRS>(t, gtid / G, q, q_stride, nq, k, max_sq, out_id, out_d2, out_xyz, out_cnt,
-                                         slots, perm);
+        knn_group_kernel<R, false><<<grid, KNN_THREADS, stacks, s>>>(t, q, q_stride, nq, k, max_sq, o, perm, entries, per_warp);
     }
 }
 
@@ -70,103 +128,18 @@ __global__ void __launch_bounds__(128) range_kernel(DevTree t, const float* __re
     search::range_body<MODE, search::RANGE_WRITE>(t, q, q_stride, radius, r_stride, qi, go, o, o_lim, ids, xyz);
 }
 
-inline unsigned blocks_for(long long n, int t) { return (unsigned)((n + t - 1) / t); }
-
-// Blocks of `fn` resident on the whole GPU (0 if the query fails).
-inline int knn_resident(const void* fn) {
-    int dev = 0, sms = 0, per_sm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, KNN_THREADS, 0) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return sms * per_sm;
-}
-
-template <int KMAX>
-void knn_launch(const DevTree& t, const float* q, int q_stride, long long nq, int k, float max_sq, int* out_id,
-                float* out_d2, float* out_xyz, int* out_cnt, int* slots, const int* perm, int lanes, cudaStream_t s,
-                bool host_out = false) {
-    const int G = lanes >= 4 ? 4 : lanes == 2 ? 2 : 1;
-    const unsigned grid = blocks_for(nq * G, KNN_THREADS);
-    if constexpr (KMAX > 0) {
-        if (G == 1) {
-            // Four slot pairs per leaf step while every block of the batch is
-            // resident at once (the occupancy of a kernel does not change:
-            // looked up once; the library drives one kind of GPU).
-            const bool staged = host_out && perm == nullptr;
-            static int resident[2] = {-1, -1};
-            int& r = resident[staged ? 1 : 0];
-            if (r < 0)
-                r = staged ? knn_resident((const void*)knn_kernel<KMAX, 1, true, 4>)
-                           : knn_resident((const void*)knn_kernel<KMAX, 1, false, 4>);
-            const bool wide = grid <= (unsigned)r;
-#define IKDG_KNN_P(ST, P)                                                                                     \
-    knn_kernel<KMAX, 1, ST, P><<<grid, KNN_THREADS, 0, s>>>(t, q, q_stride, nq, k, max_sq, out_id, out_d2, out_xyz, \
-                                                            out_cnt, slots, perm)
-            if (staged && wide)
-                IKDG_KNN_P(true, 4);
-            else if (staged)
-                IKDG_KNN_P(true, 2);
-            else if (wide)
-                IKDG_KNN_P(false, 4);
-            else
-                IKDG_KNN_P(false, 2);
-#undef IKDG_KNN_P
-            return;
-        }
-    }
-#define IKDG_KNN_G(GG)                                                                                              \
-    knn_kernel<KMAX, GG><<<grid, KNN_THREADS, 0, s>>>(t, q, q_stride, nq, k, max_sq, out_id, out_d2, out_xyz, out_cnt, \
-                                                      slots, perm)
-    if (G == 4)
-        IKDG_KNN_G(4);
-    else if (G == 2)
-        IKDG_KNN_G(2);
-    else
-        IKDG_KNN_G(1);
-#undef IKDG_KNN_G
-}
-
-// KNN_REG_MAX < k <= KNN_SMEM_MAX: each group's sorted candidate list lives
-// in shared memory, entry j of group g at [j * groups + g] (threads of a warp
-// touching the same entry hit different banks).  64 threads per CTA keep
-// 64 entries x 12 bytes x 64 groups within the default 48 KB.
-constexpr int KNN_SMEM_THREADS = 64;
-
-template <int G>
-__global__ void __launch_bounds__(KNN_SMEM_THREADS) knn_smem_kernel(DevTree t, const float* __restrict__ q,
-                                                                    int q_stride, long long nq, int k, float max_sq,
-                                                                    int* __restrict__ out_id,
-                                                                    float* __restrict__ out_d2,
-                                                                    float* __restrict__ out_xyz,
-                                                                    int* __restrict__ out_cnt,
-                                                                    const int* __restrict__ perm) {
-    extern __shared__ float knn_sm[];
-    constexpr int groups = KNN_SMEM_THREADS / G;
-    float* sd = knn_sm;
-    int* si = reinterpret_cast<int*>(sd + groups * k);
-    int* ss = si + groups * k;
-    const int g = threadIdx.x / G;
-    const long long gtid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    search::knn_body<0, G>(t, gtid / G, q, q_stride, nq, k, max_sq, out_id, out_d2, out_xyz, out_cnt, nullptr, perm,
-                           sd + g, si + g, ss + g, groups);
-}
-
-void knn_smem_launch(const DevTree& t, const float* q, int q_stride, long long nq, int k, float max_sq, int* out_id,
-                     float* out_d2, float* out_xyz, int* out_cnt, const int* perm, int lanes, cudaStream_t s) {
-    const int G = lanes >= 4 ? 4 : lanes == 2 ? 2 : 1;
-    const size_t smem = (size_t)(KNN_SMEM_THREADS / G) * k * 12;
-    const unsigned grid = blocks_for(nq * G, KNN_SMEM_THREADS);
-    if (G == 4)
-        knn_smem_kernel<4><<<grid, KNN_SMEM_THREADS, smem, s>>>(t, q, q_stride, nq, k, max_sq, out_id, out_d2,
-                                                                out_xyz, out_cnt, perm);
-    else if (G == 2)
-        knn_smem_kernel<2><<<grid, KNN_SMEM_THREADS, smem, s>>>(t, q, q_stride, nq, k, max_sq, out_id, out_d2,
-                                                                out_xyz, out_cnt, perm);
-    else
-        knn_smem_kernel<1><<<grid, KNN_SMEM_THREADS, smem, s>>>(t, q, q_stride, nq, k, max_sq, out_id, out_d2,
-                                                                out_xyz, out_cnt, perm);
+// k > 64: a thread per query, the list in its output rows.
+__global__ void __launch_bounds__(KNN_THREADS) knn_rows_kernel(DevTree t, const float* __restrict__ q, int q_stride,
+                                                               long long nq, int k, float max_sq, search::KnnOut o,
+                                                               int* __restrict__ slots, const int* __restrict__ perm) {
+    const long long tid = (long long)blockIdx.x * KNN_THREADS + threadIdx.x;
+    const bool valid = tid < nq;
+    long long qi = valid ? tid : 0;
+    if (valid && perm != nullptr) qi = __ldg(perm + tid);
+    const float qx = valid ? q[qi * q_stride + 0] : 0.f;
+    const float qy = valid ? q[qi * q_stride + 1] : 0.f;
+    const float qz = valid ? q[qi * q_stride + 2] : 0.f;
+    search::knn_rows_body(t, valid, qi, qx, qy, qz, k, max_sq, o, slots);
 }
 
 // ---- query binning -----------------------------------------------------------
@@ -207,12 +180,12 @@ __global__ void qbin_scatter_kernel(const int* __restrict__ key, long long nq, i
 size_t knn_temp_bytes(long long nq, int k) {
     size_t b = 0;
     if (nq >= QBIN_MIN_QUERIES) b += sizeof(int) * (2 * QBIN_BINS + 2 * nq) + scan_temp_bytes(QBIN_BINS) + 1024;
-    if (k > KNN_SMEM_MAX) b += sizeof(int) * nq * k + 256;
+    if (k > KNN_GROUP_MAX) b += sizeof(int) * nq * k + 256;
     return b;
 }
 
 void launch_knn(const DevTree& t, const float* q, int q_stride, long long nq, int k, float max_sq, int* out_id,
-                float* out_d2, float* out_xyz, int* out_cnt, void* temp, int lanes, int bin_bits, cudaStream_t s,
+                float* out_d2, float* out_xyz, int* out_cnt, void* temp, int bin_bits, cudaStream_t s,
                 bool host_out) {
     if (nq <= 0) return;
     char* tp = (char*)temp;
@@ -232,27 +205,24 @@ void launch_knn(const DevTree& t, const float* q, int q_stride, long long nq, in
         qbin_scatter_kernel<<<blocks_for(nq, 256), 256, 0, s>>>(key, nq, offs, pm);
         perm = pm;
     }
-    int* slots = k > KNN_SMEM_MAX ? (int*)tp : nullptr;
-#define IKDG_KNN(KM) \
-    knn_launch<KM>(t, q, q_stride, nq, k, max_sq, out_id, out_d2, out_xyz, out_cnt, slots, perm, lanes, s, host_out)
-    if (k > KNN_SMEM_MAX)
-        IKDG_KNN(0);
-    else if (k > KNN_REG_MAX)
-        knn_smem_launch(t, q, q_stride, nq, k, max_sq, out_id, out_d2, out_xyz, out_cnt, perm, lanes, s);
-    else if (k <= 1)
+    const search::KnnOut o{out_id, out_d2, out_xyz, out_cnt};
+    if (k > KNN_GROUP_MAX) {
+        knn_rows_kernel<<<blocks_for(nq, KNN_THREADS), KNN_THREADS, 0, s>>>(t, q, q_stride, nq, k, max_sq, o, (int*)tp,
+                                                                            perm);
+        return;
+    }
+    const bool staged = host_out && perm == nullptr;
+#define IKDG_KNN(R) knn_group_launch<R>(t, q, q_stride, nq, k, max_sq, o, perm, staged, s)
+    if (k <= 4)
         IKDG_KNN(1);
-    else if (k <= 2)
-        IKDG_KNN(2);
-    else if (k <= 4)
-        IKDG_KNN(4);
-    else if (k <= 5)
-        IKDG_KNN(5);
     else if (k <= 8)
-        IKDG_KNN(8);
+        IKDG_KNN(2);
     else if (k <= 16)
+        IKDG_KNN(4);
+    else if (k <= 32)
+        IKDG_KNN(8);
+    else
         IKDG_KNN(16);
-    else if constexpr (KNN_REG_MAX >= 32)
-        IKDG_KNN(32);
 #undef IKDG_KNN
 }
 

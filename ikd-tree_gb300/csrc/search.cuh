@@ -22,23 +22,74 @@ namespace search {
 
 constexpr float FINF = __builtin_huge_valf();
 
-// Two consecutive 16-byte slots from a 32-byte-aligned address, one 256-bit
-// load (read-only data: the compiler may schedule it freely).
-__device__ __forceinline__ void ld_slot_pair(const float4* p, float4& a, float4& b) {
-    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-                 : "l"(p));
+// Packed pairs of floats (two rounded operations per instruction; the results
+// are those of the scalar forms).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
 }
 
-// Slot pairs (256-bit loads) the kNN leaf scan issues together: the default
-// for the register lists is two; the per-call kNN picks four when the whole
-// batch is resident at once (measured, 1M-point map, k = 5: 100k queries
-// 0.155 -> 0.146 ms with four; 1M queries 0.851 -> 0.825 ms with two, 0.896
-// with four, whose extra registers cost resident blocks).  The shared-memory
-// and row lists take four.
-template <int KMAX>
-__host__ __device__ constexpr int knn_leaf_pairs() {
-    return KMAX > 0 ? 2 : 4;
+// 32 consecutive bytes from a 32-byte-aligned address, one 256-bit load
+// (read-only data: the compiler may schedule it freely).
+struct Quad2 {
+    f32x2 v[4];
+};
+__device__ __forceinline__ Quad2 ld_quad2(const void* p) {
+    Quad2 q;
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
+        : "=l"(q.v[0]), "=l"(q.v[1]), "=l"(q.v[2]), "=l"(q.v[3])
+        : "l"(p));
+    return q;
+}
+
+// box_dist of two children of a wide record at once: the gap of an axis is
+// max(lo - q, q - hi, 0), whose square is axis_gap's bit for bit.  The sums are
+// scalar: packed ones were contracted with the packed squares, and a bound that
+// is not rounded like sq_dist prunes points that tie with the k-th.
+__device__ __forceinline__ f32x2 gap2(f32x2 lo, f32x2 hi, f32x2 q) {
+    float a0, a1, b0, b1;
+    unpack2(sub2(lo, q), a0, a1);
+    unpack2(sub2(q, hi), b0, b1);
+    const f32x2 g = pack2(max3(a0, b0, 0.f), max3(a1, b1, 0.f));
+    return mul2(g, g);
+}
+__device__ __forceinline__ void box_dist2(f32x2 lx, f32x2 ly, f32x2 lz, f32x2 hx, f32x2 hy, f32x2 hz, f32x2 qx,
+                                          f32x2 qy, f32x2 qz, float& d0, float& d1) {
+    float x0, x1, y0, y1, z0, z1;
+    unpack2(gap2(lx, hx, qx), x0, x1);
+    unpack2(gap2(ly, hy, qy), y0, y1);
+    unpack2(gap2(lz, hz, qz), z0, z1);
+    d0 = __fadd_rn(__fadd_rn(x0, y0), z0);
+    d1 = __fadd_rn(__fadd_rn(x1, y1), z1);
+}
+
+// sq_dist(q, p) of a stored slot {x, y, z, id}, x and y packed.
+__device__ __forceinline__ float slot_dist(f32x2 qxy, float qz, f32x2 xy, float z) {
+    const f32x2 d = sub2(qxy, xy);
+    float sx, sy;
+    unpack2(mul2(d, d), sx, sy);
+    const float dz = __fsub_rn(qz, z);
+    return __fadd_rn(__fadd_rn(sx, sy), __fmul_rn(dz, dz));
 }
 
 // Leaves a warp scans per step of the range search's leaf phase.
@@ -48,88 +99,292 @@ __host__ __device__ constexpr int knn_leaf_pairs() {
 constexpr int RANGE_LEAF_BATCH = IKDG_RANGE_LEAF_BATCH;
 
 
-// Stores n floats (or int bits) from shared memory to dst with the whole warp:
-// 16-byte stores where dst is 16-byte aligned, lane-consecutive 4-byte stores
-// otherwise.  src is 16-byte aligned shared memory.
-__device__ __forceinline__ void warp_store(float* dst, const float* src, int n) {
-    const int lane = threadIdx.x & 31;
-    int done = 0;
-    if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-        const int n4 = n >> 2;
-        for (int i = lane; i < n4; i += 32)
-            reinterpret_cast<float4*>(dst)[i] = reinterpret_cast<const float4*>(src)[i];
-        done = n4 << 2;
+// ---- kNN, k <= 64: a group of four lanes per query over the wide records --------------
+//
+// A group's step is a node step (one 256-byte wide record, two children a lane)
+// or a leaf step (half a bucket, 16 slots, four a lane).  A node step goes on
+// with the nearest child; every lane stacks the rest of its own children that
+// can still hold a result, with their box distances, in a shared-memory column
+// of its own.  A leaf step inserts the slots that can enter the list, smallest
+// first, at most k of them.  The list is sorted by (distance, id) and lives in
+// the group's registers, entry lane * R + r, as (distance, slot); ids are read
+// where two distances tie and at the end.  A subtree is skipped when its box distance exceeds
+// min(max_dist^2, current k-th distance).
+//
+// The groups of a warp step together: node steps for the groups that hold a
+// record until half of them hold a leaf, then one leaf step for those (in a
+// simulated schedule over 1M points the extremes, at once and when all do, cost
+// 15 % and 6 % more).
+//
+// 1M-point map, k = 5, kernel time before (a thread per query over the binary
+// records) / now: 1 query 23.6 / 10 us, 15k 90 / 32 us, 100k 144 / 98 us (96 / 73 us
+// a call when calls on three trees overlap); 20M points, 1M queries, k = 16:
+// 1615 / 1067 us a call.
+// Bound by instruction issue (the tree is served from L2 and the chain of a
+// query is ~15 loads): a thread per query over the binary records issued less
+// per node but took 27 dependent loads a query, 96 steps a warp (its 32 queries
+// wait for one another) and one thread's time per slot.
+constexpr int KNN_G = 4;           // lanes per query
+constexpr int KNN_LEAF_STEP = 16;  // slots per leaf step
+constexpr int KNN_CTA = 128;       // threads per CTA of every kernel that uses the stacks
+
+// Entries of a lane's stack for a tree of this height: every wide record on a
+// path (the top one and one for every three levels) leaves at most the lane's
+// two children.
+__host__ __device__ constexpr int knn_stack_entries(int height) { return 2 * (1 + (height + 2) / 3) + 1; }
+
+struct KnnOut {
+    int* id;
+    float* d2;
+    float* xyz;  // nullable
+    int* cnt;    // nullable
+};
+
+struct KnnLane {
+    int lane, sl, gs;  // lane of the warp, of the group; the group's first lane
+    unsigned gmask;    // the group's lanes
+    __device__ __forceinline__ KnnLane() {
+        lane = threadIdx.x & 31;
+        sl = lane & (KNN_G - 1);
+        gs = lane & ~(KNN_G - 1);
+        gmask = ((1u << KNN_G) - 1u) << gs;
     }
-    for (int i = done + lane; i < n; i += 32) dst[i] = src[i];
+};
+
+// Searches one query per group; every lane of the warp calls it together
+// (groups without a query pass valid = false).  stk: this thread's stack
+// column in shared memory, `entries` entries KNN_CTA apart.  half_lanes: lanes
+// of half the warp's queries.  Leaves the sorted list in ld / ls (slot -1: no
+// entry).
+template <int R>
+__device__ __forceinline__ void knn_group(const DevTree& t, const KnnLane& g, bool valid, float qx, float qy, float qz,
+                                          int k, float max_sq, int2* stk, int entries, int half_lanes, float (&ld)[R],
+                                          int (&ls)[R]) {
+    constexpr int G = KNN_G, S = KNN_LEAF_STEP / G;
+    constexpr unsigned ALL = 0xffffffffu, DEAD = 0xffffffffu;
+    constexpr int DONE = 0x7fffffff;
+    static_assert(WIDE == 2 * G, "two children per lane");
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        ld[r] = FINF;
+        ls[r] = -1;
+    }
+    const f32x2 qx2 = pack2(qx, qx), qy2 = pack2(qy, qy), qz2 = pack2(qz, qz), qxy = pack2(qx, qy);
+    float lim = max_sq;  // min(max_sq, k-th distance)
+    const int wl = g.gs + (k - 1) / R, wr = (k - 1) % R;  // where the k-th entry lives
+    int sp = 0, half = 0;
+    int cur = valid ? t.start : DONE;  // a record's node, a leaf's code or DONE
+    int lev = 0;                 // level of the record `cur` (records above it on its path)
+    bool full = false;           // a stack overflowed (cannot happen: see knn_stack_entries)
+    int steps = 0;
+
+    while (true) {
+        const unsigned leaves = __ballot_sync(ALL, cur < 0);
+        const bool node = (unsigned)cur < (unsigned)DONE;
+        bool pop;
+        if (__popc(leaves) < half_lanes && __any_sync(ALL, node)) {
+            const char* a = reinterpret_cast<const char*>(t.wide + (long long)(node ? cur : 0) * 16) + 64 * g.sl;
+            const Quad2 u = ld_quad2(a), v = ld_quad2(a + 32);
+            float d0, d1, lx0, lx1, hx0, hx1, c0, c1;
+            box_dist2(u.v[0], u.v[1], u.v[2], u.v[3], v.v[0], v.v[1], qx2, qy2, qz2, d0, d1);
+            unpack2(u.v[0], lx0, lx1);
+            unpack2(u.v[3], hx0, hx1);
+            unpack2(v.v[2], c0, c1);
+            // Key: the distance with the child's index in its low three bits
+            // (they only order the visits).  Empty slots have lo > hi.
+            const bool al0 = node && d0 <= lim && lx0 <= hx0, al1 = node && d1 <= lim && lx1 <= hx1;
+            const unsigned key0 = al0 ? (__float_as_uint(d0) & ~7u) | (unsigned)(2 * g.sl) : DEAD;
+            const unsigned key1 = al1 ? (__float_as_uint(d1) & ~7u) | (unsigned)(2 * g.sl + 1) : DEAD;
+            unsigned m = min(key0, key1);
+            m = min(m, __shfl_xor_sync(ALL, m, 1));
+            m = min(m, __shfl_xor_sync(ALL, m, 2));
+            // Entry: the code, and the distance with the record's level in
+            // its low five bits.
+            const bool p0 = al0 && key0 != m, p1 = al1 && key1 != m;
+            full = full || (p0 && p1 ? sp + 1 : p0 || p1 ? sp : 0) >= entries;
+            if (p0 && sp < entries)
+                stk[KNN_CTA * sp++] = make_int2(__float_as_int(c0), (__float_as_int(d0) & ~31) | lev);
+            if (p1 && sp < entries)
+                stk[KNN_CTA * sp++] = make_int2(__float_as_int(c1), (__float_as_int(d1) & ~31) | lev);
+            const int code = __shfl_sync(ALL, __float_as_int((m & 1) ? c1 : c0), g.gs + (int)((m >> 1) & 3u));
+            pop = node && m == DEAD;
+            if (node) cur = code;
+            ++lev;
+        } else {
+            if (leaves == 0) break;
+            if (++steps > MAX_VISITS) {
+                if (cur != DONE && g.sl == 0) atomicOr(&t.st->err, ERR_LOOP);
+                break;
+            }
+            const bool act = cur < 0;
+            const int L = act ? code_leaf(cur) : 0;
+            const int j0 = half * KNN_LEAF_STEP + S * g.sl;
+            const int s0 = L * LEAF_CAP + j0;
+            const int n = act ? min(__ldg(t.leaf_n + L), LEAF_CAP) : 0;
+            unsigned key[S];
+#pragma unroll
+            for (int i = 0; i < S; ++i) key[i] = DEAD;
+            if (act) {
+#pragma unroll
+                for (int i = 0; i < S; i += 2) {
+                    const Quad2 p = ld_quad2(t.pts + (long long)s0 + i);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        float z, w;
+                        unpack2(p.v[2 * e + 1], z, w);
+                        const float d = slot_dist(qxy, qz, p.v[2 * e], z);
+                        const bool ok = j0 + i + e < n && !(__float_as_uint(w) & F_DEL) && d <= lim;
+                        key[i + e] = ok ? __float_as_uint(d) : DEAD;
+                    }
+                }
+            }
+            while (true) {
+                // The smallest candidate of each group; one with the k-th
+                // distance may still enter by its id.
+                const unsigned mine = min(min(key[0], key[1]), min(key[2], key[3]));
+                unsigned m = min(mine, __shfl_xor_sync(ALL, mine, 1));
+                m = min(m, __shfl_xor_sync(ALL, m, 2));
+                const bool go = m <= __float_as_uint(lim);  // (DEAD is above every distance)
+                if (!__any_sync(ALL, go)) break;
+                const int ml = __ffs(__ballot_sync(ALL, mine == m) & g.gmask) - 1;
+                const bool is0 = key[0] == m, is1 = key[1] == m, is2 = key[2] == m;
+                const int slot = __shfl_sync(ALL, s0 + (is0 ? 0 : is1 ? 1 : is2 ? 2 : 3), ml);
+                if (g.lane == ml) {
+                    if (is0)
+                        key[0] = DEAD;
+                    else if (is1)
+                        key[1] = DEAD;
+                    else if (is2)
+                        key[2] = DEAD;
+                    else
+                        key[3] = DEAD;
+                }
+                const float md = __uint_as_float(m);
+                float pd = __shfl_up_sync(ALL, ld[R - 1], 1, G);
+                int ps = __shfl_up_sync(ALL, ls[R - 1], 1, G);
+                if (g.sl == 0) pd = -1.f;
+                bool tie = false;
+#pragma unroll
+                for (int r = 0; r < R; ++r) tie = tie || ld[r] == md;
+                if (__any_sync(ALL, tie && go)) {
+                    // Equal distances: the smaller id first.  (ahead: entry r
+                    // stays before the candidate.)
+                    const int id = go ? (int)(__float_as_uint(__ldg(t.pts + slot).w) & ID_MASK) : 0;
+                    bool ahead[R];
+#pragma unroll
+                    for (int r = 0; r < R; ++r)
+                        ahead[r] = ld[r] < md || (ld[r] == md && ls[r] >= 0 && go &&
+                                                  (int)(__float_as_uint(__ldg(t.pts + ls[r]).w) & ID_MASK) < id);
+                    bool pa = __shfl_up_sync(ALL, ahead[R - 1], 1, G);
+                    if (g.sl == 0) pa = true;
+#pragma unroll
+                    for (int r = R - 1; r >= 0; --r) {
+                        const bool before = r > 0 ? ahead[r > 0 ? r - 1 : 0] : pa;
+                        if (go && !ahead[r]) {
+                            ld[r] = before ? md : (r > 0 ? ld[r > 0 ? r - 1 : 0] : pd);
+                            ls[r] = before ? slot : (r > 0 ? ls[r > 0 ? r - 1 : 0] : ps);
+                        }
+                    }
+                } else {
+                    // Sorted shift: an entry above the candidate takes its
+                    // predecessor, or the candidate if that is below it.
+#pragma unroll
+                    for (int r = R - 1; r >= 0; --r) {
+                        const float bd = r > 0 ? ld[r > 0 ? r - 1 : 0] : pd;
+                        const int bs = r > 0 ? ls[r > 0 ? r - 1 : 0] : ps;
+                        if (go && ld[r] > md) {
+                            ls[r] = bd > md ? bs : slot;
+                            ld[r] = fmaxf(bd, md);
+                        }
+                    }
+                }
+                float w = ld[0];
+#pragma unroll
+                for (int r = 1; r < R; ++r)
+                    if (r == wr) w = ld[r];
+                lim = fminf(max_sq, __shfl_sync(ALL, w, wl));
+            }
+            pop = act && !(half == 0 && n > KNN_LEAF_STEP);
+            if (act) half = pop ? 0 : 1;
+        }
+        // Of the columns' tops that can still hold a result, the deepest, the
+        // nearest of those: so the columns hold children of the records on
+        // one path only, two per record and lane.
+        if (__any_sync(ALL, pop)) {
+            int2 e = make_int2(DONE, 0);
+            bool dead = pop && sp > 0;
+            while (__any_sync(ALL, dead)) {  // drop what the bound has passed
+                if (dead) {
+                    e = stk[KNN_CTA * (sp - 1)];
+                    if (__int_as_float(e.y & ~31) <= lim)
+                        dead = false;
+                    else
+                        dead = --sp > 0;
+                }
+            }
+            const unsigned key =
+                pop && sp > 0 ? ((31u - (e.y & 31)) << 27) | (((unsigned)e.y >> 5) & ~3u) | (unsigned)g.sl : DEAD;
+            unsigned m = min(key, __shfl_xor_sync(ALL, key, 1));
+            m = min(m, __shfl_xor_sync(ALL, m, 2));
+            const int code = __shfl_sync(ALL, e.x, g.gs + (int)(m & 3u));
+            if (pop) {
+                cur = m == DEAD ? DONE : code;
+                lev = 32 - (int)(m >> 27);
+                if (key == m && m != DEAD) --sp;
+            }
+        }
+    }
+    if (full) atomicOr(&t.st->err, ERR_STACK);
 }
 
-// Shared-memory floats per warp for the staged kNN output (k <= kmax).
-__host__ __device__ constexpr int knn_stage_floats(int kmax) { return 32 * (5 * kmax + 1); }
+// A group's rows: entry e of query `row` at row * k + e of every array.
+template <int R>
+__device__ __forceinline__ void knn_write_rows(const DevTree& t, const KnnLane& g, bool valid, const float (&ld)[R],
+                                               const int (&ls)[R], int k, long long row, const KnnOut& o) {
+    int cnt = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int e = g.sl * R + r;
+        const bool ok = ls[r] >= 0;
+        cnt += __popc(__ballot_sync(0xffffffffu, ok && e < k) & g.gmask);
+        if (!valid || e >= k) continue;
+        const float4 p = ok ? __ldg(t.pts + ls[r]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const long long at = row * k + e;
+        o.id[at] = ok ? (int)(__float_as_uint(p.w) & ID_MASK) : -1;
+        o.d2[at] = ok ? ld[r] : FINF;
+        if (o.xyz != nullptr) {
+            o.xyz[at * 3 + 0] = p.x;
+            o.xyz[at * 3 + 1] = p.y;
+            o.xyz[at * 3 + 2] = p.z;
+        }
+    }
+    if (valid && o.cnt != nullptr && g.sl == 0) o.cnt[row] = cnt;
+}
 
+// ---- kNN, k > 64: a thread per query over the binary records -----------------------
+//
+// The sorted list lives in the query's output rows, with the slot index of each
+// entry in `slots` (k ints per query).  Nearer child first, the farther one
+// stacked with its box distance; leaves are scanned by the warp's threads
+// together, each its own.
 __device__ __forceinline__ bool cand_less(float d, int id, float d2, int id2) {
     return d < d2 || (d == d2 && id < id2);
 }
 
-// KMAX > 0: the best k candidates live sorted in registers (k <= KMAX).
-// KMAX == 0: any k; the sorted candidates live in memory: in kd / ki / ks
-// (entry j of the list at index j * kst; shared memory in the per-call
-// kernel for k <= KNN_SMEM_MAX), or, when kd is null, in the query's output
-// rows with the slot index parked in `slots` (k ints per query).
-// Traversal of one query by a group of G consecutive lanes: nearer child
-// first, the farther one pushed with its box distance; a subtree is skipped
-// when that distance exceeds min(max_dist^2, current k-th distance).  The loop
-// is "while-while": a node phase steps every group through nodes until it holds
-// a leaf (or is finished), then the warp scans leaves together, so the leaf
-// scans run with most lanes active.  The G lanes of a group keep identical
-// copies of the traversal state; in a leaf, lane s takes slots s, s+G, ...
-// and the G candidates of each round are broadcast and offered to every copy
-// in lane order, which keeps the copies identical.
-// `tid` is the query (before the optional permutation `perm`) of this
-// thread's group; every lane of the warp must call this together.
-template <int KMAX, int G, int PAIRS = knn_leaf_pairs<KMAX>()>
-__device__ __forceinline__ void knn_body(const DevTree& t, long long tid, const float* __restrict__ q, int q_stride,
-                                         long long nq, int k, float max_sq, int* __restrict__ out_id,
-                                         float* __restrict__ out_d2, float* __restrict__ out_xyz,
-                                         int* __restrict__ out_cnt, int* __restrict__ slots,
-                                         const int* __restrict__ perm, float* kd = nullptr, int* ki = nullptr,
-                                         int* ks = nullptr, int kst = 1, float* wstage = nullptr) {
-    const int sub = threadIdx.x & (G - 1);
-    const int lane = threadIdx.x & 31;
-    const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
-    const bool valid = tid < nq;
-    long long qi = valid ? tid : 0;
-    if (valid && perm != nullptr) qi = __ldg(perm + tid);
-    const float qx = valid ? q[qi * q_stride + 0] : 0.f;
-    const float qy = valid ? q[qi * q_stride + 1] : 0.f;
-    const float qz = valid ? q[qi * q_stride + 2] : 0.f;
-
-    constexpr int KR = KMAX > 0 ? KMAX : 1;
-    float bd[KR];
-    int bi[KR], bsl[KR];
-#pragma unroll
-    for (int j = 0; j < KR; ++j) {
-        bd[j] = FINF;
-        bi[j] = 0x7fffffff;
-        bsl[j] = -1;
-    }
-    const bool in_rows = kd == nullptr;
-    float* gd = in_rows ? out_d2 + qi * k : kd;
-    int* gi = in_rows ? out_id + qi * k : ki;
-    int* gs = in_rows ? (slots != nullptr ? slots + qi * k : nullptr) : ks;
-    const int gst = in_rows ? 1 : kst;
-    int gcnt = 0;
+__device__ __forceinline__ void knn_rows_body(const DevTree& t, bool valid, long long qi, float qx, float qy, float qz,
+                                              int k, float max_sq, const KnnOut& o, int* __restrict__ slots) {
+    float* gd = o.d2 + qi * k;
+    int* gi = o.id + qi * k;
+    int* gs = slots + qi * k;
+    int cnt = 0;
     float worst = FINF;
     int worst_id = 0x7fffffff;
-
     int st_code[MAX_STACK];
     float st_d[MAX_STACK];
     int sp = 0;
     int cur = 0;  // node code (>= 0; 0 = the sentinel record) or leaf code (< 0)
     bool done = !valid;
     int visits = 0;
-    const float4* __restrict__ P = t.pts;
-
-    // Next stacked subtree that can still hold a result, or done.
     auto pop = [&]() {
         const float lim = fminf(max_sq, worst);
         while (sp > 0) {
@@ -141,57 +396,7 @@ __device__ __forceinline__ void knn_body(const DevTree& t, long long tid, const 
         }
         done = true;
     };
-
-    // Offers a candidate to this lane's copy of the k best.
-    auto offer = [&](float d, int id, int sl) {
-        if (!(d <= max_sq && cand_less(d, id, worst, worst_id))) return;
-        if (KMAX == 0) {
-            // Large k: the sorted list lives in the output rows; only the
-            // group's first lane owns them.
-            if (sub == 0) {
-                int pos = gcnt < k ? gcnt : k - 1;
-                while (pos > 0 && cand_less(d, id, gd[(pos - 1) * gst], gi[(pos - 1) * gst])) {
-                    gd[pos * gst] = gd[(pos - 1) * gst];
-                    gi[pos * gst] = gi[(pos - 1) * gst];
-                    gs[pos * gst] = gs[(pos - 1) * gst];
-                    --pos;
-                }
-                gd[pos * gst] = d;
-                gi[pos * gst] = id;
-                gs[pos * gst] = sl;
-            }
-            if (gcnt < k) ++gcnt;
-            if (gcnt == k) {
-                __syncwarp(gmask);
-                worst = __shfl_sync(gmask, sub == 0 ? gd[(k - 1) * gst] : 0.f, lane & ~(G - 1));
-                worst_id = __shfl_sync(gmask, sub == 0 ? gi[(k - 1) * gst] : 0, lane & ~(G - 1));
-            }
-            return;
-        }
-        float cd = d;
-        int cid = id, cs = sl;
-#pragma unroll
-        for (int m = 0; m < KR; ++m) {
-            const bool sw = cand_less(cd, cid, bd[m], bi[m]);
-            const float td = bd[m];
-            const int ti = bi[m], ts = bsl[m];
-            bd[m] = sw ? cd : td;
-            bi[m] = sw ? cid : ti;
-            bsl[m] = sw ? cs : ts;
-            cd = sw ? td : cd;
-            cid = sw ? ti : cid;
-            cs = sw ? ts : cs;
-        }
-#pragma unroll
-        for (int m = 0; m < KR; ++m)
-            if (m == k - 1) {
-                worst = bd[m];
-                worst_id = bi[m];
-            }
-    };
-
     while (true) {
-        // Node phase.
         while (true) {
             const bool nodework = !done && cur >= 0;
             if (!__any_sync(0xffffffffu, nodework)) break;
@@ -201,7 +406,7 @@ __device__ __forceinline__ void knn_body(const DevTree& t, long long tid, const 
                 done = true;
                 continue;
             }
-            NodeRec r = load_node(t.node, cur);
+            const NodeRec r = load_node(t.node, cur);
             const int cl = r.left(), cr = r.right();
             const float lim = fminf(max_sq, worst);
             float dl = FINF, dr = FINF;
@@ -216,9 +421,8 @@ __device__ __forceinline__ void knn_body(const DevTree& t, long long tid, const 
             }
             if (vl && vr) {
                 const bool left_first = dl <= dr;
-                const int far = left_first ? cr : cl;
                 if (sp < MAX_STACK) {
-                    st_code[sp] = far;
+                    st_code[sp] = left_first ? cr : cl;
                     st_d[sp] = left_first ? dr : dl;
                     ++sp;
                 } else {
@@ -233,160 +437,51 @@ __device__ __forceinline__ void knn_body(const DevTree& t, long long tid, const 
                 pop();
             }
         }
-        // Leaf phase.
         const bool leafwork = !done && cur < 0;
         if (!__any_sync(0xffffffffu, leafwork)) break;
         if (!leafwork) continue;
         const int L = code_leaf(cur);
         const int n = min(__ldg(t.leaf_n + L), LEAF_CAP);
-        const float4* lp = P + (long long)L * LEAF_CAP;
-        if (G == 1) {
-            // Two passes.  First every slot's distance is checked against the
-            // current bound, marking the slots that can enter the list (no
-            // branch: lanes stay converged); then only the marked slots are
-            // offered, re-read from L1.  Offering in one pass made the warp run
-            // the insertion for every slot at which any lane had a candidate.
-            // The final list does not depend on the order of the offers, and
-            // the bound only tightens, so the marks miss nothing.
-            // Two slots per 256-bit load (slot pairs are 32-byte aligned), and
-            // PAIRS loads issued together before any is used.
-            // A bucket always has LEAF_CAP slots in the pool, so loads past
-            // the fill count stay inside it; their slots are ignored.
-            static_assert(LEAF_CAP % (2 * PAIRS) == 0, "a batch of pairs must not leave the bucket");
-            static_assert(LEAF_CAP <= 32, "one mark bit per slot");
-            uint32_t marks = 0;
-            for (int j0 = 0; j0 < n; j0 += 2 * PAIRS) {
-                float4 pa[PAIRS], pb[PAIRS];
-#pragma unroll
-                for (int u = 0; u < PAIRS; ++u) ld_slot_pair(lp + j0 + 2 * u, pa[u], pb[u]);
-#pragma unroll
-                for (int u = 0; u < PAIRS; ++u) {
-                    const int j = j0 + 2 * u;
-                    const uint32_t wa = __float_as_uint(pa[u].w);
-                    const float da = sq_dist(qx, qy, qz, pa[u].x, pa[u].y, pa[u].z);
-                    const bool ma = j < n && !(wa & F_DEL) && da <= max_sq &&
-                                    cand_less(da, (int)(wa & ID_MASK), worst, worst_id);
-                    const uint32_t wb = __float_as_uint(pb[u].w);
-                    const float db = sq_dist(qx, qy, qz, pb[u].x, pb[u].y, pb[u].z);
-                    const bool mb = j + 1 < n && !(wb & F_DEL) && db <= max_sq &&
-                                    cand_less(db, (int)(wb & ID_MASK), worst, worst_id);
-                    marks |= (ma ? 1u : 0u) << j;
-                    marks |= (mb ? 1u : 0u) << (j + 1);
-                }
+        for (int j = 0; j < n; ++j) {
+            const float4 p = __ldg(t.pts + (long long)L * LEAF_CAP + j);
+            const uint32_t w = __float_as_uint(p.w);
+            if (w & F_DEL) continue;
+            const float d = sq_dist(qx, qy, qz, p.x, p.y, p.z);
+            const int id = (int)(w & ID_MASK);
+            if (!(d <= max_sq && cand_less(d, id, worst, worst_id))) continue;
+            int pos = cnt < k ? cnt : k - 1;
+            while (pos > 0 && cand_less(d, id, gd[pos - 1], gi[pos - 1])) {
+                gd[pos] = gd[pos - 1];
+                gi[pos] = gi[pos - 1];
+                gs[pos] = gs[pos - 1];
+                --pos;
             }
-            while (marks) {
-                const int j = __ffs(marks) - 1;
-                marks &= marks - 1;
-                const float4 p = __ldg(lp + j);
-                const uint32_t w = __float_as_uint(p.w);
-                offer(sq_dist(qx, qy, qz, p.x, p.y, p.z), (int)(w & ID_MASK), L * LEAF_CAP + j);
+            gd[pos] = d;
+            gi[pos] = id;
+            gs[pos] = L * LEAF_CAP + j;
+            if (cnt < k) ++cnt;
+            if (cnt == k) {
+                worst = gd[k - 1];
+                worst_id = gi[k - 1];
             }
-        } else {
-          for (int j0 = 0; j0 < n; j0 += G) {
-            const int j = j0 + sub;
-            float d = FINF;
-            int id = 0x7fffffff, sl = -1;
-            if (j < n) {
-                const float4 p = __ldg(lp + j);
-                const uint32_t w = __float_as_uint(p.w);
-                if (!(w & F_DEL)) {
-                    d = sq_dist(qx, qy, qz, p.x, p.y, p.z);
-                    id = (int)(w & ID_MASK);
-                    sl = L * LEAF_CAP + j;
-                }
-            }
-            {
-#pragma unroll
-                for (int s = 0; s < G; ++s) {
-                    const int src = (lane & ~(G - 1)) + s;
-                    const float ds = __shfl_sync(gmask, d, src);
-                    const int is = __shfl_sync(gmask, id, src);
-                    const int ss = __shfl_sync(gmask, sl, src);
-                    if (ss >= 0) offer(ds, is, ss);
-                }
-            }
-          }
         }
         pop();
     }
-    if constexpr (KMAX > 0 && G == 1) {
-        if (wstage != nullptr) {
-            // The warp's 32 queries are consecutive (no permutation): their
-            // rows form one contiguous span of every output array.  Stage the
-            // rows in shared memory, then write each span with coalesced,
-            // 16-byte stores (the outputs may be host memory over the chip
-            // link, where scattered 4-byte stores are slow).
-            const long long q0 = tid - lane;
-            const int nrows = (int)min(32ll, nq - q0);
-            if (nrows <= 0) return;
-            float* s_id = wstage;
-            float* s_d2 = s_id + 32 * KMAX;
-            float* s_xyz = s_d2 + 32 * KMAX;
-            float* s_cnt = s_xyz + 96 * KMAX;
-            if (valid) {
-                int cnt = 0;
-#pragma unroll
-                for (int j = 0; j < KR; ++j) {
-                    if (j < k) {
-                        const bool ok = bsl[j] >= 0;
-                        const int id = ok ? bi[j] : -1;
-                        const float dd = ok ? bd[j] : FINF;
-                        s_id[lane * k + j] = __int_as_float(id);
-                        s_d2[lane * k + j] = dd;
-                        if (out_xyz != nullptr) {
-                            const float4 p = ok ? __ldg(P + bsl[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
-                            s_xyz[(lane * k + j) * 3 + 0] = p.x;
-                            s_xyz[(lane * k + j) * 3 + 1] = p.y;
-                            s_xyz[(lane * k + j) * 3 + 2] = p.z;
-                        }
-                        cnt += ok ? 1 : 0;
-                    }
-                }
-                s_cnt[lane] = __int_as_float(cnt);
-            }
-            __syncwarp();
-            warp_store(reinterpret_cast<float*>(out_id + q0 * k), s_id, nrows * k);
-            warp_store(out_d2 + q0 * k, s_d2, nrows * k);
-            if (out_xyz != nullptr) warp_store(out_xyz + q0 * k * 3, s_xyz, nrows * k * 3);
-            if (out_cnt != nullptr) warp_store(reinterpret_cast<float*>(out_cnt + q0), s_cnt, nrows);
-            return;
+    if (!valid) return;
+    for (int j = 0; j < k; ++j) {
+        const bool ok = j < cnt;
+        if (!ok) {
+            gi[j] = -1;
+            gd[j] = FINF;
+        }
+        if (o.xyz != nullptr) {
+            const float4 p = ok ? __ldg(t.pts + gs[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
+            o.xyz[(qi * k + j) * 3 + 0] = p.x;
+            o.xyz[(qi * k + j) * 3 + 1] = p.y;
+            o.xyz[(qi * k + j) * 3 + 2] = p.z;
         }
     }
-    if (!valid || sub != 0) return;
-
-    if (KMAX == 0) {
-        for (int j = 0; j < k; ++j) {
-            const bool ok = j < gcnt;
-            const int sl = ok ? gs[j * gst] : -1;
-            out_id[qi * k + j] = ok ? gi[j * gst] : -1;
-            out_d2[qi * k + j] = ok ? gd[j * gst] : FINF;
-            if (out_xyz != nullptr) {
-                float4 p = ok ? __ldg(P + sl) : make_float4(0.f, 0.f, 0.f, 0.f);
-                out_xyz[(qi * k + j) * 3 + 0] = p.x;
-                out_xyz[(qi * k + j) * 3 + 1] = p.y;
-                out_xyz[(qi * k + j) * 3 + 2] = p.z;
-            }
-        }
-        if (out_cnt != nullptr) out_cnt[qi] = gcnt;
-        return;
-    }
-    int cnt = 0;
-#pragma unroll
-    for (int j = 0; j < KR; ++j) {
-        if (j < k) {
-            const bool ok = bsl[j] >= 0;
-            out_id[qi * k + j] = ok ? bi[j] : -1;
-            out_d2[qi * k + j] = ok ? bd[j] : FINF;
-            if (out_xyz != nullptr) {
-                float4 p = ok ? __ldg(P + bsl[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
-                out_xyz[(qi * k + j) * 3 + 0] = p.x;
-                out_xyz[(qi * k + j) * 3 + 1] = p.y;
-                out_xyz[(qi * k + j) * 3 + 2] = p.z;
-            }
-            cnt += ok ? 1 : 0;
-        }
-    }
-    if (out_cnt != nullptr) out_cnt[qi] = cnt;
+    if (o.cnt != nullptr) o.cnt[qi] = cnt;
 }
 
 constexpr int RANGE_COUNT = 0, RANGE_WRITE = 1;

@@ -124,6 +124,7 @@ __global__ void refit_compute_kernel(DevTree t, UpdateAux a, const int* __restri
     // only by X's last walker, after every walker has arrived).  They are
     // fetched one level ahead, in the same round trip as the level below's
     // record, so each level costs the arrival and one load round trip.
+    // So is the parent's place in the wide records, where X's box also goes.
     auto invariants = [&](int X, float2& kids, int& lp, int& expect) {
         kids = __ldcg(reinterpret_cast<const float2*>(t.node + 4 * X + 3));
         lp = __ldcg(&t.nparent[X]);
@@ -140,6 +141,7 @@ __global__ void refit_compute_kernel(DevTree t, UpdateAux a, const int* __restri
         if (llp < 0) return;
         X = llp >> 1;
         if (X > 0) invariants(X, kids, lp, expect);
+        const int2 wi = __ldcg(t.winfo + X);
         int n = __ldcg(&t.leaf_n[L]);
         int m = n < LEAF_CAP ? n : LEAF_CAP;
         Box3 b = empty_box();
@@ -154,6 +156,7 @@ __global__ void refit_compute_kernel(DevTree t, UpdateAux a, const int* __restri
         }
         write_child_box(t.node, X, llp & 1, b);
         write_child_cnt(t.ncnt, X, llp & 1, n, del);
+        wide_update(t, wi, llp & 1, code, b, n - del);
         if (n > LEAF_CAP)  // an overflowing bucket must be split
             list_push(t.st, &t.st->n_viol, a.viol, a.list_cap, code);
     } else {
@@ -180,6 +183,7 @@ __global__ void refit_compute_kernel(DevTree t, UpdateAux a, const int* __restri
         int4 cc = __ldcg(t.ncnt + X);
         float2 kids_p = make_float2(0.f, 0.f);
         int lp_p = 0, expect_p = 0;
+        const int2 wi = __ldcg(t.winfo + P);
         if (P > 0) invariants(P, kids_p, lp_p, expect_p);
         Box3 b = empty_box();
         Box3 bl = r.box(0), br = r.box(1);
@@ -209,6 +213,7 @@ __global__ void refit_compute_kernel(DevTree t, UpdateAux a, const int* __restri
         }
         write_child_box(t.node, P, lp & 1, b);
         write_child_cnt(t.ncnt, P, lp & 1, slots, del);
+        wide_update(t, wi, lp & 1, X, b, slots - del);
         X = P;
         kids = kids_p;
         lp = lp_p;
@@ -847,6 +852,34 @@ __global__ void validate_nodes_kernel(DevTree t, bool at_rest, unsigned long lon
                     box_grow(b, p.x, p.y, p.z);
             }
         }
+        // the wide records: the child's own place, and its slot if it has one
+        const int2 wi = t.winfo[X];
+        const int pos = wi.y * 2 + side;
+        if (c > 0) {
+            const int2 wc = t.winfo[c], want = wide_below(wi, side, c);
+            if (wc.x != want.x || wc.y != want.y) {
+                ++nbad;
+                note_bad(t.st, 112, X, side, c, wc.x, wc.y, want.y);
+            }
+        }
+        if (pos >= WIDE || c < 0) {
+            const float* f = reinterpret_cast<const float*>(t.wide + (long long)wi.x * 16);
+            const int s0 = wide_slot(pos);
+            Box3 wb;
+            for (int a = 0; a < 3; ++a) {
+                wb.lo[a] = f[wide_at(s0, a)];
+                wb.hi[a] = f[wide_at(s0, 3 + a)];
+            }
+            bool empty_rest = true;
+            for (int s = 1; pos < WIDE && s < (8 >> (31 - __clz(pos))); ++s)
+                empty_rest = empty_rest && __float_as_int(f[wide_at(s0 + s, 6)]) == 0 &&
+                             !(f[wide_at(s0 + s, 0)] <= f[wide_at(s0 + s, 3)]);
+            const int wc = __float_as_int(f[wide_at(s0, 6)]), wv = __float_as_int(f[wide_at(s0, 7)]);
+            if (wc != c || wv != slots - del || !same_box(wb, stored) || !empty_rest) {
+                ++nbad;
+                note_bad(t.st, 113, X, side, c, wc, wv, slots - del);
+            }
+        }
         if (s2 != slots || d2 != del) {
             ++nbad;
             note_bad(t.st, 106, X, side, slots, s2, del, d2);
@@ -906,6 +939,12 @@ __global__ void validate_aux_leaves_kernel(DevTree t, UpdateAux a, unsigned long
 }
 
 __global__ void set_ll_kernel(long long* p, long long v) { *p = v; }
+
+// Empties the top wide record and places the root at position `pos` in it.
+__global__ void set_top_kernel(DevTree t, int pos) {
+    if (threadIdx.x == 0) t.winfo[0] = make_int2(0, pos / 2);
+    wide_store(t.wide, 0, threadIdx.x, empty_box(), 0, 0);
+}
 
 __global__ void snapshot_root_kernel(DevTree t) {
     int4 c = t.ncnt[0];
@@ -1590,6 +1629,8 @@ void launch_delete_points(const DevTree& t, const UpdateAux& a, const float* pts
 }
 
 void launch_snapshot_root(const DevTree& t, cudaStream_t s) { snapshot_root_kernel<<<1, 1, 0, s>>>(t); }
+
+void launch_set_top(const DevTree& t, int pos, cudaStream_t s) { set_top_kernel<<<1, WIDE, 0, s>>>(t, pos); }
 
 void launch_set_ll(long long* p, long long v, cudaStream_t s) { set_ll_kernel<<<1, 1, 0, s>>>(p, v); }
 

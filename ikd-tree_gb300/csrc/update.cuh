@@ -63,6 +63,9 @@ void launch_delete_points(const DevTree& t, const UpdateAux& a, const float* pts
                           cudaStream_t s);
 void launch_add_boxes(const DevTree& t, const UpdateAux& a, const float* boxes, long long m, cudaStream_t s);
 void launch_snapshot_root(const DevTree& t, cudaStream_t s);
+// Empties the top wide record and places the root at position pos (2, 4 or 8)
+// in it; the whole tree is then to be built.
+void launch_set_top(const DevTree& t, int pos, cudaStream_t s);
 // *p = v on the stream (no host wait; the value travels as a kernel argument).
 void launch_set_ll(long long* p, long long v, cudaStream_t s);
 void launch_route_append_dev_count(const DevTree& t, const UpdateAux& a, const float4* pts, long long n_bound,

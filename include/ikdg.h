@@ -63,10 +63,12 @@ int ikdg_set_balance_criterion_param(ikdg_tree* t, float balance_param);
 int ikdg_set_downsample_param(ikdg_tree* t, float box_length);
 /* Tuning knobs (no counterpart in the reference): points per leaf bucket
  * written by (re)builds, 8..32 (default 16); threads cooperating on one kNN
- * query, 1, 2 or 4 (default 1); tree levels used to sort a kNN batch into
- * spatially coherent order before the search: -1 (default) sorts by 16
- * levels from 262,144 queries up and not below, 0 never sorts, 1..16 sorts
- * every batch of at least 2048 queries. */
+ * query, 1, 2 or 4 (checked, without effect: the searches give every query
+ * four lanes); tree levels used to sort a kNN batch into spatially coherent
+ * order before the search: -1 (default) sorts by 14 levels where that was
+ * measured faster (524,288 queries or more, k >= 8, 12M stored points or
+ * more), 0 never sorts, 1..16 sorts every batch of at least 2048 queries.
+ * Results depend on none of them. */
 int ikdg_set_leaf_fill(ikdg_tree* t, int fill);
 int ikdg_set_knn_lanes(ikdg_tree* t, int lanes);
 int ikdg_set_knn_bin_bits(ikdg_tree* t, int bits);
@@ -163,7 +165,7 @@ int ikdg_radius_search_device(ikdg_tree* t, const float* centers, int64_t nq, in
  * points (ikdg_knn_device, ikdg_box_search_device, ikdg_radius_search_device).
  * ikdg_batch_run issues the whole list at once as one CUDA graph: the trees'
  * descriptors are refreshed, one persistent search kernel per register class
- * (kNN k <= 1, 2, 4, 8, 16 and box / radius) runs on its own graph branch, and
+ * (kNN k <= 4, 8, 16 and box / radius) runs on its own graph branch, and
  * box / radius requests then get a device prefix sum and one persistent write
  * kernel.  The graph is built at the first run after requests change.
  *
@@ -188,7 +190,8 @@ int ikdg_batch_add_box_search(ikdg_batch* b, ikdg_tree* t, const float* boxes, i
 int ikdg_batch_add_radius_search(ikdg_batch* b, ikdg_tree* t, const float* centers, int64_t nq, int32_t stride,
                                  const float* radius, int32_t radius_stride, int64_t* offsets, int32_t* ids,
                                  float* xyz, int64_t capacity, int32_t* request);
-/* Lanes per kNN query of one request (1, 2, 4; 0 = the tree's setting). */
+/* Lanes per kNN query of one request (0, 1, 2, 4): checked, without effect (as
+ * ikdg_set_knn_lanes). */
 int ikdg_batch_set_knn_lanes(ikdg_batch* b, int32_t request, int32_t lanes);
 /* use_graph 0: issue the same kernels directly at every run (no graph). */
 int ikdg_batch_set_graph(ikdg_batch* b, int use_graph);
@@ -205,11 +208,10 @@ int ikdg_batch_run(ikdg_batch* b);
  * a request's hits exceeded its capacity (those queries wrote no ids). */
 int ikdg_batch_synchronize(ikdg_batch* b, int64_t* range_totals);
 /* Autotuner: per tree of the batch, times that tree's requests alone for
- * every leaf fill in {8, 12, 16, 24, 32} (the tree is rebuilt at each) and
- * every lanes-per-kNN-query in {1, 2, 4} (median of `reps` runs), then keeps
- * the fastest pair: the tree stays rebuilt at that fill, its kNN requests get
- * those lanes.  chosen (nullable, host) receives {fill, lanes} per distinct
- * tree, in order of first use.  Results do not depend on either setting. */
+ * every leaf fill in {8, 12, 16, 24, 32} (the tree is rebuilt at each; median
+ * of `reps` runs), then keeps the fastest: the tree stays rebuilt at that
+ * fill.  chosen (nullable, host) receives {fill, lanes} per distinct tree, in
+ * order of first use (lanes is always 1).  Results do not depend on it. */
 int ikdg_batch_autotune(ikdg_batch* b, int32_t reps, int32_t* chosen);
 int ikdg_batch_num_trees(ikdg_batch* b, int32_t* n);
 int ikdg_batch_get_stream(ikdg_batch* b, void** stream);
