@@ -35,17 +35,19 @@ __device__ __forceinline__ int find_req(const long long* __restrict__ starts, in
 // per query, the list in 1, 2 or 4 registers a lane), producing their final rows;
 // KC = BATCH_RANGE_CLASS box and radius requests (per-query hit counts in
 // counts[cbase + qi]).  One kernel per class keeps each at its own register
-// count.  entries: kNN stack entries per thread (dynamic shared memory).
+// count.  entries: stack entries, per thread (kNN) or per warp (range), in dynamic
+// shared memory.
 template <int KC>
 __global__ void __launch_bounds__(BATCH_THREADS) batch_search_kernel(const DevTree* __restrict__ trees,
                                                                      const BatchReq* __restrict__ reqs,
                                                                      const long long* __restrict__ req_c1, int r0,
                                                                      int r1, long long c_begin, long long c_end,
                                                                      long long* __restrict__ counts,
+                                                                     search::RangeLog log,
                                                                      unsigned long long* __restrict__ ctr,
                                                                      int entries) {
     constexpr int G = search::KNN_G, R = KC == 0 ? 1 : KC == 1 ? 2 : 4;
-    extern __shared__ int2 batch_sm[];
+    extern __shared__ __align__(16) int2 batch_sm[];
     const int lane = threadIdx.x & 31;
     for (;;) {
         // Each warp takes its own chunk: no warp waits for another.
@@ -79,30 +81,42 @@ __global__ void __launch_bounds__(BATCH_THREADS) batch_search_kernel(const DevTr
                 search::knn_write_rows<R>(t, g, valid, ld, ls, Rq.k, qi, o);
             }
         } else {
-            // warp-collective body: every lane calls it
-            long long qi = (c - Rq.c1) * BATCH_CHUNK + lane;
-            const bool valid = qi < Rq.nq;
+            const search::RangeWarp w =
+                search::range_warp_carve<false>(reinterpret_cast<unsigned char*>(batch_sm), entries);
+            long long qi = (c - Rq.c1) * Rq.per + lane;
+            const bool valid = lane < Rq.per && qi < Rq.nq;
             if (valid && Rq.perm != nullptr) qi = __ldg(Rq.perm + qi);
-            const long long n =
-                Rq.kind == BATCH_BOX
-                    ? search::range_body<0, search::RANGE_COUNT>(t, Rq.q, Rq.q_stride, nullptr, 0, qi, valid, 0, 0,
-                                                                 nullptr, nullptr)
-                    : search::range_body<1, search::RANGE_COUNT>(t, Rq.q, Rq.q_stride, Rq.radius, Rq.r_stride, qi,
-                                                                 valid, 0, 0, nullptr, nullptr);
-            if (valid) counts[Rq.cbase + qi] = n;
+            w.cnt[lane] = 0;
+            const unsigned todo = __ballot_sync(0xffffffffu, valid);
+            search::LogCursor lc(log, Rq.c2 + (c - Rq.c1));
+            if (Rq.kind == BATCH_BOX) {
+                if (valid) search::range_put_query<0>(w, lane, Rq.q + qi * Rq.q_stride, 0.f);
+                search::range_warp<0, false>(t, w, todo, entries, log, lc, 0, 0, nullptr, nullptr);
+            } else {
+                if (valid) search::range_put_query<1>(w, lane, Rq.q + qi * Rq.q_stride, Rq.radius[qi * Rq.r_stride]);
+                search::range_warp<1, false>(t, w, todo, entries, log, lc, 0, 0, nullptr, nullptr);
+            }
+            lc.close();
+            __syncwarp();
+            if (valid) counts[Rq.cbase + qi] = w.cnt[lane];
+            __syncwarp();
         }
     }
 }
 
 // Phase 2: range requests write their CSR offsets and, where the request's
 // capacity holds the query's results, the ids / points.
-__global__ void __launch_bounds__(BATCH_THREADS) batch_write_kernel(const DevTree* __restrict__ trees,
+__global__ void __launch_bounds__(BATCH_THREADS, 6) batch_write_kernel(const DevTree* __restrict__ trees,
                                                                     const BatchReq* __restrict__ reqs,
                                                                     const int* __restrict__ ridx,
                                                                     const long long* __restrict__ req_c2, int nr,
                                                                     long long c_end,
                                                                     const long long* __restrict__ goff,
-                                                                    unsigned long long* __restrict__ ctr) {
+                                                                    search::RangeLog log,
+                                                                    unsigned long long* __restrict__ ctr, int entries) {
+    extern __shared__ __align__(16) int2 batch_sm[];
+    const search::RangeWarp w =
+        search::range_warp_carve<true>(reinterpret_cast<unsigned char*>(batch_sm), entries);
     const int lane = threadIdx.x & 31;
     for (;;) {
         long long c = 0;
@@ -116,17 +130,16 @@ __global__ void __launch_bounds__(BATCH_THREADS) batch_write_kernel(const DevTre
         if (c >= c_end) break;
         const BatchReq& R = reqs[r];
         const DevTree t = trees[R.tree];
-        const long long pos = (c - R.c2) * BATCH_CHUNK + lane;
-        const long long qi = pos < R.nq && R.perm != nullptr ? (long long)__ldg(R.perm + pos) : pos;
+        const long long at = (c - R.c2) * R.per + lane;
+        bool go = lane < R.per && at < R.nq;
+        const long long qi = go && R.perm != nullptr ? (long long)__ldg(R.perm + at) : at;
         const long long base = goff[R.cbase];
-        if (pos == 0) {
+        long long o = 0, n = 0;
+        if (go && at == 0) {
             const long long tot = goff[R.cbase + R.nq] - base;
             R.offsets[R.nq] = tot;
             if (R.total != nullptr) *R.total = tot;
         }
-        // warp-collective body: every lane calls it, lanes without work idle
-        bool go = pos < R.nq;
-        long long o = 0, n = 0;
         if (go) {
             o = goff[R.cbase + qi] - base;
             n = goff[R.cbase + qi + 1] - goff[R.cbase + qi];
@@ -138,12 +151,22 @@ __global__ void __launch_bounds__(BATCH_THREADS) batch_write_kernel(const DevTre
                 go = false;
             }
         }
-        if (R.kind == BATCH_BOX)
-            search::range_body<0, search::RANGE_WRITE>(t, R.q, R.q_stride, nullptr, 0, qi, go, o, o + n, R.ids,
-                                                       R.xyz);
-        else
-            search::range_body<1, search::RANGE_WRITE>(t, R.q, R.q_stride, R.radius, R.r_stride, qi, go, o, o + n,
-                                                       R.ids, R.xyz);
+        const unsigned todo = __ballot_sync(0xffffffffu, go);
+        if (todo == 0) continue;
+        const int2* first = log.pool + c * search::LOG_CHUNK;
+        if (todo == __ballot_sync(0xffffffffu, n > 0) && __ldg(&first->x) >= 0) {
+            search::range_replay(t, w, log, first, o, o + n, R.ids, R.xyz);
+            continue;
+        }
+        search::LogCursor lc(search::RangeLog{nullptr, nullptr, 0, 0}, 0);
+        if (R.kind == BATCH_BOX) {
+            if (go) search::range_put_query<0>(w, lane, R.q + qi * R.q_stride, 0.f);
+            search::range_warp<0, true>(t, w, todo, entries, log, lc, o, o + n, R.ids, R.xyz);
+        } else {
+            if (go) search::range_put_query<1>(w, lane, R.q + qi * R.q_stride, R.radius[qi * R.r_stride]);
+            search::range_warp<1, true>(t, w, todo, entries, log, lc, o, o + n, R.ids, R.xyz);
+        }
+        __syncwarp();
     }
 }
 
@@ -184,11 +207,18 @@ __global__ void batch_key_kernel(const DevTree* __restrict__ trees, const BatchR
 
 std::mutex g_grid_mu;
 
-// Dynamic shared memory of a search kernel class: the kNN stacks.
+// Dynamic shared memory of a search kernel class, its stack entries.
+static_assert(BATCH_THREADS == search::RANGE_CTA, "range warps per CTA");
 size_t class_smem(int kc, int height) {
     return kc < BATCH_RANGE_CLASS
                ? sizeof(int2) * search::knn_stack_entries(height) * BATCH_THREADS
-               : 0;
+               : WARPS_PER_CTA * search::range_warp_bytes(search::range_stack_entries(height), false);
+}
+int class_entries(int kc, int height) {
+    return kc < BATCH_RANGE_CLASS ? search::knn_stack_entries(height) : search::range_stack_entries(height);
+}
+size_t write_smem(int height) {
+    return WARPS_PER_CTA * search::range_warp_bytes(search::range_stack_entries(height), true);
 }
 
 int resident_grid(const void* fn, size_t smem = 0) {
@@ -202,14 +232,19 @@ int resident_grid(const void* fn, size_t smem = 0) {
     return (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
 }
 
+search::RangeLog to_log(const BatchLog& l) { return search::RangeLog{(int2*)l.pool, l.next, l.warps, l.chunks}; }
+
 typedef void (*SearchKernel)(const DevTree*, const BatchReq*, const long long*, int, int, long long, long long,
-                             long long*, unsigned long long*, int);
+                             long long*, search::RangeLog, unsigned long long*, int);
 SearchKernel search_kernel(int kc) {
     return kc == 0 ? batch_search_kernel<0> : kc == 1 ? batch_search_kernel<1> : kc == 2 ? batch_search_kernel<2>
                                                                               : batch_search_kernel<BATCH_RANGE_CLASS>;
 }
 
 }  // namespace
+
+size_t batch_log_bytes(long long chunks) { return sizeof(int2) * search::LOG_CHUNK * (size_t)chunks; }
+long long batch_log_chunks(long long warps) { return warps + (warps * 4 < 131072 ? warps * 4 : 131072); }
 
 int batch_kclass(int k) { return k <= 4 ? 0 : k <= 8 ? 1 : 2; }
 
@@ -218,19 +253,19 @@ int batch_search_grid(int kclass, int height) {
     return resident_grid((const void*)search_kernel(kclass), class_smem(kclass, height));
 }
 
-int batch_write_grid() {
+int batch_write_grid(int height) {
     std::lock_guard<std::mutex> lock(g_grid_mu);
-    return resident_grid((const void*)batch_write_kernel);
+    return resident_grid((const void*)batch_write_kernel, write_smem(height));
 }
 
 void launch_batch_search(const DevTree* trees, const BatchReq* reqs, const long long* req_c1, int r0, int r1,
                          long long c_begin, long long c_end, int kclass, int height, long long* counts,
-                         unsigned long long* ctr, int grid, cudaStream_t s) {
+                         const BatchLog& log, unsigned long long* ctr, int grid, cudaStream_t s) {
     if (c_end <= c_begin || r1 <= r0) return;
     const long long ctas = (c_end - c_begin + WARPS_PER_CTA - 1) / WARPS_PER_CTA;
     const unsigned g = (unsigned)(ctas < grid ? ctas : grid);
     search_kernel(kclass)<<<g, BATCH_THREADS, class_smem(kclass, height), s>>>(
-        trees, reqs, req_c1, r0, r1, c_begin, c_end, counts, ctr, search::knn_stack_entries(height));
+        trees, reqs, req_c1, r0, r1, c_begin, c_end, counts, to_log(log), ctr, class_entries(kclass, height));
 }
 
 void launch_batch_keys(const DevTree* trees, const BatchReq* reqs, const long long* qstart, int n, long long total,
@@ -241,11 +276,14 @@ void launch_batch_keys(const DevTree* trees, const BatchReq* reqs, const long lo
 }
 
 void launch_batch_write(const DevTree* trees, const BatchReq* reqs, const int* ridx, const long long* req_c2, int nr,
-                        long long c_end, const long long* goff, unsigned long long* ctr, int grid, cudaStream_t s) {
+                        long long c_end, int height, const long long* goff, const BatchLog& log, unsigned long long* ctr,
+                        int grid, cudaStream_t s) {
     if (c_end <= 0 || nr <= 0) return;
     const long long ctas = (c_end + WARPS_PER_CTA - 1) / WARPS_PER_CTA;
     const unsigned g = (unsigned)(ctas < grid ? ctas : grid);
-    batch_write_kernel<<<g, BATCH_THREADS, 0, s>>>(trees, reqs, ridx, req_c2, nr, c_end, goff, ctr);
+    batch_write_kernel<<<g, BATCH_THREADS, write_smem(height), s>>>(trees, reqs, ridx, req_c2, nr, c_end, goff,
+                                                                   to_log(log), ctr,
+                                                                   search::range_stack_entries(height));
 }
 
 }  // namespace ikdg

@@ -933,14 +933,15 @@ struct Tree {
         offsets[0] = 0;
         if (nq == 0) return;
         reset_counters();
+        const int logged = ids != nullptr ? RANGE_LOG : 0;
         op.ensure(align_up(sizeof(float) * nq * qs) + align_up(sizeof(float) * nq) +
-                      2 * align_up(sizeof(long long) * (nq + 1)),
+                      align_up(sizeof(long long) * (nq + 1)) + align_up(range_temp_bytes(nq, logged)),
                   stream);
         Carver c(op.p);
         float* dq = c.take<float>((size_t)nq * qs);
         float* dr = c.take<float>(nq);
-        long long* dcounts = c.take<long long>(nq + 1);
         long long* doffs = c.take<long long>(nq + 1);
+        void* temp = c.take<char>(range_temp_bytes(nq, logged));
         CK(cudaMemcpyAsync(dq, q, sizeof(float) * nq * qs, cudaMemcpyHostToDevice, stream));
         std::vector<float> rr;
         if (mode == 1) {
@@ -948,17 +949,12 @@ struct Tree {
             for (long long i = 0; i < nq; ++i) rr[i] = radius[i * rstride];
             CK(cudaMemcpyAsync(dr, rr.data(), sizeof(float) * nq, cudaMemcpyHostToDevice, stream));
         }
-        launch_range(dt, mode, dq, qs, dr, 1, nq, dcounts, nullptr, nullptr, nullptr, -1, stream);
-        std::vector<long long> counts(nq);
-        CK(cudaMemcpyAsync(counts.data(), dcounts, sizeof(long long) * nq, cudaMemcpyDeviceToHost, stream));
+        launch_range(dt, mode, dq, qs, dr, 1, nq, temp, RANGE_COUNT | logged, doffs, nullptr, nullptr, -1, nullptr,
+                     stream);
+        CK(cudaMemcpyAsync(offsets, doffs, sizeof(long long) * (nq + 1), cudaMemcpyDeviceToHost, stream));
         read_status();
         if (st->err & ERR_STACK) throw Internal{"range search: traversal stack overflow"};
-        long long acc = 0;
-        for (long long i = 0; i < nq; ++i) {
-            offsets[i] = acc;
-            acc += counts[i];
-        }
-        offsets[nq] = acc;
+        const long long acc = offsets[nq];
         *total = acc;
         if (acc > capacity || (acc > 0 && ids == nullptr)) throw CapacityFail{"range search: output too small"};
         if (acc == 0) return;
@@ -966,8 +962,7 @@ struct Tree {
         Carver o(bld.p);
         int* dids = o.take<int>(acc);
         float* dxyz = xyz ? o.take<float>(acc * 3) : nullptr;
-        CK(cudaMemcpyAsync(doffs, offsets, sizeof(long long) * (nq + 1), cudaMemcpyHostToDevice, stream));
-        launch_range(dt, mode, dq, qs, dr, 1, nq, nullptr, doffs, dids, dxyz, -1, stream);
+        launch_range(dt, mode, dq, qs, dr, 1, nq, temp, logged, doffs, dids, dxyz, -1, nullptr, stream);
         CK(cudaMemcpyAsync(ids, dids, sizeof(int) * acc, cudaMemcpyDeviceToHost, stream));
         if (xyz) CK(cudaMemcpyAsync(xyz, dxyz, sizeof(float) * acc * 3, cudaMemcpyDeviceToHost, stream));
         read_status();
@@ -990,14 +985,9 @@ struct Tree {
             if (total) CK(cudaMemsetAsync(total, 0, sizeof(long long), stream));
             return;
         }
-        small.ensure(align_up(sizeof(long long) * (nq + 1)) + align_up(scan_temp_bytes(nq + 1)) + 256, stream);
-        Carver c(small.p);
-        long long* counts = c.take<long long>(nq + 1);
-        void* temp = c.take<char>(scan_temp_bytes(nq + 1));
-        CK(cudaMemsetAsync(counts + nq, 0, sizeof(long long), stream));
-        launch_range(dt, mode, q, qs, radius, rstride, nq, counts, nullptr, nullptr, nullptr, -1, stream);
-        exclusive_scan(counts, offsets, nq + 1, total, temp, stream);
-        if (ids != nullptr) launch_range(dt, mode, q, qs, radius, rstride, nq, counts, offsets, ids, xyz, capacity, stream);
+        const int passes = ids != nullptr ? RANGE_COUNT | RANGE_LOG : RANGE_COUNT;
+        small.ensure(range_temp_bytes(nq, passes), stream);
+        launch_range(dt, mode, q, qs, radius, rstride, nq, small.p, passes, offsets, ids, xyz, capacity, total, stream);
         CK(cudaGetLastError());
     }
 
@@ -1260,6 +1250,7 @@ struct Batch {
     long long* d_totals = nullptr;
     unsigned long long* d_ctr = nullptr;
     void* d_scan = nullptr;
+    BatchLog log{};
     // query order (use_order): per request first query, keys / values of the sort
     long long n_queries = 0;
     int req_bits = 0;
@@ -1356,10 +1347,11 @@ struct Batch {
         std::vector<long long> c1(n);
         groups.clear();
         long long chunk = 0, cbase = 0;
-        // kNN queries per chunk, by class: as many as leave every resident warp
-        // four chunks (fewer trips to the shared counter), at least one step's.
-        int per[BATCH_RANGE_CLASS];
-        for (int kc = 0; kc < BATCH_RANGE_CLASS; ++kc) {
+        // Queries per chunk, by class: as many as leave every resident warp
+        // four chunks (fewer trips to the shared counter, full range windows),
+        // at least one kNN step's.
+        int per[BATCH_RANGE_CLASS + 1];
+        for (int kc = 0; kc <= BATCH_RANGE_CLASS; ++kc) {
             long long total = 0;
             for (auto& r : reqs)
                 if (req_class(r) == kc) total += r.d.nq;
@@ -1372,7 +1364,7 @@ struct Batch {
             BatchReq b = r.d;
             b.tree = tree_of[order[p]];
             const int kc = req_class(r);
-            b.per = kc < BATCH_RANGE_CLASS ? per[kc] : BATCH_CHUNK;
+            b.per = per[kc];
             b.c1 = chunk;
             b.n1 = (b.nq + b.per - 1) / b.per;
             chunk += b.n1;
@@ -1405,7 +1397,7 @@ struct Batch {
         for (size_t j = 0; j < range_reqs.size(); ++j) {
             BatchReq& b = d[pos_of[range_reqs[j]]];
             b.c2 = chunk2;
-            b.n2 = (b.nq + BATCH_CHUNK - 1) / BATCH_CHUNK;
+            b.n2 = (b.nq + b.per - 1) / b.per;
             if (b.n2 > 0) {
                 ridx.push_back(pos_of[range_reqs[j]]);
                 c2.push_back(chunk2);
@@ -1414,7 +1406,7 @@ struct Batch {
         }
         c2_end = chunk2;
         for (auto& g : groups) g.grid = batch_search_grid(g.kclass, plan_height);
-        write_grid = batch_write_grid();
+        write_grid = batch_write_grid(plan_height);
         // one allocation for the plan
         const size_t nt = trees.size(), nr = range_reqs.size();
         size_t bytes = align_up(sizeof(DevTree) * nt) + align_up(sizeof(BatchReq) * n) +
@@ -1425,6 +1417,8 @@ struct Batch {
         const long long nqo = ordered ? n_queries : 0;
         bytes += align_up(sizeof(long long) * (n + 1)) + 4 * align_up(sizeof(uint32_t) * std::max<long long>(nqo, 1)) +
                  align_up(ordered ? sort_temp_bytes(nqo, 1) : 0);
+        const long long log_chunks = c2_end > 0 ? batch_log_chunks(c2_end) : 0;
+        bytes += align_up(batch_log_bytes(log_chunks)) + align_up(sizeof(unsigned));
         CK(cudaMalloc(&dev, bytes));
         Carver c(dev);
         d_trees = c.take<DevTree>(nt);
@@ -1438,6 +1432,7 @@ struct Batch {
         d_ctr = c.take<unsigned long long>(64);
         d_scan = c.take<char>(scan_temp_bytes(cbase + 1));
         d_st = c.take<DevStatus>(1);
+        log = BatchLog{c.take<char>(batch_log_bytes(log_chunks)), c.take<unsigned>(1), c2_end, log_chunks};
         d_qstart = c.take<long long>(n + 1);
         for (int b2 = 0; b2 < 2; ++b2) {
             d_okeys[b2] = c.take<uint32_t>(std::max<long long>(nqo, 1));
@@ -1497,6 +1492,7 @@ struct Batch {
         CK(cudaMemcpyAsync(d_trees, h_trees, sizeof(DevTree) * trees.size(), cudaMemcpyHostToDevice, stream));
         CK(cudaMemsetAsync(d_ctr, 0, sizeof(unsigned long long) * 64, stream));
         CK(cudaMemsetAsync(d_st, 0, sizeof(DevStatus), stream));
+        CK(cudaMemsetAsync(log.next, 0, sizeof(unsigned), stream));
         if (ordered) {
             launch_batch_keys(d_trees, d_reqs, d_qstart, (int)reqs.size(), n_queries, req_bits, d_okeys[0],
                               d_ovals[0], stream);
@@ -1509,13 +1505,14 @@ struct Batch {
             cudaStream_t s = g == 0 ? stream : branch[g - 1];
             if (g > 0) CK(cudaStreamWaitEvent(s, ev_fork, 0));
             launch_batch_search(d_trees, d_reqs, d_c1, G.r0, G.r1, G.c_begin, G.c_end, G.kclass, plan_height, d_counts,
-                                d_ctr + g, G.grid, s);
+                                log, d_ctr + g, G.grid, s);
             if (g > 0) CK(cudaEventRecord(ev_join[g - 1], s));
         }
         for (size_t g = 1; g < groups.size(); ++g) CK(cudaStreamWaitEvent(stream, ev_join[g - 1], 0));
         if (nridx > 0) {
             exclusive_scan(d_counts, d_goff, n_range_queries + 1, nullptr, d_scan, stream);
-            launch_batch_write(d_trees, d_reqs, d_ridx, d_c2, nridx, c2_end, d_goff, d_ctr + 63, write_grid, stream);
+            launch_batch_write(d_trees, d_reqs, d_ridx, d_c2, nridx, c2_end, plan_height, d_goff, log, d_ctr + 63,
+                               write_grid, stream);
         }
         // range requests without queries: empty CSR
         for (int j : range_reqs)

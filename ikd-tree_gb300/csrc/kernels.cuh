@@ -89,15 +89,20 @@ size_t noalloc_scratch_bytes();
 void launch_knn(const DevTree& t, const float* q, int q_stride, long long nq, int k, float max_sq,
                 int* out_id, float* out_d2, float* out_xyz, int* out_cnt, void* temp, int bin_bits,
                 cudaStream_t s, bool host_out = false);
-// Box (mode 0) and radius (mode 1) search.  Pass 1 (ids == nullptr) writes
-// per-query hit counts into `counts`; pass 2 writes ids / xyz starting at
-// offsets[i].  Boxes are {min xyz, max xyz}; radius queries are {x, y, z} with
-// a per-query radius (r_stride floats apart).  With capacity >= 0, pass 2
-// reads counts and skips (raising ERR_OUTPUT) every query whose results would
-// end past `capacity`.
+// Box (mode 0) and radius (mode 1) search.  `temp` holds range_temp_bytes(nq,
+// passes) bytes.  passes: RANGE_COUNT counts the hits first (*total, nullable, receives
+// their number), without it the counts in temp are those of an earlier call
+// with the same queries; RANGE_LOG keeps the hits found while counting for the
+// writing (of this call or of that later one, which passes it too).  offsets
+// (nq + 1 entries) are written; with ids, the hits too.  Boxes are {min xyz, max
+// xyz}; radius queries are {x, y, z} with a per-query radius (r_stride floats
+// apart).  With capacity >= 0, a query whose hits would end past it is skipped
+// (raising ERR_OUTPUT).
+constexpr int RANGE_COUNT = 1, RANGE_LOG = 2;
+size_t range_temp_bytes(long long nq, int passes);
 void launch_range(const DevTree& t, int mode, const float* q, int q_stride, const float* radius, int r_stride,
-                  long long nq, long long* counts, const long long* offsets, int* ids, float* xyz,
-                  long long capacity, cudaStream_t s);
+                  long long nq, void* temp, int passes, long long* offsets, int* ids, float* xyz, long long capacity,
+                  long long* total, cudaStream_t s);
 
 // ---- batch.cu ---------------------------------------------------------------------
 // One request of a multi-tree batch: a kNN, box or radius search of nq queries
@@ -130,18 +135,29 @@ struct BatchReq {
     const int* perm;     // query at position i of the request's run order (nullptr: in order)
 };
 
+// The range requests' hit log (see RangeLog in search.cuh), one first chunk per
+// phase-2 chunk of queries.
+struct BatchLog {
+    void* pool;
+    unsigned* next;
+    long long warps, chunks;
+};
+size_t batch_log_bytes(long long chunks);
+// Chunks of the log for this many phase-2 chunks of queries.
+long long batch_log_chunks(long long warps);
+
 // Register class of a kNN request with this k (k <= BATCH_KMAX): 0..2;
 // range requests are class BATCH_RANGE_CLASS.
 int batch_kclass(int k);
 // Resident CTAs (whole GPU) of the persistent search kernel of a class;
-// `height`: the tallest tree of the batch (sizes the kNN stacks).
+// `height`: the tallest tree of the batch (sizes the stacks).
 int batch_search_grid(int kclass, int height);
-int batch_write_grid();
+int batch_write_grid(int height);
 // Phase 1 over requests [r0, r1), all of register class kclass, whose chunks
 // are [c_begin, c_end); ctr: a zeroed device counter.
 void launch_batch_search(const DevTree* trees, const BatchReq* reqs, const long long* req_c1, int r0, int r1,
                          long long c_begin, long long c_end, int kclass, int height, long long* counts,
-                         unsigned long long* ctr, int grid, cudaStream_t s);
+                         const BatchLog& log, unsigned long long* ctr, int grid, cudaStream_t s);
 // Spatial order of every request's queries: key = request position in the
 // high bits, Morton code of the query (kNN / radius: the point; box: its
 // centre) in the tree's root box below; vals = query index in its request.
@@ -151,7 +167,8 @@ void launch_batch_keys(const DevTree* trees, const BatchReq* reqs, const long lo
 // Phase 2 over the range requests listed in ridx[0..nr) (ascending c2, chunks
 // [0, c_end)); goff: exclusive scan of the batch count array.
 void launch_batch_write(const DevTree* trees, const BatchReq* reqs, const int* ridx, const long long* req_c2, int nr,
-                        long long c_end, const long long* goff, unsigned long long* ctr, int grid, cudaStream_t s);
+                        long long c_end, int height, const long long* goff, const BatchLog& log, unsigned long long* ctr,
+                        int grid, cudaStream_t s);
 
 // ---- register.cu ---------------------------------------------------------------
 // Rt_dev: 12 doubles, R row-major then t.  planes: 2 float4 per point ({n,d}

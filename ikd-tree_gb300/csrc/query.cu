@@ -97,35 +97,87 @@ void knn_group_launch(const DevTree& t, const float* q, int q_stride, long long 
     }
 }
 
-// WRITE = false stores counts[qi]; true emits at [offsets[qi],
-// offsets[qi + 1]) (offsets has nq + 1 entries).  With a capacity (>= 0), a
-// query whose results would end past it writes nothing and raises ERR_OUTPUT.
-template <int MODE, bool WRITE>
-__global__ void __launch_bounds__(128) range_kernel(DevTree t, const float* __restrict__ q, int q_stride,
-                                                    const float* __restrict__ radius, int r_stride, long long nq,
-                                                    long long* __restrict__ counts,
-                                                    const long long* __restrict__ offsets, int* __restrict__ ids,
-                                                    float* __restrict__ xyz, long long capacity) {
-    // No early exit: the search body is warp-collective.
-    const long long qi = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = qi < nq;
-    if (!WRITE) {
-        const long long c =
-            search::range_body<MODE, search::RANGE_COUNT>(t, q, q_stride, radius, r_stride, qi, valid, 0, 0, nullptr, nullptr);
-        if (valid) counts[qi] = c;
+// Box (MODE 0) and radius (MODE 1) searches, `per` consecutive queries a warp.
+// Counting: counts[qi], the warp's sum in warp_sum and, with a log, its hits.
+template <int MODE>
+__global__ void __launch_bounds__(search::RANGE_CTA) range_count_kernel(DevTree t, const float* __restrict__ q,
+                                                                        int q_stride, const float* __restrict__ radius,
+                                                                        int r_stride, long long nq, int per,
+                                                                        long long* __restrict__ counts,
+                                                                        long long* __restrict__ warp_sum,
+                                                                        search::RangeLog log, int entries) {
+    extern __shared__ __align__(16) unsigned char range_sm[];
+    const search::RangeWarp w = search::range_warp_carve<false>(range_sm, entries);
+    const int lane = threadIdx.x & 31;
+    const long long wi = ((long long)blockIdx.x * search::RANGE_CTA + threadIdx.x) >> 5;
+    const long long qi = wi * per + lane;
+    const bool valid = lane < per && qi < nq;
+    if (valid) search::range_put_query<MODE>(w, lane, q + qi * q_stride, MODE == 1 ? radius[qi * r_stride] : 0.f);
+    w.cnt[lane] = 0;
+    search::RangeLog wl = log;
+    if (wi * per >= nq) wl.pool = nullptr;  // the grid's last warps: no queries, no chunk
+    search::LogCursor lc(wl, wi);
+    search::range_warp<MODE, false>(t, w, __ballot_sync(0xffffffffu, valid), entries, wl, lc, 0, 0, nullptr, nullptr);
+    lc.close();
+    __syncwarp();
+    const int c = valid ? w.cnt[lane] : 0;
+    if (valid) counts[qi] = c;
+    long long sum = c;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0 && wi * per < nq) warp_sum[wi] = sum;
+}
+
+// The CSR offsets (nq + 1 entries) from the counts and the scanned warp sums.
+// With ids, the logged hits are written from the queries' offsets on (a warp
+// without a log searches again); with a capacity (>= 0), a query whose hits
+// would end past it writes nothing and raises ERR_OUTPUT.
+template <int MODE>
+__global__ void __launch_bounds__(search::RANGE_CTA, 8) range_write_kernel(DevTree t, const float* __restrict__ q,
+                                                                        int q_stride, const float* __restrict__ radius,
+                                                                        int r_stride, long long nq, int per,
+                                                                        const long long* __restrict__ counts,
+                                                                        const long long* __restrict__ warp_off,
+                                                                        long long* __restrict__ offsets,
+                                                                        int* __restrict__ ids, float* __restrict__ xyz,
+                                                                        long long capacity, search::RangeLog log,
+                                                                        int entries) {
+    extern __shared__ __align__(16) unsigned char range_sm[];
+    const int lane = threadIdx.x & 31;
+    const long long wi = ((long long)blockIdx.x * search::RANGE_CTA + threadIdx.x) >> 5;
+    const long long qi = wi * per + lane;
+    const bool valid = lane < per && qi < nq;
+    const long long c = valid ? counts[qi] : 0;
+    long long inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+    }
+    const long long start = (wi * per < nq ? warp_off[wi] : 0) + inc - c;
+    if (valid) {
+        offsets[qi] = start;
+        if (qi == nq - 1) offsets[nq] = start + c;
+    }
+    if (ids == nullptr) return;
+    const search::RangeWarp w = search::range_warp_carve<true>(range_sm, entries);
+    bool go = c > 0;
+    if (go && capacity >= 0 && start + c > capacity) {
+        atomicOr(&t.st->err, ERR_OUTPUT);
+        go = false;
+    }
+    const unsigned todo = __ballot_sync(0xffffffffu, go);
+    if (todo == 0) return;
+    // The log holds every query's hits: it serves unless one is to be left out.
+    const int2* first = log.pool != nullptr ? log.pool + wi * search::LOG_CHUNK : nullptr;
+    const bool all = todo == __ballot_sync(0xffffffffu, c > 0);
+    if (first != nullptr && all && __ldg(&first->x) >= 0) {
+        search::range_replay(t, w, log, first, start, start + c, ids, xyz);
         return;
     }
-    long long o = 0, o_lim = 0;
-    bool go = valid;
-    if (valid) {
-        o = offsets[qi];
-        o_lim = offsets[qi + 1];
-        if (capacity >= 0 && o_lim > capacity) {
-            atomicOr(&t.st->err, ERR_OUTPUT);
-            go = false;
-        }
-    }
-    search::range_body<MODE, search::RANGE_WRITE>(t, q, q_stride, radius, r_stride, qi, go, o, o_lim, ids, xyz);
+    if (go) search::range_put_query<MODE>(w, lane, q + qi * q_stride, MODE == 1 ? radius[qi * r_stride] : 0.f);
+    search::LogCursor lc(search::RangeLog{nullptr, nullptr, 0, 0}, 0);
+    search::range_warp<MODE, true>(t, w, todo, entries, log, lc, start, start + c, ids, xyz);
 }
 
 // k > 64: a thread per query, the list in its output rows.
@@ -259,25 +311,89 @@ cudaError_t noalloc_scratch(int device, void** ptr) {
 
 size_t noalloc_scratch_bytes() { return NOALLOC_SCRATCH_BYTES; }
 
-void launch_range(const DevTree& t, int mode, const float* q, int q_stride, const float* radius, int r_stride,
-                  long long nq, long long* counts, const long long* offsets, int* ids, float* xyz,
-                  long long capacity, cudaStream_t s) {
-    if (nq <= 0) return;
-    unsigned g = blocks_for(nq, 128);
-#define IKDG_RANGE(M, W) \
-    range_kernel<M, W><<<g, 128, 0, s>>>(t, q, q_stride, radius, r_stride, nq, counts, offsets, ids, xyz, capacity)
-    if (mode == 0) {
-        if (ids == nullptr)
-            IKDG_RANGE(0, false);
-        else
-            IKDG_RANGE(0, true);
-    } else {
-        if (ids == nullptr)
-            IKDG_RANGE(1, false);
-        else
-            IKDG_RANGE(1, true);
+namespace {
+
+// Queries per warp: as many as leave about RANGE_WARPS warps, so that small
+// batches spread over the GPU and large ones fill their warps' windows.
+constexpr long long RANGE_WARPS = 4864;  // 32 per SM
+int range_per(long long nq) {
+    int per = 1;
+    while (per < search::RANGE_QUERIES && nq / (2 * per) >= RANGE_WARPS) per *= 2;
+    return per;
+}
+
+}  // namespace
+
+namespace {
+
+// Chunks of the hit log beyond one per warp: four per warp (100k radius
+// searches of 0.5-5 m on a 1M-point map take 2.5), 64 MB at most.
+long long log_extra(long long warps) { return warps * 4 < 65536 ? warps * 4 : 65536; }
+
+struct RangeTemp {
+    long long* counts;
+    long long* sums;
+    long long* offs;
+    void* scan;
+    unsigned* next;
+    int2* pool;
+    size_t bytes;
+    RangeTemp(void* base, long long nq, long long warps, bool log) {
+        char* p = (char*)base;
+        auto take = [&](size_t b) {
+            char* r = p;
+            p += (b + 255) & ~(size_t)255;
+            return (void*)r;
+        };
+        counts = (long long*)take(sizeof(long long) * nq);
+        sums = (long long*)take(sizeof(long long) * warps);
+        offs = (long long*)take(sizeof(long long) * warps);
+        scan = take(scan_temp_bytes(warps));
+        next = (unsigned*)take(sizeof(unsigned));
+        pool = log ? (int2*)take(sizeof(int2) * search::LOG_CHUNK * (warps + log_extra(warps))) : nullptr;
+        bytes = (size_t)(p - (char*)base);
     }
-#undef IKDG_RANGE
+};
+
+long long range_warps(long long nq) { return (nq + range_per(nq) - 1) / range_per(nq); }
+
+}  // namespace
+
+size_t range_temp_bytes(long long nq, int passes) {
+    return RangeTemp(nullptr, nq, range_warps(nq), passes & RANGE_LOG).bytes + 256;
+}
+
+void launch_range(const DevTree& t, int mode, const float* q, int q_stride, const float* radius, int r_stride,
+                  long long nq, void* temp, int passes, long long* offsets, int* ids, float* xyz, long long capacity,
+                  long long* total, cudaStream_t s) {
+    if (nq <= 0) return;
+    const int per = range_per(nq);
+    const long long warps = range_warps(nq);
+    const RangeTemp w((void*)(((uintptr_t)temp + 255) & ~(uintptr_t)255), nq, warps, passes & RANGE_LOG);
+    const search::RangeLog log{w.pool, w.next, warps, warps + log_extra(warps)};
+    const unsigned grid = blocks_for(warps, search::RANGE_CTA / 32);
+    const int entries = search::range_stack_entries(t.height);
+    constexpr int WARPS = search::RANGE_CTA / 32;
+    const size_t sm_count = WARPS * search::range_warp_bytes(entries, false);
+    const size_t sm_write = ids != nullptr ? WARPS * search::range_warp_bytes(entries, true) : 0;
+    if (passes & RANGE_COUNT) {
+        if (log.pool != nullptr) cudaMemsetAsync(w.next, 0, sizeof(unsigned), s);
+        if (mode == 0)
+            range_count_kernel<0><<<grid, search::RANGE_CTA, sm_count, s>>>(t, q, q_stride, radius, r_stride, nq, per,
+                                                                            w.counts, w.sums, log, entries);
+        else
+            range_count_kernel<1><<<grid, search::RANGE_CTA, sm_count, s>>>(t, q, q_stride, radius, r_stride, nq, per,
+                                                                            w.counts, w.sums, log, entries);
+        exclusive_scan(w.sums, w.offs, warps, total, w.scan, s);
+    }
+    if (mode == 0)
+        range_write_kernel<0><<<grid, search::RANGE_CTA, sm_write, s>>>(t, q, q_stride, radius, r_stride, nq, per,
+                                                                        w.counts, w.offs, offsets, ids, xyz, capacity,
+                                                                        log, entries);
+    else
+        range_write_kernel<1><<<grid, search::RANGE_CTA, sm_write, s>>>(t, q, q_stride, radius, r_stride, nq, per,
+                                                                        w.counts, w.offs, offsets, ids, xyz, capacity,
+                                                                        log, entries);
 }
 
 }  // namespace ikdg

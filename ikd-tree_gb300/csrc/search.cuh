@@ -92,13 +92,6 @@ __device__ __forceinline__ float slot_dist(f32x2 qxy, float qz, f32x2 xy, float 
     return __fadd_rn(__fadd_rn(sx, sy), __fmul_rn(dz, dz));
 }
 
-// Leaves a warp scans per step of the range search's leaf phase.
-#ifndef IKDG_RANGE_LEAF_BATCH
-#define IKDG_RANGE_LEAF_BATCH 4
-#endif
-constexpr int RANGE_LEAF_BATCH = IKDG_RANGE_LEAF_BATCH;
-
-
 // ---- kNN, k <= 64: a group of four lanes per query over the wide records --------------
 //
 // A group's step is a node step (one 256-byte wide record, two children a lane)
@@ -117,7 +110,8 @@ constexpr int RANGE_LEAF_BATCH = IKDG_RANGE_LEAF_BATCH;
 // 15 % and 6 % more).
 //
 // 1M-point map, k = 5, kernel time before (a thread per query over the binary
-// records) / now: 1 query 23.6 / 10 us, 15k 90 / 32 us, 100k 144 / 98 us (96 / 73 us
+// records) / now: 1 query 23.6 / 13.7 us, 15k of a LiDAR scan 51 / 24 us, 100k
+// 144 / 96 us (96 / 73 us
 // a call when calls on three trees overlap); 20M points, 1M queries, k = 16:
 // 1615 / 1067 us a call.
 // Bound by instruction issue (the tree is served from L2 and the chain of a
@@ -484,180 +478,417 @@ __device__ __forceinline__ void knn_rows_body(const DevTree& t, bool valid, long
     if (o.cnt != nullptr) o.cnt[qi] = cnt;
 }
 
-constexpr int RANGE_COUNT = 0, RANGE_WRITE = 1;
+// ---- box / radius search: a warp for up to 32 queries -------------------------------
+//
+// The warp keeps one ordered stack of (subtree or leaf, query) items for all its
+// queries: query 0's root on top, below it query 1's and so on, and every
+// item's children take its place left to right.  Each step looks at the top
+// RANGE_WINDOW items.  If they start with enough leaves, those are scanned, four
+// lanes per leaf and four slots a lane; otherwise every record among them is
+// expanded in place, four lanes per record and two children a lane.  So every
+// step has work for all lanes however uneven the queries are (radii that differ
+// by ten find numbers of points that differ by a thousand; in a simulated
+// schedule 6.7-7.4 of a step's 8 items are used), and the leaves of a query still
+// come in tree order, which is the order of its hits.
+// A thread per query (the form before) kept a warp for as long as its largest
+// query: 1M-point map, 100k queries, before / now, count and write kernels: box
+// 197 + 227 us / 72 + 48 us, radius 650 + 861 us / 178 + 172 us.  Bound by
+// instruction issue.
+constexpr int RANGE_QUERIES = 32;  // queries per warp, at most
+constexpr int RANGE_WINDOW = 8;    // items per step
+constexpr int RANGE_FEW = 4;       // leading leaves that are worth a step of their own
+constexpr int RANGE_WIDE = 96;     // stack height above which one record is expanded at a time
+constexpr int RANGE_STAGE = 2 * KNN_LEAF_STEP * RANGE_WINDOW;  // hits staged at once
+constexpr int RANGE_CTA = 128;
 
-// MODE 0: box, MODE 1: radius.  OUT = RANGE_COUNT counts, RANGE_WRITE emits at
-// the query's CSR offset.
-// Box (MODE 0) / radius (MODE 1) search of query qi by this thread, with the
-// leaves scanned by the whole warp.  Every lane of the warp calls this
-// together; lanes without a query pass valid = false.  "While-while": in the
-// node phase each thread walks its own query's nodes (a fully covered subtree
-// adds its valid count from ncnt when counting, and is enumerated when
-// writing) until it holds a leaf; in the leaf phase the warp takes the held
-// leaves one at a time, one lane per slot (one 512-byte load per leaf), tests
-// the slots against the holder's query and counts them with a ballot.  So a
-// query with thousands of hits costs one warp step per leaf instead of one
-// thread step per slot, while light queries keep one thread each.
-// Returns this lane's hit count.  WRITE emits the hits at ids[o..],
-// xyz[3 o..] in traversal order, never at or past o_lim (a hit there raises
-// ERR_OUTPUT instead).  radius: one float per query, r_stride floats apart.
-template <int MODE, int OUT>
-__device__ __forceinline__ long long range_body(const DevTree& t, const float* __restrict__ q, int q_stride,
-                                                const float* __restrict__ radius, int r_stride, long long qi,
-                                                bool valid, long long o, long long o_lim, int* __restrict__ ids,
-                                                float* __restrict__ xyz) {
-    constexpr bool WRITE = OUT != RANGE_COUNT;
+// Stack entries of a warp for a tree of this height: RANGE_WIDE, one step's
+// growth, then seven per record on a path (expanded one at a time).
+__host__ __device__ constexpr int range_stack_entries(int height) {
+    return RANGE_WIDE + 7 * RANGE_WINDOW + 7 * (1 + (height + 2) / 3) + 1;
+}
+
+// A warp's shared memory (16-byte aligned parts).
+struct RangeWarp {
+    float4* q;      // [2 * RANGE_QUERIES] box {lo, hi x}, {hi y, hi z}; radius {centre, r^2}
+    float* stage;   // [4 * RANGE_STAGE] hits about to be written
+    int* cnt;       // [RANGE_QUERIES] hits (counting)
+    int2* stack;
+};
+__host__ __device__ constexpr size_t range_warp_bytes(int entries, bool write) {
+    return 2 * RANGE_QUERIES * sizeof(float4) +
+           (write ? RANGE_STAGE * sizeof(float4) : RANGE_QUERIES * sizeof(int)) +
+           ((size_t)entries * sizeof(int2) + 15) / 16 * 16;
+}
+template <bool WRITE>
+__device__ __forceinline__ RangeWarp range_warp_carve(unsigned char* base, int entries) {
+    unsigned char* p = base + (threadIdx.x >> 5) * range_warp_bytes(entries, WRITE);
+    RangeWarp w{};
+    w.q = reinterpret_cast<float4*>(p);
+    p += 2 * RANGE_QUERIES * sizeof(float4);
+    if (WRITE) {
+        w.stage = reinterpret_cast<float*>(p);
+        p += RANGE_STAGE * sizeof(float4);
+    } else {
+        w.cnt = reinterpret_cast<int*>(p);
+        p += RANGE_QUERIES * sizeof(int);
+    }
+    w.stack = reinterpret_cast<int2*>(p);
+    return w;
+}
+
+// Puts this lane's query (lane = its place among the warp's) into shared memory.
+template <int MODE>
+__device__ __forceinline__ void range_put_query(const RangeWarp& w, int lane, const float* q, float radius) {
+    if (MODE == 0) {
+        w.q[2 * lane] = make_float4(q[0], q[1], q[2], q[3]);
+        w.q[2 * lane + 1] = make_float4(q[4], q[5], 0.f, 0.f);
+    } else {
+        w.q[2 * lane] = make_float4(q[0], q[1], q[2], __fmul_rn(radius, radius));
+    }
+}
+
+// Stages a lane's hits (bits of m, slots in u and v) at places `at`, ..: points as
+// words 3 at .., ids after all points.
+__device__ __forceinline__ void range_stage(const RangeWarp& w, unsigned m, int at, const Quad2& u, const Quad2& v) {
+    float* pt = w.stage;
+    float* id = w.stage + 3 * RANGE_STAGE;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (m >> i & 1) {
+            const Quad2& s = i < 2 ? u : v;
+            float x, y, z, wd;
+            unpack2(s.v[2 * (i & 1)], x, y);
+            unpack2(s.v[2 * (i & 1) + 1], z, wd);
+            pt[3 * at] = x;
+            pt[3 * at + 1] = y;
+            pt[3 * at + 2] = z;
+            id[at] = wd;
+            ++at;
+        }
+    }
+}
+
+// The staged hits from place s0 on leave as runs of consecutive words, one per
+// query.  Groups (four lanes) with act hold one item each of query qi, their
+// first hit at place `first`; `hits` ends the last.  Lane q holds query q's pos
+// and lim.
+__device__ __forceinline__ void range_emit(const DevTree& t, const RangeWarp& w, int s0, bool act, int qi, int first,
+                                           int hits, long long& pos, long long lim, int* __restrict__ ids,
+                                           float* __restrict__ xyz) {
+    constexpr unsigned ALL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    // The query in six floats: box {lo, hi}, or radius {centre, r^2, -, -}.
-    float qa[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (valid) {
-        if (MODE == 0) {
-            for (int a = 0; a < 6; ++a) qa[a] = q[qi * q_stride + a];
-        } else {
-            for (int a = 0; a < 3; ++a) qa[a] = q[qi * q_stride + a];
-            const float r = radius[qi * r_stride];
-            qa[3] = __fmul_rn(r, r);
+    const int prev = __shfl_up_sync(ALL, qi, 4);
+    unsigned runs = __ballot_sync(ALL, act && (lane & 3) == 0 && (lane == 0 || prev != qi));
+    while (runs) {
+        const int l = __ffs(runs) - 1;
+        runs &= runs - 1;
+        const int s = __shfl_sync(ALL, first, l);
+        const int c = (runs ? __shfl_sync(ALL, first, __ffs(runs) - 1) : hits) - s;
+        if (c == 0) continue;
+        const int q = __shfl_sync(ALL, qi, l);
+        const long long o = __shfl_sync(ALL, pos, q);
+        if (__any_sync(ALL, lane == q && pos + c > lim)) {
+            if (lane == 0) atomicOr(&t.st->err, ERR_OUTPUT);
+            continue;
+        }
+        if (lane == q) pos += c;
+        const float* pt = w.stage + 3 * (s0 + s);
+        const float* id = w.stage + 3 * RANGE_STAGE + s0 + s;
+        int* io = ids + o;
+        for (int e = lane; e < c; e += 32) io[e] = (int)(__float_as_uint(id[e]) & ID_MASK);
+        if (xyz != nullptr) {
+            float* xo = xyz + 3 * o;
+            for (int e = lane; e < 3 * c; e += 32) xo[e] = pt[e];
         }
     }
-    long long count = 0;
-    int stack[MAX_STACK];
-    int sp = 0;
-    int cur = 0;  // item = code * 2 + covered; code 0 is the sentinel record
-    bool done = !valid;
-    int visits = 0;
-    const float4* __restrict__ P = t.pts;
-    auto pop = [&]() {
-        if (sp > 0)
-            cur = stack[--sp];
-        else
-            done = true;
-    };
+}
 
-    while (true) {
-        // Node phase.
-        while (true) {
-            const bool nodework = !done && (cur >> 1) >= 0;
-            if (!__any_sync(0xffffffffu, nodework)) break;
-            if (!nodework) continue;
-            if (++visits > MAX_VISITS) {
-                atomicOr(&t.st->err, ERR_LOOP);
-                done = true;
-                continue;
-            }
-            const int X = cur >> 1;
-            const bool covered = cur & 1;
-            const NodeRec r = load_node(t.node, X);
-            const int4 c4 = WRITE ? make_int4(0, 0, 0, 0) : __ldg(t.ncnt + X);
-            int next = 0;
-            bool have_next = false;
-#pragma unroll
-            for (int side = 0; side < 2; ++side) {
-                const int c = side == 0 ? r.left() : r.right();
-                if (c == 0) continue;
-                const Box3 b = r.box(side);
-                if (box_empty(b)) continue;
-                bool cov = covered;
-                if (!cov) {
-                    if (MODE == 0) {
-                        Box3 qb;
-                        for (int a = 0; a < 3; ++a) {
-                            qb.lo[a] = qa[a];
-                            qb.hi[a] = qa[3 + a];
-                        }
-                        if (qbox_disjoint(qb, b)) continue;
-                        cov = qbox_covers(qb, b);
-                    } else {
-                        if (box_dist(qa[0], qa[1], qa[2], b.lo[0], b.lo[1], b.lo[2], b.hi[0], b.hi[1], b.hi[2]) >
-                            qa[3])
-                            continue;
-                        cov = box_far(qa[0], qa[1], qa[2], b.lo[0], b.lo[1], b.lo[2], b.hi[0], b.hi[1], b.hi[2]) <=
-                              qa[3];
-                    }
-                }
-                if (cov && !WRITE) {
-                    count += side == 0 ? (c4.x - c4.y) : (c4.z - c4.w);
-                    continue;
-                }
-                const int it = c * 2 + (cov ? 1 : 0);
-                if (!have_next) {
-                    next = it;
-                    have_next = true;
-                } else if (sp < MAX_STACK) {
-                    stack[sp++] = it;
-                } else {
-                    atomicOr(&t.st->err, ERR_STACK);
-                }
-            }
-            if (have_next)
-                cur = next;
-            else
-                pop();
-        }
-        // Leaf phase: the held leaves, RANGE_LEAF_BATCH at a time, one lane per
-        // slot.  A bucket always has LEAF_CAP slots in the pool, so each slot
-        // load is issued together with the leaf's fill count.
-        const bool leafwork = !done && (cur >> 1) < 0;
-        unsigned lb = __ballot_sync(0xffffffffu, leafwork);
-        if (lb == 0) break;
-        while (lb) {
-            int src[RANGE_LEAF_BATCH];
-#pragma unroll
-            for (int u = 0; u < RANGE_LEAF_BATCH; ++u) {
-                src[u] = lb ? __ffs(lb) - 1 : -1;
-                lb &= lb - 1;
-            }
-            float4 p[RANGE_LEAF_BATCH];
-            int nl[RANGE_LEAF_BATCH], it[RANGE_LEAF_BATCH];
-#pragma unroll
-            for (int u = 0; u < RANGE_LEAF_BATCH; ++u) {
-                if (src[u] < 0) break;
-                it[u] = __shfl_sync(0xffffffffu, cur, src[u]);
-                const int L = code_leaf(it[u] >> 1);
-                p[u] = __ldg(P + (long long)L * LEAF_CAP + lane);
-                nl[u] = __ldg(t.leaf_n + L);
-            }
-#pragma unroll
-            for (int u = 0; u < RANGE_LEAF_BATCH; ++u) {
-                if (src[u] < 0) break;
-                float h[6];
-#pragma unroll
-                for (int a = 0; a < 6; ++a) h[a] = __shfl_sync(0xffffffffu, qa[a], src[u]);
-                bool hit = false;
-                if (lane < nl[u] && !(__float_as_uint(p[u].w) & F_DEL)) {
-                    if (it[u] & 1) {
-                        hit = true;
-                    } else if (MODE == 0) {
-                        hit = p[u].x >= h[0] && p[u].x < h[3] && p[u].y >= h[1] && p[u].y < h[4] &&
-                              p[u].z >= h[2] && p[u].z < h[5];
-                    } else {
-                        hit = sq_dist(p[u].x, p[u].y, p[u].z, h[0], h[1], h[2]) <= h[3];
-                    }
-                }
-                const unsigned hb = __ballot_sync(0xffffffffu, hit);
-                if (OUT == RANGE_WRITE) {
-                    const long long base = __shfl_sync(0xffffffffu, o + count, src[u]);
-                    const long long lim = __shfl_sync(0xffffffffu, o_lim, src[u]);
-                    if (hit) {
-                        const long long pos = base + __popc(hb & lt);
-                        if (pos < lim) {
-                            ids[pos] = (int)(__float_as_uint(p[u].w) & ID_MASK);
-                            if (xyz != nullptr) {
-                                xyz[pos * 3 + 0] = p[u].x;
-                                xyz[pos * 3 + 1] = p[u].y;
-                                xyz[pos * 3 + 2] = p[u].z;
-                            }
-                        } else {
-                            atomicOr(&t.st->err, ERR_OUTPUT);
-                        }
-                    }
-                }
-                if (lane == src[u]) count += __popc(hb);
-            }
-        }
-        if (leafwork) pop();
+// The hits a counting warp finds, so that the write pass need not search again:
+// one entry {leaf * 2 + half, slot mask | query << 16} per bucket half with
+// hits, in the order they are to be written, in chunks of LOG_CHUNK entries.  A
+// chunk's entry 0 is {entries used, next chunk or -1}.  Warp i starts in chunk
+// i; further chunks come from a counter.  A warp that finds none left, or that
+// meets a covered subtree of more than LOG_COVERED points (counted as a whole),
+// stores -1 used entries in its first chunk and is searched again.
+constexpr int LOG_CHUNK = 128;
+constexpr int LOG_COVERED = 1024;
+
+struct RangeLog {
+    int2* pool;              // nullptr: no log
+    unsigned* next;          // chunks taken beyond the warps' first ones
+    long long warps, chunks; // first chunks, all chunks
+};
+
+struct LogCursor {
+    int2* first;
+    int2* chunk;
+    int used;
+    bool on;
+    __device__ __forceinline__ LogCursor(const RangeLog& log, long long warp) {
+        on = log.pool != nullptr;
+        first = chunk = on ? log.pool + warp * LOG_CHUNK : nullptr;
+        used = 1;
     }
-    return count;
+    // Room for n more entries in this chunk, or in a new one (whole warp).
+    __device__ __forceinline__ void reserve(const RangeLog& log, int n) {
+        if (used + n <= LOG_CHUNK) return;
+        long long c = 0;
+        if ((threadIdx.x & 31) == 0) {
+            c = log.warps + (long long)atomicAdd(log.next, 1u);
+            if (c < log.chunks) chunk[0] = make_int2(used - 1, (int)c);
+        }
+        c = __shfl_sync(0xffffffffu, c, 0);
+        if (c >= log.chunks) {
+            on = false;
+            return;
+        }
+        chunk = log.pool + c * LOG_CHUNK;
+        used = 1;
+    }
+    __device__ __forceinline__ void close() {
+        if (first == nullptr || (threadIdx.x & 31) != 0) return;
+        if (on)
+            chunk[0] = make_int2(used - 1, -1);
+        else
+            first[0] = make_int2(-1, -1);
+    }
+};
+
+// MODE 0: box, 1: radius.  Searches the queries whose bits are set in `todo`
+// (their data in w.q) with the whole warp.  WRITE: the hits of query `lane` go
+// to ids / xyz (nullable) from `pos` on, never past `lim` (hits there raise
+// ERR_OUTPUT); otherwise they are counted in w.cnt, and logged.
+template <int MODE, bool WRITE>
+__device__ __forceinline__ void range_warp(const DevTree& t, const RangeWarp& w, unsigned todo, int entries,
+                                           const RangeLog& log, LogCursor& lc, long long pos, long long lim,
+                                           int* __restrict__ ids, float* __restrict__ xyz) {
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, j = lane >> 2, sub = lane & 3;
+    const unsigned below = (1u << lane) - 1u;
+    int sp = __popc(todo);
+    // item: {node (>= 0: its record) or leaf code, query}; the first query on top
+    if ((todo >> lane) & 1) w.stack[sp - 1 - __popc(todo & below)] = make_int2(t.start, lane);
+    __syncwarp();
+    int steps = 0;
+    while (sp > 0) {
+        if (++steps > MAX_VISITS) {
+            if (lane == 0) atomicOr(&t.st->err, ERR_LOOP);
+            break;
+        }
+        const int avail = min(sp, RANGE_WINDOW);
+        // this lane's item, and with it the window: item j in lanes 4 j ..
+        const int2 it = j < avail ? w.stack[sp - 1 - j] : make_int2(0, 0);
+        const unsigned leafm = __ballot_sync(ALL, it.x < 0);
+        int lead = (__ffs(~leafm) - 1) >> 2;  // leading leaves
+        if (leafm == ALL) lead = RANGE_WINDOW;
+        const float4 qa = w.q[2 * it.y];
+        const float4 qb = MODE == 0 ? w.q[2 * it.y + 1] : make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncwarp();  // items read before any is replaced
+        if (lead == avail || lead >= RANGE_FEW) {
+            const int L = code_leaf(it.x);
+            const f32x2 qxy = pack2(qa.x, qa.y);
+            // Hits among this lane's four slots of bucket half h, as a mask.
+            Quad2 a, b;
+            auto scan = [&](int h, int n) {
+                unsigned m = 0;
+                const float4* p = t.pts + (long long)L * LEAF_CAP + 16 * h + 4 * sub;
+                a = ld_quad2(p);
+                b = ld_quad2(p + 2);
+                const int j0 = 16 * h + 4 * sub;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const f32x2 xy = i < 2 ? a.v[2 * (i & 1)] : b.v[2 * (i & 1)];
+                    const f32x2 zw = i < 2 ? a.v[2 * (i & 1) + 1] : b.v[2 * (i & 1) + 1];
+                    float z, id;
+                    unpack2(zw, z, id);
+                    bool in = j0 + i < n && !(__float_as_uint(id) & F_DEL);
+                    if (MODE == 0) {
+                        float x, y;
+                        unpack2(xy, x, y);
+                        in = in && x >= qa.x && x < qa.w && y >= qa.y && y < qb.x && z >= qa.z && z < qb.y;
+                    } else {
+                        in = in && slot_dist(qxy, qa.z, xy, z) <= qa.w;
+                    }
+                    m |= in ? 1u << i : 0u;
+                }
+                return m;
+            };
+            int n = 0;
+            unsigned m0 = 0, m1 = 0;
+            if (j < lead) {
+                n = min(__ldg(t.leaf_n + L), LEAF_CAP);
+                m0 = scan(0, n);
+            }
+            // Buckets with more than 16 slots: half the window, both halves.
+            const bool over = __any_sync(ALL, n > KNN_LEAF_STEP);
+            Quad2 a0 = a, b0 = b;
+            if (over) {
+                lead = min(lead, RANGE_WINDOW / 2);
+                if (j >= lead) m0 = 0;
+                if (j < lead && n > KNN_LEAF_STEP) m1 = scan(1, n);
+            }
+            if (!WRITE) {
+                // the halves' slot masks, in every lane of the group
+                unsigned v = (m0 | (m1 << 16)) << (4 * sub);
+                v |= __shfl_xor_sync(ALL, v, 1);
+                v |= __shfl_xor_sync(ALL, v, 2);
+                const bool h0 = sub == 0 && (v & 0xffffu) != 0, h1 = sub == 0 && (v >> 16) != 0;
+                if (h0 || h1) atomicAdd(&w.cnt[it.y], __popc(v));
+                if (lc.on) {
+                    const unsigned e0 = __ballot_sync(ALL, h0), e1 = over ? __ballot_sync(ALL, h1) : 0u;
+                    lc.reserve(log, __popc(e0) + __popc(e1));
+                    if (lc.on) {
+                        int2* at = lc.chunk + lc.used + __popc(e0 & below) + __popc(e1 & below);
+                        if (h0) *at++ = make_int2(L * 2, (int)(v & 0xffffu) | (it.y << 16));
+                        if (h1) *at = make_int2(L * 2 + 1, (int)(v >> 16) | (it.y << 16));
+                        lc.used += __popc(e0) + __popc(e1);
+                    }
+                }
+            } else {
+                // rank of this lane's hits: leaf by leaf, first halves before second
+                const int c0 = __popc(m0), c1 = __popc(m1);
+                int x = c0 | (c1 << 16);
+                int y = __shfl_up_sync(ALL, x, 1, 4);
+                if (sub >= 1) x += y;
+                y = __shfl_up_sync(ALL, x, 2, 4);
+                if (sub >= 2) x += y;
+                const int tt = __shfl_sync(ALL, x, 3, 4);
+                const int leaf_hits = (tt & 0xffff) + (tt >> 16);
+                int z = leaf_hits;
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(ALL, z, o);
+                    if (lane >= o) z += v;
+                }
+                const int first = z - leaf_hits, hits = __shfl_sync(ALL, z, 31);
+                range_stage(w, m0, first + (x & 0xffff) - c0, a0, b0);
+                if (over) range_stage(w, m1, first + (tt & 0xffff) + (x >> 16) - c1, a, b);
+                __syncwarp();
+                range_emit(t, w, 0, j < lead, it.y, first, hits, pos, lim, ids, xyz);
+            }
+            sp -= lead;
+        } else {
+            const bool here = j < avail;
+            const bool rec = here && it.x >= 0 && (sp <= RANGE_WIDE || j == lead);
+            bool al0 = here && !rec && sub == 0, al1 = false, whole = false;
+            bool cov0 = false, cov1 = false;
+            int k0 = it.x, k1 = 0;
+            if (rec) {
+                const char* p = reinterpret_cast<const char*>(t.wide + (long long)it.x * 16) + 64 * sub;
+                const Quad2 u = ld_quad2(p), v = ld_quad2(p + 32);
+                float lx0, lx1, ly0, ly1, lz0, lz1, hx0, hx1, hy0, hy1, hz0, hz1, f0, f1, v0, v1;
+                unpack2(u.v[0], lx0, lx1);
+                unpack2(u.v[1], ly0, ly1);
+                unpack2(u.v[2], lz0, lz1);
+                unpack2(u.v[3], hx0, hx1);
+                unpack2(v.v[0], hy0, hy1);
+                unpack2(v.v[1], hz0, hz1);
+                unpack2(v.v[2], f0, f1);
+                k0 = __float_as_int(f0);
+                k1 = __float_as_int(f1);
+                if (MODE == 0) {
+                    // half-open, as qbox_disjoint
+                    al0 = lx0 <= hx0 && qa.w > lx0 && qa.x <= hx0 && qb.x > ly0 && qa.y <= hy0 && qb.y > lz0 && qa.z <= hz0;
+                    al1 = lx1 <= hx1 && qa.w > lx1 && qa.x <= hx1 && qb.x > ly1 && qa.y <= hy1 && qb.y > lz1 && qa.z <= hz1;
+                } else {
+                    float d0, d1;
+                    box_dist2(u.v[0], u.v[1], u.v[2], u.v[3], v.v[0], v.v[1], pack2(qa.x, qa.x), pack2(qa.y, qa.y),
+                              pack2(qa.z, qa.z), d0, d1);
+                    al0 = lx0 <= hx0 && d0 <= qa.w;
+                    al1 = lx1 <= hx1 && d1 <= qa.w;
+                }
+                unpack2(v.v[3], v0, v1);
+                // Covered subtrees count as a whole, except small ones whose
+                // leaves are to be logged.  (Leaves are scanned: the test costs
+                // as much.)
+                const int big = lc.on ? LOG_COVERED : 0;
+                const bool try0 = !WRITE && al0 && k0 > 0 && __float_as_int(v0) > big;
+                const bool try1 = !WRITE && al1 && k1 > 0 && __float_as_int(v1) > big;
+                if (try0 || try1) {
+                    if (MODE == 0) {
+                        cov0 = qa.x <= lx0 && qa.w > hx0 && qa.y <= ly0 && qb.x > hy0 && qa.z <= lz0 && qb.y > hz0;
+                        cov1 = qa.x <= lx1 && qa.w > hx1 && qa.y <= ly1 && qb.x > hy1 && qa.z <= lz1 && qb.y > hz1;
+                    } else {
+                        cov0 = box_far(qa.x, qa.y, qa.z, lx0, ly0, lz0, hx0, hy0, hz0) <= qa.w;
+                        cov1 = box_far(qa.x, qa.y, qa.z, lx1, ly1, lz1, hx1, hy1, hz1) <= qa.w;
+                    }
+                    cov0 = cov0 && try0;
+                    cov1 = cov1 && try1;
+                    if (cov0 || cov1) {
+                        whole = true;
+                        atomicAdd(&w.cnt[it.y], (cov0 ? __float_as_int(v0) : 0) + (cov1 ? __float_as_int(v1) : 0));
+                        al0 = al0 && !cov0;
+                        al1 = al1 && !cov1;
+                    }
+                }
+            }
+            if (!WRITE && lc.on && __any_sync(ALL, whole)) lc.on = false;
+            // The window's items are replaced in place, first on top.
+            const unsigned b0 = __ballot_sync(ALL, al0), b1 = __ballot_sync(ALL, al1);
+            const int end = sp - avail + __popc(b0) + __popc(b1);  // new height
+            const int at = end - 1 - (__popc(b0 & below) + __popc(b1 & below));
+            if (end > entries) {  // cannot happen: see range_stack_entries
+                if (lane == 0) atomicOr(&t.st->err, ERR_STACK);
+                break;
+            }
+            if (al0) w.stack[at] = make_int2(k0, it.y);
+            if (al1) w.stack[at - (al0 ? 1 : 0)] = make_int2(k1, it.y);
+            sp = end;
+        }
+        __syncwarp();
+    }
+}
+
+// Writes the hits that a counting warp logged in the chunks from `c` on: 16
+// entries a round, four lanes per entry, two entries a lane.
+__device__ __forceinline__ void range_replay(const DevTree& t, const RangeWarp& w, const RangeLog& log, const int2* c,
+                                             long long pos, long long lim, int* __restrict__ ids,
+                                             float* __restrict__ xyz) {
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, j = lane >> 2, sub = lane & 3;
+    while (true) {
+        const int2 head = __ldg(c);
+        for (int e0 = 0; e0 < head.x; e0 += 2 * RANGE_WINDOW) {
+            int2 e[2];
+            Quad2 a[2], b[2];
+            unsigned m[2];
+            bool act[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = e0 + RANGE_WINDOW * h + j;
+                act[h] = i < head.x;
+                e[h] = act[h] ? __ldg(c + 1 + i) : make_int2(0, 0);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                m[h] = ((unsigned)e[h].y >> (4 * sub)) & 15u;
+                if (!act[h]) m[h] = 0;
+                if (m[h]) {
+                    const float4* p = t.pts + (long long)(e[h].x >> 1) * LEAF_CAP + 16 * (e[h].x & 1) + 4 * sub;
+                    a[h] = ld_quad2(p);
+                    b[h] = ld_quad2(p + 2);
+                }
+            }
+            // ranks of both halves of the round in one scan
+            const int n0 = __popc(m[0]), n1 = __popc(m[1]);
+            int x = n0 | (n1 << 16);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(ALL, x, o);
+                if (lane >= o) x += v;
+            }
+            const int tot = __shfl_sync(ALL, x, 31);
+            const int f0 = (x & 0xffff) - n0, f1 = (x >> 16) - n1, t0 = tot & 0xffff;
+            range_stage(w, m[0], f0, a[0], b[0]);
+            range_stage(w, m[1], t0 + f1, a[1], b[1]);
+            __syncwarp();
+            range_emit(t, w, 0, act[0], (e[0].y >> 16) & 31, f0, t0, pos, lim, ids, xyz);
+            if (tot >> 16) range_emit(t, w, t0, act[1], (e[1].y >> 16) & 31, f1, tot >> 16, pos, lim, ids, xyz);
+            __syncwarp();
+        }
+        if (head.y < 0) break;
+        c = log.pool + (long long)head.y * LOG_CHUNK;
+    }
 }
 
 }  // namespace search
