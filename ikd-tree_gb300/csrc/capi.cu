@@ -268,6 +268,9 @@ struct Tree {
         small.release();
         if (st_dev != nullptr) cudaFree(st_dev);
         if (st != nullptr) cudaFreeHost(st);
+        if (reg_part != nullptr) cudaFreeHost(reg_part);
+        reg_part = nullptr;
+        reg_cap = 0;
         st_dev = nullptr;
         st = nullptr;
         if (own_stream && stream != nullptr) cudaStreamDestroy(stream);
@@ -992,15 +995,26 @@ struct Tree {
     }
 
     // ---- point-to-plane registration (no counterpart in the reference) -----------
-    void upload_pose(const double pose[6], double* Rt_dev) {
-        double R[9];
-        so3_exp(pose, R);
-        double h[12];
-        for (int i = 0; i < 9; ++i) h[i] = R[i];
-        for (int i = 0; i < 3; ++i) h[9 + i] = pose[3 + i];
-        CK(cudaMemcpyAsync(Rt_dev, h, sizeof(h), cudaMemcpyHostToDevice, stream));
-        CK(cudaStreamSynchronize(stream));  // h lives on this stack frame
+    static RegPose reg_pose(const double pose[6]) {
+        RegPose p;
+        so3_exp(pose, p.R);
+        for (int i = 0; i < 3; ++i) p.t[i] = pose[3 + i];
+        return p;
     }
+    // Pinned host room for the block sums of a registration step: the kernels
+    // write them there, one wait brings them.
+    double* reg_sums(size_t count) {
+        if (count > reg_cap) {
+            if (reg_part != nullptr) CK(cudaFreeHost(reg_part));
+            reg_part = nullptr;
+            reg_cap = 0;
+            CK(cudaMallocHost(&reg_part, sizeof(double) * count));
+            reg_cap = count;
+        }
+        return reg_part;
+    }
+    double* reg_part = nullptr;
+    size_t reg_cap = 0;
 
     void p2p_forward(const float* scan, long long n, const double* pose, int k, double max_dist, float thresh,
                      float* planes, float* res, int* valid, double* loss) {
@@ -1009,31 +1023,29 @@ struct Tree {
             throw BadArg{"p2p_forward: bad arguments"};
         if (loss) *loss = 0;
         if (n == 0) return;
-        reset_counters();
+        // the search reports through the error bits alone
+        zero_fields(offsetof(DevStatus, err), sizeof(int));
         const int nb = reg_blocks(n);
-        op.ensure(align_up(sizeof(double) * 12) + align_up(sizeof(float) * 3 * n) + align_up(sizeof(int) * n * k) +
+        op.ensure(align_up(sizeof(float) * 3 * n) + align_up(sizeof(int) * n * k) +
                       align_up(sizeof(float) * n * k) + align_up(sizeof(float) * 3 * n * k) + align_up(sizeof(int) * n) +
-                      align_up(sizeof(double) * nb) + align_up(knn_temp_bytes(n, k)),
+                      align_up(knn_temp_bytes(n, k)),
                   stream);
         Carver c(op.p);
-        double* Rt = c.take<double>(12);
         float* w = c.take<float>(3 * n);
         int* ids = c.take<int>((size_t)n * k);
         float* d2 = c.take<float>((size_t)n * k);
         float* nbr = c.take<float>((size_t)3 * n * k);
         int* cnt = c.take<int>(n);
-        double* part = c.take<double>(nb);
         char* temp = c.take<char>(knn_temp_bytes(n, k));
-        upload_pose(pose, Rt);
-        launch_transform(scan, n, Rt, w, stream);
+        double* part = reg_sums(nb);
+        const RegPose P = reg_pose(pose);
+        launch_transform(scan, n, P, w, stream);
         launch_knn(dt, w, 3, n, k, max_sq_threshold(max_dist), ids, d2, nbr, cnt, temp, bin_bits_for(n, k),
                    stream);
-        launch_plane_residual(scan, Rt, n, k, nbr, cnt, thresh, (float4*)planes, res, valid, part, stream);
-        std::vector<double> h(nb);
-        CK(cudaMemcpyAsync(h.data(), part, sizeof(double) * nb, cudaMemcpyDeviceToHost, stream));
+        launch_plane_residual(scan, P, n, k, nbr, cnt, thresh, (float4*)planes, res, valid, part, stream);
         read_status();
         double s = 0;
-        for (double v : h) s += v;
+        for (int b = 0; b < nb; ++b) s += part[b];
         if (loss) *loss = s;
     }
 
@@ -1045,14 +1057,10 @@ struct Tree {
         for (int i = 0; i < 6; ++i) grad_pose[i] = 0;
         if (n == 0) return;
         const int nb = reg_blocks(n);
-        op.ensure(align_up(sizeof(double) * 12) + align_up(sizeof(double) * 6 * nb), stream);
-        Carver c(op.p);
-        double* Rt = c.take<double>(12);
-        double* part = c.take<double>((size_t)6 * nb);
-        upload_pose(pose, Rt);
-        launch_adjoint(scan, n, Rt, (const float4*)planes, res, valid, (float)grad_loss, grad_points, part, stream);
-        std::vector<double> h(6 * (size_t)nb);
-        CK(cudaMemcpyAsync(h.data(), part, sizeof(double) * 6 * nb, cudaMemcpyDeviceToHost, stream));
+        const double* h = reg_sums(6 * (size_t)nb);
+        launch_adjoint(scan, n, reg_pose(pose), (const float4*)planes, res, valid, (float)grad_loss, grad_points,
+                       reg_part, stream);
+        CK(cudaGetLastError());
         CK(cudaStreamSynchronize(stream));
         double s[6] = {0, 0, 0, 0, 0, 0};
         for (int b = 0; b < nb; ++b)

@@ -171,14 +171,17 @@ void launch_batch_write(const DevTree* trees, const BatchReq* reqs, const int* r
                         int grid, cudaStream_t s);
 
 // ---- register.cu ---------------------------------------------------------------
-// Rt_dev: 12 doubles, R row-major then t.  planes: 2 float4 per point ({n,d}
-// and a point c on the plane).  partial: per-block double sums (reg_blocks(n)
-// entries of 1 (loss) or 6 (adjoint) doubles).
+// The pose travels as a kernel argument: R row-major, t.  planes: 2 float4 per
+// point ({n,d} and a point c on the plane).  partial: per-block double sums
+// (reg_blocks(n) entries of 1 (loss) or 6 (adjoint) doubles).
+struct RegPose {
+    double R[9], t[3];
+};
 int reg_blocks(long long n);
-void launch_transform(const float* p, long long n, const double* Rt_dev, float* w, cudaStream_t s);
-void launch_plane_residual(const float* p, const double* Rt_dev, long long n, int k, const float* nb, const int* cnt,
+void launch_transform(const float* p, long long n, const RegPose& pose, float* w, cudaStream_t s);
+void launch_plane_residual(const float* p, const RegPose& pose, long long n, int k, const float* nb, const int* cnt,
                            float thresh, float4* planes, float* res, int* valid, double* partial, cudaStream_t s);
-void launch_adjoint(const float* p, long long n, const double* Rt_dev, const float4* planes, const float* res,
+void launch_adjoint(const float* p, long long n, const RegPose& pose, const float4* planes, const float* res,
                     const int* valid, float dl, float* grad_p, double* partial, cudaStream_t s);
 
 // ---- update.cu --------------------------------------------------------------
