@@ -9,19 +9,15 @@
 // All jobs of a call are built together, on one of three paths chosen by the
 // largest job:
 // * small (every job <= LB_SMALL points): one CTA per job builds the whole
-//   subtree in shared memory (local_build_kernel<LB_SMALL, 256>);
+//   subtree in shared memory (local_build_kernel);
 // * medium (jobs <= MID_MAX): one launch per tree level splits every open
 //   segment of every job, one CTA per segment, down to LB_SMALL-point segments
 //   (mid_level_kernel: radix-selected median, stable partition), then the
-//   small local builder finishes them;
-// * large: each of the three coordinates is radix-sorted once; the three sorted
-//   index arrays are then stably partitioned level by level, so every segment
-//   stays a contiguous range in each array and its AABB is read off the ends of
-//   the three ranges.  Per level: one thread per segment allocates its node or
-//   leaf and links it into its parent; one thread per position marks left /
-//   right; a prefix sum and a scatter partition the three arrays.  Segments of
-//   at most LB_MAX points go, with their sorted arrays, to
-//   local_build_kernel<LB_MAX, 1024>.
+//   local builder finishes them;
+// * large: segments above SPLIT_MIN points are split one level at a time by
+//   many CTAs each (split_* kernels: histogram of the keys on the split axis,
+//   the bin that holds the median, selection among that bin's few keys, stable
+//   partition), the rest goes the medium way.
 // All three cut a segment of n points at the point of rank n / 2 on its axis,
 // ties in input order (every partition is stable), so they follow one split
 // rule.
@@ -29,47 +25,14 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
 
 #include "kernels.cuh"
 
 namespace ikdg {
 namespace {
 
-constexpr int LB_MAX = 4096;  // segments this small go to the CTA-local builder
-
-constexpr int KIND_LEAF = 0;
-constexpr int KIND_NODE = 1;
-constexpr int KIND_LOCAL = 2;  // handed to the CTA-local builder
-
 __device__ __forceinline__ float coord4(const float4& p, int a) { return a == 0 ? p.x : (a == 1 ? p.y : p.z); }
-
-__global__ void init_keys_kernel(const float4* __restrict__ pts, long long n, uint32_t* keys, uint32_t* ord) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int b = blockIdx.y;
-    if (i >= n) return;
-    float4 p = pts[i];
-    keys[b * n + i] = float_key(coord4(p, b));
-    ord[b * n + i] = (uint32_t)i;
-}
-
-__global__ void job_of_point_kernel(const int* __restrict__ job_off, int njobs, long long n, int* jp) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int lo = 0, hi = njobs - 1;  // last j with job_off[j] <= i
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (job_off[mid] <= i) lo = mid; else hi = mid - 1;
-    }
-    jp[i] = lo;
-}
-
-__global__ void job_keys_kernel(const int* __restrict__ jp, const uint32_t* __restrict__ ord, long long n,
-                                uint32_t* keys) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int b = blockIdx.y;
-    if (i >= n) return;
-    keys[b * n + i] = (uint32_t)jp[ord[b * n + i]];
-}
 
 __global__ void init_segs_kernel(const int* __restrict__ job_off, const int* __restrict__ job_link, int njobs,
                                  int4* segs, int* nseg) {
@@ -79,170 +42,23 @@ __global__ void init_segs_kernel(const int* __restrict__ job_off, const int* __r
     segs[j] = make_int4(job_off[j], job_off[j + 1], job_link[j], 0);
 }
 
-__global__ void init_segpos_kernel(const uint32_t* __restrict__ job_keys, long long n, int single, int* segpos) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    segpos[i] = single ? 0 : (int)job_keys[i];
-}
-
-// One thread per segment of the current level.
-__global__ void level_seg_kernel(DevTree t, const float4* __restrict__ pts, const uint32_t* __restrict__ ord,
-                                 long long n, const int4* __restrict__ segs, const int* nseg_cur,
-                                 int4* __restrict__ segs_next, int* nseg_next, int4* __restrict__ seginfo,
-                                 int fill, int max_next, int4* __restrict__ local_jobs, int* nlocal) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= *nseg_cur || i >= max_next) return;  // the count runs past the capacity only on overflow (flagged)
-    int4 sg = segs[i];
-    int s = sg.x, e = sg.y, link = sg.z;
-    int cnt = e - s;
-    if (cnt <= LB_MAX) {
-        int r = atomicAdd(nlocal, 1);
-        if (r >= max_next) {
-            atomicOr(&t.st->err, ERR_SEG);
-            seginfo[i] = make_int4(-1, 0, 0, 0);
-            return;
-        }
-        local_jobs[r] = make_int4(s, e, link, 0);
-        seginfo[i] = make_int4(KIND_LOCAL, 0, 0, 0);
-        return;
-    }
-    int parent = link >> 1, side = link & 1;
-    Box3 b = empty_box();
-    if (cnt > 0) {
-        for (int a = 0; a < 3; ++a) {
-            b.lo[a] = coord4(pts[ord[a * n + s]], a);
-            b.hi[a] = coord4(pts[ord[a * n + e - 1]], a);
-        }
-    }
-    if (cnt <= fill) {
-        int L = alloc_leaf(t);
-        if (L < 0) {
-            seginfo[i] = make_int4(-1, 0, 0, 0);
-            return;
-        }
-        t.leaf_n[L] = cnt;
-        t.lparent[L] = link;
-        write_child_box(t.node, parent, side, b);
-        write_child_code(t.node, parent, side, leaf_code(L));
-        write_child_cnt(t.ncnt, parent, side, cnt, 0);
-        wide_link(t, t.winfo[parent], side, leaf_code(L), b, cnt);
-        seginfo[i] = make_int4(KIND_LEAF, L, s, 0);
-        return;
-    }
-    int X = alloc_node(t);
-    if (X < 0) {
-        seginfo[i] = make_int4(-1, 0, 0, 0);
-        return;
-    }
-    float ext[3];
-    for (int a = 0; a < 3; ++a) ext[a] = __fsub_rn(b.hi[a], b.lo[a]);
-    int axis = 0;
-    if (ext[1] > ext[axis]) axis = 1;
-    if (ext[2] > ext[axis]) axis = 2;
-    int mid = s + cnt / 2;
-    float split = coord4(pts[ord[axis * n + mid]], axis);
-    float4* rec = t.node + 4 * X;
-    rec[3] = make_float4(__int_as_float(0), __int_as_float(0), split, __int_as_float(axis));
-    t.nparent[X] = link;
-    int h = 0;
-    for (int m = cnt; m > fill; m -= m / 2) ++h;
-    t.nheight[X] = h;
-    write_child_box(t.node, parent, side, b);
-    write_child_code(t.node, parent, side, X);
-    write_child_cnt(t.ncnt, parent, side, cnt, 0);
-    const int2 wi = t.winfo[parent];
-    wide_link(t, wi, side, X, b, cnt);
-    t.winfo[X] = wide_below(wi, side, X);
-    int r = atomicAdd(nseg_next, 2);
-    if (r + 1 >= max_next) {  // cannot happen with the host's bound; guard anyway
-        atomicOr(&t.st->err, ERR_SEG);
-        seginfo[i] = make_int4(-1, 0, 0, 0);
-        return;
-    }
-    segs_next[r] = make_int4(s, mid, X * 2 + 0, 0);
-    segs_next[r + 1] = make_int4(mid, e, X * 2 + 1, 0);
-    seginfo[i] = make_int4(KIND_NODE, axis, mid, r);
-}
-
-// One thread per position: leaves copy their points; internal segments mark
-// which of their points go left.
-__global__ void level_pos_kernel(DevTree t, const float4* __restrict__ pts, const uint32_t* __restrict__ ord,
-                                 long long n, const int* __restrict__ segpos, const int4* __restrict__ seginfo,
-                                 int* __restrict__ flag) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int sg = segpos[i];
-    if (sg < 0) return;
-    int4 info = seginfo[sg];
-    if (info.x == KIND_LEAF) {
-        float4 p = pts[ord[i]];
-        p.w = __uint_as_float(__float_as_uint(p.w) & ID_MASK);
-        t.pts[(long long)info.y * LEAF_CAP + (i - info.z)] = p;
-    } else if (info.x == KIND_NODE) {
-        uint32_t pt = ord[(long long)info.y * n + i];
-        flag[pt] = i < info.z ? 1 : 0;
-    }
-}
-
-__global__ void level_scanin_kernel(const uint32_t* __restrict__ ord, long long n, const int* __restrict__ segpos,
-                                    const int4* __restrict__ seginfo, const int* __restrict__ flag,
-                                    int* __restrict__ scan_in) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int b = blockIdx.y;
-    if (i >= n) return;
-    int sg = segpos[i];
-    int v = 0;
-    if (sg >= 0 && seginfo[sg].x == KIND_NODE) v = flag[ord[b * n + i]];
-    scan_in[b * n + i] = v;
-}
-
-__global__ void level_scatter_kernel(const uint32_t* __restrict__ ord, uint32_t* __restrict__ ord_next, long long n,
-                                     const int* __restrict__ segpos, int* __restrict__ segpos_next,
-                                     const int4* __restrict__ segs, const int4* __restrict__ seginfo,
-                                     const int* __restrict__ flag, const int* __restrict__ scan_out) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int b = blockIdx.y;
-    if (i >= n) return;
-    int sg = segpos[i];
-    int4 info = sg >= 0 ? seginfo[sg] : make_int4(-1, 0, 0, 0);
-    if (info.x != KIND_NODE) {
-        ord_next[b * n + i] = ord[b * n + i];  // keeps the local builder's three arrays whole
-        if (b == 0) segpos_next[i] = -1;
-        return;
-    }
-    int s = segs[sg].x, mid = info.z;
-    uint32_t pt = ord[b * n + i];
-    int in_left = flag[pt];
-    int base = scan_out[b * n + s];
-    int pl = scan_out[b * n + i] - base;
-    long long np = in_left ? (long long)s + pl : (long long)mid + (i - s - pl);
-    ord_next[b * n + np] = pt;
-    if (b == 0) segpos_next[np] = info.w + (in_left ? 0 : 1);
-}
-
 // ---- CTA-local builder ----------------------------------------------------------
-// One block builds a whole subtree of up to MAXN points in shared memory,
-// with the method of the global levels: three index arrays, each sorted on
-// one coordinate, are stably partitioned level by level, so every open
-// segment is the same position range in all three and its AABB is read off
-// the ends of the ranges.  Per level: one thread per open segment allocates
-// its node or leaf (the split point is the middle of the range on the split
-// axis, which already holds the left half in place); one pass over positions
-// marks each point's side and fills the leaves; a block prefix sum of the
-// left flags of the two other arrays and a scatter partition them.
-//
-// The arrays arrive sorted from the global levels (`idx` != nullptr: the
-// three arrays of the level scatter, stride `stride`); jobs that never went
-// through the global levels (`idx` == nullptr: points pts[x .. y)) are sorted
-// here first: one bitonic network sorts the three arrays of (coordinate key,
-// input position) together.
+// One block builds a whole subtree of up to MAXN points in shared memory:
+// three index arrays, each sorted on one coordinate (one bitonic network sorts
+// the three arrays of (coordinate key, input position) together), are stably
+// partitioned level by level, so every open segment is the same position range
+// in all three and its AABB is read off the ends of the ranges.  Per level: one
+// thread per open segment takes its node or leaf (the split point is the middle
+// of the range on the split axis, which already holds the left half in place);
+// one pass over positions marks each point's side and fills the leaves; a block
+// prefix sum of the left flags of the two other arrays and a scatter partition
+// them.
 //
 // With leaves of at most `fill` >= 8 points an open segment holds >= 9
 // points, so a level has at most 2 * MAXN / 9 < SEGS open segments.
 //
-// Two shapes: 4,096 points on 1,024 threads (about 207 KB of shared memory,
-// one block per SM) and 1,024 points on 256 threads (about 52 KB, four per
-// SM); each thread owns four positions and one open segment at most.
+// Shape: 1,024 points on 256 threads (about 55 KB of shared memory, four blocks
+// per SM); each thread owns four positions and one open segment at most.
 constexpr int LB_SMALL = 1024;
 constexpr uint16_t LB_DONE = 0xffff;
 
@@ -274,37 +90,88 @@ struct LbShared {
     int nseg[2];
     int overflow;
 };
-static_assert(sizeof(LbShared<LB_MAX, 1024>) <= 227 * 1024, "local builder shared memory");
+static_assert(4 * (sizeof(LbShared<LB_SMALL, 256>) + 1024) <= 228 * 1024, "four local builders per SM");
 
 __device__ __forceinline__ float key_float(uint32_t k) {
     uint32_t u = (k & 0x80000000u) ? (k ^ 0x80000000u) : ~k;
     return __uint_as_float(u);
 }
 
-// Ascending bitonic sort of K[a][0 .. size) for the three arrays at once,
-// size a power of two; one compare-exchange per pair, pairs spread over the
-// block.
+// Ascending bitonic sort of K[a][0 .. size) for the three arrays at once, size a
+// power of two of at most 4 * THREADS.  Thread t holds elements 4 t .. 4 t + 3 of
+// each array in registers: partners up to 64 elements apart are in the thread or
+// the warp, only longer strides go through shared memory (6 of the 55 steps for
+// 1,024 elements; every step went through it before, which bound the sort by
+// shared-memory bandwidth).
 template <int MAXN, int THREADS>
 __device__ void lb_bitonic3(unsigned long long (*K)[MAXN], int size) {
-    const int half = size >> 1;
-    for (int kk = 2; kk <= size; kk <<= 1) {
-        for (int j = kk >> 1; j > 0; j >>= 1) {
-            for (int p = threadIdx.x; p < half; p += THREADS) {
-                const int i = ((p & ~(j - 1)) << 1) | (p & (j - 1));
-                const int ixj = i | j;
-                const bool up = (i & kk) == 0;
+    static_assert(MAXN == 4 * THREADS, "four elements per thread");
+    typedef unsigned long long u64;
+    const int e0 = threadIdx.x * 4;
+    u64 v[3][4];
 #pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    const unsigned long long x = K[a][i], y = K[a][ixj];
-                    if ((x > y) == up) {
-                        K[a][i] = y;
-                        K[a][ixj] = x;
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) v[a][r] = e0 + r < size ? K[a][e0 + r] : ~0ull;
+    for (int kk = 2; kk <= size; kk <<= 1) {
+        int j = kk >> 1;
+        if (j >= 128) {
+            for (; j >= 128; j >>= 1) {
+                __syncthreads();
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) K[a][e0 + r] = v[a][r];
+                __syncthreads();
+                const bool keep_min = ((e0 & j) == 0) == ((e0 & kk) == 0);
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const u64 o = K[a][(e0 + r) ^ j];
+                        v[a][r] = (o < v[a][r]) == keep_min ? o : v[a][r];
                     }
-                }
             }
-            __syncthreads();
+        }
+        for (; j >= 4; j >>= 1) {
+            const bool keep_min = ((e0 & j) == 0) == ((e0 & kk) == 0);
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const u64 o = __shfl_xor_sync(0xffffffffu, v[a][r], j >> 2);
+                    v[a][r] = (o < v[a][r]) == keep_min ? o : v[a][r];
+                }
+        }
+        // strides 2 and 1 inside the thread
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            auto cx = [&](int x, int y, bool up) {
+                const u64 p = v[a][x], q = v[a][y];
+                const bool sw = (p > q) == up;
+                v[a][x] = sw ? q : p;
+                v[a][y] = sw ? p : q;
+            };
+            const bool up = (e0 & kk) == 0;
+            if (j == 2) {
+                cx(0, 2, up);
+                cx(1, 3, up);
+            }
+            if (kk == 2) {
+                cx(0, 1, true);
+                cx(2, 3, false);
+            } else {
+                cx(0, 1, up);
+                cx(2, 3, up);
+            }
         }
     }
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) K[a][e0 + r] = v[a][r];
+    __syncthreads();
 }
 
 // Nodes and leaves of the subtree the builders make from n points with leaf
@@ -344,8 +211,6 @@ __device__ __forceinline__ void subtree_counts(int n, int fill, int* nodes, int*
 
 template <int MAXN, int THREADS>
 __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 4) local_build_kernel(DevTree t, const float4* __restrict__ pts,
-                                                                 const uint32_t* __restrict__ idx,
-                                                                 long long stride, int* loc,
                                                                  const int4* __restrict__ jobs, const int* njobs,
                                                                  int max_jobs, int fill) {
     extern __shared__ __align__(16) unsigned char lb_raw[];
@@ -366,38 +231,26 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 4) local_build_
             if (tid == 0) atomicOr(&t.st->err, ERR_SEG);
             continue;
         }
-        if (idx == nullptr) {
-            for (int i = tid; i < n; i += THREADS) sm.P[i] = pts[(long long)jb.x + i];
-            int size = 2;
-            while (size < n) size <<= 1;
-            __syncthreads();
-            for (int i = tid; i < size; i += THREADS) {
-                if (i < n) {
-                    const float4 p = sm.P[i];
-                    sm.u.K[0][i] = ((unsigned long long)float_key(p.x) << 32) | (unsigned)i;
-                    sm.u.K[1][i] = ((unsigned long long)float_key(p.y) << 32) | (unsigned)i;
-                    sm.u.K[2][i] = ((unsigned long long)float_key(p.z) << 32) | (unsigned)i;
-                } else {
-                    sm.u.K[0][i] = sm.u.K[1][i] = sm.u.K[2][i] = ~0ull;
-                }
+        for (int i = tid; i < n; i += THREADS) sm.P[i] = pts[(long long)jb.x + i];
+        int size = 2;
+        while (size < n) size <<= 1;
+        __syncthreads();
+        for (int i = tid; i < size; i += THREADS) {
+            if (i < n) {
+                const float4 p = sm.P[i];
+                sm.u.K[0][i] = ((unsigned long long)float_key(p.x) << 32) | (unsigned)i;
+                sm.u.K[1][i] = ((unsigned long long)float_key(p.y) << 32) | (unsigned)i;
+                sm.u.K[2][i] = ((unsigned long long)float_key(p.z) << 32) | (unsigned)i;
+            } else {
+                sm.u.K[0][i] = sm.u.K[1][i] = sm.u.K[2][i] = ~0ull;
             }
-            __syncthreads();
-            lb_bitonic3<MAXN, THREADS>(sm.u.K, size);
-            for (int i = tid; i < n; i += THREADS) {
-                sm.ord0[0][i] = (uint16_t)sm.u.K[0][i];
-                sm.ord0[1][i] = (uint16_t)sm.u.K[1][i];
-                sm.ord0[2][i] = (uint16_t)sm.u.K[2][i];
-            }
-        } else {
-            for (int i = tid; i < n; i += THREADS) {
-                const uint32_t g = idx[jb.x + i];
-                sm.P[i] = pts[g];
-                sm.ord0[0][i] = (uint16_t)i;
-                loc[g] = i;
-            }
-            __syncthreads();
-            for (int b = 1; b < 3; ++b)
-                for (int i = tid; i < n; i += THREADS) sm.ord0[b][i] = (uint16_t)loc[idx[b * stride + jb.x + i]];
+        }
+        __syncthreads();
+        lb_bitonic3<MAXN, THREADS>(sm.u.K, size);
+        for (int i = tid; i < n; i += THREADS) {
+            sm.ord0[0][i] = (uint16_t)sm.u.K[0][i];
+            sm.ord0[1][i] = (uint16_t)sm.u.K[1][i];
+            sm.ord0[2][i] = (uint16_t)sm.u.K[2][i];
         }
         __syncthreads();  // the sort keys are dead from here on
         for (int i = tid; i < n; i += THREADS) sm.u.a.seg_of[i] = 0;
@@ -634,27 +487,26 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 4) local_build_
 }
 
 // ---- level-by-level splitter for medium jobs -------------------------------------------
-// Jobs of up to MID_MAX points skip the global sort: they are split one tree
-// level per launch until every open segment fits the small local builder
-// (LB_SMALL points), each open segment of a level by a block of its own (the
-// open segments of every job of the call share the launch).  Per segment: the AABB by a block reduction of
-// order-preserving keys; the median key on the longest axis by a four-pass
-// radix select (8-bit digits, shared histogram); then one stable partition
-// pass.  Keys below the median go left, keys equal to it go left in position
-// order until the left half holds n / 2 points, so the split is the same
-// (point of rank n / 2 on the axis, ties by position) as in the sorted
-// builders.  Points move between two scratch buffers (level 0 reads the
-// input); segments that fit the small local builder are copied to buffer 0
-// if they are not there and handed to it as jobs.
-constexpr int MID_MAX = 1 << 17;
-constexpr int MID_THREADS = 1024;
+// Jobs of up to MID_MAX points are split one tree level per launch until every
+// open segment holds at most SPLIT_MIN points, each open segment of a level by a
+// block of its own (the open segments of every job of the call share the
+// launch).  Per segment: the AABB by a block reduction of order-preserving keys;
+// the median key on the longest axis by a four-pass radix select (8-bit digits,
+// shared histogram); then one stable partition pass.  Keys below the median go
+// left, keys equal to it go left in position order until the left half holds n / 2
+// points, so the split is the same (point of rank n / 2 on the axis, ties by
+// position) on every path.  Points move between two scratch buffers (level 0
+// reads the input); children of at most SPLIT_MIN points go to the exit buffer
+// and to finish_split_kernel.
+constexpr int MID_MAX = 1 << 15;
+constexpr int SPLIT_MIN = 4096;  // larger segments of a large job are split by many blocks
 constexpr int MID_PPT = 4;
-constexpr int MID_TILE = MID_THREADS * MID_PPT;
 
+template <int THREADS>
 struct MidShared {
     int hist[256];
-    uint32_t red[MID_THREADS / 32][6];
-    uint32_t wsum[MID_THREADS / 32];
+    uint32_t red[THREADS / 32][6];
+    uint32_t wsum[THREADS / 32];
     uint32_t tot;
     uint32_t box[6];
     int node, axis, digit, rank;
@@ -662,8 +514,9 @@ struct MidShared {
 
 // Exclusive block prefix of a per-thread value; the block total goes to
 // *total.  The shared words are free for reuse when it returns.
-__device__ __forceinline__ uint32_t mid_block_scan(uint32_t v, uint32_t* wsum, uint32_t* tot, uint32_t* total) {
-    static_assert(MID_THREADS == 32 * 32, "one warp scans the warp sums");
+template <int THREADS>
+__device__ __forceinline__ uint32_t block_scan_u32(uint32_t v, uint32_t* wsum, uint32_t* tot, uint32_t* total) {
+    static_assert(THREADS <= 32 * 32, "one warp scans the warp sums");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t inc = v;
 #pragma unroll
@@ -674,14 +527,14 @@ __device__ __forceinline__ uint32_t mid_block_scan(uint32_t v, uint32_t* wsum, u
     if (lane == 31) wsum[warp] = inc;
     __syncthreads();
     if (warp == 0) {
-        const uint32_t w = wsum[lane];
+        const uint32_t w = lane < THREADS / 32 ? wsum[lane] : 0u;
         uint32_t wi = w;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xffffffffu, wi, o);
             if (lane >= o) wi += y;
         }
-        wsum[lane] = wi - w;
+        if (lane < THREADS / 32) wsum[lane] = wi - w;
         if (lane == 31) *tot = wi;
     }
     __syncthreads();
@@ -691,26 +544,29 @@ __device__ __forceinline__ uint32_t mid_block_scan(uint32_t v, uint32_t* wsum, u
     return r;
 }
 
+constexpr int MID_THREADS = 1024;
 __global__ void __launch_bounds__(MID_THREADS, 1) mid_level_kernel(DevTree t, const float4* src, float4* dst,
-                                                                float4* buf0, uint32_t* keys,
+                                                                float4* exits, uint32_t* keys,
                                                                 const int4* __restrict__ segs_in,
                                                                 const int* nseg_in, int4* __restrict__ segs_out,
                                                                 int* nseg_out, int max_segs,
-                                                                int4* __restrict__ local_jobs, int* nlocal,
-                                                                int max_local, int fill) {
-    __shared__ MidShared sm;
+                                                                int4* __restrict__ small, int* nsmall,
+                                                                int max_small, int fill) {
+    __shared__ MidShared<MID_THREADS> sm;
+    constexpr int MID_TILE = MID_THREADS * MID_PPT;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int S = min(*nseg_in, max_segs);
     for (int q = blockIdx.x; q < S; q += gridDim.x) {
         const int4 sg = segs_in[q];
         const int s = sg.x, e = sg.y, link = sg.z;
         const int cnt = e - s;
+        uint32_t* seg_keys = keys + s;
         __syncthreads();  // the previous segment's shared words are free again
-        if (cnt <= LB_SMALL) {  // only at level 0: a small job goes straight to the local builder
-            for (int i = s + tid; i < e; i += MID_THREADS) buf0[i] = src[i];
+        if (cnt <= SPLIT_MIN) {  // only at level 0: a small job
+            for (int i = s + tid; i < e; i += MID_THREADS) exits[i] = src[i];
             if (tid == 0) {
-                const int r = atomicAdd(nlocal, 1);
-                if (r < max_local) local_jobs[r] = make_int4(s, e, link, 0);
+                const int r = atomicAdd(nsmall, 1);
+                if (r < max_small) small[r] = make_int4(s, e, link, 0);
                 else atomicOr(&t.st->err, ERR_SEG);
             }
             continue;
@@ -781,7 +637,7 @@ __global__ void __launch_bounds__(MID_THREADS, 1) mid_level_kernel(DevTree t, co
         int rank = m;
         for (int pass = 0; pass < 4; ++pass) {
             const int shift = 24 - 8 * pass;
-            if (tid < 256) sm.hist[tid] = 0;
+            for (int i = tid; i < 256; i += MID_THREADS) sm.hist[i] = 0;
             __syncthreads();
             for (int base = s; base < e; base += MID_THREADS) {
                 const int i = base + tid;
@@ -790,9 +646,9 @@ __global__ void __launch_bounds__(MID_THREADS, 1) mid_level_kernel(DevTree t, co
                 if (i < e) {
                     if (pass == 0) {
                         k = float_key(coord4(src[i], axis));
-                        keys[i] = k;
+                        seg_keys[i - s] = k;
                     } else {
-                        k = keys[i];
+                        k = seg_keys[i - s];
                     }
                     ok = (k & pmask) == prefix;
                 }
@@ -838,6 +694,8 @@ __global__ void __launch_bounds__(MID_THREADS, 1) mid_level_kernel(DevTree t, co
                                             __int_as_float(axis));
         // Stable partition: left = keys below v, then the first `need`
         // keys equal to v.  Packed counts: below v low, equal high.
+        float4* dl = m > SPLIT_MIN ? dst : exits;
+        float4* dr = cnt - m > SPLIT_MIN ? dst : exits;
         uint32_t carry_lt = 0, carry_eq = 0;
         for (int base = s; base < e; base += MID_TILE) {
             const int i0 = base + tid * MID_PPT;
@@ -846,11 +704,11 @@ __global__ void __launch_bounds__(MID_THREADS, 1) mid_level_kernel(DevTree t, co
 #pragma unroll
             for (int r = 0; r < MID_PPT; ++r) {
                 const int i = i0 + r;
-                kk[r] = i < e ? keys[i] : 0xffffffffu;
+                kk[r] = i < e ? seg_keys[i - s] : 0xffffffffu;
                 if (i < e) sum += kk[r] < v ? 1u : (kk[r] == v ? 0x10000u : 0u);
             }
             uint32_t total;
-            const uint32_t ex = mid_block_scan(sum, sm.wsum, &sm.tot, &total);
+            const uint32_t ex = block_scan_u32<MID_THREADS>(sum, sm.wsum, &sm.tot, &total);
             uint32_t lt = carry_lt + (ex & 0xffffu), eq = carry_eq + (ex >> 16);
 #pragma unroll
             for (int r = 0; r < MID_PPT; ++r) {
@@ -860,7 +718,7 @@ __global__ void __launch_bounds__(MID_THREADS, 1) mid_level_kernel(DevTree t, co
                 const bool left = k < v || (k == v && eq < need);
                 const uint32_t lb = lt + (eq < need ? eq : need);
                 const int dest = left ? s + (int)lb : s + m + (i - s - (int)lb);
-                if (dest >= s && dest < e) dst[dest] = src[i];
+                if (dest >= s && dest < e) (left ? dl : dr)[dest] = src[i];
                 else atomicOr(&t.st->err, ERR_SEG);  // cannot happen: the select found rank m
                 if (k < v) ++lt;
                 else if (k == v) ++eq;
@@ -868,40 +726,711 @@ __global__ void __launch_bounds__(MID_THREADS, 1) mid_level_kernel(DevTree t, co
             carry_lt += total & 0xffffu;
             carry_eq += total >> 16;
         }
-        __syncthreads();  // the partition is complete before the children are read
-        // Children: small ones go to the local builder (from buffer 0),
-        // the others stay open.
-#pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
-            const int cs = c == 0 ? s : s + m, ce = c == 0 ? s + m : e;
-            if (ce - cs <= LB_SMALL) {
-                if (dst != buf0)
-                    for (int i = cs + tid; i < ce; i += MID_THREADS) buf0[i] = dst[i];
-                if (tid == 0) {
-                    const int r = atomicAdd(nlocal, 1);
-                    if (r < max_local) local_jobs[r] = make_int4(cs, ce, X * 2 + c, 0);
-                    else atomicOr(&t.st->err, ERR_SEG);
-                }
-            } else if (tid == 0) {
-                const int r = atomicAdd(nseg_out, 1);
-                if (r < max_segs) segs_out[r] = make_int4(cs, ce, X * 2 + c, 0);
-                else atomicOr(&t.st->err, ERR_SEG);
-            }
+        // Children: small ones leave, the others stay open.
+        if (tid < 2) {
+            const int cs = tid == 0 ? s : s + m, ce = tid == 0 ? s + m : e;
+            const bool open = ce - cs > SPLIT_MIN;
+            const int r = atomicAdd(open ? nseg_out : nsmall, 1);
+            if (r < (open ? max_segs : max_small)) (open ? segs_out : small)[r] = make_int4(cs, ce, X * 2 + tid, 0);
+            else atomicOr(&t.st->err, ERR_SEG);
         }
     }
 }
 
-template <int MAXN, int THREADS>
-void launch_local(unsigned grid, const DevTree& t, const float4* pts, const uint32_t* idx, long long stride, int* loc,
-                  const int4* jobs, const int* njobs, int max_jobs, int fill, cudaStream_t s) {
-    local_build_kernel<MAXN, THREADS><<<grid, THREADS, sizeof(LbShared<MAXN, THREADS>), s>>>(t, pts, idx, stride, loc,
-                                                                                          jobs, njobs, max_jobs, fill);
+// ---- segments of at most SPLIT_MIN points ------------------------------------------------
+// A block takes a whole segment into shared memory, splits it down to LB_SMALL-
+// point pieces there (at most three splits, the points of the open piece in
+// registers meanwhile) and writes the pieces out for the local builder.  Before,
+// these were two more levels of the level-by-level splitter: every pass over a
+// segment went to L2, 160 us for a 2M-point build, 61 us now.
+constexpr int FIN_THREADS = 512;
+constexpr int FIN_ROUNDS = SPLIT_MIN / FIN_THREADS;
+constexpr int FIN_WARPS = FIN_THREADS / 32;
+
+struct FinShared {
+    float4 P[SPLIT_MIN];
+    int hist[256];
+    uint32_t red[FIN_WARPS][6];
+    uint32_t cnt[FIN_ROUNDS * FIN_WARPS];  // packed (below, equal) counts, then their prefix
+    uint32_t box[6];
+    int3 open[4];                          // {s, e, link} pieces to split
+    int nopen, node, axis, digit, rank;
+};
+
+__global__ void __launch_bounds__(FIN_THREADS, 2) finish_split_kernel(DevTree t, const float4* __restrict__ src,
+                                                                      const int4* __restrict__ segs, const int* nseg,
+                                                                      int max_segs, float4* __restrict__ out,
+                                                                      int4* __restrict__ local_jobs, int* nlocal,
+                                                                      int max_local, int fill) {
+    extern __shared__ __align__(16) unsigned char fin_raw[];
+    FinShared& sm = *reinterpret_cast<FinShared*>(fin_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int S = min(*nseg, max_segs);
+    auto local = [&](int s, int e, int link) {  // one thread
+        const int r = atomicAdd(nlocal, 1);
+        if (r < max_local) local_jobs[r] = make_int4(s, e, link, 0);
+        else atomicOr(&t.st->err, ERR_SEG);
+    };
+    for (int q = blockIdx.x; q < S; q += gridDim.x) {
+        const int4 sg = segs[q];
+        const int s0 = sg.x, total = sg.y - sg.x;
+        __syncthreads();  // the previous segment's shared words are free again
+        if (total > SPLIT_MIN || total < 0) {  // cannot happen: the lists hold such segments only
+            if (tid == 0) atomicOr(&t.st->err, ERR_SEG);
+            continue;
+        }
+#pragma unroll
+        for (int r = 0; r < FIN_ROUNDS; ++r)
+            if (r * FIN_THREADS + tid < total) sm.P[r * FIN_THREADS + tid] = src[s0 + r * FIN_THREADS + tid];
+        if (tid == 0) {
+            sm.nopen = 0;
+            if (total > LB_SMALL) sm.open[sm.nopen++] = make_int3(0, total, sg.z);
+            else local(s0, s0 + total, sg.z);
+        }
+        __syncthreads();
+        while (sm.nopen > 0) {
+            const int3 o = sm.open[sm.nopen - 1];
+            const int s = o.x, cnt = o.y - o.x, m = cnt / 2, link = o.z;
+            __syncthreads();  // everyone has the piece
+            if (tid == 0) --sm.nopen;
+            float4 p[FIN_ROUNDS];
+            uint32_t mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0u, 0u, 0u};
+#pragma unroll
+            for (int r = 0; r < FIN_ROUNDS; ++r) {
+                const int i = r * FIN_THREADS + tid;
+                if (i < cnt) {
+                    p[r] = sm.P[s + i];
+                    const uint32_t kx = float_key(p[r].x), ky = float_key(p[r].y), kz = float_key(p[r].z);
+                    mn[0] = min(mn[0], kx), mx[0] = max(mx[0], kx);
+                    mn[1] = min(mn[1], ky), mx[1] = max(mx[1], ky);
+                    mn[2] = min(mn[2], kz), mx[2] = max(mx[2], kz);
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                mn[a] = __reduce_min_sync(0xffffffffu, mn[a]);
+                mx[a] = __reduce_max_sync(0xffffffffu, mx[a]);
+                if (lane == 0) sm.red[warp][a] = mn[a], sm.red[warp][3 + a] = mx[a];
+            }
+            __syncthreads();
+            if (warp == 0) {
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const uint32_t lo = __reduce_min_sync(0xffffffffu, lane < FIN_WARPS ? sm.red[lane][a] : 0xffffffffu);
+                    const uint32_t hi = __reduce_max_sync(0xffffffffu, lane < FIN_WARPS ? sm.red[lane][3 + a] : 0u);
+                    if (lane == 0) sm.box[a] = lo, sm.box[3 + a] = hi;
+                }
+                __syncwarp();
+                if (lane == 0) {
+                    Box3 b;
+                    float ext[3];
+                    for (int a = 0; a < 3; ++a) {
+                        b.lo[a] = key_float(sm.box[a]);
+                        b.hi[a] = key_float(sm.box[3 + a]);
+                        ext[a] = __fsub_rn(b.hi[a], b.lo[a]);
+                    }
+                    int axis = 0;
+                    if (ext[1] > ext[axis]) axis = 1;
+                    if (ext[2] > ext[axis]) axis = 2;
+                    const int X = alloc_node(t);
+                    sm.node = X;
+                    sm.axis = axis;
+                    if (X >= 0) {
+                        const int parent = link >> 1, side = link & 1;
+                        t.nparent[X] = link;
+                        int h = 0;
+                        for (int k = cnt; k > fill; k -= k / 2) ++h;
+                        t.nheight[X] = h;
+                        write_child_box(t.node, parent, side, b);
+                        write_child_code(t.node, parent, side, X);
+                        write_child_cnt(t.ncnt, parent, side, cnt, 0);
+                        const int2 wi = t.winfo[parent];
+                        wide_link(t, wi, side, X, b, cnt);
+                        t.winfo[X] = wide_below(wi, side, X);
+                    }
+                }
+            }
+            __syncthreads();
+            const int X = sm.node, axis = sm.axis;
+            if (X < 0) continue;  // the pool is exhausted (flagged by alloc_node): the points are dropped
+            uint32_t key[FIN_ROUNDS];
+#pragma unroll
+            for (int r = 0; r < FIN_ROUNDS; ++r)
+                key[r] = r * FIN_THREADS + tid < cnt ? float_key(coord4(p[r], axis)) : 0xffffffffu;
+            uint32_t v = 0;
+            int rank = m;
+            for (int b = 32; b > 0; b -= 8) {
+                if (tid < 256) sm.hist[tid] = 0;
+                __syncthreads();
+#pragma unroll
+                for (int r = 0; r < FIN_ROUNDS; ++r)
+                    if (r * FIN_THREADS + tid < cnt && (b < 32 ? key[r] >> b : 0u) == v)
+                        atomicAdd(&sm.hist[(key[r] >> (b - 8)) & 255u], 1);
+                __syncthreads();
+                if (warp == 0) {
+                    int c[8], sum = 0;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) c[j] = sm.hist[lane * 8 + j], sum += c[j];
+                    int inc = sum;
+#pragma unroll
+                    for (int k = 1; k < 32; k <<= 1) {
+                        const int y = __shfl_up_sync(0xffffffffu, inc, k);
+                        if (lane >= k) inc += y;
+                    }
+                    int r = rank - (inc - sum);
+                    if (r >= 0 && r < sum) {  // exactly one lane
+                        int d = 0;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            if (r < c[j]) {
+                                d = j;
+                                break;
+                            }
+                            r -= c[j];
+                        }
+                        sm.digit = lane * 8 + d;
+                        sm.rank = r;
+                    }
+                }
+                __syncthreads();
+                v = (v << 8) | (uint32_t)sm.digit;
+                rank = sm.rank;
+            }
+            if (tid == 0)
+                t.node[4 * X + 3] = make_float4(__int_as_float(0), __int_as_float(0), key_float(v), __int_as_float(axis));
+            // Stable partition: points in order of (round, thread).
+            const uint32_t need = (uint32_t)rank;  // keys equal to v that go left
+            unsigned lt[FIN_ROUNDS], eq[FIN_ROUNDS];
+#pragma unroll
+            for (int r = 0; r < FIN_ROUNDS; ++r) {
+                const bool in = r * FIN_THREADS + tid < cnt;
+                lt[r] = __ballot_sync(0xffffffffu, in && key[r] < v);
+                eq[r] = __ballot_sync(0xffffffffu, in && key[r] == v);
+                if (lane == 0) sm.cnt[r * FIN_WARPS + warp] = (uint32_t)__popc(lt[r]) | ((uint32_t)__popc(eq[r]) << 16);
+            }
+            __syncthreads();
+            if (warp == 0) {
+                constexpr int PER = FIN_ROUNDS * FIN_WARPS / 32;
+                uint32_t c[PER], sum = 0;
+#pragma unroll
+                for (int j = 0; j < PER; ++j) {
+                    c[j] = sum;
+                    sum += sm.cnt[lane * PER + j];
+                }
+                uint32_t inc = sum;
+#pragma unroll
+                for (int k = 1; k < 32; k <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, k);
+                    if (lane >= k) inc += y;
+                }
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < PER; ++j) sm.cnt[lane * PER + j] = inc - sum + c[j];
+            }
+            __syncthreads();
+            const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+            for (int r = 0; r < FIN_ROUNDS; ++r) {
+                const int i = r * FIN_THREADS + tid;
+                if (i < cnt) {
+                    const uint32_t base = sm.cnt[r * FIN_WARPS + warp];
+                    const uint32_t l = (base & 0xffffu) + __popc(lt[r] & below), q2 = (base >> 16) + __popc(eq[r] & below);
+                    const uint32_t lb = l + min(q2, need);
+                    const bool left = key[r] < v || (key[r] == v && q2 < need);
+                    sm.P[s + (left ? (int)lb : m + i - (int)lb)] = p[r];  // (left: lb < m; right: below cnt)
+                }
+            }
+            if (tid == 0) {
+                for (int c = 0; c < 2; ++c) {
+                    const int cs = c == 0 ? s : s + m, ce = c == 0 ? s + m : s + cnt;
+                    if (ce - cs > LB_SMALL) sm.open[sm.nopen++] = make_int3(cs, ce, X * 2 + c);
+                    else local(s0 + cs, s0 + ce, X * 2 + c);
+                }
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int r = 0; r < FIN_ROUNDS; ++r)
+            if (r * FIN_THREADS + tid < total) out[s0 + r * FIN_THREADS + tid] = sm.P[r * FIN_THREADS + tid];
+    }
 }
 
-// The local builders' shared memory is above the 48 KB default: opt in once
+// ---- multi-block splitter for large segments ------------------------------------------------
+// Segments above SPLIT_MIN points: one level per round of five launches, every
+// segment cut into tiles of SPLIT_TILE points, a block per (tile, segment).
+//   hist      keys on the split axis into SPLIT_BINS bins over the segment's range
+//   pick      the bin that holds the point of rank n / 2 (a block per segment)
+//   classify  per tile the points of lower bins; the picked bin's points, (key,
+//             position), into the segment's candidate list
+//   select    the (key, position) of rank n / 2 among the candidates, the tiles'
+//             left counts and their prefix sum, the node, the child segments (a
+//             block per segment)
+//   scatter   stable partition by (key, position), the children's AABBs
+// A uniform segment's candidates are ~1/1,000 of it; with many equal keys the
+// list can hold most of the segment, which only makes select slower.
+// This took the place of sorting the three coordinates once and partitioning the
+// three sorted index arrays per level with random gathers of the sides (109
+// launches): a 2M-point build moves 16 instead of ~100 bytes per point and level
+// and takes 760 us of kernels (430 of them these) against 1,950 us.  Bound by L2
+// bandwidth (level passes) and by the latency of the per-segment blocks.
+constexpr int SPLIT_THREADS = 256;
+constexpr int SPLIT_ROUNDS = 8;  // points per thread
+constexpr int SPLIT_TILE = SPLIT_THREADS * SPLIT_ROUNDS;
+constexpr int SPLIT_BINS = 2048;
+constexpr int SPLIT_CACHE = 4096;  // candidates kept in shared memory by select
+
+// The split axis of a segment (longest extent, first on ties) and its bins: equal
+// widths over the segment's range.  The bin grows with the coordinate (every
+// operation rounds monotonically), which is all the selection needs; an outlier
+// that stretches the range only makes the candidate lists longer.  (Bins of the
+// ordered keys put a quarter of an octave into each where the range spans zero:
+// select took up to 187 us on 20k candidates.)
+struct SplitAxis {
+    int axis;
+    float lo, scale;
+    __device__ __forceinline__ int bin(float x) const {
+        const int b = (int)__fmul_rn(__fsub_rn(x, lo), scale);
+        return min(max(b, 0), SPLIT_BINS - 1);
+    }
+};
+__device__ __forceinline__ SplitAxis split_axis(const uint32_t* box) {
+    float ext[3];
+    for (int a = 0; a < 3; ++a) ext[a] = __fsub_rn(key_float(box[3 + a]), key_float(box[a]));
+    SplitAxis r;
+    r.axis = 0;
+    if (ext[1] > ext[r.axis]) r.axis = 1;
+    if (ext[2] > ext[r.axis]) r.axis = 2;
+    r.lo = key_float(box[r.axis]);
+    r.scale = __fdiv_rn((float)SPLIT_BINS, ext[r.axis]);
+    return r;
+}
+
+// First tile of a segment in the tile arrays: segments hold more than SPLIT_MIN
+// = 2 tiles of points, so s / 1024 leaves room for every segment's own tiles.
+__device__ __forceinline__ int split_tile0(int s) { return s >> 10; }
+static_assert(SPLIT_TILE == 2048 && SPLIT_MIN >= 2 * SPLIT_TILE, "tile array layout");
+
+__device__ __forceinline__ void split_box_reset(uint32_t* box) {
+    for (int a = 0; a < 3; ++a) {
+        box[a] = 0xffffffffu;
+        box[3 + a] = 0u;
+    }
+}
+
+// Jobs above SPLIT_MIN points open the splitter's first level; the others go to
+// the medium list, their points copied to `exits` (a block per job).
+__global__ void __launch_bounds__(SPLIT_THREADS) split_open_kernel(const float4* __restrict__ pts,
+                                                                   const int* __restrict__ job_off,
+                                                                   const int* __restrict__ job_link, int njobs,
+                                                                   SplitLevel lv, int cap, float4* __restrict__ exits,
+                                                                   int4* __restrict__ mid, int* nmid, int max_mid,
+                                                                   DevStatus* st) {
+    __shared__ int big;
+    for (int j = blockIdx.x; j < njobs; j += gridDim.x) {
+        const int s = job_off[j], e = job_off[j + 1];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            big = e - s > SPLIT_MIN;
+            const int r = atomicAdd(big ? lv.n : nmid, 1);
+            if (r >= (big ? cap : max_mid)) {
+                atomicOr(&st->err, ERR_SEG);
+            } else if (big) {
+                lv.seg[r] = make_int4(s, e, job_link[j], 0);
+                lv.cand_n[r] = 0;
+                split_box_reset(lv.box + 6 * r);
+            } else {
+                mid[r] = make_int4(s, e, job_link[j], 0);
+            }
+        }
+        __syncthreads();
+        if (!big)
+            for (int i = s + threadIdx.x; i < e; i += SPLIT_THREADS) exits[i] = pts[i];
+    }
+}
+
+// Block-wide bounds of both sides' points into the boxes (nullptr: not wanted).
+// sm: 12 shared words holding reset boxes.
+__device__ __forceinline__ void split_grow(uint32_t* b, const float4& p) {
+    const uint32_t k[3] = {float_key(p.x), float_key(p.y), float_key(p.z)};
+    for (int a = 0; a < 3; ++a) {
+        b[a] = min(b[a], k[a]);
+        b[3 + a] = max(b[3 + a], k[a]);
+    }
+}
+__device__ __forceinline__ void split_flush(uint32_t* sm, const uint32_t* b) {
+    for (int a = 0; a < 3; ++a) {
+        const uint32_t lo = __reduce_min_sync(0xffffffffu, b[a]), hi = __reduce_max_sync(0xffffffffu, b[3 + a]);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(sm + a, lo);
+            atomicMax(sm + 3 + a, hi);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(SPLIT_THREADS) split_box_kernel(const float4* __restrict__ pts, SplitLevel lv,
+                                                                  int cap, unsigned tiles) {
+    __shared__ uint32_t sm[6];
+    const int q = (int)(blockIdx.x / tiles), tile = (int)(blockIdx.x % tiles);
+    if (q >= min(*lv.n, cap)) return;
+    const int4 sg = lv.seg[q];
+    const int t0 = sg.x + tile * SPLIT_TILE;
+    if (t0 >= sg.y) return;
+    if (threadIdx.x == 0) split_box_reset(sm);
+    __syncthreads();
+    uint32_t b[6];
+    split_box_reset(b);
+    for (int i = t0 + threadIdx.x; i < min(t0 + SPLIT_TILE, sg.y); i += SPLIT_THREADS) split_grow(b, pts[i]);
+    split_flush(sm, b);
+    __syncthreads();
+    if (threadIdx.x < 3) atomicMin(lv.box + 6 * q + threadIdx.x, sm[threadIdx.x]);
+    else if (threadIdx.x < 6) atomicMax(lv.box + 6 * q + threadIdx.x, sm[threadIdx.x]);
+}
+
+__global__ void __launch_bounds__(SPLIT_THREADS) split_hist_kernel(const float4* __restrict__ pts, SplitLevel lv,
+                                                                   int cap, unsigned tiles, int* __restrict__ hist) {
+    __shared__ int h[SPLIT_BINS];
+    const int q = (int)(blockIdx.x / tiles), tile = (int)(blockIdx.x % tiles);
+    if (q >= min(*lv.n, cap)) return;
+    const int4 sg = lv.seg[q];
+    const int t0 = sg.x + tile * SPLIT_TILE;
+    if (t0 >= sg.y) return;
+    const SplitAxis ax = split_axis(lv.box + 6 * q);
+    for (int i = threadIdx.x; i < SPLIT_BINS; i += SPLIT_THREADS) h[i] = 0;
+    __syncthreads();
+    const float* c = reinterpret_cast<const float*>(pts) + ax.axis;
+#pragma unroll
+    for (int r = 0; r < SPLIT_ROUNDS; ++r) {
+        const int i = t0 + r * SPLIT_THREADS + threadIdx.x;
+        if (i < sg.y) atomicAdd(&h[ax.bin(c[4ll * i])], 1);
+    }
+    __syncthreads();
+    int* g = hist + (long long)q * SPLIT_BINS;
+    for (int i = threadIdx.x; i < SPLIT_BINS; i += SPLIT_THREADS)
+        if (h[i]) atomicAdd(g + i, h[i]);
+}
+
+// pick[i] = {bin of the point of rank n / 2, its rank among the bin's points}.
+// The bins are left zero for the next level.
+__global__ void __launch_bounds__(SPLIT_THREADS) split_pick_kernel(SplitLevel lv, SplitLevel nx, int cap,
+                                                                   int* __restrict__ hist, int2* __restrict__ pick) {
+    __shared__ uint32_t wsum[SPLIT_THREADS / 32], tot;
+    const int q = blockIdx.x;
+    if (q == 0 && threadIdx.x == 0) *nx.n = 0;  // select fills it
+    if (q >= min(*lv.n, cap)) return;
+    const int4 sg = lv.seg[q];
+    constexpr int PER = SPLIT_BINS / SPLIT_THREADS;
+    int4* g = reinterpret_cast<int4*>(hist + (long long)q * SPLIT_BINS) + threadIdx.x * (PER / 4);
+    int c[PER], sum = 0;
+#pragma unroll
+    for (int i = 0; i < PER / 4; ++i) {
+        const int4 v = g[i];
+        c[4 * i] = v.x, c[4 * i + 1] = v.y, c[4 * i + 2] = v.z, c[4 * i + 3] = v.w;
+        sum += v.x + v.y + v.z + v.w;
+        g[i] = make_int4(0, 0, 0, 0);
+    }
+    uint32_t total;
+    int r = (sg.y - sg.x) / 2 - (int)block_scan_u32<SPLIT_THREADS>((uint32_t)sum, wsum, &tot, &total);
+    if (r >= 0 && r < sum) {  // exactly one thread
+        int d = threadIdx.x * PER;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            if (r < c[i]) {
+                d += i;
+                break;
+            }
+            r -= c[i];
+        }
+        pick[q] = make_int2(d, r);
+    }
+}
+
+__global__ void __launch_bounds__(SPLIT_THREADS) split_classify_kernel(const float4* __restrict__ pts, SplitLevel lv,
+                                                                       int cap, unsigned tiles,
+                                                                       const int2* __restrict__ pick,
+                                                                       int* __restrict__ tile_left,
+                                                                       uint2* __restrict__ cand) {
+    __shared__ int less;
+    const int q = (int)(blockIdx.x / tiles), tile = (int)(blockIdx.x % tiles);
+    if (q >= min(*lv.n, cap)) return;
+    const int4 sg = lv.seg[q];
+    const int t0 = sg.x + tile * SPLIT_TILE;
+    if (t0 >= sg.y) return;
+    const SplitAxis ax = split_axis(lv.box + 6 * q);
+    const int bin = pick[q].x;
+    if (threadIdx.x == 0) less = 0;
+    __syncthreads();
+    const float* c = reinterpret_cast<const float*>(pts) + ax.axis;
+    const int lane = threadIdx.x & 31;
+    int mine = 0;
+#pragma unroll
+    for (int r = 0; r < SPLIT_ROUNDS; ++r) {
+        const int i = t0 + r * SPLIT_THREADS + threadIdx.x;
+        const float x = i < sg.y ? c[4ll * i] : 0.f;
+        const int b = i < sg.y ? ax.bin(x) : SPLIT_BINS;
+        mine += b < bin ? 1 : 0;
+        const unsigned eq = __ballot_sync(0xffffffffu, b == bin);
+        if (eq == 0) continue;
+        int at = 0;
+        if (lane == 0) at = atomicAdd(lv.cand_n + q, __popc(eq));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(eq & ((1u << lane) - 1u));
+        if (b == bin) cand[sg.x + at] = make_uint2(float_key(x), (uint32_t)(i - sg.x));
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0 && mine) atomicAdd(&less, mine);
+    __syncthreads();
+    if (threadIdx.x == 0) tile_left[split_tile0(sg.x) + tile] = less;
+}
+
+// One 8-bit (or narrower) step of a radix selection: digit(i) of the items that
+// still match (-1: not), rank -> the digit that holds the rank, the rank inside
+// it and the items of that digit.
+struct SplitDigit {
+    int digit, rank, count;
+};
+template <int THREADS, class F>
+__device__ __forceinline__ SplitDigit split_digit(int n, int rank, int* hist, SplitDigit* out, F digit) {
+    for (int i = threadIdx.x; i < 256; i += THREADS) hist[i] = 0;
+    __syncthreads();
+    for (int base = threadIdx.x; base < n; base += 4 * THREADS) {
+        int d[4];  // four items in flight
+#pragma unroll
+        for (int u = 0; u < 4; ++u) d[u] = base + u * THREADS < n ? digit(base + u * THREADS) : -1;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (d[u] >= 0) atomicAdd(&hist[d[u]], 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int c[8], sum = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) c[j] = hist[lane * 8 + j], sum += c[j];
+        int inc = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        int r = rank - (inc - sum);
+        if (r >= 0 && r < sum) {  // exactly one lane
+            int d = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (r < c[j]) {
+                    d = j;
+                    break;
+                }
+                r -= c[j];
+            }
+            *out = SplitDigit{lane * 8 + d, r, c[d]};
+        }
+    }
+    __syncthreads();
+    const SplitDigit o = *out;
+    __syncthreads();
+    return o;
+}
+
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) split_select_kernel(DevTree t, SplitLevel lv, SplitLevel nx, int cap,
+                                                                     const int2* __restrict__ pick,
+                                                                     int* __restrict__ tile_left,
+                                                                     const uint2* __restrict__ cand,
+                                                                     uint2* __restrict__ thr, int2* __restrict__ kids,
+                                                                     int4* __restrict__ mid, int* nmid, int max_mid,
+                                                                     int fill) {
+    __shared__ uint2 cache[SPLIT_CACHE];
+    __shared__ int hist[256];
+    __shared__ SplitDigit sd;
+    __shared__ uint32_t wsum[THREADS / 32], tot, spos;
+    const int q = blockIdx.x;
+    if (q >= min(*lv.n, cap)) return;
+    const int4 sg = lv.seg[q];
+    const int s = sg.x, cnt = sg.y - sg.x, m = cnt / 2, link = sg.z;
+    const SplitAxis ax = split_axis(lv.box + 6 * q);
+    const int c = lv.cand_n[q];
+    const uint2* list = cand + s;
+    const bool cached = c <= SPLIT_CACHE;
+    if (cached) {
+        for (int i = threadIdx.x; i < c; i += THREADS) cache[i] = list[i];
+        __syncthreads();
+    }
+    auto item = [&](int i) { return cached ? cache[i] : list[i]; };
+    // The key of rank n / 2, eight bits at a time.
+    int rank = pick[q].y, same = c;
+    uint32_t v = 0;  // bits found so far
+    for (int b = 32; b > 0; b -= 8) {
+        const SplitDigit r = split_digit<THREADS>(c, rank, hist, &sd, [&](int i) {
+            const uint32_t k = item(i).x;
+            return (b < 32 ? k >> b : 0u) == v ? (int)((k >> (b - 8)) & 255u) : -1;
+        });
+        v = (v << 8) | (uint32_t)r.digit;
+        rank = r.rank;
+        same = r.count;
+    }
+    // Among equal keys the position of that rank.
+    uint32_t p = 0;
+    if (same > 1) {
+        for (int b = 32 - __clz(cnt); b > 0;) {
+            const int w = min(b, 8);
+            const SplitDigit r = split_digit<THREADS>(c, rank, hist, &sd, [&](int i) {
+                const uint2 e = item(i);
+                return e.x == v && (e.y >> b) == p ? (int)((e.y >> (b - w)) & ((1u << w) - 1u)) : -1;
+            });
+            p = (p << w) | (uint32_t)r.digit;
+            rank = r.rank;
+            b -= w;
+        }
+    } else {
+        for (int i = threadIdx.x; i < c; i += THREADS)
+            if (item(i).x == v) spos = item(i).y;
+        __syncthreads();
+        p = spos;
+    }
+    // The tiles' left counts: the lower bins', and the candidates before (v, p).
+    int* tl = tile_left + split_tile0(s);
+    for (int i = threadIdx.x; i < c; i += THREADS) {
+        const uint2 e = item(i);
+        if (e.x < v || (e.x == v && e.y < p)) atomicAdd(tl + e.y / SPLIT_TILE, 1);
+    }
+    __syncthreads();
+    const int tiles = (cnt + SPLIT_TILE - 1) / SPLIT_TILE;
+    uint32_t carry = 0;
+    for (int base = 0; base < tiles; base += THREADS) {
+        const int i = base + threadIdx.x;
+        const uint32_t x = i < tiles ? (uint32_t)__ldcg(tl + i) : 0u;
+        uint32_t total;
+        const uint32_t ex = block_scan_u32<THREADS>(x, wsum, &tot, &total);
+        if (i < tiles) tl[i] = (int)(carry + ex);
+        carry += total;
+    }
+    if (threadIdx.x != 0) return;
+    if (carry != (uint32_t)m) atomicOr(&t.st->err, ERR_SEG);  // cannot happen: the selection found rank m
+    thr[q] = make_uint2(v, p);
+    kids[q] = make_int2(-2, -2);
+    const int X = alloc_node(t);
+    if (X < 0) return;  // the pool is exhausted (flagged): the points are dropped
+    Box3 b;
+    for (int a = 0; a < 3; ++a) {
+        b.lo[a] = key_float(lv.box[6 * q + a]);
+        b.hi[a] = key_float(lv.box[6 * q + 3 + a]);
+    }
+    const int parent = link >> 1, side = link & 1;
+    t.nparent[X] = link;
+    int h = 0;
+    for (int k = cnt; k > fill; k -= k / 2) ++h;
+    t.nheight[X] = h;
+    t.node[4 * X + 3] = make_float4(__int_as_float(0), __int_as_float(0), key_float(v), __int_as_float(ax.axis));
+    write_child_box(t.node, parent, side, b);
+    write_child_code(t.node, parent, side, X);
+    write_child_cnt(t.ncnt, parent, side, cnt, 0);
+    const int2 wi = t.winfo[parent];
+    wide_link(t, wi, side, X, b, cnt);
+    t.winfo[X] = wide_below(wi, side, X);
+    // Children: the splitter's next level or the medium list (-1).
+    int kid[2];
+    for (int k = 0; k < 2; ++k) {
+        const int cs = k == 0 ? s : s + m, ce = k == 0 ? s + m : s + cnt;
+        const bool big = ce - cs > SPLIT_MIN;
+        const int r = atomicAdd(big ? nx.n : nmid, 1);
+        kid[k] = -1;
+        if (r >= (big ? cap : max_mid)) {
+            atomicOr(&t.st->err, ERR_SEG);
+        } else if (big) {
+            nx.seg[r] = make_int4(cs, ce, X * 2 + k, 0);
+            nx.cand_n[r] = 0;
+            split_box_reset(nx.box + 6 * r);
+            kid[k] = r;
+        } else {
+            mid[r] = make_int4(cs, ce, X * 2 + k, 0);
+        }
+    }
+    kids[q] = make_int2(kid[0], kid[1]);
+}
+
+// Points before (v, p) go left, the others right, both in order: to `dst`, or to
+// `exits` where the child leaves the splitter.
+__global__ void __launch_bounds__(SPLIT_THREADS) split_scatter_kernel(const float4* __restrict__ src, SplitLevel lv,
+                                                                      SplitLevel nx, int cap, unsigned tiles,
+                                                                      const int* __restrict__ tile_left,
+                                                                      const uint2* __restrict__ thr,
+                                                                      const int2* __restrict__ kids,
+                                                                      float4* __restrict__ dst,
+                                                                      float4* __restrict__ exits) {
+    constexpr int WARPS = SPLIT_THREADS / 32, WARP_PTS = SPLIT_TILE / WARPS;
+    __shared__ uint32_t sm[12];
+    __shared__ int wleft[WARPS];
+    const int q = (int)(blockIdx.x / tiles), tile = (int)(blockIdx.x % tiles);
+    if (q >= min(*lv.n, cap)) return;
+    const int4 sg = lv.seg[q];
+    const int t0 = sg.x + tile * SPLIT_TILE;
+    const int2 kd = kids[q];
+    if (t0 >= sg.y || kd.x == -2) return;
+    const int axis = split_axis(lv.box + 6 * q).axis;
+    const uint2 th = thr[q];
+    const int m = (sg.y - sg.x) / 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < 2) split_box_reset(sm + 6 * threadIdx.x);
+    // A warp's consecutive points, 32 a round.
+    const int w0 = t0 + warp * WARP_PTS;
+    float4 p[SPLIT_ROUNDS];
+    unsigned lm[SPLIT_ROUNDS];
+    int left = 0;
+#pragma unroll
+    for (int r = 0; r < SPLIT_ROUNDS; ++r) {
+        const int i = w0 + 32 * r + lane;
+        bool l = false;
+        if (i < sg.y) {
+            p[r] = src[i];
+            const uint32_t k = float_key(coord4(p[r], axis));
+            l = k < th.x || (k == th.x && (uint32_t)(i - sg.x) < th.y);
+        }
+        lm[r] = __ballot_sync(0xffffffffu, l);
+        left += __popc(lm[r]);
+    }
+    if (lane == 0) wleft[warp] = left;
+    __syncthreads();
+    int run = tile_left[split_tile0(sg.x) + tile];  // left points before this warp's
+    for (int w = 0; w < warp; ++w) run += wleft[w];
+    float4* dl = kd.x >= 0 ? dst : exits;
+    float4* dr = kd.y >= 0 ? dst : exits;
+    uint32_t bl[6], br[6];
+    split_box_reset(bl);
+    split_box_reset(br);
+#pragma unroll
+    for (int r = 0; r < SPLIT_ROUNDS; ++r) {
+        const int i = w0 + 32 * r + lane;
+        if (i < sg.y) {
+            const int before = run + __popc(lm[r] & ((1u << lane) - 1u));
+            const bool l = lm[r] >> lane & 1;
+            const int to = l ? sg.x + before : m + (i - before);
+            if (to < sg.y) (l ? dl : dr)[to] = p[r];  // (always: select checked the left count)
+            if (l && kd.x >= 0) split_grow(bl, p[r]);
+            if (!l && kd.y >= 0) split_grow(br, p[r]);
+        }
+        run += __popc(lm[r]);
+    }
+    if (kd.x >= 0) split_flush(sm, bl);
+    if (kd.y >= 0) split_flush(sm + 6, br);
+    __syncthreads();
+    if (threadIdx.x < 12) {
+        const int a = threadIdx.x % 6, kid = threadIdx.x < 6 ? kd.x : kd.y;
+        if (kid >= 0) {
+            if (a < 3) atomicMin(nx.box + 6 * kid + a, sm[threadIdx.x]);
+            else atomicMax(nx.box + 6 * kid + a, sm[threadIdx.x]);
+        }
+    }
+}
+
+void launch_local(unsigned grid, const DevTree& t, const float4* pts, const int4* jobs, const int* njobs, int max_jobs,
+                  int fill, cudaStream_t s) {
+    local_build_kernel<LB_SMALL, 256><<<grid, 256, sizeof(LbShared<LB_SMALL, 256>), s>>>(t, pts, jobs, njobs, max_jobs,
+                                                                                       fill);
+}
+
+// The local builder's shared memory is above the 48 KB default: opt in once
 // per device.  Returns the device's SM count: the block-per-job kernels run
-// one block per SM at most, each looping over jobs (idle blocks of 1,024
-// threads and 200 KB of shared memory still cost a wave each to launch).
+// one resident wave at most, each block looping over jobs.
 int lb_prepare() {
     static std::atomic<int> sms[64];
     int dev = 0;
@@ -909,10 +1438,9 @@ int lb_prepare() {
     dev &= 63;
     int n = sms[dev].load(std::memory_order_acquire);
     if (n > 0) return n;
-    cudaFuncSetAttribute(local_build_kernel<LB_MAX, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(LbShared<LB_MAX, 1024>));
     cudaFuncSetAttribute(local_build_kernel<LB_SMALL, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(LbShared<LB_SMALL, 256>));
+    cudaFuncSetAttribute(finish_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FinShared));
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
     if (n <= 0) n = 1;
     sms[dev].store(n, std::memory_order_release);
@@ -930,15 +1458,12 @@ __global__ void reset_count_kernel(int* c) { *c = 0; }
 
 inline unsigned blocks_for(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
-// Bound on the segments of a level and on the local builders' jobs of one
-// call: a level holds at most two segments per node of the level above (each
-// node has more than `fill` points); a local job is a whole job or a piece of
-// at least 512 points (half of a segment above LB_SMALL or LB_MAX points).
-long long max_segs_bound(long long n, int njobs, int fill) {
-    long long b = 2 * (n / (fill + 1)) + 2;
-    long long j = (long long)njobs + n / 512 + 2;
-    return b > j ? b : j;
-}
+// Bounds on the lists of one call: segments of the medium splitter, segments of
+// at most SPLIT_MIN points and jobs of the local builder (a whole job or a piece
+// of at least 512 points: half of a segment above LB_SMALL points); segments of
+// the large splitter.
+long long max_segs_bound(long long n, int njobs) { return (long long)njobs + n / 512 + 2; }
+long long max_split_bound(long long n) { return n / SPLIT_MIN + 2; }
 
 size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -953,128 +1478,130 @@ int build_levels(long long max_job, int fill) {
     return d + 1;
 }
 
-size_t build_scratch_bytes(long long n, int njobs, int fill) {
-    long long ms = max_segs_bound(n, njobs, fill);
-    size_t b = 0;
-    b += 2 * align_up(sizeof(uint32_t) * 3 * n);   // ord
-    b += 2 * align_up(sizeof(uint32_t) * 3 * n);   // keys
-    b += 2 * align_up(sizeof(int) * n);            // segpos
-    b += align_up(sizeof(int) * n);                // flag
-    b += 2 * align_up(sizeof(int) * 3 * n);        // scan in / out
-    b += 4 * align_up(sizeof(int4) * ms);          // segs x2, seginfo, local jobs
-    b += align_up(sizeof(int) * 4);                // nseg
-    size_t tmp = sort_temp_bytes(n, 3);
-    size_t st = scan_temp_bytes(3 * n);
-    b += align_up(tmp > st ? tmp : st);
-    return b;
+namespace {
+
+struct ScratchCarver {
+    char* base;
+    size_t off = 0;
+    template <class T>
+    T* take(size_t count) {
+        T* r = (T*)(base + off);
+        off += align_up(sizeof(T) * count);
+        return r;
+    }
+};
+
+size_t carve(void* base, long long n, int njobs, BuildScratch* bs) {
+    const long long ms = max_segs_bound(n, njobs);
+    // the large splitter's lists, only for calls that can use it
+    const long long sp = n > MID_MAX ? max_split_bound(n) : 0;
+    ScratchCarver c{(char*)base};
+    for (int i = 0; i < 3; ++i) bs->pts[i] = c.take<float4>(n);
+    bs->keys = c.take<uint32_t>(n);
+    for (int i = 0; i < 2; ++i) bs->segs[i] = c.take<int4>(ms);
+    bs->small = c.take<int4>(ms);
+    bs->local_jobs = c.take<int4>(ms);
+    bs->nseg = c.take<int>(4);
+    for (int i = 0; i < 2; ++i) {
+        bs->split[i].seg = c.take<int4>(sp);
+        bs->split[i].box = c.take<uint32_t>(6 * sp);
+        bs->split[i].cand_n = c.take<int>(sp);
+        bs->split[i].n = c.take<int>(1);
+    }
+    bs->hist = c.take<int>(SPLIT_BINS * sp);
+    bs->pick = c.take<int2>(sp);
+    bs->thr = c.take<uint2>(sp);
+    bs->kids = c.take<int2>(sp);
+    bs->tile_left = c.take<int>(sp ? n / 1024 + 2 : 0);
+    bs->cand = c.take<uint2>(sp ? n : 0);
+    return c.off;
 }
 
-void carve_build_scratch(void* base, long long n, int njobs, int fill, BuildScratch* bs) {
-    long long ms = max_segs_bound(n, njobs, fill);
-    char* p = (char*)base;
-    auto take = [&](size_t bytes) {
-        void* r = p;
-        p += align_up(bytes);
-        return r;
-    };
-    bs->ord[0] = (uint32_t*)take(sizeof(uint32_t) * 3 * n);
-    bs->ord[1] = (uint32_t*)take(sizeof(uint32_t) * 3 * n);
-    bs->keys[0] = (uint32_t*)take(sizeof(uint32_t) * 3 * n);
-    bs->keys[1] = (uint32_t*)take(sizeof(uint32_t) * 3 * n);
-    bs->segpos[0] = (int*)take(sizeof(int) * n);
-    bs->segpos[1] = (int*)take(sizeof(int) * n);
-    bs->flag = (int*)take(sizeof(int) * n);
-    bs->scan_in = (int*)take(sizeof(int) * 3 * n);
-    bs->scan_out = (int*)take(sizeof(int) * 3 * n);
-    bs->segs[0] = (int4*)take(sizeof(int4) * ms);
-    bs->segs[1] = (int4*)take(sizeof(int4) * ms);
-    bs->seginfo = (int4*)take(sizeof(int4) * ms);
-    bs->local_jobs = (int4*)take(sizeof(int4) * ms);
-    bs->nseg = (int*)take(sizeof(int) * 4);
-    bs->temp = (void*)p;
-    // The splitter of medium jobs uses none of the sort arrays: its two point
-    // buffers (32 n bytes) lie over ord[0 .. 1] and keys[0 .. 1] (>= 48 n bytes).
-    bs->mid_pts[0] = (float4*)bs->ord[0];
-    bs->mid_pts[1] = (float4*)((char*)bs->ord[0] + align_up(sizeof(float4) * n));
+}  // namespace
+
+size_t build_scratch_bytes(long long n, int njobs) {
+    BuildScratch bs;
+    return carve(nullptr, n, njobs, &bs);
 }
+
+void carve_build_scratch(void* base, long long n, int njobs, BuildScratch* bs) { carve(base, n, njobs, bs); }
 
 void build_subtrees(const DevTree& t, const float4* pts, long long n, const int* job_off, const int* job_link,
                     int njobs, long long max_job, int fill, const BuildScratch& bs, cudaStream_t s) {
     if (njobs <= 0) return;
     const long long sms = lb_prepare();
     const int T = 256;
-    long long nn = n > 0 ? n : 1;
-    long long ms = max_segs_bound(nn, njobs, fill);
-    // Block-per-job grids: the small local builder fits four blocks per SM,
-    // the splitter and the large local builder one.
+    const long long nn = n > 0 ? n : 1;
+    const long long ms = max_segs_bound(nn, njobs);
+    // Block-per-job grids: blocks of 256 threads run four per SM, the medium
+    // splitter's of 1,024 one.
     auto grid = [&](long long jobs, long long per_sm) { return (unsigned)std::min(jobs, per_sm * sms); };
     if (max_job <= LB_SMALL) {
-        // Every job fits the small local builder: one launch builds them all.
+        // Every job fits the local builder: one launch builds them all.
         init_segs_kernel<<<blocks_for(njobs, T), T, 0, s>>>(job_off, job_link, njobs, bs.segs[0], bs.nseg);
-        launch_local<LB_SMALL, 256>(grid(njobs, 4), t, pts, nullptr, 0, nullptr, bs.segs[0], bs.nseg, njobs, fill, s);
+        launch_local(grid(njobs, 4), t, pts, bs.segs[0], bs.nseg, njobs, fill, s);
         finish_alloc_kernel<<<1, 1, 0, s>>>(t.st);
         return;
     }
-    if (max_job <= MID_MAX) {
-        // Medium jobs: one launch per level splits every open segment (one
-        // block each) until all of them fit the small local builder.
-        reset_count_kernel<<<1, 1, 0, s>>>(bs.nseg + 2);
+    // Counters: medium segments of two levels, segments of at most SPLIT_MIN
+    // points, local jobs.
+    int *nsmall = bs.nseg + 2, *nlocal = bs.nseg + 3;
+    cudaMemsetAsync(bs.nseg, 0, 4 * sizeof(int), s);
+    const float4* small_pts = bs.pts[2];
+    if (max_job <= SPLIT_MIN) {
+        init_segs_kernel<<<blocks_for(njobs, T), T, 0, s>>>(job_off, job_link, njobs, bs.small, nsmall);
+        small_pts = pts;
+    } else if (max_job <= MID_MAX) {
+        // Medium segments: one launch per level splits every open one.
         init_segs_kernel<<<blocks_for(njobs, T), T, 0, s>>>(job_off, job_link, njobs, bs.segs[0], bs.nseg);
-        int levels = 0;
-        for (long long m = max_job; m > LB_SMALL; m -= m / 2) ++levels;
-        long long open = njobs;  // bound on the open segments of a level
-        for (int lv = 0; lv < std::max(levels, 1); ++lv) {
-            const float4* src = lv == 0 ? pts : ((lv & 1) ? bs.mid_pts[0] : bs.mid_pts[1]);
-            float4* dst = (lv & 1) ? bs.mid_pts[1] : bs.mid_pts[0];
-            reset_count_kernel<<<1, 1, 0, s>>>(bs.nseg + ((lv + 1) & 1));
+        long long open = njobs, size = max_job;
+        for (int lv = 0; size > SPLIT_MIN; ++lv) {
+            const float4* src = lv == 0 ? pts : bs.pts[(lv + 1) & 1];
+            int *in = bs.nseg + (lv & 1), *out = bs.nseg + ((lv + 1) & 1);
+            if (lv > 0) reset_count_kernel<<<1, 1, 0, s>>>(out);
             mid_level_kernel<<<grid(std::min(open, ms), 1), MID_THREADS, 0, s>>>(
-                t, src, dst, bs.mid_pts[0], (uint32_t*)bs.flag, bs.segs[lv & 1], bs.nseg + (lv & 1),
-                bs.segs[(lv + 1) & 1], bs.nseg + ((lv + 1) & 1), (int)ms, bs.local_jobs, bs.nseg + 2, (int)ms, fill);
+                t, src, bs.pts[lv & 1], bs.pts[2], bs.keys, bs.segs[lv & 1], in, bs.segs[(lv + 1) & 1], out, (int)ms,
+                bs.small, nsmall, (int)ms, fill);
             open = std::min(2 * open, ms);
+            size -= size / 2;
         }
-        launch_local<LB_SMALL, 256>(grid(ms, 4), t, bs.mid_pts[0], nullptr, 0, nullptr, bs.local_jobs, bs.nseg + 2,
-                                    (int)ms, fill, s);
-        finish_alloc_kernel<<<1, 1, 0, s>>>(t.st);
-        return;
+    } else {
+        // Large segments, one level per round, until all of them are small.
+        const int cap = (int)max_split_bound(nn);
+        reset_count_kernel<<<1, 1, 0, s>>>(bs.split[0].n);
+        cudaMemsetAsync(bs.hist, 0, sizeof(int) * SPLIT_BINS * (size_t)cap, s);
+        split_open_kernel<<<grid(njobs, 8), SPLIT_THREADS, 0, s>>>(pts, job_off, job_link, njobs, bs.split[0], cap,
+                                                                   bs.pts[2], bs.small, nsmall, (int)ms, t.st);
+        long long segs = std::min<long long>(njobs, cap), size = max_job;
+        for (int lv = 0; size > SPLIT_MIN; ++lv) {
+            const SplitLevel &cur = bs.split[lv & 1], &nx = bs.split[(lv + 1) & 1];
+            const float4* src = lv == 0 ? pts : bs.pts[(lv + 1) & 1];
+            float4* dst = bs.pts[lv & 1];
+            const unsigned tiles = (unsigned)((size + SPLIT_TILE - 1) / SPLIT_TILE);
+            const unsigned blocks = tiles * (unsigned)segs;
+            if (lv == 0) split_box_kernel<<<blocks, SPLIT_THREADS, 0, s>>>(src, cur, cap, tiles);
+            split_hist_kernel<<<blocks, SPLIT_THREADS, 0, s>>>(src, cur, cap, tiles, bs.hist);
+            split_pick_kernel<<<(unsigned)segs, SPLIT_THREADS, 0, s>>>(cur, nx, cap, bs.hist, bs.pick);
+            split_classify_kernel<<<blocks, SPLIT_THREADS, 0, s>>>(src, cur, cap, tiles, bs.pick, bs.tile_left, bs.cand);
+            // few segments have many candidates each
+            if (segs <= 64)
+                split_select_kernel<1024><<<(unsigned)segs, 1024, 0, s>>>(t, cur, nx, cap, bs.pick, bs.tile_left, bs.cand,
+                                                                         bs.thr, bs.kids, bs.small, nsmall, (int)ms,
+                                                                         fill);
+            else
+                split_select_kernel<256><<<(unsigned)segs, 256, 0, s>>>(t, cur, nx, cap, bs.pick, bs.tile_left, bs.cand,
+                                                                       bs.thr, bs.kids, bs.small, nsmall, (int)ms,
+                                                                       fill);
+            split_scatter_kernel<<<blocks, SPLIT_THREADS, 0, s>>>(src, cur, nx, cap, tiles, bs.tile_left, bs.thr, bs.kids,
+                                                                  dst, bs.pts[2]);
+            segs = std::min<long long>(2 * segs, cap);
+            size -= size / 2;
+        }
     }
-    init_keys_kernel<<<dim3(blocks_for(n, T), 3), T, 0, s>>>(pts, n, bs.keys[0], bs.ord[0]);
-    radix_sort_pairs(bs.keys[0], bs.ord[0], bs.keys[1], bs.ord[1], n, 3, n, 32, bs.temp, s);
-    if (njobs > 1) {
-        int* jp = bs.segpos[1];
-        job_of_point_kernel<<<blocks_for(n, T), T, 0, s>>>(job_off, njobs, n, jp);
-        job_keys_kernel<<<dim3(blocks_for(n, T), 3), T, 0, s>>>(jp, bs.ord[0], n, bs.keys[0]);
-        int bits = 8;
-        while (bits < 32 && (1ll << bits) < njobs) bits += 8;
-        radix_sort_pairs(bs.keys[0], bs.ord[0], bs.keys[1], bs.ord[1], n, 3, n, bits, bs.temp, s);
-    }
-    init_segpos_kernel<<<blocks_for(n, T), T, 0, s>>>(bs.keys[0], n, njobs == 1, bs.segpos[0]);
-    init_segs_kernel<<<blocks_for(njobs, T), T, 0, s>>>(job_off, job_link, njobs, bs.segs[0], bs.nseg);
-    reset_count_kernel<<<1, 1, 0, s>>>(bs.nseg + 2);
-    // Global levels until every segment fits the local builder.
-    int levels = build_levels(max_job, LB_MAX);
-    int cur = 0;
-    long long seg_bound = njobs;
-    for (int lv = 0; lv < levels; ++lv) {
-        int nxt = cur ^ 1;
-        reset_count_kernel<<<1, 1, 0, s>>>(bs.nseg + nxt);
-        level_seg_kernel<<<blocks_for(seg_bound, 128), 128, 0, s>>>(t, pts, bs.ord[cur], nn, bs.segs[cur],
-                                                                    bs.nseg + cur, bs.segs[nxt], bs.nseg + nxt,
-                                                                    bs.seginfo, fill, (int)ms, bs.local_jobs,
-                                                                    bs.nseg + 2);
-        level_pos_kernel<<<blocks_for(n, T), T, 0, s>>>(t, pts, bs.ord[cur], n, bs.segpos[cur], bs.seginfo, bs.flag);
-        level_scanin_kernel<<<dim3(blocks_for(n, T), 3), T, 0, s>>>(bs.ord[cur], n, bs.segpos[cur], bs.seginfo,
-                                                                   bs.flag, bs.scan_in);
-        exclusive_scan(bs.scan_in, bs.scan_out, 3 * n, nullptr, bs.temp, s);
-        level_scatter_kernel<<<dim3(blocks_for(n, T), 3), T, 0, s>>>(bs.ord[cur], bs.ord[nxt], n, bs.segpos[cur],
-                                                                    bs.segpos[nxt], bs.segs[cur], bs.seginfo,
-                                                                    bs.flag, bs.scan_out);
-        long long nb = seg_bound * 2;
-        seg_bound = nb < ms ? nb : ms;
-        cur = nxt;
-    }
-    // The three index arrays of the last level hold every local segment.
-    launch_local<LB_MAX, 1024>(grid(ms, 1), t, pts, bs.ord[cur], n, bs.flag, bs.local_jobs, bs.nseg + 2, (int)ms,
-                               fill, s);
+    finish_split_kernel<<<grid(ms, 2), FIN_THREADS, sizeof(FinShared), s>>>(t, small_pts, bs.small, nsmall, (int)ms,
+                                                                            bs.pts[0], bs.local_jobs, nlocal, (int)ms,
+                                                                            fill);
+    launch_local(grid(ms, 4), t, bs.pts[0], bs.local_jobs, nlocal, (int)ms, fill, s);
     finish_alloc_kernel<<<1, 1, 0, s>>>(t.st);
 }
 

@@ -483,12 +483,12 @@ struct Tree {
         reserve_build(total, nj);
         ensure_removed(st->removed_n + st->root_deleted + 1);
         size_t bytes = align_up(sizeof(float4) * std::max<long long>(total, 1)) +
-                       build_scratch_bytes(std::max<long long>(total, 1), nj, fill) + 4096;
+                       build_scratch_bytes(std::max<long long>(total, 1), nj) + 4096;
         bld.ensure(bytes, stream);
         float4* gathered = (float4*)bld.p;
         BuildScratch bs;
         carve_build_scratch((char*)bld.p + align_up(sizeof(float4) * std::max<long long>(total, 1)),
-                            std::max<long long>(total, 1), nj, fill, &bs);
+                            std::max<long long>(total, 1), nj, &bs);
         launch_job_gather(dt, aux, st->leaf_top, st->node_top, ovf_leaf, ovf_pts, ovf_bound, gathered, removed,
                           removed_cap, stream);
         build_subtrees(dt, gathered, total, aux.job_off, aux.job_link, nj, std::max<long long>(max_job, 1), fill, bs,
@@ -566,9 +566,9 @@ struct Tree {
         small.ensure(4096, stream);
         int* job = (int*)small.p;
         CK(cudaMemcpyAsync(job, host_job, sizeof(host_job), cudaMemcpyHostToDevice, stream));
-        bld.ensure(build_scratch_bytes(nn, 1, fill) + 4096, stream);
+        bld.ensure(build_scratch_bytes(nn, 1) + 4096, stream);
         BuildScratch bs;
-        carve_build_scratch(bld.p, nn, 1, fill, &bs);
+        carve_build_scratch(bld.p, nn, 1, &bs);
         set_top(n);
         build_subtrees(dt, pts, n, job, job + 2, 1, nn, fill, bs, stream);
         launch_snapshot_root(dt, stream);
@@ -582,12 +582,16 @@ struct Tree {
         reset_counters();
         float4* packed = nullptr;
         if (n > 0) {
-            op.ensure(align_up(sizeof(float) * n * stride) + align_up(sizeof(float4) * n), stream);
+            op.ensure(align_up(sizeof(float4) * n) + (host_mode ? 0 : align_up(sizeof(float) * n * stride)), stream);
             Carver c(op.p);
-            float* raw = c.take<float>((size_t)n * stride);
             packed = c.take<float4>(n);
-            CK(cudaMemcpyAsync(raw, xyz, sizeof(float) * n * stride, cudaMemcpyHostToDevice, stream));
-            launch_pack_points(dt, raw, stride, n, 0, packed, stream);
+            const float* src = xyz;
+            if (host_mode == 0) {
+                float* raw = c.take<float>((size_t)n * stride);
+                CK(cudaMemcpyAsync(raw, xyz, sizeof(float) * n * stride, cudaMemcpyHostToDevice, stream));
+                src = raw;
+            }
+            launch_pack_points(dt, src, stride, n, 0, packed, stream);
             read_status();
             if (st->err & ERR_INPUT) throw BadArg{"build: non-finite coordinate"};
         }

@@ -30,22 +30,30 @@ bool radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32
 // becomes a balanced subtree of leaves holding at most `fill` points, split at
 // the median of the longest AABB axis, and is linked into the child slot
 // `job_link[j]` (= parent * 2 + side) together with its AABB and counts.
-struct BuildScratch {
-    uint32_t* ord[2];    // 2 x [3 * n] point indices sorted per axis
-    uint32_t* keys[2];   // 2 x [3 * n]
-    int* segpos[2];      // 2 x [n]
-    int* flag;           // [n]
-    int* scan_in;        // [3 * n]
-    int* scan_out;       // [3 * n]
-    int4* segs[2];       // 2 x [max_segs]  {s, e, link, pad}
-    int4* seginfo;       // [max_segs]      {kind, axis/leaf, mid, child_base}
-    int4* local_jobs;    // [max_segs]      {s, e, link} for the CTA-local builder
-    int* nseg;           // [4] device counters (two levels, local jobs)
-    void* temp;          // scan / sort temp
-    float4* mid_pts[2];  // 2 x [n] points of the medium-job splitter (alias ord / keys)
+// Open segments of the large splitter at one level.
+struct SplitLevel {
+    int4* seg;       // {s, e, link, -}
+    uint32_t* box;   // 6 per segment: keys of the AABB's low, then high corner
+    int* cand_n;     // candidates listed
+    int* n;          // segments
 };
-size_t build_scratch_bytes(long long n, int njobs, int fill);
-void carve_build_scratch(void* base, long long n, int njobs, int fill, BuildScratch* bs);
+struct BuildScratch {
+    float4* pts[3];      // 3 x [n] points between levels; [2]: those of segments that left the splitters
+    uint32_t* keys;      // [n] keys of the medium splitter
+    int4* segs[2];       // medium segments of two levels  {s, e, link, -}
+    int4* small;         // segments for finish_split_kernel
+    int4* local_jobs;    // segments for the local builder
+    int* nseg;           // [4] device counters (medium segments of two levels, small, local)
+    SplitLevel split[2]; // large segments of two levels
+    int* hist;           // bins per large segment
+    int2* pick;          // {bin, rank in it}
+    uint2* thr;          // {key, position} of the split point
+    int2* kids;          // large segments of the children (-1: small, -2: dropped)
+    int* tile_left;      // left points per tile, then their prefix
+    uint2* cand;         // [n] {key, position} of the picked bins' points
+};
+size_t build_scratch_bytes(long long n, int njobs);
+void carve_build_scratch(void* base, long long n, int njobs, BuildScratch* bs);
 int build_levels(long long max_job, int fill);
 void build_subtrees(const DevTree& t, const float4* pts, long long n, const int* job_off, const int* job_link,
                     int njobs, long long max_job, int fill, const BuildScratch& bs, cudaStream_t s);

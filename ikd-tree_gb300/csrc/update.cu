@@ -1532,6 +1532,40 @@ __global__ void pack_points_kernel(DevTree t, const float* __restrict__ in, int 
     out[i] = make_float4(x, y, z, __int_as_float((int)(id & ID_MASK)));
 }
 
+// The same for tightly packed, 16-byte aligned input: a block's points come in as
+// consecutive 16-byte words (the input may be host memory over the chip link).
+constexpr int PACK_POINTS = 1024;
+__global__ void __launch_bounds__(256) pack_dense_kernel(DevTree t, const float4* __restrict__ in, long long n,
+                                                         long long first_id, float4* __restrict__ out) {
+    __shared__ float4 w[PACK_POINTS * 3 / 4];
+    const long long p0 = (long long)blockIdx.x * PACK_POINTS;
+    const int m = (int)min((long long)PACK_POINTS, n - p0);
+    const int words = m * 3 / 4;  // whole 16-byte words
+    const float4* src = in + p0 * 3 / 4;
+    float4 v[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+        if (r * 256 + (int)threadIdx.x < words) v[r] = src[r * 256 + threadIdx.x];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+        if (r * 256 + (int)threadIdx.x < words) w[r * 256 + threadIdx.x] = v[r];
+    float* f = reinterpret_cast<float*>(w);
+    if ((int)threadIdx.x < m * 3 - words * 4) f[words * 4 + threadIdx.x] = reinterpret_cast<const float*>(src)[words * 4 + threadIdx.x];
+    __syncthreads();
+    bool bad = false;
+#pragma unroll
+    for (int r = 0; r < PACK_POINTS / 256; ++r) {
+        const int i = r * 256 + threadIdx.x;
+        if (i >= m) break;
+        const float x = f[3 * i], y = f[3 * i + 1], z = f[3 * i + 2];
+        bad = bad || !(isfinite(x) && isfinite(y) && isfinite(z));
+        const long long id = first_id + p0 + i;
+        if (id > MAX_ID) atomicOr(&t.st->err, ERR_ID);
+        out[p0 + i] = make_float4(x, y, z, __int_as_float((int)(id & ID_MASK)));
+    }
+    if (bad) atomicOr(&t.st->err, ERR_INPUT);
+}
+
 __global__ void check_finite_kernel(DevTree t, const float* __restrict__ in, long long count) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
@@ -1662,6 +1696,11 @@ void launch_select_root_job(const DevTree& t, const UpdateAux& a, cudaStream_t s
 void launch_pack_points(const DevTree& t, const float* in, int stride, long long n, long long first_id, float4* out,
                         cudaStream_t s) {
     if (n <= 0) return;
+    if (stride == 3 && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {
+        pack_dense_kernel<<<blocks_for(n, PACK_POINTS), 256, 0, s>>>(t, reinterpret_cast<const float4*>(in), n, first_id,
+                                                                     out);
+        return;
+    }
     pack_points_kernel<<<blocks_for(n, 256), 256, 0, s>>>(t, in, stride, n, first_id, out);
 }
 
