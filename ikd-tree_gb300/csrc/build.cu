@@ -10,14 +10,13 @@
 // largest job:
 // * small (every job <= LB_SMALL points): one CTA per job builds the whole
 //   subtree in shared memory (local_build_kernel);
-// * medium (jobs <= MID_MAX): one launch per tree level splits every open
-//   segment of every job, one CTA per segment, down to LB_SMALL-point segments
-//   (mid_level_kernel: radix-selected median, stable partition), then the
-//   local builder finishes them;
+// * medium (jobs <= SPLIT_MIN): one CTA per job splits it in shared memory down to
+//   LB_SMALL-point segments (finish_split_kernel: radix-selected median, stable
+//   partition), then the local builder finishes them;
 // * large: segments above SPLIT_MIN points are split one level at a time by
-//   many CTAs each (split_* kernels: histogram of the keys on the split axis,
-//   the bin that holds the median, selection among that bin's few keys, stable
-//   partition), the rest goes the medium way.
+//   many CTAs each (split_* kernels: histogram of the split axis, the bin that
+//   holds the median, selection among that bin's few points, stable partition),
+//   the rest goes the medium way.
 // All three cut a segment of n points at the point of rank n / 2 on its axis,
 // ties in input order (every partition is stable), so they follow one split
 // rule.
@@ -486,31 +485,7 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 4) local_build_
     }
 }
 
-// ---- level-by-level splitter for medium jobs -------------------------------------------
-// Jobs of up to MID_MAX points are split one tree level per launch until every
-// open segment holds at most SPLIT_MIN points, each open segment of a level by a
-// block of its own (the open segments of every job of the call share the
-// launch).  Per segment: the AABB by a block reduction of order-preserving keys;
-// the median key on the longest axis by a four-pass radix select (8-bit digits,
-// shared histogram); then one stable partition pass.  Keys below the median go
-// left, keys equal to it go left in position order until the left half holds n / 2
-// points, so the split is the same (point of rank n / 2 on the axis, ties by
-// position) on every path.  Points move between two scratch buffers (level 0
-// reads the input); children of at most SPLIT_MIN points go to the exit buffer
-// and to finish_split_kernel.
-constexpr int MID_MAX = 1 << 15;
-constexpr int SPLIT_MIN = 4096;  // larger segments of a large job are split by many blocks
-constexpr int MID_PPT = 4;
-
-template <int THREADS>
-struct MidShared {
-    int hist[256];
-    uint32_t red[THREADS / 32][6];
-    uint32_t wsum[THREADS / 32];
-    uint32_t tot;
-    uint32_t box[6];
-    int node, axis, digit, rank;
-};
+constexpr int SPLIT_MIN = 4096;  // larger segments are split by many blocks
 
 // Exclusive block prefix of a per-thread value; the block total goes to
 // *total.  The shared words are free for reuse when it returns.
@@ -544,205 +519,12 @@ __device__ __forceinline__ uint32_t block_scan_u32(uint32_t v, uint32_t* wsum, u
     return r;
 }
 
-constexpr int MID_THREADS = 1024;
-__global__ void __launch_bounds__(MID_THREADS, 1) mid_level_kernel(DevTree t, const float4* src, float4* dst,
-                                                                float4* exits, uint32_t* keys,
-                                                                const int4* __restrict__ segs_in,
-                                                                const int* nseg_in, int4* __restrict__ segs_out,
-                                                                int* nseg_out, int max_segs,
-                                                                int4* __restrict__ small, int* nsmall,
-                                                                int max_small, int fill) {
-    __shared__ MidShared<MID_THREADS> sm;
-    constexpr int MID_TILE = MID_THREADS * MID_PPT;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int S = min(*nseg_in, max_segs);
-    for (int q = blockIdx.x; q < S; q += gridDim.x) {
-        const int4 sg = segs_in[q];
-        const int s = sg.x, e = sg.y, link = sg.z;
-        const int cnt = e - s;
-        uint32_t* seg_keys = keys + s;
-        __syncthreads();  // the previous segment's shared words are free again
-        if (cnt <= SPLIT_MIN) {  // only at level 0: a small job
-            for (int i = s + tid; i < e; i += MID_THREADS) exits[i] = src[i];
-            if (tid == 0) {
-                const int r = atomicAdd(nsmall, 1);
-                if (r < max_small) small[r] = make_int4(s, e, link, 0);
-                else atomicOr(&t.st->err, ERR_SEG);
-            }
-            continue;
-        }
-        // AABB.
-        uint32_t mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0u, 0u, 0u};
-        for (int i = s + tid; i < e; i += MID_THREADS) {
-            const float4 p = src[i];
-            const uint32_t kx = float_key(p.x), ky = float_key(p.y), kz = float_key(p.z);
-            mn[0] = min(mn[0], kx), mx[0] = max(mx[0], kx);
-            mn[1] = min(mn[1], ky), mx[1] = max(mx[1], ky);
-            mn[2] = min(mn[2], kz), mx[2] = max(mx[2], kz);
-        }
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            mn[a] = __reduce_min_sync(0xffffffffu, mn[a]);
-            mx[a] = __reduce_max_sync(0xffffffffu, mx[a]);
-        }
-        if (lane == 0)
-            for (int a = 0; a < 3; ++a) sm.red[warp][a] = mn[a], sm.red[warp][3 + a] = mx[a];
-        __syncthreads();
-        if (warp == 0) {
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                uint32_t lo = lane < MID_THREADS / 32 ? sm.red[lane][a] : 0xffffffffu;
-                uint32_t hi = lane < MID_THREADS / 32 ? sm.red[lane][3 + a] : 0u;
-                lo = __reduce_min_sync(0xffffffffu, lo);
-                hi = __reduce_max_sync(0xffffffffu, hi);
-                if (lane == 0) sm.box[a] = lo, sm.box[3 + a] = hi;
-            }
-        }
-        __syncthreads();
-        // The node: axis, allocation, links into its parent.
-        if (tid == 0) {
-            Box3 b;
-            for (int a = 0; a < 3; ++a) {
-                b.lo[a] = key_float(sm.box[a]);
-                b.hi[a] = key_float(sm.box[3 + a]);
-            }
-            float ext[3];
-            for (int a = 0; a < 3; ++a) ext[a] = __fsub_rn(b.hi[a], b.lo[a]);
-            int axis = 0;
-            if (ext[1] > ext[axis]) axis = 1;
-            if (ext[2] > ext[axis]) axis = 2;
-            const int X = alloc_node(t);
-            sm.node = X;
-            sm.axis = axis;
-            if (X >= 0) {
-                const int parent = link >> 1, side = link & 1;
-                t.nparent[X] = link;
-                int h = 0;
-                for (int m = cnt; m > fill; m -= m / 2) ++h;
-                t.nheight[X] = h;
-                write_child_box(t.node, parent, side, b);
-                write_child_code(t.node, parent, side, X);
-                write_child_cnt(t.ncnt, parent, side, cnt, 0);
-                const int2 wi = t.winfo[parent];
-                wide_link(t, wi, side, X, b, cnt);
-                t.winfo[X] = wide_below(wi, side, X);
-            }
-        }
-        __syncthreads();
-        const int X = sm.node, axis = sm.axis;
-        if (X < 0) continue;  // the pool is exhausted (flagged by alloc_node): the points are dropped
-        // Radix select of the key of rank m = cnt / 2.
-        const int m = cnt / 2;
-        uint32_t prefix = 0, pmask = 0;
-        int rank = m;
-        for (int pass = 0; pass < 4; ++pass) {
-            const int shift = 24 - 8 * pass;
-            for (int i = tid; i < 256; i += MID_THREADS) sm.hist[i] = 0;
-            __syncthreads();
-            for (int base = s; base < e; base += MID_THREADS) {
-                const int i = base + tid;
-                bool ok = false;
-                uint32_t k = 0;
-                if (i < e) {
-                    if (pass == 0) {
-                        k = float_key(coord4(src[i], axis));
-                        seg_keys[i - s] = k;
-                    } else {
-                        k = seg_keys[i - s];
-                    }
-                    ok = (k & pmask) == prefix;
-                }
-                const int d = ok ? (int)((k >> shift) & 255u) : 256 + lane;
-                const unsigned peers = __match_any_sync(0xffffffffu, d);
-                if (ok && lane == __ffs(peers) - 1) atomicAdd(&sm.hist[d], __popc(peers));
-            }
-            __syncthreads();
-            if (warp == 0) {
-                int c[8], sum = 0;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) c[j] = sm.hist[lane * 8 + j], sum += c[j];
-                int inc = sum;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += y;
-                }
-                const int before = inc - sum;
-                if (rank >= before && rank < inc) {  // exactly one lane
-                    int r = rank - before, d = lane * 8;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        if (r < c[j]) {
-                            d = lane * 8 + j;
-                            break;
-                        }
-                        r -= c[j];
-                    }
-                    sm.digit = d;
-                    sm.rank = r;
-                }
-            }
-            __syncthreads();
-            prefix |= (uint32_t)sm.digit << shift;
-            pmask |= 255u << shift;
-            rank = sm.rank;
-        }
-        const uint32_t v = prefix;
-        const uint32_t need = (uint32_t)rank;  // keys equal to v that go left
-        if (tid == 0)
-            t.node[4 * X + 3] = make_float4(__int_as_float(0), __int_as_float(0), key_float(v),
-                                            __int_as_float(axis));
-        // Stable partition: left = keys below v, then the first `need`
-        // keys equal to v.  Packed counts: below v low, equal high.
-        float4* dl = m > SPLIT_MIN ? dst : exits;
-        float4* dr = cnt - m > SPLIT_MIN ? dst : exits;
-        uint32_t carry_lt = 0, carry_eq = 0;
-        for (int base = s; base < e; base += MID_TILE) {
-            const int i0 = base + tid * MID_PPT;
-            uint32_t kk[MID_PPT];
-            uint32_t sum = 0;
-#pragma unroll
-            for (int r = 0; r < MID_PPT; ++r) {
-                const int i = i0 + r;
-                kk[r] = i < e ? seg_keys[i - s] : 0xffffffffu;
-                if (i < e) sum += kk[r] < v ? 1u : (kk[r] == v ? 0x10000u : 0u);
-            }
-            uint32_t total;
-            const uint32_t ex = block_scan_u32<MID_THREADS>(sum, sm.wsum, &sm.tot, &total);
-            uint32_t lt = carry_lt + (ex & 0xffffu), eq = carry_eq + (ex >> 16);
-#pragma unroll
-            for (int r = 0; r < MID_PPT; ++r) {
-                const int i = i0 + r;
-                if (i >= e) break;
-                const uint32_t k = kk[r];
-                const bool left = k < v || (k == v && eq < need);
-                const uint32_t lb = lt + (eq < need ? eq : need);
-                const int dest = left ? s + (int)lb : s + m + (i - s - (int)lb);
-                if (dest >= s && dest < e) (left ? dl : dr)[dest] = src[i];
-                else atomicOr(&t.st->err, ERR_SEG);  // cannot happen: the select found rank m
-                if (k < v) ++lt;
-                else if (k == v) ++eq;
-            }
-            carry_lt += total & 0xffffu;
-            carry_eq += total >> 16;
-        }
-        // Children: small ones leave, the others stay open.
-        if (tid < 2) {
-            const int cs = tid == 0 ? s : s + m, ce = tid == 0 ? s + m : e;
-            const bool open = ce - cs > SPLIT_MIN;
-            const int r = atomicAdd(open ? nseg_out : nsmall, 1);
-            if (r < (open ? max_segs : max_small)) (open ? segs_out : small)[r] = make_int4(cs, ce, X * 2 + tid, 0);
-            else atomicOr(&t.st->err, ERR_SEG);
-        }
-    }
-}
-
 // ---- segments of at most SPLIT_MIN points ------------------------------------------------
 // A block takes a whole segment into shared memory, splits it down to LB_SMALL-
 // point pieces there (at most three splits, the points of the open piece in
-// registers meanwhile) and writes the pieces out for the local builder.  Before,
-// these were two more levels of the level-by-level splitter: every pass over a
-// segment went to L2, 160 us for a 2M-point build, 61 us now.
+// registers meanwhile) and writes the pieces out for the local builder.  (One
+// launch per level with every pass over a segment in L2: 160 us for a 2M-point
+// build, 61 us now.)
 constexpr int FIN_THREADS = 512;
 constexpr int FIN_ROUNDS = SPLIT_MIN / FIN_THREADS;
 constexpr int FIN_WARPS = FIN_THREADS / 32;
@@ -1018,12 +800,12 @@ __device__ __forceinline__ void split_box_reset(uint32_t* box) {
 }
 
 // Jobs above SPLIT_MIN points open the splitter's first level; the others go to
-// the medium list, their points copied to `exits` (a block per job).
+// the small list, their points copied to `exits` (a block per job).
 __global__ void __launch_bounds__(SPLIT_THREADS) split_open_kernel(const float4* __restrict__ pts,
                                                                    const int* __restrict__ job_off,
                                                                    const int* __restrict__ job_link, int njobs,
                                                                    SplitLevel lv, int cap, float4* __restrict__ exits,
-                                                                   int4* __restrict__ mid, int* nmid, int max_mid,
+                                                                   int4* __restrict__ small, int* nsmall, int max_small,
                                                                    DevStatus* st) {
     __shared__ int big;
     for (int j = blockIdx.x; j < njobs; j += gridDim.x) {
@@ -1031,15 +813,15 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_open_kernel(const float4*
         __syncthreads();
         if (threadIdx.x == 0) {
             big = e - s > SPLIT_MIN;
-            const int r = atomicAdd(big ? lv.n : nmid, 1);
-            if (r >= (big ? cap : max_mid)) {
+            const int r = atomicAdd(big ? lv.n : nsmall, 1);
+            if (r >= (big ? cap : max_small)) {
                 atomicOr(&st->err, ERR_SEG);
             } else if (big) {
                 lv.seg[r] = make_int4(s, e, job_link[j], 0);
                 lv.cand_n[r] = 0;
                 split_box_reset(lv.box + 6 * r);
             } else {
-                mid[r] = make_int4(s, e, job_link[j], 0);
+                small[r] = make_int4(s, e, job_link[j], 0);
             }
         }
         __syncthreads();
@@ -1237,7 +1019,7 @@ __global__ void __launch_bounds__(THREADS) split_select_kernel(DevTree t, SplitL
                                                                      int* __restrict__ tile_left,
                                                                      const uint2* __restrict__ cand,
                                                                      uint2* __restrict__ thr, int2* __restrict__ kids,
-                                                                     int4* __restrict__ mid, int* nmid, int max_mid,
+                                                                     int4* __restrict__ small, int* nsmall, int max_small,
                                                                      int fill) {
     __shared__ uint2 cache[SPLIT_CACHE];
     __shared__ int hist[256];
@@ -1327,14 +1109,14 @@ __global__ void __launch_bounds__(THREADS) split_select_kernel(DevTree t, SplitL
     const int2 wi = t.winfo[parent];
     wide_link(t, wi, side, X, b, cnt);
     t.winfo[X] = wide_below(wi, side, X);
-    // Children: the splitter's next level or the medium list (-1).
+    // Children: the splitter's next level or the small list (-1).
     int kid[2];
     for (int k = 0; k < 2; ++k) {
         const int cs = k == 0 ? s : s + m, ce = k == 0 ? s + m : s + cnt;
         const bool big = ce - cs > SPLIT_MIN;
-        const int r = atomicAdd(big ? nx.n : nmid, 1);
+        const int r = atomicAdd(big ? nx.n : nsmall, 1);
         kid[k] = -1;
-        if (r >= (big ? cap : max_mid)) {
+        if (r >= (big ? cap : max_small)) {
             atomicOr(&t.st->err, ERR_SEG);
         } else if (big) {
             nx.seg[r] = make_int4(cs, ce, X * 2 + k, 0);
@@ -1342,7 +1124,7 @@ __global__ void __launch_bounds__(THREADS) split_select_kernel(DevTree t, SplitL
             split_box_reset(nx.box + 6 * r);
             kid[k] = r;
         } else {
-            mid[r] = make_int4(cs, ce, X * 2 + k, 0);
+            small[r] = make_int4(cs, ce, X * 2 + k, 0);
         }
     }
     kids[q] = make_int2(kid[0], kid[1]);
@@ -1458,10 +1240,9 @@ __global__ void reset_count_kernel(int* c) { *c = 0; }
 
 inline unsigned blocks_for(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
-// Bounds on the lists of one call: segments of the medium splitter, segments of
-// at most SPLIT_MIN points and jobs of the local builder (a whole job or a piece
-// of at least 512 points: half of a segment above LB_SMALL points); segments of
-// the large splitter.
+// Bounds on the lists of one call: segments of at most SPLIT_MIN points and jobs of
+// the local builder (a whole job or a piece of at least 512 points: half of a
+// segment above LB_SMALL points); segments of the large splitter.
 long long max_segs_bound(long long n, int njobs) { return (long long)njobs + n / 512 + 2; }
 long long max_split_bound(long long n) { return n / SPLIT_MIN + 2; }
 
@@ -1494,14 +1275,12 @@ struct ScratchCarver {
 size_t carve(void* base, long long n, int njobs, BuildScratch* bs) {
     const long long ms = max_segs_bound(n, njobs);
     // the large splitter's lists, only for calls that can use it
-    const long long sp = n > MID_MAX ? max_split_bound(n) : 0;
+    const long long sp = n > SPLIT_MIN ? max_split_bound(n) : 0;
     ScratchCarver c{(char*)base};
-    for (int i = 0; i < 3; ++i) bs->pts[i] = c.take<float4>(n);
-    bs->keys = c.take<uint32_t>(n);
-    for (int i = 0; i < 2; ++i) bs->segs[i] = c.take<int4>(ms);
+    for (int i = 0; i < 3; ++i) bs->pts[i] = c.take<float4>(i == 0 || sp ? n : 0);
     bs->small = c.take<int4>(ms);
     bs->local_jobs = c.take<int4>(ms);
-    bs->nseg = c.take<int>(4);
+    bs->nseg = c.take<int>(2);
     for (int i = 0; i < 2; ++i) {
         bs->split[i].seg = c.take<int4>(sp);
         bs->split[i].box = c.take<uint32_t>(6 * sp);
@@ -1533,38 +1312,22 @@ void build_subtrees(const DevTree& t, const float4* pts, long long n, const int*
     const int T = 256;
     const long long nn = n > 0 ? n : 1;
     const long long ms = max_segs_bound(nn, njobs);
-    // Block-per-job grids: blocks of 256 threads run four per SM, the medium
-    // splitter's of 1,024 one.
+    // Block-per-job grids: local builders run four per SM, finishing blocks two.
     auto grid = [&](long long jobs, long long per_sm) { return (unsigned)std::min(jobs, per_sm * sms); };
     if (max_job <= LB_SMALL) {
         // Every job fits the local builder: one launch builds them all.
-        init_segs_kernel<<<blocks_for(njobs, T), T, 0, s>>>(job_off, job_link, njobs, bs.segs[0], bs.nseg);
-        launch_local(grid(njobs, 4), t, pts, bs.segs[0], bs.nseg, njobs, fill, s);
+        init_segs_kernel<<<blocks_for(njobs, T), T, 0, s>>>(job_off, job_link, njobs, bs.local_jobs, bs.nseg);
+        launch_local(grid(njobs, 4), t, pts, bs.local_jobs, bs.nseg, njobs, fill, s);
         finish_alloc_kernel<<<1, 1, 0, s>>>(t.st);
         return;
     }
-    // Counters: medium segments of two levels, segments of at most SPLIT_MIN
-    // points, local jobs.
-    int *nsmall = bs.nseg + 2, *nlocal = bs.nseg + 3;
-    cudaMemsetAsync(bs.nseg, 0, 4 * sizeof(int), s);
+    // Counters: segments of at most SPLIT_MIN points, local jobs.
+    int *nsmall = bs.nseg, *nlocal = bs.nseg + 1;
+    cudaMemsetAsync(bs.nseg, 0, 2 * sizeof(int), s);
     const float4* small_pts = bs.pts[2];
     if (max_job <= SPLIT_MIN) {
         init_segs_kernel<<<blocks_for(njobs, T), T, 0, s>>>(job_off, job_link, njobs, bs.small, nsmall);
         small_pts = pts;
-    } else if (max_job <= MID_MAX) {
-        // Medium segments: one launch per level splits every open one.
-        init_segs_kernel<<<blocks_for(njobs, T), T, 0, s>>>(job_off, job_link, njobs, bs.segs[0], bs.nseg);
-        long long open = njobs, size = max_job;
-        for (int lv = 0; size > SPLIT_MIN; ++lv) {
-            const float4* src = lv == 0 ? pts : bs.pts[(lv + 1) & 1];
-            int *in = bs.nseg + (lv & 1), *out = bs.nseg + ((lv + 1) & 1);
-            if (lv > 0) reset_count_kernel<<<1, 1, 0, s>>>(out);
-            mid_level_kernel<<<grid(std::min(open, ms), 1), MID_THREADS, 0, s>>>(
-                t, src, bs.pts[lv & 1], bs.pts[2], bs.keys, bs.segs[lv & 1], in, bs.segs[(lv + 1) & 1], out, (int)ms,
-                bs.small, nsmall, (int)ms, fill);
-            open = std::min(2 * open, ms);
-            size -= size / 2;
-        }
     } else {
         // Large segments, one level per round, until all of them are small.
         const int cap = (int)max_split_bound(nn);

@@ -38,12 +38,10 @@ struct SplitLevel {
     int* n;          // segments
 };
 struct BuildScratch {
-    float4* pts[3];      // 3 x [n] points between levels; [2]: those of segments that left the splitters
-    uint32_t* keys;      // [n] keys of the medium splitter
-    int4* segs[2];       // medium segments of two levels  {s, e, link, -}
-    int4* small;         // segments for finish_split_kernel
+    float4* pts[3];      // 3 x [n] points between levels; [2]: those of segments that left the splitter
+    int4* small;         // segments for finish_split_kernel  {s, e, link, -}
     int4* local_jobs;    // segments for the local builder
-    int* nseg;           // [4] device counters (medium segments of two levels, small, local)
+    int* nseg;           // [2] device counters (small, local)
     SplitLevel split[2]; // large segments of two levels
     int* hist;           // bins per large segment
     int2* pick;          // {bin, rank in it}

@@ -1,5 +1,5 @@
 """Builds at the edges of the builder's paths (whole-block finish up to 4,096
-points, medium splitter up to 32,768, multi-block splitter above) and on inputs
+points, multi-block splitter above) and on inputs
 that make its selection long: lattices (many equal keys), all points equal, two
 values, a far outlier that puts nearly every point into one bin.  The structure
 is validated, the stored points are the input, and searches equal the model."""
@@ -20,7 +20,7 @@ GEN = {
 
 
 @pytest.mark.parametrize("kind", sorted(GEN))
-@pytest.mark.parametrize("n", [4095, 4096, 4097, 8193, 32767, 32769, 65537, 140001])
+@pytest.mark.parametrize("n", [4095, 4096, 4097, 8192, 8193, 32769, 65537, 140001])
 def test_paths_and_degenerate_inputs(ikdg_mod, n, kind):
     rng = np.random.default_rng(n)
     pts = GEN[kind](rng, n).astype(np.float32)
