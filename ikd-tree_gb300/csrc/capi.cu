@@ -20,6 +20,8 @@
 #include <string>
 #include <vector>
 
+#include <unistd.h>
+
 #include "ikdg.h"
 #include "kernels.cuh"
 #include "search.cuh"
@@ -182,9 +184,23 @@ struct Tree {
     }
     // On Grace-Blackwell the GPU reads and writes pageable host memory through
     // NVLink-C2C with the CPU's page tables (cudaDevAttrPageableMemoryAccess).
-    // Host-pointer searches then run their kernels directly on the caller's
-    // buffers instead of staging copies.  IKDG_HOST_STAGING=1 forces copies.
-    int host_mode = 0;  // 0: staging copies, 1: direct reads + staged results, 2: all direct
+    // Host-pointer calls then run their kernels directly on the caller's
+    // buffers: the transfer overlaps the search and no copy follows it (15k
+    // queries k = 5 from and to ordinary arrays 106 us with copies back, 62 us
+    // without; 200k 349 / 208 us).  IKDG_HOST_STAGING=1 forces copies.
+    bool direct = false;
+    // Pages of output arrays that nobody has touched yet are brought in here,
+    // by the CPU: a GPU page fault each would cost far more.
+    static void touch_pages(void* p, size_t bytes) {
+        if (p == nullptr || bytes == 0) return;
+        static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+        volatile char* c = (volatile char*)p;
+        for (size_t o = 0; o < bytes; o += page) c[o] = 0;
+        c[bytes - 1] = 0;
+    }
+    // Kernels that run on host buffers report errors into pinned host memory:
+    // no copy brings the bits.
+    DevStatus* host_st = nullptr;
 
     DevTree dt{};
     UpdateAux aux{};
@@ -225,9 +241,9 @@ struct Tree {
             cudaGetLastError();
             pageable = 0;
         }
-        host_mode = pageable != 0 ? 1 : 0;
-        if (const char* m = std::getenv("IKDG_HOST_MODE")) host_mode = pageable != 0 ? std::atoi(m) : 0;
-        if (std::getenv("IKDG_HOST_STAGING") != nullptr) host_mode = 0;
+        direct = pageable != 0 && std::getenv("IKDG_HOST_STAGING") == nullptr;
+        CK(cudaMallocHost(&host_st, sizeof(DevStatus)));
+        std::memset(host_st, 0, sizeof(DevStatus));
         ensure_pools(64, 64);
         reset_tree();
         CK(cudaStreamSynchronize(stream));
@@ -268,6 +284,8 @@ struct Tree {
         small.release();
         if (st_dev != nullptr) cudaFree(st_dev);
         if (st != nullptr) cudaFreeHost(st);
+        if (host_st != nullptr) cudaFreeHost(host_st);
+        host_st = nullptr;
         if (reg_part != nullptr) cudaFreeHost(reg_part);
         reg_part = nullptr;
         reg_cap = 0;
@@ -582,15 +600,10 @@ struct Tree {
         reset_counters();
         float4* packed = nullptr;
         if (n > 0) {
-            op.ensure(align_up(sizeof(float4) * n) + (host_mode ? 0 : align_up(sizeof(float) * n * stride)), stream);
+            op.ensure(align_up(sizeof(float4) * n) + input_bytes((size_t)n * stride), stream);
             Carver c(op.p);
             packed = c.take<float4>(n);
-            const float* src = xyz;
-            if (host_mode == 0) {
-                float* raw = c.take<float>((size_t)n * stride);
-                CK(cudaMemcpyAsync(raw, xyz, sizeof(float) * n * stride, cudaMemcpyHostToDevice, stream));
-                src = raw;
-            }
+            const float* src = input(xyz, (size_t)n * stride, c.take<float>(0));
             launch_pack_points(dt, src, stride, n, 0, packed, stream);
             read_status();
             if (st->err & ERR_INPUT) throw BadArg{"build: non-finite coordinate"};
@@ -614,16 +627,13 @@ struct Tree {
         reset_counters();
         if (debug_validate) check_valid("start of Add_Points");
         if (!downsample) {
-            op.ensure(align_up(sizeof(float) * n * stride) + 2 * align_up(sizeof(float4) * n) +
-                          align_up(sizeof(int4) * n),
+            op.ensure(input_bytes((size_t)n * stride) + 2 * align_up(sizeof(float4) * n) + align_up(sizeof(int4) * n),
                       stream);
             Carver c(op.p);
-            float* raw = c.take<float>((size_t)n * stride);
             float4* packed = c.take<float4>(n);
             int4* ovf_leaf = c.take<int4>(n);
             float4* ovf_pts = c.take<float4>(n);
-            CK(cudaMemcpyAsync(raw, xyz, sizeof(float) * n * stride, cudaMemcpyHostToDevice, stream));
-            launch_pack_points(dt, raw, stride, n, next_id, packed, stream);
+            launch_pack_points(dt, input(xyz, (size_t)n * stride, c.take<float>(0)), stride, n, next_id, packed, stream);
             if (st->root_code == 0) {
                 read_status();
                 if (st->err & ERR_INPUT) throw BadArg{"add_points: non-finite coordinate"};
@@ -649,17 +659,16 @@ struct Tree {
         // the walking deletion that takes over when the list overflows).
         long long pair_cap = std::min<long long>((long long)st->root_slots + n + 65536, INT_MAX / 2);
         if (const char* e = std::getenv("IKDG_DS_PAIR_CAP")) pair_cap = std::max(1ll, std::min(pair_cap, std::atoll(e)));
-        op.ensure(align_up(sizeof(float) * n * stride) + ds_scratch_bytes(n, pair_cap) + align_up(sizeof(float4) * n) +
+        op.ensure(input_bytes((size_t)n * stride) + ds_scratch_bytes(n, pair_cap) + align_up(sizeof(float4) * n) +
                       align_up(sizeof(int4) * n) + 4096,
                   stream);
         Carver c(op.p);
-        float* raw = c.take<float>((size_t)n * stride);
+        float* raw = c.take<float>(direct ? 0 : (size_t)n * stride);
         int4* ovf_leaf = c.take<int4>(n);
         float4* ovf_pts = c.take<float4>(n);
         DsScratch d;
         carve_ds_scratch(op.p == nullptr ? nullptr : (char*)op.p + c.off, n, pair_cap, &d);
-        CK(cudaMemcpyAsync(raw, xyz, sizeof(float) * n * stride, cudaMemcpyHostToDevice, stream));
-        launch_ds_prepare(dt, raw, stride, n, ds_size, d, stream);
+        launch_ds_prepare(dt, input(xyz, (size_t)n * stride, raw), stride, n, ds_size, d, stream);
         // No status read between the phases of a sub-batch: the kernels read
         // the group count, the sub-batch end and the non-finite flag on the
         // device (n bounds the group count for their grids), and the status
@@ -711,10 +720,8 @@ struct Tree {
         if (n < 0 || stride < 3 || (n > 0 && xyz == nullptr)) throw BadArg{"delete_points: bad arguments"};
         if (n == 0 || st->root_code == 0) return;
         reset_counters();
-        op.ensure(align_up(sizeof(float) * n * stride), stream);
-        float* raw = (float*)op.p;
-        CK(cudaMemcpyAsync(raw, xyz, sizeof(float) * n * stride, cudaMemcpyHostToDevice, stream));
-        launch_delete_points(dt, aux, raw, stride, n, stream);
+        op.ensure(input_bytes((size_t)n * stride), stream);
+        launch_delete_points(dt, aux, input(xyz, (size_t)n * stride, (float*)op.p), stride, n, stream);
         finish_update(nullptr, nullptr, 0);
     }
 
@@ -723,7 +730,7 @@ struct Tree {
         if (m == 0 || st->root_code == 0) return 0;
         reset_counters();
         op.ensure(align_up(sizeof(float) * m * 6), stream);
-        float* raw = (float*)op.p;
+        float* raw = (float*)op.p;  // (every block reads its box several times: a copy in HBM)
         CK(cudaMemcpyAsync(raw, boxes, sizeof(float) * m * 6, cudaMemcpyHostToDevice, stream));
         launch_delete_boxes(dt, aux, raw, m, F_DEL, (long long*)((char*)st_dev + offsetof(DevStatus, count)),
                             stream);
@@ -744,6 +751,15 @@ struct Tree {
         finish_update(nullptr, nullptr, 0);
     }
 
+    // The caller's input array as the kernels read it: in place, or copied to
+    // `staged` (device room for it).
+    const float* input(const float* in, size_t floats, float* staged) {
+        if (direct) return in;
+        CK(cudaMemcpyAsync(staged, in, sizeof(float) * floats, cudaMemcpyHostToDevice, stream));
+        return staged;
+    }
+    size_t input_bytes(size_t floats) const { return direct ? 0 : align_up(sizeof(float) * floats); }
+
     // True when every non-null pointer is page-locked host memory (registered
     // with or allocated by CUDA).
     static bool all_pinned(std::initializer_list<const void*> ptrs) {
@@ -760,10 +776,10 @@ struct Tree {
     }
 
     // ---- concurrent small searches ------------------------------------------------
-    // A search context: a stream, a device buffer (a status block for the
-    // kernel's error bits, the result rows, the kNN scratch) and a pinned host
-    // mirror of the status and rows, so one device-to-host copy returns
-    // everything.  Contexts are pooled per tree and reused.
+    // A search context: a stream, a device buffer (staged queries and rows, the
+    // kNN scratch) and a pinned host block (a status block for the kernel's
+    // error bits; staged queries and rows).  Contexts are pooled per tree and
+    // reused.
     struct SearchCtx {
         cudaStream_t s = nullptr;
         char* d = nullptr;
@@ -832,41 +848,47 @@ struct Tree {
             throw BadArg{"knn: bad arguments"};
         if (nq == 0) return;
         const size_t nk = (size_t)nq * k;
-        const size_t o_ids = align_up(sizeof(DevStatus));
-        const size_t o_d2 = o_ids + align_up(sizeof(int) * nk);
+        const size_t tmp = knn_temp_bytes(nq, k);
+        const size_t o_rows = align_up(sizeof(DevStatus));  // the status comes first
+        const size_t o_d2 = o_rows + align_up(sizeof(int) * nk);
         const size_t o_xyz = o_d2 + align_up(sizeof(float) * nk);
         const size_t o_cnt = o_xyz + (xyz ? align_up(sizeof(float) * 3 * nk) : 0);
-        const size_t o_end = o_cnt + (cnt ? align_up(sizeof(int) * nq) : 0);
-        const size_t o_q = o_end;
-        const size_t o_tmp = o_q + (host_mode == 0 ? align_up(sizeof(float) * nq * stride) : 0);
-        const size_t dneed = o_tmp + align_up(knn_temp_bytes(nq, k) + 256);
-        const size_t hneed = std::max(o_end, o_tmp);
+        const size_t o_q = o_cnt + (cnt ? align_up(sizeof(int) * nq) : 0);
+        const size_t o_tmp = o_q + align_up(sizeof(float) * nq * stride);
+        const int bits = bin_bits_for(nq, k);
+        const bool direct = this->direct && bits == 0;  // (a sorted batch's rows would leave one by one)
         SearchCtx* c = take_ctx();
         try {
-            ctx_reserve(c, dneed, hneed);
+            ctx_reserve(c, direct ? 0 : o_tmp + align_up(tmp + 256), direct ? o_rows : o_tmp);
             DevTree t = dt;
-            t.st = (DevStatus*)c->d;  // this call's error bits land in its own status block
-            CK(cudaMemsetAsync(c->d + offsetof(DevStatus, err), 0, sizeof(int), c->s));
-            const float* qsrc = q;
-            if (host_mode == 0) {
+            t.st = (DevStatus*)c->h;  // this call's error bits land in its own status block
+            t.st->err = 0;
+            if (direct) {
+                touch_pages(ids, sizeof(int) * nk);
+                touch_pages(d2, sizeof(float) * nk);
+                touch_pages(xyz, sizeof(float) * 3 * nk);
+                touch_pages(cnt, sizeof(int) * nq);
+                launch_knn(t, q, stride, nq, k, max_sq_threshold(max_dist), ids, d2, xyz, cnt, nullptr, 0, c->s,
+                           /*host_out=*/true);
+                CK(cudaGetLastError());
+                CK(cudaStreamSynchronize(c->s));
+            } else {
                 std::memcpy(c->h + o_q, q, sizeof(float) * nq * stride);
-                CK(cudaMemcpyAsync(c->d + o_q, c->h + o_q, sizeof(float) * nq * stride, cudaMemcpyHostToDevice,
-                                   c->s));
-                qsrc = (const float*)(c->d + o_q);
+                CK(cudaMemcpyAsync(c->d + o_q, c->h + o_q, sizeof(float) * nq * stride, cudaMemcpyHostToDevice, c->s));
+                launch_knn(t, (const float*)(c->d + o_q), stride, nq, k, max_sq_threshold(max_dist),
+                           (int*)(c->d + o_rows), (float*)(c->d + o_d2), xyz ? (float*)(c->d + o_xyz) : nullptr,
+                           cnt ? (int*)(c->d + o_cnt) : nullptr, c->d + o_tmp, bits, c->s);
+                CK(cudaGetLastError());
+                CK(cudaMemcpyAsync(c->h + o_rows, c->d + o_rows, o_q - o_rows, cudaMemcpyDeviceToHost, c->s));
+                CK(cudaStreamSynchronize(c->s));
+                std::memcpy(ids, c->h + o_rows, sizeof(int) * nk);
+                std::memcpy(d2, c->h + o_d2, sizeof(float) * nk);
+                if (xyz) std::memcpy(xyz, c->h + o_xyz, sizeof(float) * 3 * nk);
+                if (cnt) std::memcpy(cnt, c->h + o_cnt, sizeof(int) * nq);
             }
-            launch_knn(t, qsrc, stride, nq, k, max_sq_threshold(max_dist), (int*)(c->d + o_ids),
-                       (float*)(c->d + o_d2), xyz ? (float*)(c->d + o_xyz) : nullptr,
-                       cnt ? (int*)(c->d + o_cnt) : nullptr, c->d + o_tmp, bin_bits_for(nq, k), c->s);
-            CK(cudaGetLastError());
-            CK(cudaMemcpyAsync(c->h, c->d, o_end, cudaMemcpyDeviceToHost, c->s));
-            CK(cudaStreamSynchronize(c->s));
             const DevStatus* hs = (const DevStatus*)c->h;
             if (hs->err & ERR_STACK) throw Internal{"knn: traversal stack overflow"};
             if (hs->err & ERR_LOOP) throw Internal{"knn: loop cap reached"};
-            std::memcpy(ids, c->h + o_ids, sizeof(int) * nk);
-            std::memcpy(d2, c->h + o_d2, sizeof(float) * nk);
-            if (xyz) std::memcpy(xyz, c->h + o_xyz, sizeof(float) * 3 * nk);
-            if (cnt) std::memcpy(cnt, c->h + o_cnt, sizeof(int) * nq);
         } catch (...) {
             give_ctx(c);
             throw;
@@ -888,20 +910,29 @@ struct Tree {
             CK(cudaGetLastError());
             return;
         }
-        // the search reports through the error bits alone
-        zero_fields(offsetof(DevStatus, err), sizeof(int));
-        if (host_mode == 2 || (host_mode == 1 && all_pinned({ids, d2, xyz, cnt}))) {
+        if (direct && k <= KNN_GROUP_MAX && bin_bits_for(nq, k) == 0) {
             // Kernels read the queries and write the results in host memory:
-            // each warp's rows leave as coalesced 16-byte spans, so the
-            // transfer over the chip link overlaps the search instead of
-            // following it as one copy.
-            small.ensure(knn_temp_bytes(nq, k) + 256, stream);
-            launch_knn(dt, q, stride, nq, k, lim, ids, d2, xyz, cnt, small.p, bin_bits_for(nq, k), stream,
-                       /*host_out=*/true);
-            read_status();
-            if (st->err & ERR_STACK) throw Internal{"knn: traversal stack overflow"};
+            // each CTA's rows leave as coalesced 16-byte spans.  (A sorted
+            // batch's rows would leave one by one, and lists in the output rows
+            // would be worked on there: those are staged.)
+            if (!all_pinned({ids, d2, xyz, cnt})) {
+                touch_pages(ids, sizeof(int) * nk);
+                touch_pages(d2, sizeof(float) * nk);
+                touch_pages(xyz, sizeof(float) * 3 * nk);
+                touch_pages(cnt, sizeof(int) * nq);
+            }
+            DevTree t = dt;
+            t.st = host_st;
+            host_st->err = 0;
+            launch_knn(t, q, stride, nq, k, lim, ids, d2, xyz, cnt, nullptr, 0, stream, /*host_out=*/true);
+            CK(cudaGetLastError());
+            CK(cudaStreamSynchronize(stream));
+            if (host_st->err & ERR_STACK) throw Internal{"knn: traversal stack overflow"};
+            if (host_st->err & ERR_LOOP) throw Internal{"device error: loop cap reached;"};
             return;
         }
+        // the search reports through the error bits alone
+        zero_fields(offsetof(DevStatus, err), sizeof(int));
         op.ensure(align_up(sizeof(float) * nq * stride) + align_up(sizeof(int) * nk) + align_up(sizeof(float) * nk) +
                       align_up(sizeof(float) * nk * 3) + align_up(sizeof(int) * nq) + align_up(knn_temp_bytes(nq, k)),
                   stream);
@@ -912,14 +943,8 @@ struct Tree {
         float* dxyz = xyz ? c.take<float>(nk * 3) : nullptr;
         int* dcnt = cnt ? c.take<int>(nq) : nullptr;
         char* temp = c.take<char>(knn_temp_bytes(nq, k));
-        // Mode 1: the kernel reads the (small, in-order) queries straight from
-        // host memory; the results come back by DMA.
-        const float* qsrc = q;
-        if (host_mode == 0) {
-            CK(cudaMemcpyAsync(dq, q, sizeof(float) * nq * stride, cudaMemcpyHostToDevice, stream));
-            qsrc = dq;
-        }
-        launch_knn(dt, qsrc, stride, nq, k, lim, dids, dd2, dxyz, dcnt, temp, bin_bits_for(nq, k), stream);
+        CK(cudaMemcpyAsync(dq, q, sizeof(float) * nq * stride, cudaMemcpyHostToDevice, stream));
+        launch_knn(dt, dq, stride, nq, k, lim, dids, dd2, dxyz, dcnt, temp, bin_bits_for(nq, k), stream);
         CK(cudaMemcpyAsync(ids, dids, sizeof(int) * nk, cudaMemcpyDeviceToHost, stream));
         CK(cudaMemcpyAsync(d2, dd2, sizeof(float) * nk, cudaMemcpyDeviceToHost, stream));
         if (xyz) CK(cudaMemcpyAsync(xyz, dxyz, sizeof(float) * nk * 3, cudaMemcpyDeviceToHost, stream));
@@ -939,42 +964,55 @@ struct Tree {
         *total = 0;
         offsets[0] = 0;
         if (nq == 0) return;
-        reset_counters();
         const int logged = ids != nullptr ? RANGE_LOG : 0;
-        op.ensure(align_up(sizeof(float) * nq * qs) + align_up(sizeof(float) * nq) +
-                      align_up(sizeof(long long) * (nq + 1)) + align_up(range_temp_bytes(nq, logged)),
+        op.ensure(input_bytes((size_t)nq * qs) + input_bytes((size_t)nq * (mode == 1 ? std::max(rstride, 1) : 0)) +
+                      (direct ? 0 : align_up(sizeof(long long) * (nq + 1))) + align_up(range_temp_bytes(nq, logged)) + 512,
                   stream);
         Carver c(op.p);
-        float* dq = c.take<float>((size_t)nq * qs);
-        float* dr = c.take<float>(nq);
-        long long* doffs = c.take<long long>(nq + 1);
+        const size_t rfloats = mode == 1 ? (size_t)(nq - 1) * rstride + 1 : 0;
+        const float* dq = input(q, (size_t)nq * qs, c.take<float>(direct ? 0 : (size_t)nq * qs));
+        const float* dr = mode == 1 ? input(radius, rfloats, c.take<float>(direct ? 0 : rfloats)) : nullptr;
+        long long* doffs = direct ? offsets : c.take<long long>(nq + 1);
         void* temp = c.take<char>(range_temp_bytes(nq, logged));
-        CK(cudaMemcpyAsync(dq, q, sizeof(float) * nq * qs, cudaMemcpyHostToDevice, stream));
-        std::vector<float> rr;
-        if (mode == 1) {
-            rr.resize(nq);
-            for (long long i = 0; i < nq; ++i) rr[i] = radius[i * rstride];
-            CK(cudaMemcpyAsync(dr, rr.data(), sizeof(float) * nq, cudaMemcpyHostToDevice, stream));
-        }
-        launch_range(dt, mode, dq, qs, dr, 1, nq, temp, RANGE_COUNT | logged, doffs, nullptr, nullptr, -1, nullptr,
+        DevTree t = dt;
+        t.st = host_st;
+        host_st->err = 0;
+        if (direct) touch_pages(offsets, sizeof(long long) * (nq + 1));
+        launch_range(t, mode, dq, qs, dr, rstride, nq, temp, RANGE_COUNT | logged, doffs, nullptr, nullptr, -1, nullptr,
                      stream);
-        CK(cudaMemcpyAsync(offsets, doffs, sizeof(long long) * (nq + 1), cudaMemcpyDeviceToHost, stream));
-        read_status();
-        if (st->err & ERR_STACK) throw Internal{"range search: traversal stack overflow"};
+        if (!direct)
+            CK(cudaMemcpyAsync(offsets, doffs, sizeof(long long) * (nq + 1), cudaMemcpyDeviceToHost, stream));
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(stream));
+        if (host_st->err & ERR_STACK) throw Internal{"range search: traversal stack overflow"};
+        if (host_st->err & ERR_LOOP) throw Internal{"device error: loop cap reached;"};
         const long long acc = offsets[nq];
         *total = acc;
         if (acc > capacity || (acc > 0 && ids == nullptr)) throw CapacityFail{"range search: output too small"};
         if (acc == 0) return;
-        bld.ensure(align_up(sizeof(int) * acc) + align_up(sizeof(float) * acc * 3), stream);
-        Carver o(bld.p);
-        int* dids = o.take<int>(acc);
-        float* dxyz = xyz ? o.take<float>(acc * 3) : nullptr;
-        launch_range(dt, mode, dq, qs, dr, 1, nq, temp, logged, doffs, dids, dxyz, -1, nullptr, stream);
-        CK(cudaMemcpyAsync(ids, dids, sizeof(int) * acc, cudaMemcpyDeviceToHost, stream));
-        if (xyz) CK(cudaMemcpyAsync(xyz, dxyz, sizeof(float) * acc * 3, cudaMemcpyDeviceToHost, stream));
-        read_status();
-        if (st->err & ERR_OUTPUT) throw Internal{"range search: hits differ between the count and write passes"};
+        // Few hits are written where the caller wants them; many come by copy.
+        const bool in_place = direct && acc <= RANGE_DIRECT_HITS;
+        int* dids = ids;
+        float* dxyz = xyz;
+        if (in_place) {
+            touch_pages(ids, sizeof(int) * acc);
+            touch_pages(xyz, sizeof(float) * acc * 3);
+        } else {
+            bld.ensure(align_up(sizeof(int) * acc) + align_up(sizeof(float) * acc * 3), stream);
+            Carver o(bld.p);
+            dids = o.take<int>(acc);
+            dxyz = xyz ? o.take<float>(acc * 3) : nullptr;
+        }
+        launch_range(t, mode, dq, qs, dr, rstride, nq, temp, logged, doffs, dids, dxyz, -1, nullptr, stream);
+        if (!in_place) {
+            CK(cudaMemcpyAsync(ids, dids, sizeof(int) * acc, cudaMemcpyDeviceToHost, stream));
+            if (xyz) CK(cudaMemcpyAsync(xyz, dxyz, sizeof(float) * acc * 3, cudaMemcpyDeviceToHost, stream));
+        }
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(stream));
+        if (host_st->err & ERR_OUTPUT) throw Internal{"range search: hits differ between the count and write passes"};
     }
+    static constexpr long long RANGE_DIRECT_HITS = 1 << 18;
 
     // Device-pointer range search, asynchronous on the tree's stream: count
     // pass, device prefix sum into offsets (offsets[nq] = total), write pass.
