@@ -1229,13 +1229,6 @@ int lb_prepare() {
     return n;
 }
 
-__global__ void finish_alloc_kernel(DevStatus* st) {
-    st->free_node_n = max(0, st->free_node_n - st->free_node_taken);
-    st->free_leaf_n = max(0, st->free_leaf_n - st->free_leaf_taken);
-    st->free_node_taken = 0;
-    st->free_leaf_taken = 0;
-}
-
 __global__ void reset_count_kernel(int* c) { *c = 0; }
 
 inline unsigned blocks_for(long long n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -1318,7 +1311,6 @@ void build_subtrees(const DevTree& t, const float4* pts, long long n, const int*
         // Every job fits the local builder: one launch builds them all.
         init_segs_kernel<<<blocks_for(njobs, T), T, 0, s>>>(job_off, job_link, njobs, bs.local_jobs, bs.nseg);
         launch_local(grid(njobs, 4), t, pts, bs.local_jobs, bs.nseg, njobs, fill, s);
-        finish_alloc_kernel<<<1, 1, 0, s>>>(t.st);
         return;
     }
     // Counters: segments of at most SPLIT_MIN points, local jobs.
@@ -1365,7 +1357,6 @@ void build_subtrees(const DevTree& t, const float4* pts, long long n, const int*
                                                                             bs.pts[0], bs.local_jobs, nlocal, (int)ms,
                                                                             fill);
     launch_local(grid(ms, 4), t, bs.pts[0], bs.local_jobs, nlocal, (int)ms, fill, s);
-    finish_alloc_kernel<<<1, 1, 0, s>>>(t.st);
 }
 
 }  // namespace ikdg

@@ -223,6 +223,7 @@ struct Tree {
     // mutation (slow; for tests and debugging).
     bool debug_validate = std::getenv("IKDG_DEBUG_VALIDATE") != nullptr;
     std::string dbg_note;
+    int sm_count = 1;
     int dbg_round = 0;
 
     // ---- lifetime -------------------------------------------------------------
@@ -241,6 +242,7 @@ struct Tree {
             cudaGetLastError();
             pageable = 0;
         }
+        CK(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
         direct = pageable != 0 && std::getenv("IKDG_HOST_STAGING") == nullptr;
         CK(cudaMallocHost(&host_st, sizeof(DevStatus)));
         std::memset(host_st, 0, sizeof(DevStatus));
@@ -378,6 +380,10 @@ struct Tree {
     void read_status() {
         CK(cudaMemcpyAsync(st, st_dev, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream));
         CK(cudaStreamSynchronize(stream));
+        take_status();
+    }
+    // Looks at the status that has arrived in st.
+    void take_status() {
         set_search_start();
         if (st->err & ERR_ANY_INTERNAL) {
             int e = st->err;
@@ -401,11 +407,9 @@ struct Tree {
     void zero_fields(size_t off, size_t bytes) {
         CK(cudaMemsetAsync((char*)st_dev + off, 0, bytes, stream));
     }
-    // Clears the per-call counters (everything but the pool state and removed_n).
+    // Clears the per-call counters.
     void reset_counters() {
-        zero_fields(offsetof(DevStatus, err), offsetof(DevStatus, root_code) - offsetof(DevStatus, err));
-        zero_fields(offsetof(DevStatus, count), 2 * sizeof(long long));
-        zero_fields(offsetof(DevStatus, job_total), sizeof(long long) + 8 * sizeof(int));
+        zero_fields(offsetof(DevStatus, err), offsetof(DevStatus, bad) - offsetof(DevStatus, err));
     }
     void set_status_ll(size_t off, long long v) {
         CK(cudaMemcpyAsync((char*)st_dev + off, &v, sizeof(v), cudaMemcpyHostToDevice, stream));
@@ -448,19 +452,10 @@ struct Tree {
     // ---- rebuild jobs ---------------------------------------------------------------
     Criteria criteria() const { return Criteria{del_param, bal_param, min_size, fill}; }
 
-    // Runs the jobs selected in aux (st->n_jobs on the device, nj here):
-    // gather their valid points (plus overflow points), rebuild, relink and
-    // refit their ancestors.
-    // bound: an upper bound on the jobs selected (the violator count); the
-    // job counts, totals and sizes come back in one status read.
-    // counted: the jobs were selected and counted before the last status read
-    // (launch_select_and_count), which brought their count and sizes back.
-    void run_jobs(int bound, const int4* ovf_leaf, const float4* ovf_pts, int ovf_bound, bool counted = false) {
-        if (!counted) {
-            small.ensure(scan_temp_bytes(bound + 1) + 1024, stream);
-            launch_job_count(dt, aux, st->leaf_top, st->node_top, ovf_leaf, ovf_bound, bound, small.p, stream);
-            read_status();
-        }
+    // Runs the jobs selected in aux (their number and sizes are in st): gather
+    // their valid points (plus overflow points), rebuild, relink and refit their
+    // ancestors.
+    void run_jobs(const int4* ovf_leaf, const float4* ovf_pts, int ovf_bound) {
         const int nj = st->n_jobs;
         if (nj == 0) throw Internal{"violators without a topmost job"};
         if (debug_validate) {
@@ -511,10 +506,7 @@ struct Tree {
                           removed_cap, stream);
         build_subtrees(dt, gathered, total, aux.job_off, aux.job_link, nj, std::max<long long>(max_job, 1), fill, bs,
                        stream);
-        zero_fields(offsetof(DevStatus, n_items), sizeof(int));
-        zero_fields(offsetof(DevStatus, n_viol), sizeof(int));
-        launch_job_finish(dt, aux, nj, stream);
-        zero_fields(offsetof(DevStatus, n_jobs), sizeof(int));
+        launch_job_finish(dt, aux, stream);
         launch_refit(dt, aux, aux.items, &st_dev->n_items, nj, criteria(), stream);
     }
 
@@ -526,50 +518,28 @@ struct Tree {
             launch_refit(dt, aux, aux.items, &st_dev->n_items, bound, criteria(), stream);
             if (debug_validate) check_valid("after the refit of a mutation", /*at_rest=*/false);
         }
-        // The dirty list is consumed: the next update starts a fresh one.
-        zero_fields(offsetof(DevStatus, n_items), sizeof(int));
         // Rebuilding a subtree can unbalance its ancestors; each round moves
-        // the violations up, so a few rounds settle the tree.  The root
-        // snapshot is taken before every status read: when the read finds no
-        // violators it is already the final status of the call.
-        bool settled = false;
+        // the violations up, so a few rounds settle the tree.  One launch after
+        // each refit takes the root's snapshot and, where there are violators,
+        // selects and sizes the rebuild jobs, so one wait brings everything:
+        // without violators it is the final status of the call.
         for (int round = 0; round < 8; ++round) {
-            launch_snapshot_root(dt, stream);
-            // The first round selects and counts its rebuild jobs before the
-            // status read (nothing happens on the device when there are no
-            // violators), so one read brings the violators, the jobs and
-            // their sizes.  After a mutation no build ran since the last
-            // read, so the host's pool tops bound the leaf and node scans;
-            // later rounds, and the call after rebuild_all's build, read
-            // first.
-            const bool ahead = round == 0 && refit_first;
-            if (ahead) launch_select_and_count(dt, aux, st->leaf_top, st->node_top, ovf_leaf, ovf_bound, stream);
-            read_status();
-            int nv = st->n_viol;
-            if (nv == 0) {
-                settled = true;
-                break;
-            }
-            if (round == 7) {
-                // Still unsettled: clear the flags; the next call retries.
-                launch_clear_viol(dt, aux, nv, stream);
-                break;
-            }
-            if (!ahead) launch_select_jobs(dt, aux, nv, stream);
+            const bool first = round == 0;
+            // unsettled after seven rounds: clear the flags; the next call retries
+            const bool select = round < 7;
+            // (two blocks per SM fit; the device's own counts bound its loops)
+            const long long work = (long long)st->leaf_top + st->node_top;
+            const int blocks = (int)std::min<long long>(2 * sm_count, std::max(1ll, (work + 1023) / 1024));
+            CK(launch_settle(dt, aux, first ? ovf_leaf : nullptr, first ? ovf_bound : 0, select, st, blocks, stream));
+            CK(cudaStreamSynchronize(stream));
+            take_status();
+            if (st->n_viol == 0 || !select) break;
             dbg_round = round;
-            // at most nv jobs: run_jobs reads the job count with its own sizes
-            run_jobs(nv, round == 0 ? ovf_leaf : nullptr, round == 0 ? ovf_pts : nullptr, round == 0 ? ovf_bound : 0,
-                     ahead);
-            zero_fields(offsetof(DevStatus, n_items), sizeof(int));
+            run_jobs(first ? ovf_leaf : nullptr, first ? ovf_pts : nullptr, first ? ovf_bound : 0);
             if (debug_validate) {
                 read_status();
                 if (st->n_viol == 0) check_valid("after a rebuild round");
             }
-        }
-        if (!settled) {
-            zero_fields(offsetof(DevStatus, n_viol), sizeof(int));
-            launch_snapshot_root(dt, stream);
-            read_status();
         }
         if (st->err & ERR_STACK) throw Internal{"tree deeper than the traversal stack"};
         if (debug_validate) check_valid("end of update");
@@ -678,10 +648,9 @@ struct Tree {
         next_id += n;  // taken even if a later step fails: ids are never reused
         long long a = 0;
         while (a < n) {
-            launch_set_ll((long long*)((char*)st_dev + offsetof(DevStatus, count)), n, stream);
+            if (a > 0) launch_set_ll((long long*)((char*)st_dev + offsetof(DevStatus, count)), n, stream);
             if (debug_validate) check_valid("start of a downsampling sub-batch");
             launch_ds_search(dt, n, ds_size, a, d, n_bound, stream);
-            zero_fields(offsetof(DevStatus, n_ins), sizeof(int));
             launch_ds_fold(dt, aux, n, a, first_id, d, n_bound, stream);
             if (debug_validate) {
                 read_status();
@@ -1200,10 +1169,8 @@ struct Tree {
     void rebuild_all() {
         if (st->root_code == 0) return;
         reset_counters();
-        launch_select_root_job(dt, aux, stream);
+        launch_select_root(dt, aux, stream);
         set_top((long long)st->root_slots - st->root_deleted);
-        run_jobs(1, nullptr, nullptr, 0);
-        // run_jobs already refit the root's parent (the sentinel: nothing to do)
         finish_update(nullptr, nullptr, 0, /*refit_first=*/false);
     }
 

@@ -61,7 +61,8 @@ __host__ __device__ inline bool code_is_leaf(int c) { return c < 0; }
 __host__ __device__ inline int code_leaf(int c) { return -c - 1; }
 __host__ __device__ inline int leaf_code(int l) { return -(l + 1); }
 
-// Device-resident counters, read back by the host after each API call.
+// Device-resident counters, read back by the host after each API call.  The
+// fields from `err` to `dbg` are cleared at the start of a call.
 struct DevStatus {
     int node_top;         // bump pointer of the node pool
     int leaf_top;         // bump pointer of the leaf pool
@@ -69,6 +70,11 @@ struct DevStatus {
     int free_leaf_n;
     int free_node_taken;  // pops during the current build
     int free_leaf_taken;
+    int root_code;        // snapshot of the sentinel's left child
+    int root_slots;       // size(): stored slots, deleted ones included
+    int root_deleted;     // deleted slots; validnum() = slots - deleted
+    int root_height;
+    long long removed_n;  // deleted points dropped by rebuilds, not yet drained
     int err;              // ERR_* bits
     int n_items;          // refit start codes queued
     int n_jobs;           // rebuild jobs selected
@@ -77,14 +83,10 @@ struct DevStatus {
     int n_ins;            // downsampling winners to insert
     int n_groups;         // downsampling voxel groups
     int max_job;          // largest rebuild job (points)
-    int root_code;        // snapshot of the sentinel's left child
-    int root_slots;       // size(): stored slots, deleted ones included
-    int root_deleted;     // deleted slots; validnum() = slots - deleted
-    int root_height;
     long long count;      // generic result counter
     long long count2;
-    long long removed_n;  // deleted points dropped by rebuilds, not yet drained
     long long job_total;  // points gathered for rebuild jobs
+    unsigned barrier;     // arrivals at settle_kernel's grid barriers
     int dbg[8];           // details of the first internal error (diagnostics)
     long long bad;        // structural violations found by the validator
 };

@@ -29,7 +29,8 @@ bool radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32
 // (job j = [job_off[j], job_off[j+1])), each as {x, y, z, id}.  Every job
 // becomes a balanced subtree of leaves holding at most `fill` points, split at
 // the median of the longest AABB axis, and is linked into the child slot
-// `job_link[j]` (= parent * 2 + side) together with its AABB and counts.
+// `job_link[j]` (= parent * 2 + side) together with its AABB and counts.  The pools'
+// free stacks are settled by the snapshot or job-finish kernel that follows.
 // Open segments of the large splitter at one level.
 struct SplitLevel {
     int4* seg;       // {s, e, link, -}

@@ -39,23 +39,16 @@ void launch_route_append(const DevTree& t, const UpdateAux& a, const float4* pts
 // clears the dirty flags of the listed leaves.
 void launch_refit(const DevTree& t, const UpdateAux& a, const int* items, const int* n_items, int max_items,
                   const Criteria& c, cudaStream_t s);
-// Select topmost violators as rebuild jobs (st->n_jobs = job count).
-void launch_select_jobs(const DevTree& t, const UpdateAux& a, int max_viol, cudaStream_t s);
-// Clears the criterion flags of the recorded violators without selecting jobs.
-void launch_clear_viol(const DevTree& t, const UpdateAux& a, int max_viol, cudaStream_t s);
-// Count / gather the valid points of every job (plus overflow points).
-void launch_job_count(const DevTree& t, const UpdateAux& a, int leaf_top, int node_top, const int4* ovf_leaf,
-                      int max_ovf, int max_jobs, void* scan_temp, cudaStream_t s);
-// Job selection and counting launched before the host knows the violator
-// count (st->n_viol, st->n_jobs read on the device; nothing happens when they
-// are zero): one status read then returns the violators, the jobs and their
-// sizes.  leaf_top / node_top must be current (no build since the last read).
-void launch_select_and_count(const DevTree& t, const UpdateAux& a, int leaf_top, int node_top, const int4* ovf_leaf,
-                             int max_ovf, cudaStream_t s);
+// After a refit: root snapshot, selection of the topmost violators as rebuild
+// jobs, their sizes; the status goes to `host` (pinned).  `blocks`: at most two
+// per SM (cooperative launch).
+cudaError_t launch_settle(const DevTree& t, const UpdateAux& a, const int4* ovf_leaf, int max_ovf, bool select,
+                          DevStatus* host, int blocks, cudaStream_t s);
+// Gathers the valid points of every job (plus overflow points).
 void launch_job_gather(const DevTree& t, const UpdateAux& a, int leaf_top, int node_top, const int4* ovf_leaf,
                        const float4* ovf_pts, int max_ovf, float4* out, float4* removed, long long removed_cap,
                        cudaStream_t s);
-void launch_job_finish(const DevTree& t, const UpdateAux& a, int max_jobs, cudaStream_t s);
+void launch_job_finish(const DevTree& t, const UpdateAux& a, cudaStream_t s);
 // Delete every valid point inside each box; `flags` = F_DEL or F_DEL|F_DSDEL.
 void launch_delete_boxes(const DevTree& t, const UpdateAux& a, const float* boxes, long long m, uint32_t flags,
                          long long* total, cudaStream_t s);
@@ -86,8 +79,8 @@ void launch_stored_ids(const DevTree& t, int* out, long long cap, long long* cou
 // (between calls) also requires cleared violation / job tags and leaves within
 // their slots.
 void launch_validate(const DevTree& t, const UpdateAux& a, bool at_rest, long long* bad, cudaStream_t s);
-// Makes the whole tree the single rebuild job (st->n_jobs = 1).
-void launch_select_root_job(const DevTree& t, const UpdateAux& a, cudaStream_t s);
+// Makes the whole tree the only violator.
+void launch_select_root(const DevTree& t, const UpdateAux& a, cudaStream_t s);
 
 // ---- voxel downsampling ----------------------------------------------------
 struct DsScratch {

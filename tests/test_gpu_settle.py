@@ -1,0 +1,46 @@
+"""Mutations that end without a rebuild, with one job, with many jobs, with the
+whole tree as the job, and with overflow points, on trees of one leaf up to more
+leaves than the settling launch has threads.  The structure is validated and the
+stored points equal the model's."""
+import numpy as np
+import pytest
+
+import spec
+
+pytestmark = pytest.mark.gpu
+
+
+def same(tree, ref, rng):
+    assert tree.validate() == 0 and tree.validnum() == ref.validnum()
+    if ref.validnum() == 0:
+        return
+    q = rng.uniform(-55, 55, (12, 3)).astype(np.float32)
+    ids, d2, _, _ = tree.knn(q, 6)
+    rid, rd2 = ref.knn(q, 6)
+    assert np.array_equal(ids, rid) and np.array_equal(d2, rd2)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 2000, 40000, 700001])
+def test_edit_sequences(ikdg_mod, n):
+    rng = np.random.default_rng(n)
+    pts = rng.uniform(-50, 50, (n, 3)).astype(np.float32)
+    tree, ref = ikdg_mod.KDTree(0.3, 0.6, 0.5), spec.SpecTree(0.5)
+    for t in (tree, ref):
+        t.Build(pts)
+    # one spot takes many points: full buckets overflow into a rebuild
+    steps = [rng.uniform(49, 50, (600, 3)), rng.uniform(-50, 50, (3, 3)), rng.uniform(-50, 50, (n // 8 + 1, 3))]
+    for add in steps:
+        for t in (tree, ref):
+            t.Add_Points(add.astype(np.float32), False)
+        same(tree, ref, rng)
+    # nothing hit; a few points; scattered slabs (many jobs); all that is left
+    slabs = np.array([[x, -50, -50, x + 2.5, 50, 50] for x in range(-48, 48, 6)], np.float32)
+    for boxes in (np.array([[60, 60, 60, 61, 61, 61]], np.float32), np.array([[0, 0, 0, 3, 3, 3]], np.float32), slabs,
+                  np.array([[-60, -60, -60, 60, 60, 60]], np.float32)):
+        assert tree.Delete_Point_Boxes(boxes) == ref.Delete_Point_Boxes(boxes)
+        same(tree, ref, rng)
+    for t in (tree, ref):
+        t.Add_Points(pts[:100], False)
+    tree.rebuild()
+    same(tree, ref, rng)
+    tree.close()
