@@ -267,6 +267,7 @@ struct Tree {
         free_array(dt.free_leaf);
         free_array(aux.pend);
         free_array(aux.arrive);
+        free_array(aux.mail);
         free_array(aux.viol_flag);
         free_array(aux.job_of_node);
         free_array(aux.node_job);
@@ -314,6 +315,7 @@ struct Tree {
             grow_array(dt.free_node, old_n, new_n, -1, stream);
             grow_array(aux.pend, old_n, new_n, 0, stream);
             grow_array(aux.arrive, old_n, new_n, 0, stream);
+            grow_array(aux.mail, (size_t)old_n * 4, (size_t)new_n * 4, 0, stream);
             grow_array(aux.viol_flag, old_n, new_n, 0, stream);
             grow_array(aux.job_of_node, old_n, new_n, 0xff, stream);
             grow_array(aux.node_job, old_n, new_n, 0xff, stream);

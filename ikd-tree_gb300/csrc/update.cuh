@@ -7,15 +7,16 @@ namespace ikdg {
 // Per-node / per-leaf bookkeeping arrays used by mutations (sized with the
 // pools; all entries idle at 0 or -1 between calls).
 struct UpdateAux {
-    int* pend;          // [node_cap] refit: number of dirty children    (0)
-    int* arrive;        // [node_cap] refit: arrivals so far            (0)
+    int* pend;          // [node_cap] refit: number of changing children (0)
+    int* arrive;        // [node_cap] refit: the first child's height    (0)
+    uint4* mail;        // [node_cap * 4] refit: per side, box and counts      (0)
     int* viol_flag;     // [node_cap] criterion violated                (0)
     int* job_of_node;   // [node_cap] job rooted here                   (-1)
     int* node_job;      // [node_cap] scratch: job containing the node
     int* dirty_flag;    // [leaf_cap] leaf queued for refit             (0)
     int* job_of_leaf;   // [leaf_cap] job rooted at this leaf           (-1)
     int* leaf_job;      // [leaf_cap] scratch: job containing the leaf
-    int* items;         // [leaf_cap + node_cap] refit start codes
+    int* items;         // [leaf_cap + node_cap] refit start: leaf codes, links of subtrees
     int* viol;          // [leaf_cap + node_cap] violator codes
     int* jobs;          // [leaf_cap + node_cap] job root codes
     int* job_link;      // [leaf_cap + node_cap]

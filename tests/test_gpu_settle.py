@@ -44,3 +44,24 @@ def test_edit_sequences(ikdg_mod, n):
     tree.rebuild()
     same(tree, ref, rng)
     tree.close()
+
+
+@pytest.mark.parametrize("hit", [1, 7, 400, 9000, 30000])
+def test_refit_meetings(ikdg_mod, hit):
+    """From one dirty bucket up to every bucket of the map: walks that meet at no
+    node, at the upper nodes, at every node; twice on the same nodes."""
+    rng = np.random.default_rng(hit)
+    pts = rng.uniform(-50, 50, (30000, 3)).astype(np.float32)
+    tree, ref = ikdg_mod.KDTree(0.9, 0.95, 0.5), spec.SpecTree(0.5)  # (nothing is rebuilt but full buckets)
+    for t in (tree, ref):
+        t.Build(pts)
+    for seed in range(2):
+        sel = rng.permutation(len(pts))[:hit]
+        for t in (tree, ref):
+            t.Delete_Points(pts[sel])
+        same(tree, ref, rng)
+        assert np.array_equal(np.asarray(tree.tree_range()).reshape(-1), ref.tree_range())
+        for t in (tree, ref):
+            t.Add_Points(pts[sel], False)
+        same(tree, ref, rng)
+    tree.close()
