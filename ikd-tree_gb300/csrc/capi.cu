@@ -701,10 +701,11 @@ struct Tree {
         if (m == 0 || st->root_code == 0) return 0;
         reset_counters();
         op.ensure(align_up(sizeof(float) * m * 6), stream);
-        float* raw = (float*)op.p;  // (every block reads its box several times: a copy in HBM)
+        float* raw = (float*)op.p;  // (every warp of a box reads it: a copy in HBM)
         CK(cudaMemcpyAsync(raw, boxes, sizeof(float) * m * 6, cudaMemcpyHostToDevice, stream));
-        launch_delete_boxes(dt, aux, raw, m, F_DEL, (long long*)((char*)st_dev + offsetof(DevStatus, count)),
-                            stream);
+        // (the root's place in the top record leaves it 4, 2 or all 8 slots)
+        launch_delete_boxes(dt, aux, raw, m, top_pos == 2 ? 2 : top_pos == 4 ? 1 : 3, F_DEL,
+                            (long long*)((char*)st_dev + offsetof(DevStatus, count)), stream);
         // The rebuild rounds leave `count` alone: its value arrives with the
         // status reads of finish_update.
         finish_update(nullptr, nullptr, 0);

@@ -50,9 +50,10 @@ void launch_job_gather(const DevTree& t, const UpdateAux& a, int leaf_top, int n
                        const float4* ovf_pts, int max_ovf, float4* out, float4* removed, long long removed_cap,
                        cudaStream_t s);
 void launch_job_finish(const DevTree& t, const UpdateAux& a, cudaStream_t s);
-// Delete every valid point inside each box; `flags` = F_DEL or F_DEL|F_DSDEL.
-void launch_delete_boxes(const DevTree& t, const UpdateAux& a, const float* boxes, long long m, uint32_t flags,
-                         long long* total, cudaStream_t s);
+// Delete every valid point inside each box; `flags` = F_DEL or F_DEL|F_DSDEL;
+// top_bits = log2 of the slots the record at t.start may use.
+void launch_delete_boxes(const DevTree& t, const UpdateAux& a, const float* boxes, long long m, int top_bits,
+                         uint32_t flags, long long* total, cudaStream_t s);
 void launch_delete_points(const DevTree& t, const UpdateAux& a, const float* pts, int stride, long long n,
                           cudaStream_t s);
 void launch_add_boxes(const DevTree& t, const UpdateAux& a, const float* boxes, long long m, cudaStream_t s);

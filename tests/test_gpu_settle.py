@@ -65,3 +65,54 @@ def test_refit_meetings(ikdg_mod, hit):
             t.Add_Points(pts[sel], False)
         same(tree, ref, rng)
     tree.close()
+
+
+@pytest.mark.parametrize("n", [1, 5, 40, 300, 5000, 120000])
+@pytest.mark.parametrize("dup", [False, True])
+def test_box_and_point_deletion_walks(ikdg_mod, n, dup):
+    """One to many boxes a call (the deletion splits the tree over more warps the fewer
+    there are), covering all, touching faces, far off, overlapping; point deletions
+    with several stored points within the match distance."""
+    rng = np.random.default_rng(n)
+    pts = rng.uniform(-50, 50, (n, 3)).astype(np.float32)
+    if dup:
+        pts[n // 2:] = pts[: n - n // 2]  # pairs of equal points
+    tree, ref = ikdg_mod.KDTree(0.5, 0.6, 0.5), spec.SpecTree(0.5)
+    for t in (tree, ref):
+        t.Build(pts)
+    lo = rng.uniform(-55, 50, (1500, 3))
+    many = np.c_[lo, lo + rng.uniform(0, 4, (1500, 3))].astype(np.float32)
+    face = np.r_[pts[0], pts[0] + 3][None].astype(np.float32)  # half-open: pts[0] is inside
+    face2 = np.r_[pts[n // 3] - 3, pts[n // 3]][None].astype(np.float32)  # and outside here
+    for boxes in (face, face2, many[:3], many[:130], many, np.array([[-60, -60, -60, 0, 60, 60]], np.float32)):
+        assert tree.Delete_Point_Boxes(boxes) == ref.Delete_Point_Boxes(boxes)
+        same(tree, ref, rng)
+    for t in (tree, ref):
+        t.Add_Points(pts[: n // 2], False)
+    gone = np.r_[pts[:: max(1, n // 200)], pts[:3] + 3e-7, rng.uniform(-50, 50, (20, 3)).astype(np.float32)]
+    for t in (tree, ref):
+        t.Delete_Points(gone.astype(np.float32))
+    assert tree.validate() == 0 and tree.validnum() == ref.validnum()
+    every = np.array([[-60, -60, -60, 60, 60, 60]], np.float32)
+    assert tree.Delete_Point_Boxes(every) == ref.Delete_Point_Boxes(every)
+    assert tree.validnum() == 0 and tree.validate() == 0
+    tree.close()
+
+
+@pytest.mark.parametrize("spread", [0.05, 0.6, 6.0])
+def test_voxel_search_teams(ikdg_mod, monkeypatch, spread):
+    """Downsampling insertion where voxels hold many, a few and no stored points, with
+    and without room for the pair list."""
+    rng = np.random.default_rng(3)
+    pts = rng.uniform(-4, 4, (9001, 3)).astype(np.float32)
+    for cap in (None, "16"):
+        if cap:
+            monkeypatch.setenv("IKDG_DS_PAIR_CAP", cap)
+        tree, ref = ikdg_mod.KDTree(0.5, 0.6, 0.5), spec.SpecTree(0.5)
+        for t in (tree, ref):
+            t.Build(pts)
+        for seed in range(2):
+            add = (rng.normal(0, spread, (301, 3))).astype(np.float32)
+            assert tree.Add_Points(add, True) == ref.Add_Points(add, True)
+            same(tree, ref, rng)
+        tree.close()
