@@ -33,8 +33,9 @@ namespace {
 
 __device__ __forceinline__ float coord4(const float4& p, int a) { return a == 0 ? p.x : (a == 1 ? p.y : p.z); }
 
-__global__ void init_segs_kernel(const int* __restrict__ job_off, const int* __restrict__ job_link, int njobs,
+__global__ void init_segs_kernel(const int* job_off, const int* job_link, int njobs,
                                  int4* segs, int* nseg) {
+    chain_begin();
     int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j == 0) nseg[0] = njobs;
     if (j >= njobs) return;
@@ -209,9 +210,10 @@ __device__ __forceinline__ void subtree_counts(int n, int fill, int* nodes, int*
 }
 
 template <int MAXN, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 4) local_build_kernel(DevTree t, const float4* __restrict__ pts,
-                                                                 const int4* __restrict__ jobs, const int* njobs,
+__global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 4) local_build_kernel(DevTree t, const float4* pts,
+                                                                 const int4* jobs, const int* njobs,
                                                                  int max_jobs, int fill) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char lb_raw[];
     constexpr int PPT = MAXN / THREADS;
     constexpr int SEGS = THREADS;
@@ -539,11 +541,12 @@ struct FinShared {
     int nopen, node, axis, digit, rank;
 };
 
-__global__ void __launch_bounds__(FIN_THREADS, 2) finish_split_kernel(DevTree t, const float4* __restrict__ src,
-                                                                      const int4* __restrict__ segs, const int* nseg,
+__global__ void __launch_bounds__(FIN_THREADS, 2) finish_split_kernel(DevTree t, const float4* src,
+                                                                      const int4* segs, const int* nseg,
                                                                       int max_segs, float4* __restrict__ out,
                                                                       int4* __restrict__ local_jobs, int* nlocal,
                                                                       int max_local, int fill) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char fin_raw[];
     FinShared& sm = *reinterpret_cast<FinShared*>(fin_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -801,12 +804,13 @@ __device__ __forceinline__ void split_box_reset(uint32_t* box) {
 
 // Jobs above SPLIT_MIN points open the splitter's first level; the others go to
 // the small list, their points copied to `exits` (a block per job).
-__global__ void __launch_bounds__(SPLIT_THREADS) split_open_kernel(const float4* __restrict__ pts,
-                                                                   const int* __restrict__ job_off,
-                                                                   const int* __restrict__ job_link, int njobs,
+__global__ void __launch_bounds__(SPLIT_THREADS) split_open_kernel(const float4* pts,
+                                                                   const int* job_off,
+                                                                   const int* job_link, int njobs,
                                                                    SplitLevel lv, int cap, float4* __restrict__ exits,
                                                                    int4* __restrict__ small, int* nsmall, int max_small,
                                                                    DevStatus* st) {
+    chain_begin();
     __shared__ int big;
     for (int j = blockIdx.x; j < njobs; j += gridDim.x) {
         const int s = job_off[j], e = job_off[j + 1];
@@ -849,8 +853,9 @@ __device__ __forceinline__ void split_flush(uint32_t* sm, const uint32_t* b) {
     }
 }
 
-__global__ void __launch_bounds__(SPLIT_THREADS) split_box_kernel(const float4* __restrict__ pts, SplitLevel lv,
+__global__ void __launch_bounds__(SPLIT_THREADS) split_box_kernel(const float4* pts, SplitLevel lv,
                                                                   int cap, unsigned tiles) {
+    chain_begin();
     __shared__ uint32_t sm[6];
     const int q = (int)(blockIdx.x / tiles), tile = (int)(blockIdx.x % tiles);
     if (q >= min(*lv.n, cap)) return;
@@ -868,8 +873,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_box_kernel(const float4* 
     else if (threadIdx.x < 6) atomicMax(lv.box + 6 * q + threadIdx.x, sm[threadIdx.x]);
 }
 
-__global__ void __launch_bounds__(SPLIT_THREADS) split_hist_kernel(const float4* __restrict__ pts, SplitLevel lv,
+__global__ void __launch_bounds__(SPLIT_THREADS) split_hist_kernel(const float4* pts, SplitLevel lv,
                                                                    int cap, unsigned tiles, int* __restrict__ hist) {
+    chain_begin();
     __shared__ int h[SPLIT_BINS];
     const int q = (int)(blockIdx.x / tiles), tile = (int)(blockIdx.x % tiles);
     if (q >= min(*lv.n, cap)) return;
@@ -895,6 +901,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_hist_kernel(const float4*
 // The bins are left zero for the next level.
 __global__ void __launch_bounds__(SPLIT_THREADS) split_pick_kernel(SplitLevel lv, SplitLevel nx, int cap,
                                                                    int* __restrict__ hist, int2* __restrict__ pick) {
+    chain_begin();
     __shared__ uint32_t wsum[SPLIT_THREADS / 32], tot;
     const int q = blockIdx.x;
     if (q == 0 && threadIdx.x == 0) *nx.n = 0;  // select fills it
@@ -926,11 +933,12 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_pick_kernel(SplitLevel lv
     }
 }
 
-__global__ void __launch_bounds__(SPLIT_THREADS) split_classify_kernel(const float4* __restrict__ pts, SplitLevel lv,
+__global__ void __launch_bounds__(SPLIT_THREADS) split_classify_kernel(const float4* pts, SplitLevel lv,
                                                                        int cap, unsigned tiles,
-                                                                       const int2* __restrict__ pick,
+                                                                       const int2* pick,
                                                                        int* __restrict__ tile_left,
                                                                        uint2* __restrict__ cand) {
+    chain_begin();
     __shared__ int less;
     const int q = (int)(blockIdx.x / tiles), tile = (int)(blockIdx.x % tiles);
     if (q >= min(*lv.n, cap)) return;
@@ -1015,12 +1023,13 @@ __device__ __forceinline__ SplitDigit split_digit(int n, int rank, int* hist, Sp
 
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) split_select_kernel(DevTree t, SplitLevel lv, SplitLevel nx, int cap,
-                                                                     const int2* __restrict__ pick,
+                                                                     const int2* pick,
                                                                      int* __restrict__ tile_left,
-                                                                     const uint2* __restrict__ cand,
+                                                                     const uint2* cand,
                                                                      uint2* __restrict__ thr, int2* __restrict__ kids,
                                                                      int4* __restrict__ small, int* nsmall, int max_small,
                                                                      int fill) {
+    chain_begin();
     __shared__ uint2 cache[SPLIT_CACHE];
     __shared__ int hist[256];
     __shared__ SplitDigit sd;
@@ -1132,13 +1141,14 @@ __global__ void __launch_bounds__(THREADS) split_select_kernel(DevTree t, SplitL
 
 // Points before (v, p) go left, the others right, both in order: to `dst`, or to
 // `exits` where the child leaves the splitter.
-__global__ void __launch_bounds__(SPLIT_THREADS) split_scatter_kernel(const float4* __restrict__ src, SplitLevel lv,
+__global__ void __launch_bounds__(SPLIT_THREADS) split_scatter_kernel(const float4* src, SplitLevel lv,
                                                                       SplitLevel nx, int cap, unsigned tiles,
-                                                                      const int* __restrict__ tile_left,
-                                                                      const uint2* __restrict__ thr,
-                                                                      const int2* __restrict__ kids,
+                                                                      const int* tile_left,
+                                                                      const uint2* thr,
+                                                                      const int2* kids,
                                                                       float4* __restrict__ dst,
                                                                       float4* __restrict__ exits) {
+    chain_begin();
     constexpr int WARPS = SPLIT_THREADS / 32, WARP_PTS = SPLIT_TILE / WARPS;
     __shared__ uint32_t sm[12];
     __shared__ int wleft[WARPS];
@@ -1206,7 +1216,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_scatter_kernel(const floa
 
 void launch_local(unsigned grid, const DevTree& t, const float4* pts, const int4* jobs, const int* njobs, int max_jobs,
                   int fill, cudaStream_t s) {
-    local_build_kernel<LB_SMALL, 256><<<grid, 256, sizeof(LbShared<LB_SMALL, 256>), s>>>(t, pts, jobs, njobs, max_jobs,
+    launch_chain(local_build_kernel<LB_SMALL, 256>, grid, 256, sizeof(LbShared<LB_SMALL, 256>), s, t, pts, jobs, njobs, max_jobs,
                                                                                        fill);
 }
 
@@ -1229,7 +1239,7 @@ int lb_prepare() {
     return n;
 }
 
-__global__ void reset_count_kernel(int* c) { *c = 0; }
+__global__ void reset_count_kernel(int* c) { chain_begin(); *c = 0; }
 
 inline unsigned blocks_for(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
@@ -1309,7 +1319,7 @@ void build_subtrees(const DevTree& t, const float4* pts, long long n, const int*
     auto grid = [&](long long jobs, long long per_sm) { return (unsigned)std::min(jobs, per_sm * sms); };
     if (max_job <= LB_SMALL) {
         // Every job fits the local builder: one launch builds them all.
-        init_segs_kernel<<<blocks_for(njobs, T), T, 0, s>>>(job_off, job_link, njobs, bs.local_jobs, bs.nseg);
+        launch_chain(init_segs_kernel, blocks_for(njobs, T), T, 0, s, job_off, job_link, njobs, bs.local_jobs, bs.nseg);
         launch_local(grid(njobs, 4), t, pts, bs.local_jobs, bs.nseg, njobs, fill, s);
         return;
     }
@@ -1318,14 +1328,14 @@ void build_subtrees(const DevTree& t, const float4* pts, long long n, const int*
     cudaMemsetAsync(bs.nseg, 0, 2 * sizeof(int), s);
     const float4* small_pts = bs.pts[2];
     if (max_job <= SPLIT_MIN) {
-        init_segs_kernel<<<blocks_for(njobs, T), T, 0, s>>>(job_off, job_link, njobs, bs.small, nsmall);
+        launch_chain(init_segs_kernel, blocks_for(njobs, T), T, 0, s, job_off, job_link, njobs, bs.small, nsmall);
         small_pts = pts;
     } else {
         // Large segments, one level per round, until all of them are small.
         const int cap = (int)max_split_bound(nn);
-        reset_count_kernel<<<1, 1, 0, s>>>(bs.split[0].n);
+        launch_chain(reset_count_kernel, 1, 1, 0, s, bs.split[0].n);
         cudaMemsetAsync(bs.hist, 0, sizeof(int) * SPLIT_BINS * (size_t)cap, s);
-        split_open_kernel<<<grid(njobs, 8), SPLIT_THREADS, 0, s>>>(pts, job_off, job_link, njobs, bs.split[0], cap,
+        launch_chain(split_open_kernel, grid(njobs, 8), SPLIT_THREADS, 0, s, pts, job_off, job_link, njobs, bs.split[0], cap,
                                                                    bs.pts[2], bs.small, nsmall, (int)ms, t.st);
         long long segs = std::min<long long>(njobs, cap), size = max_job;
         for (int lv = 0; size > SPLIT_MIN; ++lv) {
@@ -1334,26 +1344,26 @@ void build_subtrees(const DevTree& t, const float4* pts, long long n, const int*
             float4* dst = bs.pts[lv & 1];
             const unsigned tiles = (unsigned)((size + SPLIT_TILE - 1) / SPLIT_TILE);
             const unsigned blocks = tiles * (unsigned)segs;
-            if (lv == 0) split_box_kernel<<<blocks, SPLIT_THREADS, 0, s>>>(src, cur, cap, tiles);
-            split_hist_kernel<<<blocks, SPLIT_THREADS, 0, s>>>(src, cur, cap, tiles, bs.hist);
-            split_pick_kernel<<<(unsigned)segs, SPLIT_THREADS, 0, s>>>(cur, nx, cap, bs.hist, bs.pick);
-            split_classify_kernel<<<blocks, SPLIT_THREADS, 0, s>>>(src, cur, cap, tiles, bs.pick, bs.tile_left, bs.cand);
+            if (lv == 0) launch_chain(split_box_kernel, blocks, SPLIT_THREADS, 0, s, src, cur, cap, tiles);
+            launch_chain(split_hist_kernel, blocks, SPLIT_THREADS, 0, s, src, cur, cap, tiles, bs.hist);
+            launch_chain(split_pick_kernel, (unsigned)segs, SPLIT_THREADS, 0, s, cur, nx, cap, bs.hist, bs.pick);
+            launch_chain(split_classify_kernel, blocks, SPLIT_THREADS, 0, s, src, cur, cap, tiles, bs.pick, bs.tile_left, bs.cand);
             // few segments have many candidates each
             if (segs <= 64)
-                split_select_kernel<1024><<<(unsigned)segs, 1024, 0, s>>>(t, cur, nx, cap, bs.pick, bs.tile_left, bs.cand,
+                launch_chain(split_select_kernel<1024>, (unsigned)segs, 1024, 0, s, t, cur, nx, cap, bs.pick, bs.tile_left, bs.cand,
                                                                          bs.thr, bs.kids, bs.small, nsmall, (int)ms,
                                                                          fill);
             else
-                split_select_kernel<256><<<(unsigned)segs, 256, 0, s>>>(t, cur, nx, cap, bs.pick, bs.tile_left, bs.cand,
+                launch_chain(split_select_kernel<256>, (unsigned)segs, 256, 0, s, t, cur, nx, cap, bs.pick, bs.tile_left, bs.cand,
                                                                        bs.thr, bs.kids, bs.small, nsmall, (int)ms,
                                                                        fill);
-            split_scatter_kernel<<<blocks, SPLIT_THREADS, 0, s>>>(src, cur, nx, cap, tiles, bs.tile_left, bs.thr, bs.kids,
+            launch_chain(split_scatter_kernel, blocks, SPLIT_THREADS, 0, s, src, cur, nx, cap, tiles, bs.tile_left, bs.thr, bs.kids,
                                                                   dst, bs.pts[2]);
             segs = std::min<long long>(2 * segs, cap);
             size -= size / 2;
         }
     }
-    finish_split_kernel<<<grid(ms, 2), FIN_THREADS, sizeof(FinShared), s>>>(t, small_pts, bs.small, nsmall, (int)ms,
+    launch_chain(finish_split_kernel, grid(ms, 2), FIN_THREADS, sizeof(FinShared), s, t, small_pts, bs.small, nsmall, (int)ms,
                                                                             bs.pts[0], bs.local_jobs, nlocal, (int)ms,
                                                                             fill);
     launch_local(grid(ms, 4), t, bs.pts[0], bs.local_jobs, nlocal, (int)ms, fill, s);

@@ -1,17 +1,57 @@
 // Host-side launchers shared between the translation units of libikdg.
 #pragma once
 #include <cuda_runtime.h>
+
+#include <utility>
 #include <stdint.h>
 
 #include "common.cuh"
 
 namespace ikdg {
 
+// A mutation or a build is a chain of short launches in one stream, each needing the
+// one before.  launch_chain lets a kernel's blocks come up while its predecessor
+// drains (programmatic stream serialization); every kernel launched so calls
+// chain_begin first, which waits until all earlier work of the stream is complete and
+// visible, then lets the next one come up.  What
+// the chain writes is read with plain or L2 loads, never as read-only data
+// (const __restrict__, __ldg): the reader is up while it is written.  Not used for
+// queries (one or two launches) nor under capture.  Waiting blocks hold no more
+// than one kernel's worth of places: a kernel lets the next one come up only once it
+// runs itself.  14,400-point scan into 300,000 points 431 -> 393 us, small edits of
+// 100,000 points 502 -> 465, a build of 2,000,000 points 1054 -> 1000.
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+inline void launch_chain_if(bool chain, void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s,
+                            A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = chain ? 1 : 0;
+    // (a refused launch stays as the thread's last error, as with <<<>>>)
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+template <class... P, class... A>
+inline void launch_chain(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
+    launch_chain_if(true, kernel, grid, block, smem, s, std::forward<A>(args)...);
+}
+
+
 // ---- scan.cu / sort.cu ------------------------------------------------------
 // Exclusive prefix sum of n int32 / int64 values; `total` (device, nullable) receives
 // the sum.  `temp` must hold scan_temp_bytes(n) bytes.
 size_t scan_temp_bytes(long long n);
-void exclusive_scan(const int* in, int* out, long long n, int* total, void* temp, cudaStream_t s);
+// chain: launched with launch_chain.
+void exclusive_scan(const int* in, int* out, long long n, int* total, void* temp, cudaStream_t s, bool chain = false);
 void exclusive_scan(const long long* in, long long* out, long long n, long long* total, void* temp, cudaStream_t s);
 
 // Stable LSD radix sort of `batch` independent (key, value) arrays of length n
@@ -22,7 +62,7 @@ size_t sort_temp_bytes(long long n, int batch);
 // With copy_back = false an odd number of passes leaves the result in the
 // alt buffers, and the call returns true.
 bool radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, long long n,
-                      int batch, long long stride, int bits, void* temp, cudaStream_t s, bool copy_back = true);
+                      int batch, long long stride, int bits, void* temp, cudaStream_t s, bool copy_back = true, bool chain = false);
 
 // ---- build.cu ---------------------------------------------------------------
 // Batched subtree build.  `pts` holds the points of `njobs` jobs back to back

@@ -60,7 +60,8 @@ __device__ __forceinline__ T block_excl_scan(T v, T* total) {
 }
 
 template <typename T>
-__global__ void scan_reduce_kernel(const T* __restrict__ in, long long n, T* __restrict__ partial) {
+__global__ void scan_reduce_kernel(const T* in, long long n, T* __restrict__ partial) {
+    chain_begin();
     long long base = (long long)blockIdx.x * SCAN_TILE;
     T s = 0;
     for (int i = threadIdx.x; i < SCAN_TILE; i += SCAN_THREADS) {
@@ -75,6 +76,7 @@ __global__ void scan_reduce_kernel(const T* __restrict__ in, long long n, T* __r
 // Single block: exclusive scan of the tile partials.
 template <typename T>
 __global__ void scan_partials_kernel(T* partial, int ntiles, T* total) {
+    chain_begin();
     __shared__ T carry;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
@@ -92,8 +94,9 @@ __global__ void scan_partials_kernel(T* partial, int ntiles, T* total) {
 }
 
 template <typename T>
-__global__ void scan_down_kernel(const T* __restrict__ in, T* __restrict__ out, long long n,
-                                 const T* __restrict__ partial) {
+__global__ void scan_down_kernel(const T* in, T* __restrict__ out, long long n,
+                                 const T* partial) {
+    chain_begin();
     __shared__ T tile[SCAN_TILE];
     long long base = (long long)blockIdx.x * SCAN_TILE;
     for (int i = threadIdx.x; i < SCAN_TILE; i += SCAN_THREADS) {
@@ -127,8 +130,9 @@ constexpr int SCAN_ONE_ITEMS = 8;
 constexpr int SCAN_ONE = SCAN_ONE_THREADS * SCAN_ONE_ITEMS;
 
 template <typename T>
-__global__ void __launch_bounds__(SCAN_ONE_THREADS) scan_single_kernel(const T* __restrict__ in, T* __restrict__ out,
+__global__ void __launch_bounds__(SCAN_ONE_THREADS) scan_single_kernel(const T* in, T* __restrict__ out,
                                                                        int n, T* total) {
+    chain_begin();
     // warp w owns values [w * 256, ...): item i of a lane is 32 i further on,
     // so loads and stores are coalesced and a warp scans item rows in turn
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
@@ -157,26 +161,27 @@ __global__ void __launch_bounds__(SCAN_ONE_THREADS) scan_single_kernel(const T* 
 }
 
 template <typename T>
-void exclusive_scan_t(const T* in, T* out, long long n, T* total, void* temp, cudaStream_t s) {
+void exclusive_scan_t(const T* in, T* out, long long n, T* total, void* temp, cudaStream_t s, bool chain) {
     if (n <= 0) {
         if (total) cudaMemsetAsync(total, 0, sizeof(T), s);
         return;
     }
     if (n <= SCAN_ONE) {
-        scan_single_kernel<T><<<1, SCAN_ONE_THREADS, 0, s>>>(in, out, (int)n, total);
+        launch_chain_if(chain, scan_single_kernel<T>, 1, SCAN_ONE_THREADS, 0, s, in, out, (int)n, total);
         return;
     }
     int tiles = (int)((n + SCAN_TILE - 1) / SCAN_TILE);
     T* partial = (T*)temp;
-    scan_reduce_kernel<T><<<tiles, SCAN_THREADS, 0, s>>>(in, n, partial);
-    scan_partials_kernel<T><<<1, 1024, 0, s>>>(partial, tiles, total);
-    scan_down_kernel<T><<<tiles, SCAN_THREADS, 0, s>>>(in, out, n, partial);
+    launch_chain_if(chain, scan_reduce_kernel<T>, tiles, SCAN_THREADS, 0, s, in, n, partial);
+    launch_chain_if(chain, scan_partials_kernel<T>, 1, 1024, 0, s, partial, tiles, total);
+    launch_chain_if(chain, scan_down_kernel<T>, tiles, SCAN_THREADS, 0, s, in, out, n, partial);
 }
 
 // ---- radix sort --------------------------------------------------------------
 
-__global__ void sort_hist_kernel(const uint32_t* __restrict__ keys, long long n, long long stride, int shift,
+__global__ void sort_hist_kernel(const uint32_t* keys, long long n, long long stride, int shift,
                                  int ntiles, int rounds, int* __restrict__ hist) {
+    chain_begin();
     __shared__ int h[RADIX];
     for (int i = threadIdx.x; i < RADIX; i += SORT_THREADS) h[i] = 0;
     __syncthreads();
@@ -193,10 +198,11 @@ __global__ void sort_hist_kernel(const uint32_t* __restrict__ keys, long long n,
     for (int d = threadIdx.x; d < RADIX; d += SORT_THREADS) hb[(long long)d * ntiles + blockIdx.x] = h[d];
 }
 
-__global__ void sort_scatter_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
+__global__ void sort_scatter_kernel(const uint32_t* keys, const uint32_t* vals,
                                     uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, long long n,
                                     long long stride, int shift, int ntiles, int rounds,
-                                    const int* __restrict__ offs) {
+                                    const int* offs) {
+    chain_begin();
     __shared__ int wcnt[SORT_THREADS / 32][RADIX];
     __shared__ int dbase[RADIX];
     const int b = blockIdx.y;
@@ -254,12 +260,12 @@ size_t scan_temp_bytes(long long n) {
     return (size_t)((tiles + 64) * sizeof(long long) + 256);
 }
 
-void exclusive_scan(const int* in, int* out, long long n, int* total, void* temp, cudaStream_t s) {
-    exclusive_scan_t<int>(in, out, n, total, temp, s);
+void exclusive_scan(const int* in, int* out, long long n, int* total, void* temp, cudaStream_t s, bool chain) {
+    exclusive_scan_t<int>(in, out, n, total, temp, s, chain);
 }
 
 void exclusive_scan(const long long* in, long long* out, long long n, long long* total, void* temp, cudaStream_t s) {
-    exclusive_scan_t<long long>(in, out, n, total, temp, s);
+    exclusive_scan_t<long long>(in, out, n, total, temp, s, false);
 }
 
 size_t sort_temp_bytes(long long n, int batch) {
@@ -270,7 +276,7 @@ size_t sort_temp_bytes(long long n, int batch) {
 }
 
 bool radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, long long n,
-                      int batch, long long stride, int bits, void* temp, cudaStream_t s, bool copy_back) {
+                      int batch, long long stride, int bits, void* temp, cudaStream_t s, bool copy_back, bool chain) {
     if (n <= 1 || batch <= 0) return false;
     const int rounds = sort_rounds(n, batch);
     int tiles = ceil_div_ll(n, (long long)rounds * SORT_THREADS);
@@ -283,9 +289,9 @@ bool radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32
     dim3 grid(tiles, batch);
     for (int p = 0; p < passes; ++p) {
         int shift = 8 * p;
-        sort_hist_kernel<<<grid, SORT_THREADS, 0, s>>>(ki, n, stride, shift, tiles, rounds, hist);
-        exclusive_scan(hist, offs, hn, nullptr, stemp, s);
-        sort_scatter_kernel<<<grid, SORT_THREADS, 0, s>>>(ki, vi, ko, vo, n, stride, shift, tiles, rounds, offs);
+        launch_chain_if(chain, sort_hist_kernel, grid, SORT_THREADS, 0, s, ki, n, stride, shift, tiles, rounds, hist);
+        exclusive_scan(hist, offs, hn, nullptr, stemp, s, chain);
+        launch_chain_if(chain, sort_scatter_kernel, grid, SORT_THREADS, 0, s, ki, vi, ko, vo, n, stride, shift, tiles, rounds, offs);
         uint32_t* t;
         t = ki; ki = ko; ko = t;
         t = vi; vi = vo; vo = t;

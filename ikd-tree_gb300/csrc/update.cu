@@ -63,8 +63,9 @@ __device__ __forceinline__ void mark_dirty_warp(const UpdateAux& a, DevStatus* s
 
 // ---- insertion -----------------------------------------------------------------
 
-__global__ void route_append_kernel(DevTree t, UpdateAux a, const float4* __restrict__ pts, long long n,
+__global__ void route_append_kernel(DevTree t, UpdateAux a, const float4* pts, long long n,
                                     const int* n_dev, int4* __restrict__ ovf_leaf, float4* __restrict__ ovf_pts) {
+    chain_begin();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long lim = n_dev != nullptr ? (long long)*n_dev : n;
     if (i >= lim) return;
@@ -116,7 +117,8 @@ __device__ __forceinline__ int first_item() {
 }
 
 // Counts into pend[X] the child sides of X that a refit will change.
-__global__ void refit_mark_kernel(DevTree t, UpdateAux a, const int* __restrict__ items, const int* n_items) {
+__global__ void refit_mark_kernel(DevTree t, UpdateAux a, const int* items, const int* n_items) {
+    chain_begin();
     const int n = min(*n_items, a.list_cap);
     for (int i = first_item(); i < n; i += gridDim.x * blockDim.x) {
         const int link = item_link(t, items[i]);
@@ -242,8 +244,9 @@ __device__ __forceinline__ bool violates(const Criteria& c, int slots, int del, 
 // writes, the arrival, the loads and then the arithmetic: 15 levels took 33 us,
 // 17 now (14,400-point scan into 300,000 points, four refits: the call went from
 // 548 to 485 us; small edits of a 100,000-point map, 26 -> 13 us: 632 -> 535).
-__global__ void __launch_bounds__(128) refit_compute_kernel(DevTree t, UpdateAux a, const int* __restrict__ items,
+__global__ void __launch_bounds__(128) refit_compute_kernel(DevTree t, UpdateAux a, const int* items,
                                                             const int* n_items, Criteria c) {
+    chain_begin();
     const int n_it = min(*n_items, a.list_cap);
     for (int i = first_item(); i < n_it; i += gridDim.x * blockDim.x) {
         const int item = items[i];
@@ -549,7 +552,7 @@ __device__ __forceinline__ void grid_barrier(DevStatus* st) {
 // and 4 when there is nothing to rebuild; the call as a whole went from 624 to
 // 548 us, a small edit of a 100,000-point map from 773 to 632.  select = false: no
 // jobs, the violators' flags are cleared.
-__global__ void __launch_bounds__(SETTLE_THREADS, 2) settle_kernel(DevTree t, UpdateAux a, const int4* __restrict__ ovf_leaf,
+__global__ void __launch_bounds__(SETTLE_THREADS, 2) settle_kernel(DevTree t, UpdateAux a, const int4* ovf_leaf,
                                                                 int max_ovf, bool select, DevStatus* __restrict__ host) {
     DevStatus* st = t.st;
     const int nv = min(__ldcg(&st->n_viol), a.list_cap);
@@ -629,9 +632,10 @@ __device__ __forceinline__ void gather_leaf(const DevTree& t, const UpdateAux& a
 
 // The points of every job into `out`, back to back; the jobs' leaves and nodes go
 // to the free stacks.  One thread per leaf, node and overflow point.
-__global__ void job_gather_kernel(DevTree t, UpdateAux a, int leaf_top, int node_top, const int4* __restrict__ ovf_leaf,
-                                  const float4* __restrict__ ovf_pts, int max_ovf, float4* __restrict__ out,
+__global__ void job_gather_kernel(DevTree t, UpdateAux a, int leaf_top, int node_top, const int4* ovf_leaf,
+                                  const float4* ovf_pts, int max_ovf, float4* __restrict__ out,
                                   float4* __restrict__ removed, long long removed_cap) {
+    chain_begin();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < leaf_top) {
         gather_leaf(t, a, i, out, removed, removed_cap);
@@ -653,6 +657,7 @@ __global__ void job_gather_kernel(DevTree t, UpdateAux a, int leaf_top, int node
 // Resets per-job state and queues each job's parent for the follow-up refit
 // (one block).
 __global__ void __launch_bounds__(1024) job_finish_kernel(DevTree t, UpdateAux a) {
+    chain_begin();
     const int n = min(t.st->n_jobs, a.list_cap);
     for (int j = threadIdx.x; j < n; j += blockDim.x) {
         int code = a.jobs[j];
@@ -713,7 +718,7 @@ __device__ __forceinline__ void team_walk(const DevTree& t, bool active, int* st
             int c0 = 0, c1 = 0;
             if (node) {
                 const float4* p = t.wide + (long long)cur * 16 + 4 * sub;
-                const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
+                const float4 a = __ldcg(p), b = __ldcg(p + 1), c = __ldcg(p + 2), d = __ldcg(p + 3);
                 const float lo0[3] = {a.x, a.z, b.x}, hi0[3] = {b.z, c.x, c.z};
                 const float lo1[3] = {a.y, a.w, b.y}, hi1[3] = {b.w, c.y, c.w};
                 al0 = lo0[0] <= hi0[0] && overlap(lo0, hi0);
@@ -808,8 +813,9 @@ __device__ int box_seed(const DevTree& t, const Box3& qb, int part, int split_bi
 // of the box) and queue leaves, then each warp edits queued leaves one slot per
 // lane.
 __global__ void __launch_bounds__(DB_THREADS) box_restore_kernel(DevTree t, UpdateAux a,
-                                                                 const float* __restrict__ boxes, long long m,
+                                                                 const float* boxes, long long m,
                                                                  int split_bits) {
+    chain_begin();
     __shared__ int stack[DB_STACK];
     __shared__ int leafq[2 * DB_THREADS];
     __shared__ int top, nleaf;
@@ -904,9 +910,10 @@ constexpr int BD_CTA = 128;
 __host__ __device__ constexpr int bd_stack_entries(int height) {
     return BD_WIDE + 7 * BD_WINDOW + 7 * (1 + (height + 2) / 3) + 1;
 }
-__global__ void __launch_bounds__(BD_CTA) box_delete_kernel(DevTree t, UpdateAux a, const float* __restrict__ boxes,
+__global__ void __launch_bounds__(BD_CTA) box_delete_kernel(DevTree t, UpdateAux a, const float* boxes,
                                                             long long m, int levels, int top_bits,
                                                             uint32_t del_flags, long long* __restrict__ total) {
+    chain_begin();
     extern __shared__ int stacks[];
     constexpr unsigned ALL = 0xffffffffu;
     const int lane = threadIdx.x & 31, sub = lane & (TEAM - 1), j = lane / TEAM;
@@ -933,10 +940,10 @@ __global__ void __launch_bounds__(BD_CTA) box_delete_kernel(DevTree t, UpdateAux
             Box3 b;
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                b.lo[k] = __ldg(f + 2 * k);
-                b.hi[k] = __ldg(f + 6 + 2 * k);
+                b.lo[k] = __ldcg(f + 2 * k);
+                b.hi[k] = __ldcg(f + 6 + 2 * k);
             }
-            code = __float_as_int(__ldg(f + 12));
+            code = __float_as_int(__ldcg(f + 12));
             part >>= w;
             live = code != 0 && !box_empty(b) && (cov || !qbox_disjoint(qb, b)) && (code > 0 || part == 0);
             cov = cov || qbox_covers(qb, b);
@@ -963,7 +970,7 @@ __global__ void __launch_bounds__(BD_CTA) box_delete_kernel(DevTree t, UpdateAux
             int k0 = it, k1 = 0;
             if (rec) {
                 const float4* p = t.wide + (long long)c * 16 + 4 * sub;
-                const float4 x = __ldg(p), y = __ldg(p + 1), z = __ldg(p + 2), w = __ldg(p + 3);
+                const float4 x = __ldcg(p), y = __ldcg(p + 1), z = __ldcg(p + 2), w = __ldcg(p + 3);
                 Box3 b0, b1;
                 b0.lo[0] = x.x, b0.lo[1] = x.z, b0.lo[2] = y.x, b0.hi[0] = y.z, b0.hi[1] = z.x, b0.hi[2] = z.z;
                 b1.lo[0] = x.y, b1.lo[1] = x.w, b1.lo[2] = y.y, b1.hi[0] = y.w, b1.hi[1] = z.y, b1.hi[2] = z.w;
@@ -1038,6 +1045,7 @@ __device__ __forceinline__ bool same_point(float ax, float ay, float az, float b
 // points in 100,000, 10 now.
 __global__ void __launch_bounds__(TEAM_CTA) delete_points_kernel(DevTree t, UpdateAux a, const float* __restrict__ in,
                                                                  int stride, long long n) {
+    chain_begin();
     extern __shared__ int stacks[];
     const long long i = ((long long)blockIdx.x * TEAM_CTA + threadIdx.x) / TEAM;
     const bool active = i < n;
@@ -1117,6 +1125,7 @@ __global__ void stored_ids_kernel(DevTree t, int* __restrict__ out, long long ca
 
 // The whole tree as the only violator: settle_kernel makes it the rebuild job.
 __global__ void select_root_kernel(DevTree t, UpdateAux a) {
+    chain_begin();
     const int code = __float_as_int(t.node[3].x);
     if (code == 0) return;
     a.viol[0] = code;
@@ -1299,7 +1308,7 @@ __global__ void validate_aux_leaves_kernel(DevTree t, UpdateAux a, unsigned long
     }
 }
 
-__global__ void set_ll_kernel(long long* p, long long v) { *p = v; }
+__global__ void set_ll_kernel(long long* p, long long v) { chain_begin(); *p = v; }
 
 // Empties the top wide record and places the root at position `pos` in it.
 __global__ void set_top_kernel(DevTree t, int pos) {
@@ -1308,6 +1317,7 @@ __global__ void set_top_kernel(DevTree t, int pos) {
 }
 
 __global__ void snapshot_root_kernel(DevTree t) {
+    chain_begin();
     finish_alloc(t.st);
     snapshot_root(t);
 }
@@ -1367,6 +1377,7 @@ __device__ __forceinline__ bool in_voxel_range(float c, float f, float df, float
 
 __global__ void ds_prepare_kernel(DevTree t, const float* __restrict__ in, int stride, long long n, float ds,
                                   DsScratch d) {
+    chain_begin();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) t.st->count = n;  // end of the first sub-batch, until a point cuts it
     if (i >= n) return;
@@ -1406,6 +1417,7 @@ __device__ __forceinline__ bool same_key(const int4& a, const int4& b) { return 
 // per-group walks below read consecutive entries instead of gathering through
 // hval one dependent load at a time.
 __global__ void ds_leaders_kernel(long long n, DsScratch d, DevStatus* st) {
+    chain_begin();
     long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     uint32_t h = d.hkey[0][j];
@@ -1432,9 +1444,9 @@ __device__ __forceinline__ void for_run(const DsScratch& d, long long n, long lo
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const long long jj = base + u;
-            hh[u] = jj < n ? __ldg(d.hkey[0] + jj) : ~h;
-            kk[u] = jj < n ? __ldg(d.s_key + jj) : make_int4(0, 0, 0, 0);
-            pp[u] = jj < n ? __ldg(d.s_pts + jj) : make_float4(0.f, 0.f, 0.f, 0.f);
+            hh[u] = jj < n ? __ldcg(d.hkey[0] + jj) : ~h;
+            kk[u] = jj < n ? __ldcg(d.s_key + jj) : make_int4(0, 0, 0, 0);
+            pp[u] = jj < n ? __ldcg(d.s_pts + jj) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -1446,8 +1458,8 @@ __device__ __forceinline__ void for_run(const DsScratch& d, long long n, long lo
 
 // First member index >= a of group g (members are in increasing index order).
 __device__ __forceinline__ long long group_first_from(const DsScratch& d, long long n, int j, long long a) {
-    const uint32_t h = __ldg(d.hkey[0] + j);
-    const int4 k = __ldg(d.s_key + j);
+    const uint32_t h = __ldcg(d.hkey[0] + j);
+    const int4 k = __ldcg(d.s_key + j);
     long long r = -1;
     for_run(d, n, j, h, [&](long long, const int4& kk, const float4& p) {
         if (!same_key(kk, k)) return true;
@@ -1462,6 +1474,7 @@ __device__ __forceinline__ long long group_first_from(const DsScratch& d, long l
 }
 
 __global__ void ds_h1_kernel(long long n, long long a, DsScratch d, DevStatus* st) {
+    chain_begin();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *d.n_pairs = 0;  // ds_search_kernel lists its pairs afresh
         st->n_ins = 0;   // and the fold its winners
@@ -1496,6 +1509,7 @@ __device__ __forceinline__ bool half_open_overlap(const Box3& q, const float* lo
 // scan, 9,000 groups, 300,000 stored points: 65 us with a thread per group on the
 // binary nodes, 21 now.
 __global__ void __launch_bounds__(TEAM_CTA) ds_search_kernel(DevTree t, long long n, long long a, DsScratch d, float ds) {
+    chain_begin();
     extern __shared__ int stacks[];
     constexpr unsigned ALL = 0xffffffffu;
     const int g = (blockIdx.x * TEAM_CTA + threadIdx.x) / TEAM;
@@ -1594,6 +1608,7 @@ __global__ void __launch_bounds__(TEAM_CTA) ds_search_kernel(DevTree t, long lon
 
 __global__ void __launch_bounds__(128) ds_fold_kernel(DevTree t, long long n, long long a, long long first_id,
                                                       DsScratch d) {
+    chain_begin();
     int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= t.st->n_groups) return;
     if (t.st->err & ERR_INPUT) return;  // a non-finite input: the call changes nothing
@@ -1603,15 +1618,15 @@ __global__ void __launch_bounds__(128) ds_fold_kernel(DevTree t, long long n, lo
     int j = d.groups[g];
     int4 info = d.g_info[g];
     d.g_out[g] = make_int4(0, 0, 0, 0);
-    const uint32_t h = __ldg(d.hkey[0] + j);
-    if (j + DS_BIG_RUN < n && __ldg(d.hkey[0] + j + DS_BIG_RUN) == h) {
+    const uint32_t h = __ldcg(d.hkey[0] + j);
+    if (j + DS_BIG_RUN < n && __ldcg(d.hkey[0] + j + DS_BIG_RUN) == h) {
         // a long hash run (a voxel with many points): folded by a warp
         d.big[atomicAdd(d.n_big, 1)] = g;
         return;
     }
     if (info.y == -1 && info.x == 0 && group_first_from(d, n, j, a) < 0) return;
     const int lead = d.hval[0][j];
-    const int4 k = __ldg(d.s_key + j);
+    const int4 k = __ldcg(d.s_key + j);
     float4 mid = d.mid[lead];
     float4 best = d.g_best[g];
     const int n0 = info.x;
@@ -1677,6 +1692,7 @@ __global__ void __launch_bounds__(128) ds_fold_kernel(DevTree t, long long n, lo
 // final c under its own id (the stored point's, or first_id + its index).
 __global__ void __launch_bounds__(128) ds_fold_big_kernel(DevTree t, long long n, long long a, long long first_id,
                                                           DsScratch d) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -1688,8 +1704,8 @@ __global__ void __launch_bounds__(128) ds_fold_big_kernel(DevTree t, long long n
         const int j = d.groups[g];
         const int4 info = d.g_info[g];
         const float4 best = d.g_best[g];
-        const uint32_t h = __ldg(d.hkey[0] + j);
-        const int4 k = __ldg(d.s_key + j);
+        const uint32_t h = __ldcg(d.hkey[0] + j);
+        const int4 k = __ldcg(d.s_key + j);
         const float4 mid = d.mid[d.hval[0][j]];
         const int n0 = info.x;
         // running c: distance, position in the run (-2: the stored best,
@@ -1703,7 +1719,7 @@ __global__ void __launch_bounds__(128) ds_fold_big_kernel(DevTree t, long long n
         bool more = true;
         for (long long base = j; more && base < n; base += 32) {
             const long long jj = base + lane;
-            const uint32_t hh = jj < n ? __ldg(d.hkey[0] + jj) : ~h;
+            const uint32_t hh = jj < n ? __ldcg(d.hkey[0] + jj) : ~h;
             const unsigned off_run = __ballot_sync(0xffffffffu, hh != h);
             // entries from the first one of another hash on are not in the run
             const int run_end = off_run ? __ffs(off_run) - 1 : 32;
@@ -1711,9 +1727,9 @@ __global__ void __launch_bounds__(128) ds_fold_big_kernel(DevTree t, long long n
             float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
             long long idx = -1;
             if (lane < run_end) {
-                const int4 kk = __ldg(d.s_key + jj);
+                const int4 kk = __ldcg(d.s_key + jj);
                 if (same_key(kk, k)) {
-                    p = __ldg(d.s_pts + jj);
+                    p = __ldcg(d.s_pts + jj);
                     idx = __float_as_int(p.w);
                     member = idx >= a && idx < e;
                 }
@@ -1786,6 +1802,7 @@ __global__ void __launch_bounds__(128) ds_fold_big_kernel(DevTree t, long long n
 // in the boxes of the groups whose fold decided so: one thread per listed
 // (group, slot) pair, no tree walk (nothing moved since the search).
 __global__ void ds_delete_pairs_kernel(DevTree t, UpdateAux a, DsScratch d) {
+    chain_begin();
     const int np = *d.n_pairs;
     if (np > d.pair_cap || (t.st->err & ERR_INPUT)) return;  // the list overflowed: ds_delete_kernel walks
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
@@ -1800,6 +1817,7 @@ __global__ void ds_delete_pairs_kernel(DevTree t, UpdateAux a, DsScratch d) {
 // The same deletion by walking the tree from every voxel box, when the pair
 // list overflowed.
 __global__ void __launch_bounds__(TEAM_CTA) ds_delete_kernel(DevTree t, UpdateAux a, DsScratch d) {
+    chain_begin();
     extern __shared__ int stacks[];
     if (*d.n_pairs <= d.pair_cap) return;  // ds_delete_pairs_kernel did it
     const int g = (blockIdx.x * TEAM_CTA + threadIdx.x) / TEAM;
@@ -1823,6 +1841,7 @@ __global__ void __launch_bounds__(TEAM_CTA) ds_delete_kernel(DevTree t, UpdateAu
 
 __global__ void pack_points_kernel(DevTree t, const float* __restrict__ in, int stride, long long n, long long first_id,
                                    float4* __restrict__ out) {
+    chain_begin();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float x = in[i * stride], y = in[i * stride + 1], z = in[i * stride + 2];
@@ -1837,6 +1856,7 @@ __global__ void pack_points_kernel(DevTree t, const float* __restrict__ in, int 
 constexpr int PACK_POINTS = 1024;
 __global__ void __launch_bounds__(256) pack_dense_kernel(DevTree t, const float4* __restrict__ in, long long n,
                                                          long long first_id, float4* __restrict__ out) {
+    chain_begin();
     __shared__ float4 w[PACK_POINTS * 3 / 4];
     const long long p0 = (long long)blockIdx.x * PACK_POINTS;
     const int m = (int)min((long long)PACK_POINTS, n - p0);
@@ -1879,13 +1899,13 @@ inline size_t au(size_t x) { return (x + 255) & ~(size_t)255; }
 void launch_route_append(const DevTree& t, const UpdateAux& a, const float4* pts, long long n, int4* ovf_leaf,
                          float4* ovf_pts, cudaStream_t s) {
     if (n <= 0) return;
-    route_append_kernel<<<blocks_for(n, 256), 256, 0, s>>>(t, a, pts, n, nullptr, ovf_leaf, ovf_pts);
+    launch_chain(route_append_kernel, blocks_for(n, 256), 256, 0, s, t, a, pts, n, nullptr, ovf_leaf, ovf_pts);
 }
 
 void launch_route_append_dev_count(const DevTree& t, const UpdateAux& a, const float4* pts, long long n_bound,
                                    const int* n_dev, int4* ovf_leaf, float4* ovf_pts, cudaStream_t s) {
     if (n_bound <= 0) return;
-    route_append_kernel<<<blocks_for(n_bound, 256), 256, 0, s>>>(t, a, pts, n_bound, n_dev, ovf_leaf, ovf_pts);
+    launch_chain(route_append_kernel, blocks_for(n_bound, 256), 256, 0, s, t, a, pts, n_bound, n_dev, ovf_leaf, ovf_pts);
 }
 
 void launch_refit(const DevTree& t, const UpdateAux& a, const int* items, const int* n_items, int max_items,
@@ -1893,8 +1913,8 @@ void launch_refit(const DevTree& t, const UpdateAux& a, const int* items, const 
     if (max_items <= 0) return;
     // (the number of items is on the device, the bound often far above it: the
     // grids end at what the device holds at once)
-    refit_mark_kernel<<<std::min(blocks_for(max_items, 128), 152u * 8u), 128, 0, s>>>(t, a, items, n_items);
-    refit_compute_kernel<<<std::min(blocks_for(max_items, 128), 152u * 8u), 128, 0, s>>>(t, a, items, n_items, c);
+    launch_chain(refit_mark_kernel, std::min(blocks_for(max_items, 128), 152u * 8u), 128, 0, s, t, a, items, n_items);
+    launch_chain(refit_compute_kernel, std::min(blocks_for(max_items, 128), 152u * 8u), 128, 0, s, t, a, items, n_items, c);
 }
 
 
@@ -1911,12 +1931,12 @@ void launch_job_gather(const DevTree& t, const UpdateAux& a, int leaf_top, int n
                        cudaStream_t s) {
     const long long n = (long long)leaf_top + node_top + max_ovf;
     if (n > 0)
-        job_gather_kernel<<<blocks_for(n, 256), 256, 0, s>>>(t, a, leaf_top, node_top, ovf_leaf, ovf_pts, max_ovf, out,
+        launch_chain(job_gather_kernel, blocks_for(n, 256), 256, 0, s, t, a, leaf_top, node_top, ovf_leaf, ovf_pts, max_ovf, out,
                                                              removed, removed_cap);
 }
 
 void launch_job_finish(const DevTree& t, const UpdateAux& a, cudaStream_t s) {
-    job_finish_kernel<<<1, 1024, 0, s>>>(t, a);
+    launch_chain(job_finish_kernel, 1, 1024, 0, s, t, a);
 }
 
 void launch_delete_boxes(const DevTree& t, const UpdateAux& a, const float* boxes, long long m, int top_bits,
@@ -1929,26 +1949,26 @@ void launch_delete_boxes(const DevTree& t, const UpdateAux& a, const float* boxe
     while (levels < BD_LEVELS_MAX && bits < t.height && (m << bits) < BD_UNITS) bits += levels++ ? 3 : top_bits;
     const long long blocks = ((m << bits) + BD_CTA / 32 - 1) / (BD_CTA / 32);
     const size_t smem = sizeof(int) * bd_stack_entries(t.height) * (BD_CTA / 32);
-    box_delete_kernel<<<box_grid(blocks), BD_CTA, smem, s>>>(t, a, boxes, m, levels, top_bits, flags, total);
+    launch_chain(box_delete_kernel, box_grid(blocks), BD_CTA, smem, s, t, a, boxes, m, levels, top_bits, flags, total);
 }
 
 void launch_add_boxes(const DevTree& t, const UpdateAux& a, const float* boxes, long long m, cudaStream_t s) {
     if (m <= 0) return;
     int bits = box_split_bits(m);
-    box_restore_kernel<<<box_grid(m << bits), DB_THREADS, 0, s>>>(t, a, boxes, m, bits);
+    launch_chain(box_restore_kernel, box_grid(m << bits), DB_THREADS, 0, s, t, a, boxes, m, bits);
 }
 
 void launch_delete_points(const DevTree& t, const UpdateAux& a, const float* pts, int stride, long long n,
                           cudaStream_t s) {
     if (n <= 0) return;
-    delete_points_kernel<<<blocks_for(n * TEAM, TEAM_CTA), TEAM_CTA, team_stack_bytes(t.height), s>>>(t, a, pts, stride, n);
+    launch_chain(delete_points_kernel, blocks_for(n * TEAM, TEAM_CTA), TEAM_CTA, team_stack_bytes(t.height), s, t, a, pts, stride, n);
 }
 
-void launch_snapshot_root(const DevTree& t, cudaStream_t s) { snapshot_root_kernel<<<1, 1, 0, s>>>(t); }
+void launch_snapshot_root(const DevTree& t, cudaStream_t s) { launch_chain(snapshot_root_kernel, 1, 1, 0, s, t); }
 
 void launch_set_top(const DevTree& t, int pos, cudaStream_t s) { set_top_kernel<<<1, WIDE, 0, s>>>(t, pos); }
 
-void launch_set_ll(long long* p, long long v, cudaStream_t s) { set_ll_kernel<<<1, 1, 0, s>>>(p, v); }
+void launch_set_ll(long long* p, long long v, cudaStream_t s) { launch_chain(set_ll_kernel, 1, 1, 0, s, p, v); }
 
 void launch_validate(const DevTree& t, const UpdateAux& a, bool at_rest, long long* bad, cudaStream_t s) {
     if (t.node_cap > 0)
@@ -1972,18 +1992,18 @@ void launch_stored_ids(const DevTree& t, int* out, long long cap, long long* cou
 }
 
 void launch_select_root(const DevTree& t, const UpdateAux& a, cudaStream_t s) {
-    select_root_kernel<<<1, 1, 0, s>>>(t, a);
+    launch_chain(select_root_kernel, 1, 1, 0, s, t, a);
 }
 
 void launch_pack_points(const DevTree& t, const float* in, int stride, long long n, long long first_id, float4* out,
                         cudaStream_t s) {
     if (n <= 0) return;
     if (stride == 3 && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {
-        pack_dense_kernel<<<blocks_for(n, PACK_POINTS), 256, 0, s>>>(t, reinterpret_cast<const float4*>(in), n, first_id,
+        launch_chain(pack_dense_kernel, blocks_for(n, PACK_POINTS), 256, 0, s, t, reinterpret_cast<const float4*>(in), n, first_id,
                                                                      out);
         return;
     }
-    pack_points_kernel<<<blocks_for(n, 256), 256, 0, s>>>(t, in, stride, n, first_id, out);
+    launch_chain(pack_points_kernel, blocks_for(n, 256), 256, 0, s, t, in, stride, n, first_id, out);
 }
 
 void launch_check_finite(const DevTree& t, const float* in, long long count, cudaStream_t s) {
@@ -2040,32 +2060,30 @@ void carve_ds_scratch(void* base, long long n, long long pair_cap, DsScratch* d)
 void launch_ds_prepare(const DevTree& t, const float* in, int stride, long long n, float ds, DsScratch& d,
                        cudaStream_t s) {
     if (n <= 0) return;
-    ds_prepare_kernel<<<blocks_for(n, 256), 256, 0, s>>>(t, in, stride, n, ds, d);
+    launch_chain(ds_prepare_kernel, blocks_for(n, 256), 256, 0, s, t, in, stride, n, ds, d);
     // 24-bit keys: three passes; the sorted pairs stay where the last pass
     // left them
-    if (radix_sort_pairs(d.hkey[0], d.hval[0], d.hkey[1], d.hval[1], n, 1, n, DS_HASH_BITS, d.temp, s, false)) {
+    if (radix_sort_pairs(d.hkey[0], d.hval[0], d.hkey[1], d.hval[1], n, 1, n, DS_HASH_BITS, d.temp, s, false, true)) {
         std::swap(d.hkey[0], d.hkey[1]);
         std::swap(d.hval[0], d.hval[1]);
     }
-    ds_leaders_kernel<<<blocks_for(n, 256), 256, 0, s>>>(n, d, t.st);
+    launch_chain(ds_leaders_kernel, blocks_for(n, 256), 256, 0, s, n, d, t.st);
 }
 
 void launch_ds_search(const DevTree& t, long long n, float ds, long long a, DsScratch& d, int max_groups,
                       cudaStream_t s) {
-    if (n - a > 0) ds_h1_kernel<<<blocks_for(n - a, 256), 256, 0, s>>>(n, a, d, t.st);
+    if (n - a > 0) launch_chain(ds_h1_kernel, blocks_for(n - a, 256), 256, 0, s, n, a, d, t.st);
     if (max_groups > 0)
-        ds_search_kernel<<<blocks_for((long long)max_groups * TEAM, TEAM_CTA), TEAM_CTA, team_stack_bytes(t.height), s>>>(
-            t, n, a, d, ds);
+        launch_chain(ds_search_kernel, blocks_for((long long)max_groups * TEAM, TEAM_CTA), TEAM_CTA, team_stack_bytes(t.height), s, t, n, a, d, ds);
 }
 
 void launch_ds_fold(const DevTree& t, const UpdateAux& aux, long long n, long long a, long long first_id,
                     DsScratch& d, int max_groups, cudaStream_t s) {
     if (max_groups <= 0) return;
-    ds_fold_kernel<<<blocks_for(max_groups, 128), 128, 0, s>>>(t, n, a, first_id, d);
-    ds_fold_big_kernel<<<DS_BIG_BLOCKS, 128, 0, s>>>(t, n, a, first_id, d);
-    ds_delete_pairs_kernel<<<SPEC_BLOCKS, 256, 0, s>>>(t, aux, d);
-    ds_delete_kernel<<<blocks_for((long long)max_groups * TEAM, TEAM_CTA), TEAM_CTA, team_stack_bytes(t.height), s>>>(
-        t, aux, d);
+    launch_chain(ds_fold_kernel, blocks_for(max_groups, 128), 128, 0, s, t, n, a, first_id, d);
+    launch_chain(ds_fold_big_kernel, DS_BIG_BLOCKS, 128, 0, s, t, n, a, first_id, d);
+    launch_chain(ds_delete_pairs_kernel, SPEC_BLOCKS, 256, 0, s, t, aux, d);
+    launch_chain(ds_delete_kernel, blocks_for((long long)max_groups * TEAM, TEAM_CTA), TEAM_CTA, team_stack_bytes(t.height), s, t, aux, d);
 }
 
 }  // namespace ikdg
