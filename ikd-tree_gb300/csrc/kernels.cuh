@@ -18,7 +18,7 @@ namespace ikdg {
 // (const __restrict__, __ldg): the reader is up while it is written.  Not used for
 // queries (one or two launches) nor under capture.  Waiting blocks hold no more
 // than one kernel's worth of places: a kernel lets the next one come up only once it
-// runs itself.  14,400-point scan into 300,000 points 431 -> 393 us, small edits of
+// runs itself.  14,400-point scan into 500,000 points 431 -> 393 us, small edits of
 // 100,000 points 502 -> 465, a build of 2,000,000 points 1054 -> 1000.
 __device__ __forceinline__ void chain_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");

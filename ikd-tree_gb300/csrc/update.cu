@@ -109,7 +109,7 @@ __device__ __forceinline__ int item_link(const DevTree& t, int item) {
 
 // Items are dealt out over the warps before the lanes, so a few thousand walks run
 // one to a warp: walks of one warp diverge at each meeting and wait for one another
-// (14,400-point scan into 300,000 points: 40 us with the items packed into full
+// (14,400-point scan into 500,000 points: 40 us with the items packed into full
 // warps, 17 dealt out).
 __device__ __forceinline__ int first_item() {
     const int warps = gridDim.x * (blockDim.x >> 5);
@@ -242,7 +242,7 @@ __device__ __forceinline__ bool violates(const Criteria& c, int slots, int del, 
 // check runs while its exchange is in flight.  The stored boxes and counts are
 // read by nobody in this launch.  Before, each level cost the release of its
 // writes, the arrival, the loads and then the arithmetic: 15 levels took 33 us,
-// 17 now (14,400-point scan into 300,000 points, four refits: the call went from
+// 17 now (14,400-point scan into 500,000 points, four refits: the call went from
 // 548 to 485 us; small edits of a 100,000-point map, 26 -> 13 us: 632 -> 535).
 __global__ void __launch_bounds__(128) refit_compute_kernel(DevTree t, UpdateAux a, const int* items,
                                                             const int* n_items, Criteria c) {
@@ -548,7 +548,7 @@ __device__ __forceinline__ void grid_barrier(DevStatus* st) {
 // Bound by the walks up the tree (select_job, find_job_up): chains of dependent
 // loads, so every leaf and node gets its own thread where the device has them.
 // One cooperative launch with three grid barriers replaces eight small launches
-// and a copy: 60 us of kernels became 33 (14,400-point scan into 300,000 points),
+// and a copy: 60 us of kernels became 33 (14,400-point scan into 500,000 points),
 // and 4 when there is nothing to rebuild; the call as a whole went from 624 to
 // 548 us, a small edit of a 100,000-point map from 773 to 632.  select = false: no
 // jobs, the violators' flags are cleared.
@@ -718,7 +718,7 @@ __device__ __forceinline__ void team_walk(const DevTree& t, bool active, int* st
             int c0 = 0, c1 = 0;
             if (node) {
                 const float4* p = t.wide + (long long)cur * 16 + 4 * sub;
-                const float4 a = __ldcg(p), b = __ldcg(p + 1), c = __ldcg(p + 2), d = __ldcg(p + 3);
+                const float4 a = p[0], b = p[1], c = p[2], d = p[3];  // (the top records stay in L1)
                 const float lo0[3] = {a.x, a.z, b.x}, hi0[3] = {b.z, c.x, c.z};
                 const float lo1[3] = {a.y, a.w, b.y}, hi1[3] = {b.w, c.y, c.w};
                 al0 = lo0[0] <= hi0[0] && overlap(lo0, hi0);
@@ -901,7 +901,7 @@ __global__ void __launch_bounds__(DB_THREADS) box_restore_kernel(DevTree t, Upda
 // two children per lane, or four slots of a bucket half.  Above BD_WIDE entries only
 // one record a step is expanded, which bounds the stack (bd_stack_entries).  Bound by
 // the chain of records; the kernel it replaces walked binary nodes with four block
-// barriers a level: 37 us for six boxes in 300,000 points, 13 now.
+// barriers a level: 37 us for six boxes in 500,000 points, 13 now.
 constexpr int BD_WINDOW = 8;
 constexpr int BD_WIDE = 96;
 constexpr int BD_LEVELS_MAX = 4;
@@ -940,10 +940,10 @@ __global__ void __launch_bounds__(BD_CTA) box_delete_kernel(DevTree t, UpdateAux
             Box3 b;
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                b.lo[k] = __ldcg(f + 2 * k);
-                b.hi[k] = __ldcg(f + 6 + 2 * k);
+                b.lo[k] = f[2 * k];
+                b.hi[k] = f[6 + 2 * k];
             }
-            code = __float_as_int(__ldcg(f + 12));
+            code = __float_as_int(f[12]);
             part >>= w;
             live = code != 0 && !box_empty(b) && (cov || !qbox_disjoint(qb, b)) && (code > 0 || part == 0);
             cov = cov || qbox_covers(qb, b);
@@ -970,7 +970,7 @@ __global__ void __launch_bounds__(BD_CTA) box_delete_kernel(DevTree t, UpdateAux
             int k0 = it, k1 = 0;
             if (rec) {
                 const float4* p = t.wide + (long long)c * 16 + 4 * sub;
-                const float4 x = __ldcg(p), y = __ldcg(p + 1), z = __ldcg(p + 2), w = __ldcg(p + 3);
+                const float4 x = p[0], y = p[1], z = p[2], w = p[3];  // (the top records stay in L1)
                 Box3 b0, b1;
                 b0.lo[0] = x.x, b0.lo[1] = x.z, b0.lo[2] = y.x, b0.hi[0] = y.z, b0.hi[1] = z.x, b0.hi[2] = z.z;
                 b1.lo[0] = x.y, b1.lo[1] = x.w, b1.lo[2] = y.y, b1.hi[0] = y.w, b1.hi[1] = z.y, b1.hi[2] = z.w;
@@ -1035,8 +1035,8 @@ unsigned box_grid(long long units) { return (unsigned)(units < (1LL << 20) ? uni
 // same_point (ikd_Tree.cpp:1368-1371): |a - b| < 1e-6 per axis, the float
 // difference compared in double.
 __device__ __forceinline__ bool same_point(float ax, float ay, float az, float bx, float by, float bz) {
-    return (double)fabsf(__fsub_rn(ax, bx)) < 1e-6 && (double)fabsf(__fsub_rn(ay, by)) < 1e-6 &&
-           (double)fabsf(__fsub_rn(az, bz)) < 1e-6;
+    // 1e-6f is the largest float below 1e-6: the same test without doubles
+    return fabsf(__fsub_rn(ax, bx)) <= 1e-6f && fabsf(__fsub_rn(ay, by)) <= 1e-6f && fabsf(__fsub_rn(az, bz)) <= 1e-6f;
 }
 
 // One team per point: the first match in the walk's order that no other team has
@@ -1343,12 +1343,15 @@ __global__ void snapshot_root_kernel(DevTree t) {
 // point i of the batch gets id first_id + i.
 
 // Bits of the voxel hash the grouper sorts by (and compares: entries of one
-// hash run are the sorted neighbours with equal masked hash).
-constexpr int DS_HASH_BITS = 24;
+// hash run are the sorted neighbours with equal masked hash): three sort passes, or two where the points are so few that
+// two voxels rarely share one of 65,536 values (a run with several voxels costs its
+// readers a comparison per member).  14,400 points: the sort 36 -> 24 us.
+constexpr long long DS_SHORT_HASH = 32768;
+inline int ds_hash_bits(long long n) { return n <= DS_SHORT_HASH ? 16 : 24; }
 // Hash runs longer than this go to ds_fold_big_kernel (a warp per group,
 // DS_BIG_BLOCKS blocks of four warps walking the deferred list).
-constexpr int DS_BIG_RUN = 64;
-constexpr int DS_BIG_BLOCKS = 38;
+constexpr int DS_BIG_RUN = 16;
+constexpr int DS_BIG_BLOCKS = 152;
 // Blocks of the deletion by pairs (their number is only on the device).
 constexpr int SPEC_BLOCKS = 152;
 
@@ -1376,7 +1379,7 @@ __device__ __forceinline__ bool in_voxel_range(float c, float f, float df, float
 }
 
 __global__ void ds_prepare_kernel(DevTree t, const float* __restrict__ in, int stride, long long n, float ds,
-                                  DsScratch d) {
+                                  int hash_bits, DsScratch d) {
     chain_begin();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) t.st->count = n;  // end of the first sub-batch, until a point cuts it
@@ -1407,7 +1410,7 @@ __global__ void ds_prepare_kernel(DevTree t, const float* __restrict__ in, int s
     // ~16 bits and put up to 7 voxels on one hash).
     uint32_t h = mix32((uint32_t)kb[2] ^ 0x9e3779b9u);
     h = mix32(h ^ (uint32_t)kb[1]);
-    d.hkey[0][i] = mix32(h ^ (uint32_t)kb[0]) & ((1u << DS_HASH_BITS) - 1u);
+    d.hkey[0][i] = mix32(h ^ (uint32_t)kb[0]) & ((1u << hash_bits) - 1u);
     d.hval[0][i] = (uint32_t)i;
 }
 
@@ -1506,7 +1509,7 @@ __device__ __forceinline__ bool half_open_overlap(const Box3& q, const float* lo
 // float-rounding sliver: the group is then folded alone).
 // One team per group; bound by the chain of its walk and, before, by one atomic on
 // the pair counter per bucket with hits: now one per warp and step.  14,400-point
-// scan, 9,000 groups, 300,000 stored points: 65 us with a thread per group on the
+// scan, 9,000 groups, 500,000 stored points: 65 us with a thread per group on the
 // binary nodes, 21 now.
 __global__ void __launch_bounds__(TEAM_CTA) ds_search_kernel(DevTree t, long long n, long long a, DsScratch d, float ds) {
     chain_begin();
@@ -1609,74 +1612,87 @@ __global__ void __launch_bounds__(TEAM_CTA) ds_search_kernel(DevTree t, long lon
 __global__ void __launch_bounds__(128) ds_fold_kernel(DevTree t, long long n, long long a, long long first_id,
                                                       DsScratch d) {
     chain_begin();
-    int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= t.st->n_groups) return;
-    if (t.st->err & ERR_INPUT) return;  // a non-finite input: the call changes nothing
-    // the sub-batch ends where ds_h1_kernel found the first point that must
-    // be folded alone (st->count), and holds at least one point
-    const long long e = min(max((long long)t.st->count, a + 1), n);
-    int j = d.groups[g];
-    int4 info = d.g_info[g];
-    d.g_out[g] = make_int4(0, 0, 0, 0);
-    const uint32_t h = __ldcg(d.hkey[0] + j);
-    if (j + DS_BIG_RUN < n && __ldcg(d.hkey[0] + j + DS_BIG_RUN) == h) {
-        // a long hash run (a voxel with many points): folded by a warp
-        d.big[atomicAdd(d.n_big, 1)] = g;
-        return;
-    }
-    if (info.y == -1 && info.x == 0 && group_first_from(d, n, j, a) < 0) return;
-    const int lead = d.hval[0][j];
-    const int4 k = __ldcg(d.s_key + j);
-    float4 mid = d.mid[lead];
-    float4 best = d.g_best[g];
-    const int n0 = info.x;
-    bool s_is_s0 = true, del_s0 = false, have_ins = false;
-    float cx = 0.f, cy = 0.f, cz = 0.f, cd = 0.f;
-    long long cid = -1;  // id of the current winner c: a stored point keeps its id
-    int triggers = 0;
-    for_run(d, n, j, h, [&](long long, const int4& kk, const float4& p) {
-        if (!same_key(kk, k)) return true;
-        const long long idx = __float_as_int(p.w);
-        if (idx < a) return true;
-        if (idx >= e) return false;  // members come in increasing index order
-        float pd = sq_dist(p.x, p.y, p.z, mid.x, mid.y, mid.z);
-        float wx = p.x, wy = p.y, wz = p.z, wd = pd;
-        long long wid = first_id + idx;
-        bool trig;
-        if (s_is_s0) {
-            if (n0 > 0 && best.w < pd) {
-                wx = best.x; wy = best.y; wz = best.z; wd = best.w;
-                wid = info.z;
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, n_groups = t.st->n_groups, all = gridDim.x * blockDim.x;
+    // Groups are dealt out over the warps before the lanes (first_item): their runs
+    // differ in length and the lanes of a warp wait for the longest.  14,400 points:
+    // 25 us with full warps and runs of up to 64 entries, 14 + 6 (ds_fold_big_kernel)
+    // with up to 16.
+    for (int g0 = first_item() - lane * (all >> 5); g0 < n_groups; g0 += all) {
+        const int g = g0 + lane * (all >> 5);
+        bool have_ins = false;
+        float cx = 0.f, cy = 0.f, cz = 0.f, cd = 0.f;
+        long long cid = -1;  // id of the current winner c: a stored point keeps its id
+        int triggers = 0;
+        // (a non-finite input: the call changes nothing)
+        if (g < n_groups && !(t.st->err & ERR_INPUT)) [&] {
+            // the sub-batch ends where ds_h1_kernel found the first point that must
+            // be folded alone (st->count), and holds at least one point
+            const long long e = min(max((long long)t.st->count, a + 1), n);
+            int j = d.groups[g];
+            int4 info = d.g_info[g];
+            d.g_out[g] = make_int4(0, 0, 0, 0);
+            const uint32_t h = __ldcg(d.hkey[0] + j);
+            if (j + DS_BIG_RUN < n && __ldcg(d.hkey[0] + j + DS_BIG_RUN) == h) {
+                // a long hash run (a voxel with many points): folded by a warp
+                d.big[atomicAdd(d.n_big, 1)] = g;
+                return;
             }
-            trig = n0 > 1 || same_point(p.x, p.y, p.z, wx, wy, wz);
-            if (trig) {
-                del_s0 = n0 > 0;
-                s_is_s0 = false;
-            }
-        } else {
-            if (cd < pd) {
-                wx = cx; wy = cy; wz = cz; wd = cd;
-                wid = cid;
-            }
-            trig = same_point(p.x, p.y, p.z, wx, wy, wz);
-        }
-        if (trig) {
-            ++triggers;
-            cx = wx; cy = wy; cz = wz; cd = wd;
-            cid = wid;
-            have_ins = true;
-        }
-        return true;
-    });
-    d.g_out[g] = make_int4(del_s0 ? 1 : 0, have_ins ? 1 : 0, triggers, 0);
-    if (triggers) atomicAdd((unsigned long long*)&t.st->count2, (unsigned long long)triggers);
-    if (have_ins) {
-        if (cid > MAX_ID) {
+            if (info.y == -1 && info.x == 0 && group_first_from(d, n, j, a) < 0) return;
+            const int lead = d.hval[0][j];
+            const int4 k = __ldcg(d.s_key + j);
+            float4 mid = d.mid[lead];
+            float4 best = d.g_best[g];
+            const int n0 = info.x;
+            bool s_is_s0 = true, del_s0 = false;
+            for_run(d, n, j, h, [&](long long, const int4& kk, const float4& p) {
+                if (!same_key(kk, k)) return true;
+                const long long idx = __float_as_int(p.w);
+                if (idx < a) return true;
+                if (idx >= e) return false;  // members come in increasing index order
+                float pd = sq_dist(p.x, p.y, p.z, mid.x, mid.y, mid.z);
+                float wx = p.x, wy = p.y, wz = p.z, wd = pd;
+                long long wid = first_id + idx;
+                bool trig;
+                if (s_is_s0) {
+                    if (n0 > 0 && best.w < pd) {
+                        wx = best.x; wy = best.y; wz = best.z; wd = best.w;
+                        wid = info.z;
+                    }
+                    trig = n0 > 1 || same_point(p.x, p.y, p.z, wx, wy, wz);
+                    if (trig) {
+                        del_s0 = n0 > 0;
+                        s_is_s0 = false;
+                    }
+                } else {
+                    if (cd < pd) {
+                        wx = cx; wy = cy; wz = cz; wd = cd;
+                        wid = cid;
+                    }
+                    trig = same_point(p.x, p.y, p.z, wx, wy, wz);
+                }
+                if (trig) {
+                    ++triggers;
+                    cx = wx; cy = wy; cz = wz; cd = wd;
+                    cid = wid;
+                    have_ins = true;
+                }
+                return true;
+            });
+            d.g_out[g] = make_int4(del_s0 ? 1 : 0, have_ins ? 1 : 0, triggers, 0);
+        }();
+        // one addition per warp to each counter
+        const int trig = __reduce_add_sync(ALL, triggers);
+        if (lane == 0 && trig) atomicAdd((unsigned long long*)&t.st->count2, (unsigned long long)trig);
+        if (have_ins && cid > MAX_ID) {
             atomicOr(&t.st->err, ERR_ID);
-            return;
+            have_ins = false;
         }
-        int q = atomicAdd(&t.st->n_ins, 1);
-        d.ins[q] = make_float4(cx, cy, cz, __int_as_float((int)cid));
+        const unsigned ins = __ballot_sync(ALL, have_ins);
+        int q = 0;
+        if (lane == 0 && ins) q = atomicAdd(&t.st->n_ins, __popc(ins));
+        q = __shfl_sync(ALL, q, 0) + __popc(ins & ((1u << lane) - 1u));
+        if (have_ins) d.ins[q] = make_float4(cx, cy, cz, __int_as_float((int)cid));
     }
 }
 
@@ -1943,7 +1959,7 @@ void launch_delete_boxes(const DevTree& t, const UpdateAux& a, const float* boxe
                          uint32_t flags, long long* total, cudaStream_t s) {
     if (m <= 0) return;
     // The tree is split below the top until there are units for the whole device
-    // (six boxes in 300,000 points: 33 us with units of 128 buckets, 13 with
+    // (six boxes in 500,000 points: 33 us with units of 128 buckets, 13 with
     // 16); many boxes: not at all.
     int levels = 0, bits = 0;
     while (levels < BD_LEVELS_MAX && bits < t.height && (m << bits) < BD_UNITS) bits += levels++ ? 3 : top_bits;
@@ -2060,10 +2076,9 @@ void carve_ds_scratch(void* base, long long n, long long pair_cap, DsScratch* d)
 void launch_ds_prepare(const DevTree& t, const float* in, int stride, long long n, float ds, DsScratch& d,
                        cudaStream_t s) {
     if (n <= 0) return;
-    launch_chain(ds_prepare_kernel, blocks_for(n, 256), 256, 0, s, t, in, stride, n, ds, d);
-    // 24-bit keys: three passes; the sorted pairs stay where the last pass
-    // left them
-    if (radix_sort_pairs(d.hkey[0], d.hval[0], d.hkey[1], d.hval[1], n, 1, n, DS_HASH_BITS, d.temp, s, false, true)) {
+    launch_chain(ds_prepare_kernel, blocks_for(n, 256), 256, 0, s, t, in, stride, n, ds, ds_hash_bits(n), d);
+    // (the sorted pairs stay where the last pass left them)
+    if (radix_sort_pairs(d.hkey[0], d.hval[0], d.hkey[1], d.hval[1], n, 1, n, ds_hash_bits(n), d.temp, s, false, true)) {
         std::swap(d.hkey[0], d.hkey[1]);
         std::swap(d.hval[0], d.hval[1]);
     }
@@ -2080,7 +2095,7 @@ void launch_ds_search(const DevTree& t, long long n, float ds, long long a, DsSc
 void launch_ds_fold(const DevTree& t, const UpdateAux& aux, long long n, long long a, long long first_id,
                     DsScratch& d, int max_groups, cudaStream_t s) {
     if (max_groups <= 0) return;
-    launch_chain(ds_fold_kernel, blocks_for(max_groups, 128), 128, 0, s, t, n, a, first_id, d);
+    launch_chain(ds_fold_kernel, std::min(blocks_for(max_groups, 4), 152u * 8u), 128, 0, s, t, n, a, first_id, d);
     launch_chain(ds_fold_big_kernel, DS_BIG_BLOCKS, 128, 0, s, t, n, a, first_id, d);
     launch_chain(ds_delete_pairs_kernel, SPEC_BLOCKS, 256, 0, s, t, aux, d);
     launch_chain(ds_delete_kernel, blocks_for((long long)max_groups * TEAM, TEAM_CTA), TEAM_CTA, team_stack_bytes(t.height), s, t, aux, d);

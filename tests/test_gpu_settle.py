@@ -116,3 +116,25 @@ def test_voxel_search_teams(ikdg_mod, monkeypatch, spread):
             assert tree.Add_Points(add, True) == ref.Add_Points(add, True)
             same(tree, ref, rng)
         tree.close()
+
+
+@pytest.mark.parametrize("n", [400, 32768, 32769])
+def test_voxel_groups_of_every_length(ikdg_mod, n):
+    """New points at both hash widths of the grouper, voxels with 1 to 40 of them
+    (folded by a thread or by a warp)."""
+    rng = np.random.default_rng(n)
+    reps = np.resize([1, 1, 2, 3, 15, 16, 17, 18, 33, 40], n)
+    vox = np.repeat(np.arange(n), reps)[:n]
+    corner = np.stack([vox % 37, vox // 37 % 41, vox // (37 * 41)], 1) * 0.5
+    pts = (corner + rng.uniform(0.02, 0.48, (n, 3)))[rng.permutation(n)].astype(np.float32)
+    tree, ref = ikdg_mod.KDTree(0.5, 0.6, 0.5), spec.SpecTree(0.5)
+    base = rng.uniform(0, 20, (200, 3)).astype(np.float32)
+    for t in (tree, ref):
+        t.Build(base)
+    assert tree.Add_Points(pts, True) == ref.Add_Points(pts, True)
+    same(tree, ref, rng)
+    xyz, ids = tree.flatten(with_ids=True)
+    want, wid = ref.valid_points()
+    assert np.array_equal(np.sort(ids), np.sort(wid))
+    assert np.array_equal(xyz[np.argsort(ids)], want[np.argsort(wid)])
+    tree.close()
