@@ -532,7 +532,7 @@ struct Tree {
             // (two blocks per SM fit; the device's own counts bound its loops)
             const long long work = (long long)st->leaf_top + st->node_top;
             const int blocks = (int)std::min<long long>(2 * sm_count, std::max(1ll, (work + 1023) / 1024));
-            CK(launch_settle(dt, aux, first ? ovf_leaf : nullptr, first ? ovf_bound : 0, select, st, blocks, stream));
+            CK(launch_settle(dt, aux, select, st, blocks, stream));
             CK(cudaStreamSynchronize(stream));
             take_status();
             if (st->n_viol == 0 || !select) break;

@@ -140,6 +140,15 @@ __device__ __forceinline__ int child_height(const DevTree& t, int code) {
     return code > 0 ? __ldcg(&t.nheight[code]) : 0;
 }
 
+// A leaf that must be rebuilt (a full bucket that took more points) carries this in
+// job_of_leaf from the moment it is listed until the jobs are chosen.
+constexpr int LEAF_VIOL = -2;
+
+__device__ __forceinline__ void list_leaf_violator(const DevTree& t, const UpdateAux& a, int L) {
+    a.job_of_leaf[L] = LEAF_VIOL;
+    list_push(t.st, &t.st->n_viol, a.viol, a.list_cap, leaf_code(L));
+}
+
 // What a child side tells its node.
 struct Arrival {
     Box3 b;
@@ -293,8 +302,7 @@ __global__ void __launch_bounds__(128) refit_compute_kernel(DevTree t, UpdateAux
             }
             m.slots = n;
             m.height = 0;
-            if (n > LEAF_CAP)  // an overflowing bucket must be split
-                list_push(t.st, &t.st->n_viol, a.viol, a.list_cap, item);
+            if (n > LEAF_CAP) list_leaf_violator(t, a, L);  // an overflowing bucket must be split
         } else {  // the builder wrote the subtree's box and counts into X
             code = side ? r.right() : r.left();
             m.b = r.box(side);
@@ -358,87 +366,92 @@ __global__ void __launch_bounds__(128) refit_compute_kernel(DevTree t, UpdateAux
 
 constexpr int SETTLE_THREADS = 1024;
 
-__device__ __forceinline__ void select_job(const DevTree& t, const UpdateAux& a, int i) {
-    int code = a.viol[i];
-    int link = code < 0 ? t.lparent[code_leaf(code)] : t.nparent[code];
-    if (link < 0) return;
-    int X = link >> 1;
+// The topmost violator on the way from node X up to the root, X included (0: none).
+__device__ __forceinline__ int top_violator(const DevTree& t, const UpdateAux& a, int X) {
+    int top = 0;
     for (int steps = 0; X > 0; ++steps) {
         if (steps > MAX_WALK) {
             atomicOr(&t.st->err, ERR_LOOP);
-            return;
+            return 0;
         }
-        const int flag = a.viol_flag[X], up = t.nparent[X];  // (one round trip for both)
-        if (flag) return;  // an ancestor is rebuilt instead
+        const int flag = __ldcg(a.viol_flag + X), up = __ldcg(t.nparent + X);  // one round trip for both
+        if (flag) top = X;
         X = up >> 1;
     }
-    // One job per subtree even if the violator was listed twice.
-    int* tag = code < 0 ? &a.job_of_leaf[code_leaf(code)] : &a.job_of_node[code];
-    if (atomicCAS(tag, -1, -2) != -1) return;
-    int j = atomicAdd(&t.st->n_jobs, 1);
+    return top;
+}
+
+// A rebuild job for the subtree `code` below `link`; its index, or -1.
+__device__ __forceinline__ int new_job(const DevTree& t, const UpdateAux& a, int code, int link) {
+    const int j = atomicAdd(&t.st->n_jobs, 1);
     if (j >= a.list_cap) {
         atomicOr(&t.st->err, ERR_LIST);
-        return;
+        return -1;
     }
     a.jobs[j] = code;
     a.job_link[j] = link;
-    if (code < 0)
-        a.job_of_leaf[code_leaf(code)] = j;
-    else
-        a.job_of_node[code] = j;
+    return j;
 }
 
-__device__ __forceinline__ int find_job_up(const DevTree& t, const UpdateAux& a, int X) {
-    for (int steps = 0; X > 0; ++steps) {
-        if (steps > MAX_WALK) {
-            atomicOr(&t.st->err, ERR_LOOP);
-            return -1;
-        }
-        const int j = a.job_of_node[X], up = t.nparent[X];  // (one round trip for both)
-        if (j >= 0) return j;
-        X = up >> 1;
+// First pass over leaf L / node X: what it belongs to, into leaf_job / node_job: a
+// violating node (> 0), its own job (-1 - index; leaves only) or nothing (0).  A
+// violator without one above makes its job.
+__device__ __forceinline__ void choose_leaf(const DevTree& t, const UpdateAux& a, int L) {
+    const int lp = __ldcg(t.lparent + L), mark = __ldcg(a.job_of_leaf + L);
+    int top = lp >= 0 ? top_violator(t, a, lp >> 1) : 0;
+    if (mark == LEAF_VIOL) {
+        int j = -1;
+        if (top == 0 && lp >= 0) j = new_job(t, a, leaf_code(L), lp);
+        a.job_of_leaf[L] = j;
+        if (j >= 0) top = -1 - j;
     }
-    return -1;
+    a.leaf_job[L] = top;
+}
+__device__ __forceinline__ void choose_node(const DevTree& t, const UpdateAux& a, int X) {
+    const int link = __ldcg(t.nparent + X);
+    const int top = link >= 0 ? top_violator(t, a, X) : 0;
+    if (top == X) a.job_of_node[X] = new_job(t, a, X, link);
+    a.node_job[X] = top;
 }
 
-__device__ __forceinline__ int count_valid(const DevTree& t, int L) {
-    int n = t.leaf_n[L];
-    int m = n < LEAF_CAP ? n : LEAF_CAP;
-    int v = 0;
+// Valid points among leaf L's first m slots, and those whose deletion is reported
+// (acquire_removed_points).
+__device__ __forceinline__ void count_slots(const DevTree& t, int L, int m, int& valid, int& reported) {
     const float* lw = reinterpret_cast<const float*>(t.pts + (long long)L * LEAF_CAP) + 3;
+    valid = reported = 0;
     // eight flag words in flight (slots past the fill count stay in the bucket)
     for (int j0 = 0; j0 < m; j0 += 8) {
         float w[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) w[u] = lw[4 * (j0 + u)];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v += (j0 + u < m && !(__float_as_uint(w[u]) & F_DEL)) ? 1 : 0;
+        for (int u = 0; u < 8; ++u) {
+            const unsigned f = __float_as_uint(w[u]);
+            if (j0 + u >= m) continue;
+            valid += (f & F_DEL) ? 0 : 1;
+            reported += (f & (F_DEL | F_DSDEL)) == F_DEL ? 1 : 0;
+        }
     }
-    return v;
+}
+__device__ __forceinline__ int count_valid(const DevTree& t, int L) {
+    int valid, reported;
+    count_slots(t, L, min(t.leaf_n[L], LEAF_CAP), valid, reported);
+    return valid;
 }
 
-// The job (or -1) that leaf L / node X belongs to; a leaf's valid points are
-// added to its job's count.
+// Second pass: the index of the job (or -1) of leaf L / node X; a leaf's valid points
+// are added to its job's count, as are those that found its bucket full (leaf_n counts
+// them too).
 __device__ __forceinline__ void count_leaf(const DevTree& t, const UpdateAux& a, int L) {
-    const int lp = t.lparent[L];
-    int j = -1;
-    if (lp >= 0) {
-        j = a.job_of_leaf[L];
-        if (j < 0) j = find_job_up(t, a, lp >> 1);
-    }
+    const int top = a.leaf_job[L];
+    const int j = top > 0 ? __ldcg(a.job_of_node + top) : top < 0 ? -1 - top : -1;
     a.leaf_job[L] = j;
-    if (j >= 0) atomicAdd(&a.job_count[j], count_valid(t, L));
-}
-__device__ __forceinline__ void count_node(const DevTree& t, const UpdateAux& a, int X) {
-    a.node_job[X] = t.nparent[X] < 0 ? -1 : find_job_up(t, a, X);
-}
-// An overflow point joins the job that splits its bucket.
-__device__ __forceinline__ void count_ovf(const DevTree& t, const UpdateAux& a, int L) {
-    const int j = __ldcg(a.leaf_job + L);
+    const int over = t.leaf_n[L] - LEAF_CAP;
     if (j >= 0) {
-        atomicAdd(&a.job_count[j], 1);
+        atomicAdd(&a.job_count[j], count_valid(t, L) + max(over, 0));
         return;
     }
+    if (over <= 0) return;
     atomicOr(&t.st->err, ERR_OVF_JOB);
     int* d = t.st->dbg;
     if (atomicCAS(&d[0], 0, 1) == 0) {
@@ -451,6 +464,10 @@ __device__ __forceinline__ void count_ovf(const DevTree& t, const UpdateAux& a, 
         d[6] = lp >= 0 ? a.viol_flag[lp >> 1] : -7;
         d[7] = t.st->n_ovf;
     }
+}
+__device__ __forceinline__ void count_node(const DevTree& t, const UpdateAux& a, int X) {
+    const int top = a.node_job[X];
+    a.node_job[X] = top > 0 ? __ldcg(a.job_of_node + top) : -1;
 }
 
 // job_off = exclusive prefix sum of job_count over the selected jobs,
@@ -545,15 +562,16 @@ __device__ __forceinline__ void grid_barrier(DevStatus* st) {
 // After a refit: the root's snapshot and, if the refit recorded violators, the
 // rebuild jobs (topmost violators), the job every leaf and node belongs to, the
 // jobs' sizes and offsets; the status block goes to pinned host memory at `host`.
-// Bound by the walks up the tree (select_job, find_job_up): chains of dependent
-// loads, so every leaf and node gets its own thread where the device has them.
-// One cooperative launch with three grid barriers replaces eight small launches
-// and a copy: 60 us of kernels became 33 (14,400-point scan into 500,000 points),
-// and 4 when there is nothing to rebuild; the call as a whole went from 624 to
-// 548 us, a small edit of a 100,000-point map from 773 to 632.  select = false: no
-// jobs, the violators' flags are cleared.
-__global__ void __launch_bounds__(SETTLE_THREADS, 2) settle_kernel(DevTree t, UpdateAux a, const int4* ovf_leaf,
-                                                                int max_ovf, bool select, DevStatus* __restrict__ host) {
+// Bound by the walk up the tree, a chain of dependent loads, so every leaf and node
+// gets its own thread where the device has them, and there is one walk: it finds the
+// topmost violator, which is the job.  One cooperative launch with two grid barriers
+// replaces eight small launches and a copy (500,000 points: 60 us of kernels became
+// 34 with a walk per choice and three barriers, 26 with one and two; 4 when
+// there is nothing to rebuild).  14,400-point scan into 500,000 points, with two
+// such launches: 624 -> 548 us, later 344 -> 338; small edits of 100,000 points
+// 773 -> 632, later 455 -> 418.  select = false: no jobs, the marks are cleared.
+__global__ void __launch_bounds__(SETTLE_THREADS, 2) settle_kernel(DevTree t, UpdateAux a, bool select,
+                                                                   DevStatus* __restrict__ host) {
     DevStatus* st = t.st;
     const int nv = min(__ldcg(&st->n_viol), a.list_cap);
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
@@ -562,28 +580,34 @@ __global__ void __launch_bounds__(SETTLE_THREADS, 2) settle_kernel(DevTree t, Up
         st->n_items = 0;  // the dirty list is consumed
     }
     if (nv > 0 && select) {
-        for (int i = i0; i < nv; i += step) select_job(t, a, i);
-        grid_barrier(st);
         const int leaf_top = min(__ldcg(&st->leaf_top), t.leaf_cap), node_top = min(__ldcg(&st->node_top), t.node_cap);
+        const int all = leaf_top + node_top;
+        for (int i = i0; i < all; i += step) {
+            if (i < leaf_top)
+                choose_leaf(t, a, i);
+            else if (i > leaf_top)
+                choose_node(t, a, i - leaf_top);
+        }
+        grid_barrier(st);
         for (int i = i0; i < nv; i += step) {
             const int code = a.viol[i];
             if (code > 0) a.viol_flag[code] = 0;
         }
-        for (int i = i0; i < leaf_top + node_top; i += step) {
+        for (int i = i0; i < all; i += step) {
             if (i < leaf_top)
                 count_leaf(t, a, i);
             else if (i > leaf_top)
                 count_node(t, a, i - leaf_top);
         }
         grid_barrier(st);
-        const int no = min(__ldcg(&st->n_ovf), max_ovf);
-        for (int o = i0; o < no; o += step) count_ovf(t, a, ovf_leaf[o].x);
-        grid_barrier(st);
         if (blockIdx.x == 0) job_scan(t, a);
     } else if (nv > 0) {
         for (int i = i0; i < nv; i += step) {
             const int code = a.viol[i];
-            if (code > 0) a.viol_flag[code] = 0;
+            if (code > 0)
+                a.viol_flag[code] = 0;
+            else
+                a.job_of_leaf[code_leaf(code)] = -1;
         }
         grid_barrier(st);  // every block has read n_viol
     }
@@ -596,15 +620,11 @@ __global__ void __launch_bounds__(SETTLE_THREADS, 2) settle_kernel(DevTree t, Up
     if (threadIdx.x == 0) st->n_viol = 0;  // the next refit records afresh
 }
 
-__device__ __forceinline__ void gather_leaf(const DevTree& t, const UpdateAux& a, int L, float4* __restrict__ out,
-                                            float4* __restrict__ removed, long long removed_cap) {
-    int j = a.leaf_job[L];
-    if (j < 0) return;
-    int n = t.leaf_n[L];
-    int m = n < LEAF_CAP ? n : LEAF_CAP;
+// The points of leaf L's job from place `pos` of out on, its deleted ones from `rem` of
+// removed on.
+__device__ __forceinline__ void gather_leaf(const DevTree& t, int L, int m, float4* __restrict__ out, int pos,
+                                            float4* __restrict__ removed, long long rem, long long removed_cap) {
     const float4* lp = t.pts + (long long)L * LEAF_CAP;
-    int nv = count_valid(t, L);
-    int pos = a.job_off[j] + atomicAdd(&a.job_fill[j], nv);
     for (int s0 = 0; s0 < m; s0 += 8) {
         float4 pb[8];  // eight slots in flight (the bucket always has LEAF_CAP slots)
 #pragma unroll
@@ -619,39 +639,71 @@ __device__ __forceinline__ void gather_leaf(const DevTree& t, const UpdateAux& a
             } else if (!(w & F_DSDEL)) {
                 // Dropped deleted points are kept for acquire_removed_points
                 // (flatten with DELETE_POINTS_REC, ikd_Tree.cpp:1338-1342).
-                long long r = atomicAdd((unsigned long long*)&t.st->removed_n, 1ull);
-                if (r < removed_cap) removed[r] = make_float4(p.x, p.y, p.z, __uint_as_float(w & ID_MASK));
+                if (rem < removed_cap) removed[rem] = make_float4(p.x, p.y, p.z, __uint_as_float(w & ID_MASK));
+                ++rem;
             }
         }
     }
-    t.lparent[L] = -1;
-    t.leaf_n[L] = 0;
-    int f = atomicAdd(&t.st->free_leaf_n, 1);
-    t.free_leaf[f] = L;
+}
+
+// A place for each lane that wants n of something counted at `counter`: one addition
+// per warp.
+template <class T>
+__device__ __forceinline__ T warp_places(T* counter, int n) {
+    const int lane = threadIdx.x & 31;
+    int inc = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    T base = 0;
+    if (lane == 31 && inc) base = atomicAdd(counter, (T)inc);
+    return __shfl_sync(0xffffffffu, base, 31) + (T)(inc - n);
 }
 
 // The points of every job into `out`, back to back; the jobs' leaves and nodes go
-// to the free stacks.  One thread per leaf, node and overflow point.
+// to the free stacks.  One thread per leaf, node and overflow point; the shared
+// counters take one addition per warp (500,000 points: 13 -> 8 us).
 __global__ void job_gather_kernel(DevTree t, UpdateAux a, int leaf_top, int node_top, const int4* ovf_leaf,
                                   const float4* ovf_pts, int max_ovf, float4* __restrict__ out,
                                   float4* __restrict__ removed, long long removed_cap) {
     chain_begin();
+    constexpr unsigned ALL = 0xffffffffu;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < leaf_top) {
-        gather_leaf(t, a, i, out, removed, removed_cap);
-        return;
+    // leaves, then nodes: whole warps stay together for the shared additions
+    const int j = i < leaf_top ? a.leaf_job[i] : -1;
+    if (__any_sync(ALL, j >= 0)) {
+        int m = 0, nv = 0, nd = 0;
+        if (j >= 0) {
+            m = min(t.leaf_n[i], LEAF_CAP);
+            count_slots(t, i, m, nv, nd);
+        }
+        const int pos = j >= 0 ? a.job_off[j] + atomicAdd(&a.job_fill[j], nv) : 0;
+        const long long rem = (long long)warp_places((unsigned long long*)&t.st->removed_n, nd);
+        const int f = warp_places(&t.st->free_leaf_n, j >= 0 ? 1 : 0);
+        if (j >= 0) {
+            gather_leaf(t, i, m, out, pos, removed, rem, removed_cap);
+            t.lparent[i] = -1;
+            t.leaf_n[i] = 0;
+            t.free_leaf[f] = i;
+        }
     }
-    i -= leaf_top;
-    if (i < node_top) {
-        if (i < 1 || a.node_job[i] < 0) return;
-        t.nparent[i] = -1;
-        t.free_node[atomicAdd(&t.st->free_node_n, 1)] = i;
-        return;
+    const int X = i - leaf_top;
+    const bool node = X >= 1 && X < node_top && a.node_job[X] >= 0;
+    if (__any_sync(ALL, node)) {
+        const int f = warp_places(&t.st->free_node_n, node ? 1 : 0);
+        if (node) {
+            t.nparent[X] = -1;
+            t.free_node[f] = X;
+        }
     }
+    if (X < node_top) return;
+    i = X;
     i -= node_top;
     if (i >= min(max_ovf, t.st->n_ovf)) return;
-    const int j = a.leaf_job[ovf_leaf[i].x];
-    if (j >= 0) out[a.job_off[j] + atomicAdd(&a.job_fill[j], 1)] = ovf_pts[i];
+    const int jo = a.leaf_job[ovf_leaf[i].x];
+    if (jo >= 0) out[a.job_off[jo] + atomicAdd(&a.job_fill[jo], 1)] = ovf_pts[i];
 }
 
 // Resets per-job state and queues each job's parent for the follow-up refit
@@ -1128,6 +1180,11 @@ __global__ void select_root_kernel(DevTree t, UpdateAux a) {
     chain_begin();
     const int code = __float_as_int(t.node[3].x);
     if (code == 0) return;
+    if (code < 0) {
+        list_leaf_violator(t, a, code_leaf(code));
+        return;
+    }
+    a.viol_flag[code] = 1;
     a.viol[0] = code;
     t.st->n_viol = 1;
 }
@@ -1299,10 +1356,10 @@ __global__ void validate_aux_nodes_kernel(DevTree t, UpdateAux a, bool at_rest, 
     }
 }
 
-__global__ void validate_aux_leaves_kernel(DevTree t, UpdateAux a, unsigned long long* bad) {
+__global__ void validate_aux_leaves_kernel(DevTree t, UpdateAux a, bool at_rest, unsigned long long* bad) {
     int L = blockIdx.x * blockDim.x + threadIdx.x;
     if (L >= t.leaf_cap) return;
-    if (a.dirty_flag[L] != 0 || a.job_of_leaf[L] != -1) {
+    if (a.dirty_flag[L] != 0 || (a.job_of_leaf[L] != -1 && (at_rest || a.job_of_leaf[L] != LEAF_VIOL))) {
         atomicAdd(bad, 1ull);
         note_bad(t.st, 111, L, a.dirty_flag[L], a.job_of_leaf[L], L < t.st->leaf_top ? t.lparent[L] : -9, 0, 0);
     }
@@ -1934,11 +1991,11 @@ void launch_refit(const DevTree& t, const UpdateAux& a, const int* items, const 
 }
 
 
-cudaError_t launch_settle(const DevTree& t, const UpdateAux& a, const int4* ovf_leaf, int max_ovf, bool select,
-                          DevStatus* host, int blocks, cudaStream_t s) {
+cudaError_t launch_settle(const DevTree& t, const UpdateAux& a, bool select, DevStatus* host, int blocks,
+                          cudaStream_t s) {
     DevTree tt = t;
     UpdateAux aa = a;
-    void* args[] = {&tt, &aa, &ovf_leaf, &max_ovf, &select, &host};
+    void* args[] = {&tt, &aa, &select, &host};
     return cudaLaunchCooperativeKernel((const void*)settle_kernel, dim3(blocks), dim3(SETTLE_THREADS), args, 0, s);
 }
 
@@ -1994,7 +2051,7 @@ void launch_validate(const DevTree& t, const UpdateAux& a, bool at_rest, long lo
     if (t.node_cap > 0)
         validate_aux_nodes_kernel<<<blocks_for(t.node_cap, 256), 256, 0, s>>>(t, a, at_rest, (unsigned long long*)bad);
     if (t.leaf_cap > 0)
-        validate_aux_leaves_kernel<<<blocks_for(t.leaf_cap, 256), 256, 0, s>>>(t, a, (unsigned long long*)bad);
+        validate_aux_leaves_kernel<<<blocks_for(t.leaf_cap, 256), 256, 0, s>>>(t, a, at_rest, (unsigned long long*)bad);
 }
 
 void launch_flatten(const DevTree& t, float4* out, long long* counter, cudaStream_t s) {

@@ -43,8 +43,8 @@ void launch_refit(const DevTree& t, const UpdateAux& a, const int* items, const 
 // After a refit: root snapshot, selection of the topmost violators as rebuild
 // jobs, their sizes; the status goes to `host` (pinned).  `blocks`: at most two
 // per SM (cooperative launch).
-cudaError_t launch_settle(const DevTree& t, const UpdateAux& a, const int4* ovf_leaf, int max_ovf, bool select,
-                          DevStatus* host, int blocks, cudaStream_t s);
+cudaError_t launch_settle(const DevTree& t, const UpdateAux& a, bool select, DevStatus* host, int blocks,
+                          cudaStream_t s);
 // Gathers the valid points of every job (plus overflow points).
 void launch_job_gather(const DevTree& t, const UpdateAux& a, int leaf_top, int node_top, const int4* ovf_leaf,
                        const float4* ovf_pts, int max_ovf, float4* out, float4* removed, long long removed_cap,
