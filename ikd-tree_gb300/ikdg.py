@@ -493,7 +493,7 @@ class Batch:
         return tot[:n_range]
 
     def autotune(self, reps: int = 3) -> np.ndarray:
-        """Picks leaf fill and kNN lanes per tree; returns {fill, lanes} rows."""
+        """Picks the leaf fill per tree; returns {fill, lanes} rows (lanes is 1)."""
         n = C.c_int32()
         self._check(self.lib.ikdg_batch_num_trees(self.h, C.byref(n)), "batch_num_trees")
         out = np.zeros((max(n.value, 1), 2), np.int32)
