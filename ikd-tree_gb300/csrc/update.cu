@@ -365,6 +365,7 @@ __global__ void __launch_bounds__(128) refit_compute_kernel(DevTree t, UpdateAux
 // ---- rebuild jobs ----------------------------------------------------------------
 
 constexpr int SETTLE_THREADS = 1024;
+constexpr int LIST_THREADS = 512;  // (settle_kernel<true>, which needs the registers)
 
 // The topmost violator on the way from node X up to the root, X included (0: none).
 __device__ __forceinline__ int top_violator(const DevTree& t, const UpdateAux& a, int X) {
@@ -559,6 +560,100 @@ __device__ __forceinline__ void grid_barrier(DevStatus* st) {
     __syncthreads();
 }
 
+// A place for each lane that wants n of something counted at `counter`: one addition
+// per warp.
+template <class T>
+__device__ __forceinline__ T warp_places(T* counter, int n) {
+    const int lane = threadIdx.x & 31;
+    int inc = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    T base = 0;
+    if (lane == 31 && inc) base = atomicAdd(counter, (T)inc);
+    return __shfl_sync(0xffffffffu, base, 31) + (T)(inc - n);
+}
+
+// ---- the same on a map with more leaves and nodes than the device has threads: from
+// the violators up, then from the jobs down
+
+// Violator i becomes a job unless one of its ancestors violates too.
+__device__ __forceinline__ void choose_violator(const DevTree& t, const UpdateAux& a, int i) {
+    const int code = a.viol[i], L = code < 0 ? code_leaf(code) : 0;
+    const int link = code < 0 ? __ldcg(t.lparent + L) : __ldcg(t.nparent + code);
+    int j = -1;
+    if (link >= 0 && top_violator(t, a, link >> 1) == 0) j = new_job(t, a, code, link);
+    if (code < 0) {
+        a.job_of_leaf[L] = j;
+        if (j >= 0) a.leaf_job[L] = j;
+    } else if (j >= 0) {
+        a.job_of_node[code] = j;
+        a.node_job[code] = j;
+    }
+}
+
+// Everything below the jobs into a.items: leaf codes, and 2 * node + 1 for nodes whose
+// children are listed too (2 * node: in the next round).  A round takes three levels, a
+// thread per node; its entries follow those of the rounds before.  Ends with a grid
+// barrier; returns the number of entries.
+constexpr int LIST_ROUNDS = sizeof(DevStatus::level_n) / sizeof(int);
+static_assert(3 * (LIST_ROUNDS - 1) > MAX_STACK, "a round takes three levels");
+__device__ int list_jobs(const DevTree& t, const UpdateAux& a, int i0, int step) {
+    DevStatus* st = t.st;
+    const int lane = threadIdx.x & 31;
+    int begin = 0, end = min(__ldcg(&st->n_jobs), a.list_cap);
+    for (int i = i0; i < end; i += step) {
+        const int c = __ldcg(a.jobs + i);
+        a.items[i] = c < 0 ? c : 2 * c;
+    }
+    for (int r = 0; r < LIST_ROUNDS && end > begin; ++r) {
+        for (int i = begin + i0; i - lane < end; i += step) {  // (whole warps: one reservation each)
+            const int item = i < end ? __ldcg(a.items + i) : -1;
+            const bool open = item > 0 && !(item & 1);
+            // children, grandchildren and theirs: the loads of one level go out together
+            int c[14];
+            int j = 0, n = 0;
+            auto kids = [&](int X, int at) {
+                float2 k = make_float2(0.f, 0.f);
+                if (X > 0) k = __ldcg(reinterpret_cast<const float2*>(t.node + 4 * X + 3));
+                c[at] = __float_as_int(k.x);
+                c[at + 1] = __float_as_int(k.y);
+            };
+            if (open) j = __ldcg(a.node_job + (item >> 1));
+            kids(open ? item >> 1 : 0, 0);
+#pragma unroll
+            for (int u = 0; u < 6; ++u) kids(c[u], 2 + 2 * u);
+#pragma unroll
+            for (int u = 0; u < 14; ++u) n += c[u] != 0 ? 1 : 0;
+            int at = end + warp_places(&st->level_n[r], n);
+            if (n > 0 && at + n > a.list_cap) {
+                atomicOr(&st->err, ERR_LIST);
+                continue;
+            }
+#pragma unroll
+            for (int u = 0; u < 14; ++u) {
+                if (c[u] == 0) continue;
+                if (c[u] < 0)
+                    a.leaf_job[code_leaf(c[u])] = j;
+                else
+                    a.node_job[c[u]] = j;
+                a.items[at++] = c[u] < 0 ? c[u] : 2 * c[u] + (u < 6 ? 1 : 0);
+            }
+        }
+        grid_barrier(st);
+        begin = end;
+        end = min(end + __ldcg(&st->level_n[r]), a.list_cap);
+    }
+    return end;
+}
+
+// A listed leaf's points, those that found its bucket full included.
+__device__ __forceinline__ void count_listed(const DevTree& t, const UpdateAux& a, int L) {
+    atomicAdd(&a.job_count[__ldcg(a.leaf_job + L)], count_valid(t, L) + max(__ldcg(t.leaf_n + L) - LEAF_CAP, 0));
+}
+
 // After a refit: the root's snapshot and, if the refit recorded violators, the
 // rebuild jobs (topmost violators), the job every leaf and node belongs to, the
 // jobs' sizes and offsets; the status block goes to pinned host memory at `host`.
@@ -569,8 +664,11 @@ __device__ __forceinline__ void grid_barrier(DevStatus* st) {
 // 34 with a walk per choice and three barriers, 26 with one and two; 4 when
 // there is nothing to rebuild).  14,400-point scan into 500,000 points, with two
 // such launches: 624 -> 548 us, later 344 -> 338; small edits of 100,000 points
-// 773 -> 632, later 455 -> 418.  select = false: no jobs, the marks are cleared.
-__global__ void __launch_bounds__(SETTLE_THREADS, 2) settle_kernel(DevTree t, UpdateAux a, bool select,
+// 773 -> 632, later 455 -> 418.  LIST: from the violators up and from the jobs down
+// (list_jobs), for maps where a walk from every leaf costs more than that chain of
+// rounds.  select = false: no jobs, the marks are cleared.
+template <bool LIST>
+__global__ void __launch_bounds__(LIST ? LIST_THREADS : SETTLE_THREADS, 2) settle_kernel(DevTree t, UpdateAux a, bool select,
                                                                    DevStatus* __restrict__ host) {
     DevStatus* st = t.st;
     const int nv = min(__ldcg(&st->n_viol), a.list_cap);
@@ -582,22 +680,35 @@ __global__ void __launch_bounds__(SETTLE_THREADS, 2) settle_kernel(DevTree t, Up
     if (nv > 0 && select) {
         const int leaf_top = min(__ldcg(&st->leaf_top), t.leaf_cap), node_top = min(__ldcg(&st->node_top), t.node_cap);
         const int all = leaf_top + node_top;
-        for (int i = i0; i < all; i += step) {
-            if (i < leaf_top)
-                choose_leaf(t, a, i);
-            else if (i > leaf_top)
-                choose_node(t, a, i - leaf_top);
+        if (LIST) {
+            for (int i = i0; i < nv; i += step) choose_violator(t, a, i);
+        } else {
+            for (int i = i0; i < all; i += step) {
+                if (i < leaf_top)
+                    choose_leaf(t, a, i);
+                else if (i > leaf_top)
+                    choose_node(t, a, i - leaf_top);
+            }
         }
         grid_barrier(st);
         for (int i = i0; i < nv; i += step) {
             const int code = a.viol[i];
             if (code > 0) a.viol_flag[code] = 0;
         }
-        for (int i = i0; i < all; i += step) {
-            if (i < leaf_top)
-                count_leaf(t, a, i);
-            else if (i > leaf_top)
-                count_node(t, a, i - leaf_top);
+        if (LIST) {
+            const int n = list_jobs(t, a, i0, step);
+            for (int i = i0; i < n; i += step) {
+                const int item = __ldcg(a.items + i);
+                if (item < 0) count_listed(t, a, code_leaf(item));
+            }
+            if (i0 == 0) st->n_queue = n;
+        } else {
+            for (int i = i0; i < all; i += step) {
+                if (i < leaf_top)
+                    count_leaf(t, a, i);
+                else if (i > leaf_top)
+                    count_node(t, a, i - leaf_top);
+            }
         }
         grid_barrier(st);
         if (blockIdx.x == 0) job_scan(t, a);
@@ -646,64 +757,57 @@ __device__ __forceinline__ void gather_leaf(const DevTree& t, int L, int m, floa
     }
 }
 
-// A place for each lane that wants n of something counted at `counter`: one addition
-// per warp.
-template <class T>
-__device__ __forceinline__ T warp_places(T* counter, int n) {
-    const int lane = threadIdx.x & 31;
-    int inc = n;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
-    }
-    T base = 0;
-    if (lane == 31 && inc) base = atomicAdd(counter, (T)inc);
-    return __shfl_sync(0xffffffffu, base, 31) + (T)(inc - n);
-}
-
 // The points of every job into `out`, back to back; the jobs' leaves and nodes go
-// to the free stacks.  One thread per leaf, node and overflow point; the shared
+// to the free stacks.  One thread per leaf and node (n_queue
+// of them listed in a.items, or, below zero, all of the map's) and overflow point; the shared
 // counters take one addition per warp (500,000 points: 13 -> 8 us).
-__global__ void job_gather_kernel(DevTree t, UpdateAux a, int leaf_top, int node_top, const int4* ovf_leaf,
+__global__ void job_gather_kernel(DevTree t, UpdateAux a, int n_queue, int leaf_top, int node_top, const int4* ovf_leaf,
                                   const float4* ovf_pts, int max_ovf, float4* __restrict__ out,
                                   float4* __restrict__ removed, long long removed_cap) {
     chain_begin();
     constexpr unsigned ALL = 0xffffffffu;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    // leaves, then nodes: whole warps stay together for the shared additions
-    const int j = i < leaf_top ? a.leaf_job[i] : -1;
-    if (__any_sync(ALL, j >= 0)) {
-        int m = 0, nv = 0, nd = 0;
-        if (j >= 0) {
-            m = min(t.leaf_n[i], LEAF_CAP);
-            count_slots(t, i, m, nv, nd);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int all = n_queue >= 0 ? n_queue : leaf_top + node_top;
+    // this thread's leaf L or node X, -1: none; whole warps stay together for the
+    // shared additions
+    int L = -1, X = -1;
+    if (n_queue >= 0) {
+        const int item = i < all ? a.items[i] : 0;
+        if (item < 0) L = code_leaf(item);
+        if (item > 0) X = item >> 1;
+    } else if (i < leaf_top) {
+        if (a.leaf_job[i] >= 0) L = i;
+    } else if (i > leaf_top && i < all && a.node_job[i - leaf_top] >= 0) {
+        X = i - leaf_top;
+    }
+    if (__any_sync(ALL, L >= 0)) {
+        int m = 0, nv = 0, nd = 0, pos = 0;
+        if (L >= 0) {
+            const int j = a.leaf_job[L];
+            m = min(t.leaf_n[L], LEAF_CAP);
+            count_slots(t, L, m, nv, nd);
+            pos = a.job_off[j] + atomicAdd(&a.job_fill[j], nv);
         }
-        const int pos = j >= 0 ? a.job_off[j] + atomicAdd(&a.job_fill[j], nv) : 0;
         const long long rem = (long long)warp_places((unsigned long long*)&t.st->removed_n, nd);
-        const int f = warp_places(&t.st->free_leaf_n, j >= 0 ? 1 : 0);
-        if (j >= 0) {
-            gather_leaf(t, i, m, out, pos, removed, rem, removed_cap);
-            t.lparent[i] = -1;
-            t.leaf_n[i] = 0;
-            t.free_leaf[f] = i;
+        const int f = warp_places(&t.st->free_leaf_n, L >= 0 ? 1 : 0);
+        if (L >= 0) {
+            gather_leaf(t, L, m, out, pos, removed, rem, removed_cap);
+            t.lparent[L] = -1;
+            t.leaf_n[L] = 0;
+            t.free_leaf[f] = L;
         }
     }
-    const int X = i - leaf_top;
-    const bool node = X >= 1 && X < node_top && a.node_job[X] >= 0;
-    if (__any_sync(ALL, node)) {
-        const int f = warp_places(&t.st->free_node_n, node ? 1 : 0);
-        if (node) {
+    if (__any_sync(ALL, X >= 0)) {
+        const int f = warp_places(&t.st->free_node_n, X >= 0 ? 1 : 0);
+        if (X >= 0) {
             t.nparent[X] = -1;
             t.free_node[f] = X;
         }
     }
-    if (X < node_top) return;
-    i = X;
-    i -= node_top;
-    if (i >= min(max_ovf, t.st->n_ovf)) return;
-    const int jo = a.leaf_job[ovf_leaf[i].x];
-    if (jo >= 0) out[a.job_off[jo] + atomicAdd(&a.job_fill[jo], 1)] = ovf_pts[i];
+    const int o = i - all;
+    if (o < 0 || o >= min(max_ovf, t.st->n_ovf)) return;
+    const int jo = a.leaf_job[ovf_leaf[o].x];
+    if (jo >= 0) out[a.job_off[jo] + atomicAdd(&a.job_fill[jo], 1)] = ovf_pts[o];
 }
 
 // Resets per-job state and queues each job's parent for the follow-up refit
@@ -729,6 +833,8 @@ __global__ void __launch_bounds__(1024) job_finish_kernel(DevTree t, UpdateAux a
         t.st->n_ovf = 0;
         t.st->n_jobs = 0;
         t.st->barrier = 0;  // the next settle_kernel may have another grid
+        t.st->n_queue = 0;
+        for (int r = 0; r < LIST_ROUNDS; ++r) t.st->level_n[r] = 0;
     }
 }
 
@@ -1991,21 +2097,22 @@ void launch_refit(const DevTree& t, const UpdateAux& a, const int* items, const 
 }
 
 
-cudaError_t launch_settle(const DevTree& t, const UpdateAux& a, bool select, DevStatus* host, int blocks,
+cudaError_t launch_settle(const DevTree& t, const UpdateAux& a, bool select, DevStatus* host, bool list, int blocks,
                           cudaStream_t s) {
     DevTree tt = t;
     UpdateAux aa = a;
     void* args[] = {&tt, &aa, &select, &host};
-    return cudaLaunchCooperativeKernel((const void*)settle_kernel, dim3(blocks), dim3(SETTLE_THREADS), args, 0, s);
+    return cudaLaunchCooperativeKernel(list ? (const void*)settle_kernel<true> : (const void*)settle_kernel<false>,
+                                       dim3(blocks), dim3(list ? LIST_THREADS : SETTLE_THREADS), args, 0, s);
 }
 
-void launch_job_gather(const DevTree& t, const UpdateAux& a, int leaf_top, int node_top, const int4* ovf_leaf,
-                       const float4* ovf_pts, int max_ovf, float4* out, float4* removed, long long removed_cap,
-                       cudaStream_t s) {
-    const long long n = (long long)leaf_top + node_top + max_ovf;
+void launch_job_gather(const DevTree& t, const UpdateAux& a, int n_queue, int leaf_top, int node_top,
+                       const int4* ovf_leaf, const float4* ovf_pts, int max_ovf, float4* out, float4* removed,
+                       long long removed_cap, cudaStream_t s) {
+    const long long n = (n_queue >= 0 ? (long long)n_queue : (long long)leaf_top + node_top) + max_ovf;
     if (n > 0)
-        launch_chain(job_gather_kernel, blocks_for(n, 256), 256, 0, s, t, a, leaf_top, node_top, ovf_leaf, ovf_pts, max_ovf, out,
-                                                             removed, removed_cap);
+        launch_chain(job_gather_kernel, blocks_for(n, 256), 256, 0, s, t, a, n_queue, leaf_top, node_top, ovf_leaf,
+                     ovf_pts, max_ovf, out, removed, removed_cap);
 }
 
 void launch_job_finish(const DevTree& t, const UpdateAux& a, cudaStream_t s) {

@@ -40,14 +40,17 @@ void launch_route_append(const DevTree& t, const UpdateAux& a, const float4* pts
 // clears the dirty flags of the listed leaves.
 void launch_refit(const DevTree& t, const UpdateAux& a, const int* items, const int* n_items, int max_items,
                   const Criteria& c, cudaStream_t s);
+constexpr long long SETTLE_LIST = 131072;  // leaves and nodes above which the jobs list theirs
 // After a refit: root snapshot, selection of the topmost violators as rebuild
 // jobs, their sizes; the status goes to `host` (pinned).  `blocks`: at most two
-// per SM (cooperative launch).
-cudaError_t launch_settle(const DevTree& t, const UpdateAux& a, bool select, DevStatus* host, int blocks,
-                          cudaStream_t s);
-// Gathers the valid points of every job (plus overflow points).
-void launch_job_gather(const DevTree& t, const UpdateAux& a, int leaf_top, int node_top, const int4* ovf_leaf,
-                       const float4* ovf_pts, int max_ovf, float4* out, float4* removed, long long removed_cap,
+// per SM (cooperative launch).  list: the jobs' leaves and nodes are listed in a.items
+// (st->n_queue) instead of marked in leaf_job / node_job of the whole map.
+cudaError_t launch_settle(const DevTree& t, const UpdateAux& a, bool select, DevStatus* host, bool list,
+                          int blocks, cudaStream_t s);
+// Gathers the valid points of every job (its leaves: n_queue listed ones, or below zero
+// the marked ones of the map) (plus overflow points).
+void launch_job_gather(const DevTree& t, const UpdateAux& a, int n_queue, int leaf_top, int node_top,
+                       const int4* ovf_leaf, const float4* ovf_pts, int max_ovf, float4* out, float4* removed, long long removed_cap,
                        cudaStream_t s);
 void launch_job_finish(const DevTree& t, const UpdateAux& a, cudaStream_t s);
 // Delete every valid point inside each box; `flags` = F_DEL or F_DEL|F_DSDEL;

@@ -20,7 +20,7 @@ def same(tree, ref, rng):
     assert np.array_equal(ids, rid) and np.array_equal(d2, rd2)
 
 
-@pytest.mark.parametrize("n", [1, 31, 33, 2000, 40000, 700001])
+@pytest.mark.parametrize("n", [1, 31, 33, 2000, 40000, 700001, 1060000])
 def test_edit_sequences(ikdg_mod, n):
     rng = np.random.default_rng(n)
     pts = rng.uniform(-50, 50, (n, 3)).astype(np.float32)
@@ -137,4 +137,28 @@ def test_voxel_groups_of_every_length(ikdg_mod, n):
     want, wid = ref.valid_points()
     assert np.array_equal(np.sort(ids), np.sort(wid))
     assert np.array_equal(xyz[np.argsort(ids)], want[np.argsort(wid)])
+    tree.close()
+
+
+def test_rebuild_jobs_of_a_large_map(ikdg_mod):
+    """So many leaves and nodes that the jobs list what is below them.  Overflowing buckets, scattered jobs, one large job, the whole tree."""
+    rng = np.random.default_rng(8)
+    n = 2_900_000
+    pts = rng.uniform(-50, 50, (n, 3)).astype(np.float32)
+    tree, ref = ikdg_mod.KDTree(0.3, 0.6, 0.5), spec.SpecTree(0.5)
+    for t in (tree, ref):
+        t.Build(pts)
+    spot = rng.uniform(10, 10.4, (3000, 3)).astype(np.float32)
+    for t in (tree, ref):
+        t.Add_Points(spot, False)
+    same(tree, ref, rng)
+    cubes = rng.uniform(-50, 47, (60, 3))
+    for boxes in (np.c_[cubes, cubes + 3], np.array([[-50, -50, -50, -20, 50, 50]]), np.array([[0, 0, 0, 1e-3, 1, 1]])):
+        boxes = boxes.astype(np.float32)
+        assert tree.Delete_Point_Boxes(boxes) == ref.Delete_Point_Boxes(boxes)
+        same(tree, ref, rng)
+    tree.rebuild()
+    same(tree, ref, rng)
+    gone = tree.acquire_removed_points()
+    assert len(gone) + tree.validnum() == n + len(spot)
     tree.close()
