@@ -533,9 +533,11 @@ struct Tree {
             // jobs list theirs (an insertion of 5,000 points with rebuilds: 100,000
             // points 123 us looking, 128 listing; 1,000,000: 139 and 134; 20,000,000:
             // 681 and 168).
+            // Free pool entries cost the walk one load each.
             const long long work = (long long)st->leaf_top + st->node_top;
-            const bool list = work > SETTLE_LIST;
-            const int blocks = list ? sm_count : (int)std::max(1ll, (work + 1023) / 1024);
+            const long long live = work - st->free_leaf_n - st->free_node_n;
+            const bool list = live > SETTLE_LIST || work > 8 * SETTLE_LIST;
+            const int blocks = list ? sm_count : (int)std::min(2ll * sm_count, std::max(1ll, (work + 1023) / 1024));
             CK(launch_settle(dt, aux, select, st, list, blocks, stream));
             CK(cudaStreamSynchronize(stream));
             take_status();

@@ -40,7 +40,7 @@ void launch_route_append(const DevTree& t, const UpdateAux& a, const float4* pts
 // clears the dirty flags of the listed leaves.
 void launch_refit(const DevTree& t, const UpdateAux& a, const int* items, const int* n_items, int max_items,
                   const Criteria& c, cudaStream_t s);
-constexpr long long SETTLE_LIST = 131072;  // leaves and nodes above which the jobs list theirs
+constexpr long long SETTLE_LIST = 131072;  // live leaves and nodes above which the jobs list theirs
 // After a refit: root snapshot, selection of the topmost violators as rebuild
 // jobs, their sizes; the status goes to `host` (pinned).  `blocks`: at most two
 // per SM (cooperative launch).  list: the jobs' leaves and nodes are listed in a.items
