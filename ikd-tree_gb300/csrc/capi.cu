@@ -413,10 +413,6 @@ struct Tree {
     void reset_counters() {
         zero_fields(offsetof(DevStatus, err), offsetof(DevStatus, bad) - offsetof(DevStatus, err));
     }
-    void set_status_ll(size_t off, long long v) {
-        CK(cudaMemcpyAsync((char*)st_dev + off, &v, sizeof(v), cudaMemcpyHostToDevice, stream));
-        CK(cudaStreamSynchronize(stream));  // v lives on this stack frame
-    }
 
     // Empty tree: pools cleared, sentinel with no children.
     void reset_tree() {

@@ -367,15 +367,5 @@ __device__ __forceinline__ int pool_pick(const PoolRun& r, const int* free_list,
     }
     return x;
 }
-__device__ __forceinline__ int alloc_leaf(const DevTree& t) {
-    int k = atomicAdd(&t.st->free_leaf_taken, 1);
-    if (k < t.st->free_leaf_n) return t.free_leaf[t.st->free_leaf_n - 1 - k];
-    int n = atomicAdd(&t.st->leaf_top, 1);
-    if (n >= t.leaf_cap) {
-        atomicOr(&t.st->err, ERR_POOL_LEAF);
-        return -1;
-    }
-    return n;
-}
 
 }  // namespace ikdg

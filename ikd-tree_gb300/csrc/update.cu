@@ -2065,12 +2065,6 @@ __global__ void __launch_bounds__(256) pack_dense_kernel(DevTree t, const float4
     if (bad) atomicOr(&t.st->err, ERR_INPUT);
 }
 
-__global__ void check_finite_kernel(DevTree t, const float* __restrict__ in, long long count) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    if (!isfinite(in[i])) atomicOr(&t.st->err, ERR_INPUT);
-}
-
 inline size_t au(size_t x) { return (x + 255) & ~(size_t)255; }
 
 }  // namespace
@@ -2184,11 +2178,6 @@ void launch_pack_points(const DevTree& t, const float* in, int stride, long long
         return;
     }
     launch_chain(pack_points_kernel, blocks_for(n, 256), 256, 0, s, t, in, stride, n, first_id, out);
-}
-
-void launch_check_finite(const DevTree& t, const float* in, long long count, cudaStream_t s) {
-    if (count <= 0) return;
-    check_finite_kernel<<<blocks_for(count, 256), 256, 0, s>>>(t, in, count);
 }
 
 size_t ds_scratch_bytes(long long n, long long pair_cap) {

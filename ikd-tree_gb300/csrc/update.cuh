@@ -72,8 +72,6 @@ void launch_route_append_dev_count(const DevTree& t, const UpdateAux& a, const f
 // coordinates (st->err |= ERR_INPUT).
 void launch_pack_points(const DevTree& t, const float* in, int stride, long long n, long long first_id, float4* out,
                         cudaStream_t s);
-// Flags non-finite values among n * width floats (st->err |= ERR_INPUT).
-void launch_check_finite(const DevTree& t, const float* in, long long count, cudaStream_t s);
 // Copies every valid point ({x, y, z, id}) to out; *counter += count.
 void launch_flatten(const DevTree& t, float4* out, long long* counter, cudaStream_t s);
 // Writes the id of every stored slot (valid or deleted) to out[0 .. cap);
