@@ -756,12 +756,16 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) finish_split_kernel(DevTree t,
 // This took the place of sorting the three coordinates once and partitioning the
 // three sorted index arrays per level with random gathers of the sides (109
 // launches): a 2M-point build moves 16 instead of ~100 bytes per point and level
-// and takes 760 us of kernels (430 of them these) against 1,950 us.  Bound by L2
+// and takes 700 us of kernels (370 of them these) against 1,950 us.  Bound by L2
 // bandwidth (level passes) and by the latency of the per-segment blocks.
 constexpr int SPLIT_THREADS = 256;
 constexpr int SPLIT_ROUNDS = 8;  // points per thread
 constexpr int SPLIT_TILE = SPLIT_THREADS * SPLIT_ROUNDS;
 constexpr int SPLIT_BINS = 2048;
+// The histogram takes larger tiles: with one point per bin on average (2,048 points) a
+// tile's flush was an addition in L2 per point.  2M points, nine levels: 88 -> 66 us.
+constexpr int HIST_THREADS = 1024;
+constexpr int HIST_TILE = HIST_THREADS * SPLIT_ROUNDS;
 constexpr int SPLIT_CACHE = 4096;  // candidates kept in shared memory by select
 
 // The split axis of a segment (longest extent, first on ties) and its bins: equal
@@ -779,14 +783,13 @@ struct SplitAxis {
     }
 };
 __device__ __forceinline__ SplitAxis split_axis(const uint32_t* box) {
-    float ext[3];
-    for (int a = 0; a < 3; ++a) ext[a] = __fsub_rn(key_float(box[3 + a]), key_float(box[a]));
-    SplitAxis r;
-    r.axis = 0;
-    if (ext[1] > ext[r.axis]) r.axis = 1;
-    if (ext[2] > ext[r.axis]) r.axis = 2;
-    r.lo = key_float(box[r.axis]);
-    r.scale = __fdiv_rn((float)SPLIT_BINS, ext[r.axis]);
+    const float x = key_float(box[0]), y = key_float(box[1]), z = key_float(box[2]);
+    float ext = __fsub_rn(key_float(box[3]), x);
+    const float ey = __fsub_rn(key_float(box[4]), y), ez = __fsub_rn(key_float(box[5]), z);
+    SplitAxis r{0, x, 0.f};
+    if (ey > ext) r.axis = 1, r.lo = y, ext = ey;
+    if (ez > ext) r.axis = 2, r.lo = z, ext = ez;
+    r.scale = __fdiv_rn((float)SPLIT_BINS, ext);
     return r;
 }
 
@@ -873,27 +876,27 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_box_kernel(const float4* 
     else if (threadIdx.x < 6) atomicMax(lv.box + 6 * q + threadIdx.x, sm[threadIdx.x]);
 }
 
-__global__ void __launch_bounds__(SPLIT_THREADS) split_hist_kernel(const float4* pts, SplitLevel lv,
+__global__ void __launch_bounds__(HIST_THREADS) split_hist_kernel(const float4* pts, SplitLevel lv,
                                                                    int cap, unsigned tiles, int* __restrict__ hist) {
     chain_begin();
     __shared__ int h[SPLIT_BINS];
     const int q = (int)(blockIdx.x / tiles), tile = (int)(blockIdx.x % tiles);
     if (q >= min(*lv.n, cap)) return;
     const int4 sg = lv.seg[q];
-    const int t0 = sg.x + tile * SPLIT_TILE;
+    const int t0 = sg.x + tile * HIST_TILE;
     if (t0 >= sg.y) return;
     const SplitAxis ax = split_axis(lv.box + 6 * q);
-    for (int i = threadIdx.x; i < SPLIT_BINS; i += SPLIT_THREADS) h[i] = 0;
+    for (int i = threadIdx.x; i < SPLIT_BINS; i += HIST_THREADS) h[i] = 0;
     __syncthreads();
     const float* c = reinterpret_cast<const float*>(pts) + ax.axis;
 #pragma unroll
     for (int r = 0; r < SPLIT_ROUNDS; ++r) {
-        const int i = t0 + r * SPLIT_THREADS + threadIdx.x;
+        const int i = t0 + r * HIST_THREADS + threadIdx.x;
         if (i < sg.y) atomicAdd(&h[ax.bin(c[4ll * i])], 1);
     }
     __syncthreads();
     int* g = hist + (long long)q * SPLIT_BINS;
-    for (int i = threadIdx.x; i < SPLIT_BINS; i += SPLIT_THREADS)
+    for (int i = threadIdx.x; i < SPLIT_BINS; i += HIST_THREADS)
         if (h[i]) atomicAdd(g + i, h[i]);
 }
 
@@ -1140,8 +1143,9 @@ __global__ void __launch_bounds__(THREADS) split_select_kernel(DevTree t, SplitL
 }
 
 // Points before (v, p) go left, the others right, both in order: to `dst`, or to
-// `exits` where the child leaves the splitter.
-__global__ void __launch_bounds__(SPLIT_THREADS) split_scatter_kernel(const float4* src, SplitLevel lv,
+// `exits` where the child leaves the splitter.  64 registers, so that four blocks share
+// an SM (2M points, nine levels: 157 us with 74, 130).
+__global__ void __launch_bounds__(SPLIT_THREADS, 4) split_scatter_kernel(const float4* src, SplitLevel lv,
                                                                       SplitLevel nx, int cap, unsigned tiles,
                                                                       const int* tile_left,
                                                                       const uint2* thr,
@@ -1158,6 +1162,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_scatter_kernel(const floa
     const int t0 = sg.x + tile * SPLIT_TILE;
     const int2 kd = kids[q];
     if (t0 >= sg.y || kd.x == -2) return;
+    int run = tile_left[split_tile0(sg.x) + tile];  // left points before this warp's
     const int axis = split_axis(lv.box + 6 * q).axis;
     const uint2 th = thr[q];
     const int m = (sg.y - sg.x) / 2;
@@ -1182,7 +1187,6 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_scatter_kernel(const floa
     }
     if (lane == 0) wleft[warp] = left;
     __syncthreads();
-    int run = tile_left[split_tile0(sg.x) + tile];  // left points before this warp's
     for (int w = 0; w < warp; ++w) run += wleft[w];
     float4* dl = kd.x >= 0 ? dst : exits;
     float4* dr = kd.y >= 0 ? dst : exits;
@@ -1345,7 +1349,8 @@ void build_subtrees(const DevTree& t, const float4* pts, long long n, const int*
             const unsigned tiles = (unsigned)((size + SPLIT_TILE - 1) / SPLIT_TILE);
             const unsigned blocks = tiles * (unsigned)segs;
             if (lv == 0) launch_chain(split_box_kernel, blocks, SPLIT_THREADS, 0, s, src, cur, cap, tiles);
-            launch_chain(split_hist_kernel, blocks, SPLIT_THREADS, 0, s, src, cur, cap, tiles, bs.hist);
+            const unsigned htiles = (unsigned)((size + HIST_TILE - 1) / HIST_TILE);
+            launch_chain(split_hist_kernel, htiles * (unsigned)segs, HIST_THREADS, 0, s, src, cur, cap, htiles, bs.hist);
             launch_chain(split_pick_kernel, (unsigned)segs, SPLIT_THREADS, 0, s, cur, nx, cap, bs.hist, bs.pick);
             launch_chain(split_classify_kernel, blocks, SPLIT_THREADS, 0, s, src, cur, cap, tiles, bs.pick, bs.tile_left, bs.cand);
             // few segments have many candidates each
