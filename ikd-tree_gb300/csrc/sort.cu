@@ -1,4 +1,4 @@
-// Prefix sums and LSD radix sort used by the tree builder, the query sorter and
+// Prefix sums and LSD radix sort used by the searches, the query sorter and
 // the downsampling grouper.  Both are three-phase (per-tile reduce, scan of the
 // tile partials, per-tile downsweep / scatter): no block ever waits on
 // another, so nothing here can spin.
