@@ -198,6 +198,9 @@ struct Tree {
         for (size_t o = 0; o < bytes; o += page) c[o] = 0;
         c[bytes - 1] = 0;
     }
+    // IKDG_MAX_VISITS lowers the cap of the traversals (tests use it to run into
+    // the cap on a sound tree).
+    int visit_cap = 0;
     // Kernels that run on host buffers report errors into pinned host memory:
     // no copy brings the bits.
     DevStatus* host_st = nullptr;
@@ -244,6 +247,7 @@ struct Tree {
         }
         CK(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
         direct = pageable != 0 && std::getenv("IKDG_HOST_STAGING") == nullptr;
+        if (const char* e = std::getenv("IKDG_MAX_VISITS")) visit_cap = std::atoi(e);
         CK(cudaMallocHost(&host_st, sizeof(DevStatus)));
         std::memset(host_st, 0, sizeof(DevStatus));
         ensure_pools(64, 64);
@@ -331,6 +335,8 @@ struct Tree {
             grow_array(aux.leaf_job, old_l, new_l, 0xff, stream);
             dt.leaf_cap = new_l;
         }
+        dt.max_visits = walk_cap(dt.node_cap, dt.leaf_cap);
+        if (visit_cap > 0) dt.max_visits = std::min(dt.max_visits, visit_cap);
         int need_list = dt.node_cap + dt.leaf_cap + 2;
         if (need_list > list_cap) {
             grow_array(aux.items, list_cap, need_list, -1, stream);

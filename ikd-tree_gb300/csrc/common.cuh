@@ -51,11 +51,17 @@ constexpr int ERR_LIST = 1024;     // a work list would exceed its capacity
 constexpr int ERR_ANY_INTERNAL = ERR_POOL | ERR_LOOP | ERR_POOL_LEAF | ERR_SEG | ERR_ROUTE | ERR_OVF_JOB | ERR_LIST;
 
 // Caps on every device loop that follows tree links: a walk to the root takes
-// at most MAX_WALK steps, a traversal at most MAX_VISITS node / leaf visits.
-// Hitting a cap sets ERR_LOOP and ends the loop (never expected; it turns a
-// corrupted tree into an error instead of a hung GPU).
+// at most MAX_WALK steps, a traversal at most DevTree::max_visits steps, those on
+// nodes and those on leaves counted alike.  Hitting a cap sets ERR_LOOP and ends
+// the loop (never expected; it turns a corrupted tree into an error instead of a
+// hung GPU).  A step takes at least one record or half a bucket of one query off a
+// warp's list, a warp has up to 32 queries, and a sound tree shows each of them
+// every record and half bucket at most once.
 constexpr int MAX_WALK = 4 * MAX_STACK;
-constexpr int MAX_VISITS = 1 << 26;
+inline int walk_cap(long long nodes, long long leaves) {
+    const long long c = 32 * (nodes + 2 * leaves) + 1024;
+    return c < 0x7fffffff ? (int)c : 0x7fffffff - 1;
+}
 
 __host__ __device__ inline bool code_is_leaf(int c) { return c < 0; }
 __host__ __device__ inline int code_leaf(int c) { return -c - 1; }
@@ -109,6 +115,7 @@ struct DevTree {
     int leaf_cap;
     int height;          // levels below the root (set by the host after every mutation)
     int start;           // wide record every search starts at (host): 0 or the root's own
+    int max_visits;      // steps a traversal may take (host: walk_cap of the pools)
     DevStatus* st;
 };
 

@@ -173,6 +173,10 @@ __device__ __forceinline__ void knn_group(const DevTree& t, const KnnLane& g, bo
     int steps = 0;
 
     while (true) {
+        if (++steps > t.max_visits) {
+            if (cur != DONE && g.sl == 0) atomicOr(&t.st->err, ERR_LOOP);
+            break;
+        }
         const unsigned leaves = __ballot_sync(ALL, cur < 0);
         const bool node = (unsigned)cur < (unsigned)DONE;
         bool pop;
@@ -206,10 +210,6 @@ __device__ __forceinline__ void knn_group(const DevTree& t, const KnnLane& g, bo
             ++lev;
         } else {
             if (leaves == 0) break;
-            if (++steps > MAX_VISITS) {
-                if (cur != DONE && g.sl == 0) atomicOr(&t.st->err, ERR_LOOP);
-                break;
-            }
             const bool act = cur < 0;
             const int L = act ? code_leaf(cur) : 0;
             const int j0 = half * KNN_LEAF_STEP + S * g.sl;
@@ -395,7 +395,7 @@ __device__ __forceinline__ void knn_rows_body(const DevTree& t, bool valid, long
             const bool nodework = !done && cur >= 0;
             if (!__any_sync(0xffffffffu, nodework)) break;
             if (!nodework) continue;
-            if (++visits > MAX_VISITS) {
+            if (++visits > t.max_visits) {
                 atomicOr(&t.st->err, ERR_LOOP);
                 done = true;
                 continue;
@@ -671,7 +671,7 @@ __device__ __forceinline__ void range_warp(const DevTree& t, const RangeWarp& w,
     __syncwarp();
     int steps = 0;
     while (sp > 0) {
-        if (++steps > MAX_VISITS) {
+        if (++steps > t.max_visits) {
             if (lane == 0) atomicOr(&t.st->err, ERR_LOOP);
             break;
         }

@@ -865,7 +865,7 @@ __device__ __forceinline__ void team_walk(const DevTree& t, bool active, int* st
     int sp = active ? 1 : 0;
     int cur = t.start;  // the top of the stack, in every lane of the team
     for (int steps = 0;; ++steps) {
-        if (steps > MAX_VISITS) {
+        if (steps > t.max_visits) {
             if (sp > 0) atomicOr(&t.st->err, ERR_LOOP);
             break;
         }
@@ -997,7 +997,7 @@ __global__ void __launch_bounds__(DB_THREADS) box_restore_kernel(DevTree t, Upda
         for (int rounds = 0;; ++rounds) {
             int cur_top = top;
             if (cur_top == 0) break;
-            if (rounds > MAX_VISITS / DB_THREADS) {
+            if (rounds > t.max_visits) {
                 if (threadIdx.x == 0) atomicOr(&t.st->err, ERR_LOOP);
                 break;
             }
@@ -1112,7 +1112,7 @@ __global__ void __launch_bounds__(BD_CTA) box_delete_kernel(DevTree t, UpdateAux
         if (lane == 0) stack[0] = code * 2 + cov;
         __syncwarp();
         for (int steps = 0; sp > 0; ++steps) {
-            if (steps > MAX_VISITS) {
+            if (steps > t.max_visits) {
                 if (lane == 0) atomicOr(&t.st->err, ERR_LOOP);
                 break;
             }
