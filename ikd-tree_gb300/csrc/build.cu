@@ -27,6 +27,7 @@
 #include <climits>
 
 #include "kernels.cuh"
+#include "split_grid.h"
 
 namespace ikdg {
 namespace {
@@ -487,8 +488,6 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 4) local_build_
     }
 }
 
-constexpr int SPLIT_MIN = 4096;  // larger segments are split by many blocks
-
 // Exclusive block prefix of a per-thread value; the block total goes to
 // *total.  The shared words are free for reuse when it returns.
 template <int THREADS>
@@ -742,7 +741,7 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) finish_split_kernel(DevTree t,
 
 // ---- multi-block splitter for large segments ------------------------------------------------
 // Segments above SPLIT_MIN points: one level per round of five launches, every
-// segment cut into tiles of SPLIT_TILE points, a block per (tile, segment).
+// segment cut into tiles of SPLIT_TILE points, a block per tile (split_grid.h).
 //   hist      keys on the split axis into SPLIT_BINS bins over the segment's range
 //   pick      the bin that holds the point of rank n / 2 (a block per segment)
 //   classify  per tile the points of lower bins; the picked bin's points, (key,
@@ -760,12 +759,9 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) finish_split_kernel(DevTree t,
 // bandwidth (level passes) and by the latency of the per-segment blocks.
 constexpr int SPLIT_THREADS = 256;
 constexpr int SPLIT_ROUNDS = 8;  // points per thread
-constexpr int SPLIT_TILE = SPLIT_THREADS * SPLIT_ROUNDS;
 constexpr int SPLIT_BINS = 2048;
-// The histogram takes larger tiles: with one point per bin on average (2,048 points) a
-// tile's flush was an addition in L2 per point.  2M points, nine levels: 88 -> 66 us.
 constexpr int HIST_THREADS = 1024;
-constexpr int HIST_TILE = HIST_THREADS * SPLIT_ROUNDS;
+static_assert(SPLIT_TILE == SPLIT_THREADS * SPLIT_ROUNDS && HIST_TILE == HIST_THREADS * SPLIT_ROUNDS, "points per thread");
 constexpr int SPLIT_CACHE = 4096;  // candidates kept in shared memory by select
 
 // The split axis of a segment (longest extent, first on ties) and its bins: equal
@@ -805,6 +801,39 @@ __device__ __forceinline__ void split_box_reset(uint32_t* box) {
     }
 }
 
+// A level's counters in one word, so that one addition gives a new segment its index and
+// the places of its tiles: segments from bit 42 on, tiles from bit 21, htiles below (n is
+// below 2^30, so there are at most 2^18 segments and 2^20 tiles).
+struct SplitCount {
+    int segs, tiles, htiles;
+};
+__device__ __forceinline__ SplitCount split_unpack(unsigned long long v) {
+    return SplitCount{(int)(v >> 42), (int)(v >> 21 & 0x1fffffu), (int)(v & 0x1fffffu)};
+}
+// Opens segment [s, e) below `link` (one thread); its index, or -1 when the list is full
+// (flagged), and where its tiles go.
+__device__ __forceinline__ SplitCount split_take(const SplitLevel& lv, int cap, int s, int e, int link, DevStatus* st) {
+    const int tiles = (e - s + SPLIT_TILE - 1) / SPLIT_TILE, htiles = (e - s + HIST_TILE - 1) / HIST_TILE;
+    SplitCount c = split_unpack(atomicAdd(lv.n, (1ull << 42) | (unsigned long long)tiles << 21 | (unsigned long long)htiles));
+    if (c.segs >= cap) {  // cannot happen: see split_grid.h
+        atomicOr(&st->err, ERR_SEG);
+        c.segs = -1;
+        return c;
+    }
+    lv.seg[c.segs] = make_int4(s, e, link, 0);
+    lv.cand_n[c.segs] = 0;
+    split_box_reset(lv.box + 6 * c.segs);
+    return c;
+}
+// Lists the tiles of a segment split_take opened (the whole block).
+template <int THREADS>
+__device__ __forceinline__ void split_list(const SplitLevel& lv, const SplitCount& c, int s, int e) {
+    const int tiles = (e - s + SPLIT_TILE - 1) / SPLIT_TILE, htiles = (e - s + HIST_TILE - 1) / HIST_TILE;
+    for (int i = threadIdx.x; i < tiles; i += THREADS) lv.tile[c.tiles + i] = make_int4(s, e, c.segs, i);
+    for (int i = threadIdx.x; i < htiles; i += THREADS) lv.htile[c.htiles + i] = make_int4(s, e, c.segs, i);
+}
+__device__ __forceinline__ int split_segs(const SplitLevel& lv, int cap) { return min(split_unpack(*lv.n).segs, cap); }
+
 // Jobs above SPLIT_MIN points open the splitter's first level; the others go to
 // the small list, their points copied to `exits` (a block per job).
 __global__ void __launch_bounds__(SPLIT_THREADS) split_open_kernel(const float4* pts,
@@ -814,26 +843,27 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_open_kernel(const float4*
                                                                    int4* __restrict__ small, int* nsmall, int max_small,
                                                                    DevStatus* st) {
     chain_begin();
-    __shared__ int big;
+    __shared__ SplitCount at;
     for (int j = blockIdx.x; j < njobs; j += gridDim.x) {
         const int s = job_off[j], e = job_off[j + 1];
+        const bool big = e - s > SPLIT_MIN;
         __syncthreads();
         if (threadIdx.x == 0) {
-            big = e - s > SPLIT_MIN;
-            const int r = atomicAdd(big ? lv.n : nsmall, 1);
-            if (r >= (big ? cap : max_small)) {
-                atomicOr(&st->err, ERR_SEG);
-            } else if (big) {
-                lv.seg[r] = make_int4(s, e, job_link[j], 0);
-                lv.cand_n[r] = 0;
-                split_box_reset(lv.box + 6 * r);
+            if (big) {
+                at = split_take(lv, cap, s, e, job_link[j], st);
             } else {
-                small[r] = make_int4(s, e, job_link[j], 0);
+                const int r = atomicAdd(nsmall, 1);
+                if (r >= max_small)
+                    atomicOr(&st->err, ERR_SEG);
+                else
+                    small[r] = make_int4(s, e, job_link[j], 0);
             }
         }
         __syncthreads();
         if (!big)
             for (int i = s + threadIdx.x; i < e; i += SPLIT_THREADS) exits[i] = pts[i];
+        else if (at.segs >= 0)
+            split_list<SPLIT_THREADS>(lv, at, s, e);
     }
 }
 
@@ -857,14 +887,12 @@ __device__ __forceinline__ void split_flush(uint32_t* sm, const uint32_t* b) {
 }
 
 __global__ void __launch_bounds__(SPLIT_THREADS) split_box_kernel(const float4* pts, SplitLevel lv,
-                                                                  int cap, unsigned tiles) {
+                                                                  int max_tiles) {
     chain_begin();
     __shared__ uint32_t sm[6];
-    const int q = (int)(blockIdx.x / tiles), tile = (int)(blockIdx.x % tiles);
-    if (q >= min(*lv.n, cap)) return;
-    const int4 sg = lv.seg[q];
-    const int t0 = sg.x + tile * SPLIT_TILE;
-    if (t0 >= sg.y) return;
+    const int4 sg = lv.tile[blockIdx.x];
+    if ((int)blockIdx.x >= min(split_unpack(*lv.n).tiles, max_tiles)) return;
+    const int q = sg.z, t0 = sg.x + sg.w * SPLIT_TILE;
     if (threadIdx.x == 0) split_box_reset(sm);
     __syncthreads();
     uint32_t b[6];
@@ -877,14 +905,12 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_box_kernel(const float4* 
 }
 
 __global__ void __launch_bounds__(HIST_THREADS) split_hist_kernel(const float4* pts, SplitLevel lv,
-                                                                   int cap, unsigned tiles, int* __restrict__ hist) {
+                                                                   int max_tiles, int* __restrict__ hist) {
     chain_begin();
     __shared__ int h[SPLIT_BINS];
-    const int q = (int)(blockIdx.x / tiles), tile = (int)(blockIdx.x % tiles);
-    if (q >= min(*lv.n, cap)) return;
-    const int4 sg = lv.seg[q];
-    const int t0 = sg.x + tile * HIST_TILE;
-    if (t0 >= sg.y) return;
+    const int4 sg = lv.htile[blockIdx.x];
+    if ((int)blockIdx.x >= min(split_unpack(*lv.n).htiles, max_tiles)) return;
+    const int q = sg.z, t0 = sg.x + sg.w * HIST_TILE;
     const SplitAxis ax = split_axis(lv.box + 6 * q);
     for (int i = threadIdx.x; i < SPLIT_BINS; i += HIST_THREADS) h[i] = 0;
     __syncthreads();
@@ -908,7 +934,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_pick_kernel(SplitLevel lv
     __shared__ uint32_t wsum[SPLIT_THREADS / 32], tot;
     const int q = blockIdx.x;
     if (q == 0 && threadIdx.x == 0) *nx.n = 0;  // select fills it
-    if (q >= min(*lv.n, cap)) return;
+    if (q >= split_segs(lv, cap)) return;
     const int4 sg = lv.seg[q];
     constexpr int PER = SPLIT_BINS / SPLIT_THREADS;
     int4* g = reinterpret_cast<int4*>(hist + (long long)q * SPLIT_BINS) + threadIdx.x * (PER / 4);
@@ -937,17 +963,15 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_pick_kernel(SplitLevel lv
 }
 
 __global__ void __launch_bounds__(SPLIT_THREADS) split_classify_kernel(const float4* pts, SplitLevel lv,
-                                                                       int cap, unsigned tiles,
+                                                                       int max_tiles,
                                                                        const int2* pick,
                                                                        int* __restrict__ tile_left,
                                                                        uint2* __restrict__ cand) {
     chain_begin();
     __shared__ int less;
-    const int q = (int)(blockIdx.x / tiles), tile = (int)(blockIdx.x % tiles);
-    if (q >= min(*lv.n, cap)) return;
-    const int4 sg = lv.seg[q];
-    const int t0 = sg.x + tile * SPLIT_TILE;
-    if (t0 >= sg.y) return;
+    const int4 sg = lv.tile[blockIdx.x];
+    if ((int)blockIdx.x >= min(split_unpack(*lv.n).tiles, max_tiles)) return;
+    const int q = sg.z, tile = sg.w, t0 = sg.x + tile * SPLIT_TILE;
     const SplitAxis ax = split_axis(lv.box + 6 * q);
     const int bin = pick[q].x;
     if (threadIdx.x == 0) less = 0;
@@ -1038,7 +1062,7 @@ __global__ void __launch_bounds__(THREADS) split_select_kernel(DevTree t, SplitL
     __shared__ SplitDigit sd;
     __shared__ uint32_t wsum[THREADS / 32], tot, spos;
     const int q = blockIdx.x;
-    if (q >= min(*lv.n, cap)) return;
+    if (q >= split_segs(lv, cap)) return;
     const int4 sg = lv.seg[q];
     const int s = sg.x, cnt = sg.y - sg.x, m = cnt / 2, link = sg.z;
     const SplitAxis ax = split_axis(lv.box + 6 * q);
@@ -1098,55 +1122,59 @@ __global__ void __launch_bounds__(THREADS) split_select_kernel(DevTree t, SplitL
         if (i < tiles) tl[i] = (int)(carry + ex);
         carry += total;
     }
-    if (threadIdx.x != 0) return;
-    if (carry != (uint32_t)m) atomicOr(&t.st->err, ERR_SEG);  // cannot happen: the selection found rank m
-    thr[q] = make_uint2(v, p);
-    kids[q] = make_int2(-2, -2);
-    const int X = alloc_node(t);
-    if (X < 0) return;  // the pool is exhausted (flagged): the points are dropped
-    Box3 b;
-    for (int a = 0; a < 3; ++a) {
-        b.lo[a] = key_float(lv.box[6 * q + a]);
-        b.hi[a] = key_float(lv.box[6 * q + 3 + a]);
-    }
-    const int parent = link >> 1, side = link & 1;
-    t.nparent[X] = link;
-    int h = 0;
-    for (int k = cnt; k > fill; k -= k / 2) ++h;
-    t.nheight[X] = h;
-    t.node[4 * X + 3] = make_float4(__int_as_float(0), __int_as_float(0), key_float(v), __int_as_float(ax.axis));
-    write_child_box(t.node, parent, side, b);
-    write_child_code(t.node, parent, side, X);
-    write_child_cnt(t.ncnt, parent, side, cnt, 0);
-    const int2 wi = t.winfo[parent];
-    wide_link(t, wi, side, X, b, cnt);
-    t.winfo[X] = wide_below(wi, side, X);
-    // Children: the splitter's next level or the small list (-1).
-    int kid[2];
-    for (int k = 0; k < 2; ++k) {
-        const int cs = k == 0 ? s : s + m, ce = k == 0 ? s + m : s + cnt;
-        const bool big = ce - cs > SPLIT_MIN;
-        const int r = atomicAdd(big ? nx.n : nsmall, 1);
-        kid[k] = -1;
-        if (r >= (big ? cap : max_small)) {
-            atomicOr(&t.st->err, ERR_SEG);
-        } else if (big) {
-            nx.seg[r] = make_int4(cs, ce, X * 2 + k, 0);
-            nx.cand_n[r] = 0;
-            split_box_reset(nx.box + 6 * r);
-            kid[k] = r;
-        } else {
-            small[r] = make_int4(cs, ce, X * 2 + k, 0);
+    // The node and its children: the splitter's next level or the small list.
+    __shared__ SplitCount open[2];
+    if (threadIdx.x == 0) {
+        open[0].segs = open[1].segs = -1;
+        if (carry != (uint32_t)m) atomicOr(&t.st->err, ERR_SEG);  // cannot happen: the selection found rank m
+        thr[q] = make_uint2(v, p);
+        const int X = alloc_node(t);
+        int2 kid = make_int2(-2, -2);  // the pool is exhausted (flagged): the points are dropped
+        if (X >= 0) {
+            Box3 b;
+            for (int a = 0; a < 3; ++a) {
+                b.lo[a] = key_float(lv.box[6 * q + a]);
+                b.hi[a] = key_float(lv.box[6 * q + 3 + a]);
+            }
+            const int parent = link >> 1, side = link & 1;
+            t.nparent[X] = link;
+            int h = 0;
+            for (int k = cnt; k > fill; k -= k / 2) ++h;
+            t.nheight[X] = h;
+            t.node[4 * X + 3] =
+                make_float4(__int_as_float(0), __int_as_float(0), key_float(v), __int_as_float(ax.axis));
+            write_child_box(t.node, parent, side, b);
+            write_child_code(t.node, parent, side, X);
+            write_child_cnt(t.ncnt, parent, side, cnt, 0);
+            const int2 wi = t.winfo[parent];
+            wide_link(t, wi, side, X, b, cnt);
+            t.winfo[X] = wide_below(wi, side, X);
+            for (int k = 0; k < 2; ++k) {
+                const int cs = k == 0 ? s : s + m, ce = k == 0 ? s + m : s + cnt;
+                if (ce - cs > SPLIT_MIN) {
+                    open[k] = split_take(nx, cap, cs, ce, X * 2 + k, t.st);
+                } else {
+                    const int r = atomicAdd(nsmall, 1);
+                    if (r >= max_small)
+                        atomicOr(&t.st->err, ERR_SEG);
+                    else
+                        small[r] = make_int4(cs, ce, X * 2 + k, 0);
+                }
+            }
+            kid = make_int2(open[0].segs, open[1].segs);
         }
+        kids[q] = kid;
     }
-    kids[q] = make_int2(kid[0], kid[1]);
+    __syncthreads();
+    for (int k = 0; k < 2; ++k)
+        if (open[k].segs >= 0) split_list<THREADS>(nx, open[k], k == 0 ? s : s + m, k == 0 ? s + m : s + cnt);
 }
 
 // Points before (v, p) go left, the others right, both in order: to `dst`, or to
 // `exits` where the child leaves the splitter.  64 registers, so that four blocks share
 // an SM (2M points, nine levels: 157 us with 74, 130).
 __global__ void __launch_bounds__(SPLIT_THREADS, 4) split_scatter_kernel(const float4* src, SplitLevel lv,
-                                                                      SplitLevel nx, int cap, unsigned tiles,
+                                                                      SplitLevel nx, int max_tiles,
                                                                       const int* tile_left,
                                                                       const uint2* thr,
                                                                       const int2* kids,
@@ -1156,12 +1184,11 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 4) split_scatter_kernel(const f
     constexpr int WARPS = SPLIT_THREADS / 32, WARP_PTS = SPLIT_TILE / WARPS;
     __shared__ uint32_t sm[12];
     __shared__ int wleft[WARPS];
-    const int q = (int)(blockIdx.x / tiles), tile = (int)(blockIdx.x % tiles);
-    if (q >= min(*lv.n, cap)) return;
-    const int4 sg = lv.seg[q];
-    const int t0 = sg.x + tile * SPLIT_TILE;
+    const int4 sg = lv.tile[blockIdx.x];
+    if ((int)blockIdx.x >= min(split_unpack(*lv.n).tiles, max_tiles)) return;
+    const int q = sg.z, tile = sg.w, t0 = sg.x + tile * SPLIT_TILE;
     const int2 kd = kids[q];
-    if (t0 >= sg.y || kd.x == -2) return;
+    if (kd.x == -2) return;
     int run = tile_left[split_tile0(sg.x) + tile];  // left points before this warp's
     const int axis = split_axis(lv.box + 6 * q).axis;
     const uint2 th = thr[q];
@@ -1243,7 +1270,7 @@ int lb_prepare() {
     return n;
 }
 
-__global__ void reset_count_kernel(int* c) { chain_begin(); *c = 0; }
+__global__ void reset_count_kernel(unsigned long long* c) { chain_begin(); *c = 0; }
 
 inline unsigned blocks_for(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
@@ -1251,7 +1278,6 @@ inline unsigned blocks_for(long long n, int t) { return (unsigned)((n + t - 1) /
 // the local builder (a whole job or a piece of at least 512 points: half of a
 // segment above LB_SMALL points); segments of the large splitter.
 long long max_segs_bound(long long n, int njobs) { return (long long)njobs + n / 512 + 2; }
-long long max_split_bound(long long n) { return n / SPLIT_MIN + 2; }
 
 size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -1282,7 +1308,7 @@ struct ScratchCarver {
 size_t carve(void* base, long long n, int njobs, BuildScratch* bs) {
     const long long ms = max_segs_bound(n, njobs);
     // the large splitter's lists, only for calls that can use it
-    const long long sp = n > SPLIT_MIN ? max_split_bound(n) : 0;
+    const long long sp = n > SPLIT_MIN ? split_segs_cap(n) : 0;
     ScratchCarver c{(char*)base};
     for (int i = 0; i < 3; ++i) bs->pts[i] = c.take<float4>(i == 0 || sp ? n : 0);
     bs->small = c.take<int4>(ms);
@@ -1292,7 +1318,9 @@ size_t carve(void* base, long long n, int njobs, BuildScratch* bs) {
         bs->split[i].seg = c.take<int4>(sp);
         bs->split[i].box = c.take<uint32_t>(6 * sp);
         bs->split[i].cand_n = c.take<int>(sp);
-        bs->split[i].n = c.take<int>(1);
+        bs->split[i].tile = c.take<int4>(sp ? split_tiles_cap(n) : 0);
+        bs->split[i].htile = c.take<int4>(sp ? split_htiles_cap(n) : 0);
+        bs->split[i].n = c.take<unsigned long long>(1);
     }
     bs->hist = c.take<int>(SPLIT_BINS * sp);
     bs->pick = c.take<int2>(sp);
@@ -1336,35 +1364,34 @@ void build_subtrees(const DevTree& t, const float4* pts, long long n, const int*
         small_pts = pts;
     } else {
         // Large segments, one level per round, until all of them are small.
-        const int cap = (int)max_split_bound(nn);
+        const int cap = (int)split_segs_cap(nn);
         launch_chain(reset_count_kernel, 1, 1, 0, s, bs.split[0].n);
         cudaMemsetAsync(bs.hist, 0, sizeof(int) * SPLIT_BINS * (size_t)cap, s);
         launch_chain(split_open_kernel, grid(njobs, 8), SPLIT_THREADS, 0, s, pts, job_off, job_link, njobs, bs.split[0], cap,
                                                                    bs.pts[2], bs.small, nsmall, (int)ms, t.st);
-        long long segs = std::min<long long>(njobs, cap), size = max_job;
+        long long size = max_job;
         for (int lv = 0; size > SPLIT_MIN; ++lv) {
+            const SplitGrid g = split_grid(nn, njobs, lv);
+            const unsigned segs = (unsigned)g.segs, blocks = (unsigned)g.tiles, hblocks = (unsigned)g.htiles;
+            const int mt = (int)g.tiles, mh = (int)g.htiles;
             const SplitLevel &cur = bs.split[lv & 1], &nx = bs.split[(lv + 1) & 1];
             const float4* src = lv == 0 ? pts : bs.pts[(lv + 1) & 1];
             float4* dst = bs.pts[lv & 1];
-            const unsigned tiles = (unsigned)((size + SPLIT_TILE - 1) / SPLIT_TILE);
-            const unsigned blocks = tiles * (unsigned)segs;
-            if (lv == 0) launch_chain(split_box_kernel, blocks, SPLIT_THREADS, 0, s, src, cur, cap, tiles);
-            const unsigned htiles = (unsigned)((size + HIST_TILE - 1) / HIST_TILE);
-            launch_chain(split_hist_kernel, htiles * (unsigned)segs, HIST_THREADS, 0, s, src, cur, cap, htiles, bs.hist);
-            launch_chain(split_pick_kernel, (unsigned)segs, SPLIT_THREADS, 0, s, cur, nx, cap, bs.hist, bs.pick);
-            launch_chain(split_classify_kernel, blocks, SPLIT_THREADS, 0, s, src, cur, cap, tiles, bs.pick, bs.tile_left, bs.cand);
+            if (lv == 0) launch_chain(split_box_kernel, blocks, SPLIT_THREADS, 0, s, src, cur, mt);
+            launch_chain(split_hist_kernel, hblocks, HIST_THREADS, 0, s, src, cur, mh, bs.hist);
+            launch_chain(split_pick_kernel, segs, SPLIT_THREADS, 0, s, cur, nx, cap, bs.hist, bs.pick);
+            launch_chain(split_classify_kernel, blocks, SPLIT_THREADS, 0, s, src, cur, mt, bs.pick, bs.tile_left, bs.cand);
             // few segments have many candidates each
             if (segs <= 64)
-                launch_chain(split_select_kernel<1024>, (unsigned)segs, 1024, 0, s, t, cur, nx, cap, bs.pick, bs.tile_left, bs.cand,
+                launch_chain(split_select_kernel<1024>, segs, 1024, 0, s, t, cur, nx, cap, bs.pick, bs.tile_left, bs.cand,
                                                                          bs.thr, bs.kids, bs.small, nsmall, (int)ms,
                                                                          fill);
             else
-                launch_chain(split_select_kernel<256>, (unsigned)segs, 256, 0, s, t, cur, nx, cap, bs.pick, bs.tile_left, bs.cand,
+                launch_chain(split_select_kernel<256>, segs, 256, 0, s, t, cur, nx, cap, bs.pick, bs.tile_left, bs.cand,
                                                                        bs.thr, bs.kids, bs.small, nsmall, (int)ms,
                                                                        fill);
-            launch_chain(split_scatter_kernel, blocks, SPLIT_THREADS, 0, s, src, cur, nx, cap, tiles, bs.tile_left, bs.thr, bs.kids,
+            launch_chain(split_scatter_kernel, blocks, SPLIT_THREADS, 0, s, src, cur, nx, mt, bs.tile_left, bs.thr, bs.kids,
                                                                   dst, bs.pts[2]);
-            segs = std::min<long long>(2 * segs, cap);
             size -= size / 2;
         }
     }

@@ -386,6 +386,7 @@ struct Tree {
 
     // ---- status ------------------------------------------------------------------
     void read_status() {
+        CK(take_chain_refused());
         CK(cudaMemcpyAsync(st, st_dev, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream));
         CK(cudaStreamSynchronize(stream));
         take_status();
@@ -540,6 +541,7 @@ struct Tree {
             const long long live = work - st->free_leaf_n - st->free_node_n;
             const bool list = live > SETTLE_LIST || work > 8 * SETTLE_LIST;
             const int blocks = list ? sm_count : (int)std::min(2ll * sm_count, std::max(1ll, (work + 1023) / 1024));
+            CK(take_chain_refused());
             CK(launch_settle(dt, aux, select, st, list, blocks, stream));
             CK(cudaStreamSynchronize(stream));
             take_status();

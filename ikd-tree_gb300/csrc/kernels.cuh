@@ -24,6 +24,16 @@ __device__ __forceinline__ void chain_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// The first launch of this thread's chains that was refused since the last look.  A
+// chain with a launch missing leaves a wrong tree: the call that issued it looks before
+// it waits.
+inline thread_local cudaError_t chain_refused = cudaSuccess;
+inline cudaError_t take_chain_refused() {
+    const cudaError_t e = chain_refused;
+    chain_refused = cudaSuccess;
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
 template <class... P, class... A>
 inline void launch_chain_if(bool chain, void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s,
                             A&&... args) {
@@ -37,8 +47,8 @@ inline void launch_chain_if(bool chain, void (*kernel)(P...), dim3 grid, unsigne
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = chain ? 1 : 0;
-    // (a refused launch stays as the thread's last error, as with <<<>>>)
-    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+    if (e != cudaSuccess && chain_refused == cudaSuccess) chain_refused = e;
 }
 template <class... P, class... A>
 inline void launch_chain(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
@@ -71,12 +81,15 @@ bool radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32
 // the median of the longest AABB axis, and is linked into the child slot
 // `job_link[j]` (= parent * 2 + side) together with its AABB and counts.  The pools'
 // free stacks are settled by the snapshot or job-finish kernel that follows.
-// Open segments of the large splitter at one level.
+// Open segments of the large splitter at one level, and their tiles: a block of a
+// launch over tiles b takes tile[b] = {s, e, segment, tile of the segment}.
 struct SplitLevel {
     int4* seg;       // {s, e, link, -}
     uint32_t* box;   // 6 per segment: keys of the AABB's low, then high corner
     int* cand_n;     // candidates listed
-    int* n;          // segments
+    int4* tile;      // tiles of SPLIT_TILE points
+    int4* htile;     // tiles of HIST_TILE points
+    unsigned long long* n;  // segments, tiles, htiles in one word (split_take)
 };
 struct BuildScratch {
     float4* pts[3];      // 3 x [n] points between levels; [2]: those of segments that left the splitter
