@@ -2,9 +2,10 @@
 // per-call orchestration of the kernels, and the extern "C" entry points
 // declared in include/ikdg.h.
 //
-// Every call runs on the tree's CUDA stream.  Host-pointer calls copy their
-// inputs in, run the kernels, copy the results out and synchronise; the
-// reference API is synchronous (it returns counts), so are these.
+// Every call runs on the tree's CUDA stream.  Host-pointer calls run the kernels on
+// the caller's buffers where the GPU can address them, or on copies (see `direct`
+// below), and synchronise; the reference API is synchronous (it returns counts), so
+// are these.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -201,6 +202,30 @@ struct Tree {
     // IKDG_MAX_VISITS lowers the cap of the traversals (tests use it to run into
     // the cap on a sound tree).
     int visit_cap = 0;
+    // The results are those of the inputs as they were when the call began: where an
+    // output shares memory with an input, the inputs are copied first.
+    struct Span {
+        const void* p;
+        size_t bytes;
+    };
+    static bool apart(std::initializer_list<Span> outs, std::initializer_list<Span> ins) {
+        for (const Span& o : outs)
+            for (const Span& i : ins) {
+                if (o.p == nullptr || i.p == nullptr || o.bytes == 0 || i.bytes == 0) continue;
+                const uintptr_t a = (uintptr_t)o.p, b = (uintptr_t)i.p;
+                if (a < b + i.bytes && b < a + o.bytes) return false;
+            }
+        return true;
+    }
+    static size_t rows_bytes(long long n, int stride, int width) {
+        return n > 0 ? sizeof(float) * ((size_t)(n - 1) * stride + width) : 0;
+    }
+    static bool knn_apart(const float* q, long long nq, int stride, int k, const int* ids, const float* d2,
+                          const float* xyz, const int* cnt) {
+        const size_t rows = sizeof(float) * (size_t)nq * k;
+        return apart({{ids, rows}, {d2, rows}, {xyz, 3 * rows}, {cnt, sizeof(int) * (size_t)nq}},
+                     {{q, rows_bytes(nq, stride, 3)}});
+    }
     // Kernels that run on host buffers report errors into pinned host memory:
     // no copy brings the bits.
     DevStatus* host_st = nullptr;
@@ -735,8 +760,8 @@ struct Tree {
 
     // The caller's input array as the kernels read it: in place, or copied to
     // `staged` (device room for it).
-    const float* input(const float* in, size_t floats, float* staged) {
-        if (direct) return in;
+    const float* input(const float* in, size_t floats, float* staged) { return direct ? in : stage(in, floats, staged); }
+    const float* stage(const float* in, size_t floats, float* staged) {
         CK(cudaMemcpyAsync(staged, in, sizeof(float) * floats, cudaMemcpyHostToDevice, stream));
         return staged;
     }
@@ -838,7 +863,8 @@ struct Tree {
         const size_t o_q = o_cnt + (cnt ? align_up(sizeof(int) * nq) : 0);
         const size_t o_tmp = o_q + align_up(sizeof(float) * nq * stride);
         const int bits = bin_bits_for(nq, k);
-        const bool direct = this->direct && bits == 0;  // (a sorted batch's rows would leave one by one)
+        // (a sorted batch's rows would leave one by one)
+        const bool direct = this->direct && bits == 0 && knn_apart(q, nq, stride, k, ids, d2, xyz, cnt);
         SearchCtx* c = take_ctx();
         try {
             ctx_reserve(c, direct ? 0 : o_tmp + align_up(tmp + 256), direct ? o_rows : o_tmp);
@@ -892,7 +918,7 @@ struct Tree {
             CK(cudaGetLastError());
             return;
         }
-        if (direct && k <= KNN_GROUP_MAX && bin_bits_for(nq, k) == 0) {
+        if (direct && k <= KNN_GROUP_MAX && bin_bits_for(nq, k) == 0 && knn_apart(q, nq, stride, k, ids, d2, xyz, cnt)) {
             // Kernels read the queries and write the results in host memory:
             // each CTA's rows leave as coalesced 16-byte spans.  (A sorted
             // batch's rows would leave one by one, and lists in the output rows
@@ -944,16 +970,26 @@ struct Tree {
             throw BadArg{"radius search: bad arguments"};
         int qs = mode == 0 ? 6 : stride;
         *total = 0;
-        offsets[0] = 0;
-        if (nq == 0) return;
+        if (nq == 0) {
+            offsets[0] = 0;
+            return;
+        }
         const int logged = ids != nullptr ? RANGE_LOG : 0;
-        op.ensure(input_bytes((size_t)nq * qs) + input_bytes((size_t)nq * (mode == 1 ? std::max(rstride, 1) : 0)) +
+        const size_t qfloats = (size_t)nq * qs, rfloats = mode == 1 ? (size_t)(nq - 1) * rstride + 1 : 0;
+        const size_t room = capacity > 0 ? (size_t)capacity : 0;
+        const bool in_place_in =
+            direct && apart({{offsets, sizeof(long long) * (nq + 1)}, {ids, sizeof(int) * room}, {xyz, sizeof(float) * 3 * room}},
+                            {{q, rows_bytes(nq, qs, mode == 0 ? 6 : 3)}, {radius, sizeof(float) * rfloats}});
+        op.ensure((in_place_in ? 0 : align_up(sizeof(float) * qfloats) + align_up(sizeof(float) * rfloats)) +
                       (direct ? 0 : align_up(sizeof(long long) * (nq + 1))) + align_up(range_temp_bytes(nq, logged)) + 512,
                   stream);
         Carver c(op.p);
-        const size_t rfloats = mode == 1 ? (size_t)(nq - 1) * rstride + 1 : 0;
-        const float* dq = input(q, (size_t)nq * qs, c.take<float>(direct ? 0 : (size_t)nq * qs));
-        const float* dr = mode == 1 ? input(radius, rfloats, c.take<float>(direct ? 0 : rfloats)) : nullptr;
+        const float *dq = q, *dr = radius;
+        if (!in_place_in) {
+            dq = stage(q, qfloats, c.take<float>(qfloats));
+            if (mode == 1) dr = stage(radius, rfloats, c.take<float>(rfloats));
+            if (direct) CK(cudaStreamSynchronize(stream));  // outputs are touched by the host below
+        }
         long long* doffs = direct ? offsets : c.take<long long>(nq + 1);
         void* temp = c.take<char>(range_temp_bytes(nq, logged));
         DevTree t = dt;

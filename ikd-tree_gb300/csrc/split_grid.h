@@ -6,7 +6,7 @@
 // each and the points of a level are at most n, so there are at most n / (SPLIT_MIN + 1)
 // of them, and each has less than one tile more than its points fill.  (The largest
 // job's tiles times the number of jobs, the bound before, is the same for one job; one
-// job of 3M points beside 2,000 small ones got 2.7M blocks a launch for 1,500 tiles.)
+// job of 3M points beside 2,000 small ones got 1.1M blocks a launch for 1,500 tiles.)
 #pragma once
 
 namespace ikdg {

@@ -18,6 +18,9 @@
  *   - Functions taking host pointers are synchronous.  *_device variants take
  *     device pointers and are asynchronous on the tree's stream.
  *   - All functions return an ikdg_status code.
+ *   - Outputs of a host-pointer call may share memory with its inputs (the results are
+ *     those of the inputs as they were when the call began), not with one another.
+ *     Outputs of a device-pointer call share memory with nothing.
  *
  * Thread safety: calls on one tree are serialised by an internal mutex; the
  * reference's concurrent Nearest_Search callers (ikd_Tree.cpp:875-884) are
