@@ -1000,10 +1000,7 @@ struct Tree {
                      stream);
         if (!direct)
             CK(cudaMemcpyAsync(offsets, doffs, sizeof(long long) * (nq + 1), cudaMemcpyDeviceToHost, stream));
-        CK(cudaGetLastError());
-        CK(cudaStreamSynchronize(stream));
-        if (host_st->err & ERR_STACK) throw Internal{"range search: traversal stack overflow"};
-        if (host_st->err & ERR_LOOP) throw Internal{"device error: loop cap reached;"};
+        wait_range();
         const long long acc = offsets[nq];
         *total = acc;
         if (acc > capacity || (acc > 0 && ids == nullptr)) throw CapacityFail{"range search: output too small"};
@@ -1026,9 +1023,15 @@ struct Tree {
             CK(cudaMemcpyAsync(ids, dids, sizeof(int) * acc, cudaMemcpyDeviceToHost, stream));
             if (xyz) CK(cudaMemcpyAsync(xyz, dxyz, sizeof(float) * acc * 3, cudaMemcpyDeviceToHost, stream));
         }
+        wait_range();  // (a warp without a hit log searches again)
+        if (host_st->err & ERR_OUTPUT) throw Internal{"range search: hits differ between the count and write passes"};
+    }
+    // Waits for a pass of a host range search and looks at its error bits.
+    void wait_range() {
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(stream));
-        if (host_st->err & ERR_OUTPUT) throw Internal{"range search: hits differ between the count and write passes"};
+        if (host_st->err & ERR_STACK) throw Internal{"range search: traversal stack overflow"};
+        if (host_st->err & ERR_LOOP) throw Internal{"device error: loop cap reached;"};
     }
     static constexpr long long RANGE_DIRECT_HITS = 1 << 18;
 

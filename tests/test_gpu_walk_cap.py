@@ -55,6 +55,18 @@ def test_batch_and_range_searches_count(ikdg_mod, monkeypatch):
     tree.close()
 
 
+def test_write_pass_of_a_range_search_reports(ikdg_mod, monkeypatch):
+    # The counting pass takes subtrees that the box covers as a whole, a handful of
+    # steps; the write pass has every bucket to go through, 800 steps at the least.
+    tree, pts = pair(ikdg_mod, monkeypatch, 400)
+    box = np.array([[-30, -30, -30, 30, 30, 30]], np.float32)
+    with pytest.raises(ikdg_mod.IkdgError, match="loop cap"):
+        tree.box_search(box)
+    with pytest.raises(ikdg_mod.IkdgError, match="loop cap"):
+        tree.radius_search(np.zeros((1, 3), np.float32), 60.0)
+    tree.close()
+
+
 def test_default_cap_allows_the_longest_searches(ikdg_mod):
     # every point equally far: no subtree can be skipped, eight such queries a warp
     pts = np.full((20000, 3), 1.5, np.float32)
