@@ -202,6 +202,14 @@ struct Tree {
     // IKDG_MAX_VISITS lowers the cap of the traversals (tests use it to run into
     // the cap on a sound tree).
     int visit_cap = 0;
+    // The searches' stacks are sized for a tree of at most this many levels.  The
+    // height guard of the rebuilds keeps trees far below; should one grow past it all
+    // the same, its searches are refused until a rebuild.  (IKDG_MAX_LEVELS lowers it,
+    // for tests.)
+    int max_levels = MAX_STACK;
+    void check_levels() const {
+        if (dt.height > max_levels) throw Internal{"tree deeper than the traversal stack"};
+    }
     // The results are those of the inputs as they were when the call began: where an
     // output shares memory with an input, the inputs are copied first.
     struct Span {
@@ -273,6 +281,7 @@ struct Tree {
         CK(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
         direct = pageable != 0 && std::getenv("IKDG_HOST_STAGING") == nullptr;
         if (const char* e = std::getenv("IKDG_MAX_VISITS")) visit_cap = std::atoi(e);
+        if (const char* e = std::getenv("IKDG_MAX_LEVELS")) max_levels = std::min(std::atoi(e), MAX_STACK);
         CK(cudaMallocHost(&host_st, sizeof(DevStatus)));
         std::memset(host_st, 0, sizeof(DevStatus));
         ensure_pools(64, 64);
@@ -854,6 +863,7 @@ struct Tree {
         if (nq < 0 || stride < 3 || k < 1 || (nq > 0 && (q == nullptr || ids == nullptr || d2 == nullptr)))
             throw BadArg{"knn: bad arguments"};
         if (nq == 0) return;
+        check_levels();
         const size_t nk = (size_t)nq * k;
         const size_t tmp = knn_temp_bytes(nq, k);
         const size_t o_rows = align_up(sizeof(DevStatus));  // the status comes first
@@ -910,6 +920,7 @@ struct Tree {
             throw BadArg{"knn: bad arguments"};
         if (nq == 0) return;
         if ((long long)nq * k > (1ll << 31)) throw BadArg{"knn: nq * k too large"};
+        check_levels();
         float lim = max_sq_threshold(max_dist);
         size_t nk = (size_t)nq * k;
         if (device_ptrs) {
@@ -974,6 +985,7 @@ struct Tree {
             offsets[0] = 0;
             return;
         }
+        check_levels();
         const int logged = ids != nullptr ? RANGE_LOG : 0;
         const size_t qfloats = (size_t)nq * qs, rfloats = mode == 1 ? (size_t)(nq - 1) * rstride + 1 : 0;
         const size_t room = capacity > 0 ? (size_t)capacity : 0;
@@ -1051,6 +1063,7 @@ struct Tree {
             if (total) CK(cudaMemsetAsync(total, 0, sizeof(long long), stream));
             return;
         }
+        check_levels();
         const int passes = ids != nullptr ? RANGE_COUNT | RANGE_LOG : RANGE_COUNT;
         small.ensure(range_temp_bytes(nq, passes), stream);
         launch_range(dt, mode, q, qs, radius, rstride, nq, small.p, passes, offsets, ids, xyz, capacity, total, stream);
@@ -1086,6 +1099,7 @@ struct Tree {
             throw BadArg{"p2p_forward: bad arguments"};
         if (loss) *loss = 0;
         if (n == 0) return;
+        check_levels();
         // the search reports through the error bits alone
         zero_fields(offsetof(DevStatus, err), sizeof(int));
         const int nb = reg_blocks(n);
@@ -1593,6 +1607,7 @@ struct Batch {
         int h = 0;
         for (auto& r : reqs) {
             std::unique_lock<std::shared_mutex> lock(r.tree->mu);
+            r.tree->check_levels();
             h = std::max(h, r.tree->dt.height);
         }
         return h;
@@ -1608,6 +1623,7 @@ struct Batch {
             for (size_t i = 0; i < trees.size(); ++i) {
                 Tree* t = trees[i];
                 std::unique_lock<std::shared_mutex> lock(t->mu);
+                t->check_levels();  // (so a new plan always has room for it)
                 h_trees[i] = t->dt;
                 h_trees[i].st = d_st;
                 height = std::max(height, t->dt.height);
@@ -1929,6 +1945,7 @@ int ikdg_knn_device_noalloc(ikdg_tree* h, const float* q, int64_t nq, int32_t st
             throw ikdg::BadArg{"knn_device_noalloc: at most " + std::to_string(ikdg::NOALLOC_MAX_QUERIES) +
                                " queries per call (size of the static scratch array)"};
         if (nq == 0) return;
+        t.check_levels();
         void* scratch = nullptr;
         CK(ikdg::noalloc_scratch(t.device, &scratch));
         if (ikdg::knn_temp_bytes(nq, k) > ikdg::noalloc_scratch_bytes())

@@ -646,6 +646,11 @@ __device__ int list_jobs(const DevTree& t, const UpdateAux& a, int i0, int step)
         begin = end;
         end = min(end + __ldcg(&st->level_n[r]), a.list_cap);
     }
+    // (a taller tree than the rounds reach: its points must not be dropped)
+    for (int i = begin + i0; i < end; i += step) {
+        const int item = __ldcg(a.items + i);
+        if (item > 0 && !(item & 1)) atomicOr(&st->err, ERR_LIST);
+    }
     return end;
 }
 
