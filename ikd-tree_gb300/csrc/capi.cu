@@ -210,6 +210,19 @@ struct Tree {
     void check_levels() const {
         if (dt.height > max_levels) throw Internal{"tree deeper than the traversal stack"};
     }
+    // The tree as a search on its stream gets it.  A captured search may run again after
+    // a mutation that kept the pools: it starts at the top record, which stays where it
+    // is, and has stacks for any height.
+    DevTree search_tree() const {
+        DevTree t = dt;
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) cudaGetLastError();
+        if (cs != cudaStreamCaptureStatusNone) {
+            t.start = 0;
+            t.height = MAX_STACK;
+        }
+        return t;
+    }
     // The results are those of the inputs as they were when the call began: where an
     // output shares memory with an input, the inputs are copied first.
     struct Span {
@@ -925,7 +938,7 @@ struct Tree {
         size_t nk = (size_t)nq * k;
         if (device_ptrs) {
             small.ensure(knn_temp_bytes(nq, k) + 256, stream);
-            launch_knn(dt, q, stride, nq, k, lim, ids, d2, xyz, cnt, small.p, bin_bits_for(nq, k), stream);
+            launch_knn(search_tree(), q, stride, nq, k, lim, ids, d2, xyz, cnt, small.p, bin_bits_for(nq, k), stream);
             CK(cudaGetLastError());
             return;
         }
@@ -1066,7 +1079,8 @@ struct Tree {
         check_levels();
         const int passes = ids != nullptr ? RANGE_COUNT | RANGE_LOG : RANGE_COUNT;
         small.ensure(range_temp_bytes(nq, passes), stream);
-        launch_range(dt, mode, q, qs, radius, rstride, nq, small.p, passes, offsets, ids, xyz, capacity, total, stream);
+        launch_range(search_tree(), mode, q, qs, radius, rstride, nq, small.p, passes, offsets, ids, xyz, capacity, total,
+                     stream);
         CK(cudaGetLastError());
     }
 
@@ -1953,7 +1967,7 @@ int ikdg_knn_device_noalloc(ikdg_tree* h, const float* q, int64_t nq, int32_t st
         // Batches of QBIN_MIN_QUERIES or more are sorted (bins at QBIN_BITS
         // levels): the sort is the part that needs scratch.  Smaller batches
         // run unsorted and touch no scratch.  Nothing here allocates.
-        ikdg::launch_knn(t.dt, q, stride, nq, k, ikdg::max_sq_threshold(max_dist), ids, d2, xyz, cnt, scratch,
+        ikdg::launch_knn(t.search_tree(), q, stride, nq, k, ikdg::max_sq_threshold(max_dist), ids, d2, xyz, cnt, scratch,
                          ikdg::QBIN_BITS, t.stream);
         CK(cudaGetLastError());
     });

@@ -17,6 +17,10 @@
  *     ids; distance ties are broken by the smaller id.
  *   - Functions taking host pointers are synchronous.  *_device variants take
  *     device pointers and are asynchronous on the tree's stream.
+ *   - *_device searches may be captured into a CUDA graph on the tree's stream after one
+ *     such call has run.  The graph holds the addresses of the tree's arrays: it answers
+ *     for the tree as it is at a replay, until a call that makes the arrays grow (Build,
+ *     insertions, rebuilds; larger *_device searches).
  *   - All functions return an ikdg_status code.
  *   - Outputs of a host-pointer call may share memory with its inputs (the results are
  *     those of the inputs as they were when the call began), not with one another.
