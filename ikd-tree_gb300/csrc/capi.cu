@@ -753,16 +753,19 @@ struct Tree {
         finish_update(nullptr, nullptr, 0);
     }
 
+    // Subtrees the units of a box deletion can pass on (a unit passes on some 100).
+    static constexpr int SPILL = 1 << 16;
     long long delete_boxes(const float* boxes, long long m) {
         if (m < 0 || (m > 0 && boxes == nullptr)) throw BadArg{"delete_boxes: bad arguments"};
         if (m == 0 || st->root_code == 0) return 0;
         reset_counters();
-        op.ensure(align_up(sizeof(float) * m * 6), stream);
+        op.ensure(align_up(sizeof(float) * m * 6) + sizeof(int2) * SPILL, stream);
         float* raw = (float*)op.p;  // (every warp of a box reads it: a copy in HBM)
+        int2* spill = (int2*)((char*)op.p + align_up(sizeof(float) * m * 6));
         CK(cudaMemcpyAsync(raw, boxes, sizeof(float) * m * 6, cudaMemcpyHostToDevice, stream));
         // (the root's place in the top record leaves it 4, 2 or all 8 slots)
         launch_delete_boxes(dt, aux, raw, m, top_pos == 2 ? 2 : top_pos == 4 ? 1 : 3, F_DEL,
-                            (long long*)((char*)st_dev + offsetof(DevStatus, count)), stream);
+                            (long long*)((char*)st_dev + offsetof(DevStatus, count)), spill, SPILL, stream);
         // The rebuild rounds leave `count` alone: its value arrives with the
         // status reads of finish_update.
         finish_update(nullptr, nullptr, 0);

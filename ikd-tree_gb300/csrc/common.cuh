@@ -94,6 +94,7 @@ struct DevStatus {
     long long job_total;  // points gathered for rebuild jobs
     unsigned barrier;     // arrivals at settle_kernel's grid barriers
     int n_queue;          // nodes and leaves listed under the rebuild jobs
+    int n_spill;          // subtrees a box deletion passed on (box_delete_kernel)
     int level_n[24];      // of them, found by each round of the listing
     int dbg[8];           // details of the first internal error (diagnostics)
     long long bad;        // structural violations found by the validator

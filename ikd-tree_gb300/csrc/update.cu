@@ -1065,17 +1065,30 @@ __global__ void __launch_bounds__(DB_THREADS) box_restore_kernel(DevTree t, Upda
 // one record a step is expanded, which bounds the stack (bd_stack_entries).  Bound by
 // the chain of records; the kernel it replaces walked binary nodes with four block
 // barriers a level: 37 us for six boxes in 500,000 points, 13 now.
+// Where many boxes leave each of them few units, a unit that is not through after
+// `limit` steps puts what is on its stack on the list `spill` (as much as fits: the
+// bottom, which are the largest subtrees) and a second launch takes the list, a warp per
+// entry (`list`).  8,000,000 points, the call, a box of a million among 300 / 3,000 small
+// ones: 10.1 / 38.2 ms without the list, 1.2 / 2.7 with it; a box of everything 18.5 /
+// 283 ms and 1.8 / 17.1.
 constexpr int BD_WINDOW = 8;
 constexpr int BD_WIDE = 96;
 constexpr int BD_LEVELS_MAX = 4;
 constexpr long long BD_UNITS = 2048;
 constexpr int BD_CTA = 128;
+// Units per box below which a unit's work is limited (from there on the units are small
+// themselves), and the limit: boxes of up to some 5,000 points stay where they are.  The
+// second launch costs a call 1-2 us.
+constexpr int BD_FEW_UNITS = 256;
+constexpr int BD_LIMIT = 64;
+constexpr int BD_SPILL_BLOCKS = 152 * 8;
 __host__ __device__ constexpr int bd_stack_entries(int height) {
     return BD_WIDE + 7 * BD_WINDOW + 7 * (1 + (height + 2) / 3) + 1;
 }
 __global__ void __launch_bounds__(BD_CTA) box_delete_kernel(DevTree t, UpdateAux a, const float* boxes,
                                                             long long m, int levels, int top_bits,
-                                                            uint32_t del_flags, long long* __restrict__ total) {
+                                                            uint32_t del_flags, long long* __restrict__ total,
+                                                            bool list, int limit, int2* spill, int spill_cap) {
     chain_begin();
     extern __shared__ int stacks[];
     constexpr unsigned ALL = 0xffffffffu;
@@ -1084,19 +1097,21 @@ __global__ void __launch_bounds__(BD_CTA) box_delete_kernel(DevTree t, UpdateAux
     const int entries = bd_stack_entries(t.height);
     int* stack = stacks + (threadIdx.x >> 5) * entries;
     const int bits = levels > 0 ? top_bits + 3 * (levels - 1) : 0;
-    const long long units = m << bits, warps = (long long)gridDim.x * (BD_CTA / 32);
+    const long long units = list ? min(t.st->n_spill, spill_cap) : m << bits, warps = (long long)gridDim.x * (BD_CTA / 32);
     int count = 0;
     for (long long u = (long long)blockIdx.x * (BD_CTA / 32) + (threadIdx.x >> 5); u < units; u += warps) {
-        const float* bx = boxes + (u >> bits) * 6;
+        const int2 sp_in = list ? spill[u] : make_int2(0, 0);
+        const long long bi = list ? sp_in.y : u >> bits;
+        const float* bx = boxes + bi * 6;
         Box3 qb;
         for (int k = 0; k < 3; ++k) {
             qb.lo[k] = bx[k];
             qb.hi[k] = bx[3 + k];
         }
         // down to the unit's subtree (the whole warp reads the same words)
-        int part = (int)(u & ((1 << bits) - 1)), code = t.start, cov = 0;
+        int part = (int)(u & ((1 << bits) - 1)), code = list ? sp_in.x >> 1 : t.start, cov = list ? sp_in.x & 1 : 0;
         bool live = true;
-        for (int d = 0; d < levels && live && code >= 0; ++d) {
+        for (int d = 0; !list && d < levels && live && code >= 0; ++d) {
             const int w = d == 0 ? top_bits : 3;
             const float* f =
                 reinterpret_cast<const float*>(t.wide + (long long)code * 16) + wide_at(part & ((1 << w) - 1), 0);
@@ -1120,6 +1135,21 @@ __global__ void __launch_bounds__(BD_CTA) box_delete_kernel(DevTree t, UpdateAux
             if (steps > t.max_visits) {
                 if (lane == 0) atomicOr(&t.st->err, ERR_LOOP);
                 break;
+            }
+            if (limit > 0 && steps == limit) {
+                int base = 0;
+                if (lane == 0) base = atomicAdd(&t.st->n_spill, sp);
+                base = __shfl_sync(ALL, base, 0);
+                const int k = base < spill_cap ? min(sp, spill_cap - base) : 0;
+                for (int i = lane; i < k; i += 32) spill[base + i] = make_int2(stack[i], (int)bi);
+                sp -= k;
+                for (int i = lane; i - lane < sp; i += 32) {
+                    const int v = i < sp ? stack[i + k] : 0;
+                    __syncwarp();
+                    if (i < sp) stack[i] = v;
+                    __syncwarp();
+                }
+                if (sp == 0) break;
             }
             const int avail = min(sp, BD_WINDOW);
             const bool here = j < avail;
@@ -2119,7 +2149,7 @@ void launch_job_finish(const DevTree& t, const UpdateAux& a, cudaStream_t s) {
 }
 
 void launch_delete_boxes(const DevTree& t, const UpdateAux& a, const float* boxes, long long m, int top_bits,
-                         uint32_t flags, long long* total, cudaStream_t s) {
+                         uint32_t flags, long long* total, int2* spill, int spill_cap, cudaStream_t s) {
     if (m <= 0) return;
     // The tree is split below the top until there are units for the whole device
     // (six boxes in 500,000 points: 33 us with units of 128 buckets, 13 with
@@ -2128,7 +2158,12 @@ void launch_delete_boxes(const DevTree& t, const UpdateAux& a, const float* boxe
     while (levels < BD_LEVELS_MAX && bits < t.height && (m << bits) < BD_UNITS) bits += levels++ ? 3 : top_bits;
     const long long blocks = ((m << bits) + BD_CTA / 32 - 1) / (BD_CTA / 32);
     const size_t smem = sizeof(int) * bd_stack_entries(t.height) * (BD_CTA / 32);
-    launch_chain(box_delete_kernel, box_grid(blocks), BD_CTA, smem, s, t, a, boxes, m, levels, top_bits, flags, total);
+    const bool few = (1 << bits) < BD_FEW_UNITS && spill_cap > 0;
+    launch_chain(box_delete_kernel, box_grid(blocks), BD_CTA, smem, s, t, a, boxes, m, levels, top_bits, flags, total,
+                 false, few ? BD_LIMIT : 0, spill, spill_cap);
+    if (few)
+        launch_chain(box_delete_kernel, BD_SPILL_BLOCKS, BD_CTA, smem, s, t, a, boxes, m, 0, top_bits, flags, total, true,
+                     0, spill, spill_cap);
 }
 
 void launch_add_boxes(const DevTree& t, const UpdateAux& a, const float* boxes, long long m, cudaStream_t s) {

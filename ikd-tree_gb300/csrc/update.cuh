@@ -56,7 +56,7 @@ void launch_job_finish(const DevTree& t, const UpdateAux& a, cudaStream_t s);
 // Delete every valid point inside each box; `flags` = F_DEL or F_DEL|F_DSDEL;
 // top_bits = log2 of the slots the record at t.start may use.
 void launch_delete_boxes(const DevTree& t, const UpdateAux& a, const float* boxes, long long m, int top_bits,
-                         uint32_t flags, long long* total, cudaStream_t s);
+                         uint32_t flags, long long* total, int2* spill, int spill_cap, cudaStream_t s);
 void launch_delete_points(const DevTree& t, const UpdateAux& a, const float* pts, int stride, long long n,
                           cudaStream_t s);
 void launch_add_boxes(const DevTree& t, const UpdateAux& a, const float* boxes, long long m, cudaStream_t s);
