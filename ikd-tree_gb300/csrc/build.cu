@@ -20,6 +20,7 @@
 // All three cut a segment of n points at the point of rank n / 2 on its axis,
 // ties in input order (every partition is stable), so they follow one split
 // rule.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -750,8 +751,8 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) finish_split_kernel(DevTree t,
 //             left counts and their prefix sum, the node, the child segments (a
 //             block per segment)
 //   scatter   stable partition by (key, position), the children's AABBs
-// A uniform segment's candidates are ~1/1,000 of it; with many equal keys the
-// list can hold most of the segment, which only makes select slower.
+// A uniform segment's candidates are ~1/1,000 of it; a stray point far away or many
+// equal keys put most of the segment on the list (select_large).
 // This took the place of sorting the three coordinates once and partitioning the
 // three sorted index arrays per level with random gathers of the sides (109
 // launches): a 2M-point build moves 16 instead of ~100 bytes per point and level
@@ -767,9 +768,9 @@ constexpr int SPLIT_CACHE = 4096;  // candidates kept in shared memory by select
 // The split axis of a segment (longest extent, first on ties) and its bins: equal
 // widths over the segment's range.  The bin grows with the coordinate (every
 // operation rounds monotonically), which is all the selection needs; an outlier
-// that stretches the range only makes the candidate lists longer.  (Bins of the
+// that stretches the range makes the candidate lists longer.  (Bins of the
 // ordered keys put a quarter of an octave into each where the range spans zero:
-// select took up to 187 us on 20k candidates.)
+// 20k candidates also where the points are even.)
 struct SplitAxis {
     int axis;
     float lo, scale;
@@ -978,19 +979,29 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_classify_kernel(const flo
     __syncthreads();
     const float* c = reinterpret_cast<const float*>(pts) + ax.axis;
     const int lane = threadIdx.x & 31;
-    int mine = 0;
+    int mine = 0, picked = 0;
+    float x[SPLIT_ROUNDS];
+    unsigned eq[SPLIT_ROUNDS];
 #pragma unroll
     for (int r = 0; r < SPLIT_ROUNDS; ++r) {
         const int i = t0 + r * SPLIT_THREADS + threadIdx.x;
-        const float x = i < sg.y ? c[4ll * i] : 0.f;
-        const int b = i < sg.y ? ax.bin(x) : SPLIT_BINS;
+        x[r] = i < sg.y ? c[4ll * i] : 0.f;
+        const int b = i < sg.y ? ax.bin(x[r]) : SPLIT_BINS;
         mine += b < bin ? 1 : 0;
-        const unsigned eq = __ballot_sync(0xffffffffu, b == bin);
-        if (eq == 0) continue;
+        eq[r] = __ballot_sync(0xffffffffu, b == bin);
+        picked += __popc(eq[r]);
+    }
+    if (picked) {  // one addition per warp: the bin can hold all of the tile
         int at = 0;
-        if (lane == 0) at = atomicAdd(lv.cand_n + q, __popc(eq));
-        at = __shfl_sync(0xffffffffu, at, 0) + __popc(eq & ((1u << lane) - 1u));
-        if (b == bin) cand[sg.x + at] = make_uint2(float_key(x), (uint32_t)(i - sg.x));
+        if (lane == 0) at = atomicAdd(lv.cand_n + q, picked);
+        at = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+        for (int r = 0; r < SPLIT_ROUNDS; ++r) {
+            const int i = t0 + r * SPLIT_THREADS + threadIdx.x;
+            if (eq[r] >> lane & 1)
+                cand[sg.x + at + __popc(eq[r] & ((1u << lane) - 1u))] = make_uint2(float_key(x[r]), (uint32_t)(i - sg.x));
+            at += __popc(eq[r]);
+        }
     }
     mine = __reduce_add_sync(0xffffffffu, mine);
     if (lane == 0 && mine) atomicAdd(&less, mine);
@@ -998,12 +1009,117 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_classify_kernel(const flo
     if (threadIdx.x == 0) tile_left[split_tile0(sg.x) + tile] = less;
 }
 
-// One 8-bit (or narrower) step of a radix selection: digit(i) of the items that
-// still match (-1: not), rank -> the digit that holds the rank, the rank inside
-// it and the items of that digit.
+// A bin with more points than select keeps in shared memory: a stray point far away, heavy
+// tails, towns far apart or many equal coordinates put nearly all of a segment into one.
+// The list is then read by a cluster of blocks, with every thread's next eight items in
+// flight, in digits of 11 bits (three of the key, at most three of the position), and
+// the tiles' counts take one addition per warp and tile.  A build of 2M points, one block
+// and digits of 8 bits / this: one point at 1e9 m 6861 / 1437 us, four towns 5346 / 1324,
+// Cauchy 8012 / 1510, all equal 10526 / 1544 (evenly spread: 874 / 870).
 struct SplitDigit {
     int digit, rank, count;
 };
+constexpr int SELECT_BITS = 11;
+constexpr int SELECT_BINS = 1 << SELECT_BITS;
+constexpr int SELECT_CLUSTER = 8;      // blocks, at most, for a segment
+constexpr long long SELECT_SHARE = 32768;  // points per block (every block reads all the others' bins)
+
+// f(item) for this block's share of the list.
+template <int THREADS, class F>
+__device__ __forceinline__ void select_each(const uint2* list, int c, int blocks, int block, F f) {
+    const int step = blocks * THREADS;
+    for (int base = block * THREADS + threadIdx.x; base - (int)threadIdx.x < c; base += 8 * step) {
+        uint2 e[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            e[u] = base + u * step < c ? list[base + u * step] : make_uint2(0u, 0xffffffffu);  // (no such position)
+#pragma unroll
+        for (int u = 0; u < 8; ++u) f(e[u]);
+    }
+}
+
+// The key and position of rank `rank` among the c items of a list, and the left counts of
+// the tiles (tl) for those before it: by all blocks of the cluster.  mem: 2 * SELECT_BINS
+// ints of shared memory.
+template <int THREADS>
+__device__ void select_large(const uint2* list, int c, int cnt, int rank, int* tl, int* mem, uint32_t* wsum,
+                             uint32_t* tot, SplitDigit* sd, uint32_t& v, uint32_t& p) {
+    const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const int blocks = (int)cl.num_blocks(), block = (int)cl.block_rank();
+    constexpr int PER = SELECT_BINS / THREADS;
+    int pass = 0;
+    // One digit: digit(item), -1 for an item that no longer matches.  The histograms of
+    // two passes take turns, so one cluster barrier a pass will do.
+    auto step = [&](auto digit) {
+        int* h = mem + (pass++ & 1) * SELECT_BINS;
+        for (int i = threadIdx.x; i < SELECT_BINS; i += THREADS) h[i] = 0;
+        __syncthreads();
+        select_each<THREADS>(list, c, blocks, block, [&](const uint2& e) {
+            const int d = e.y == 0xffffffffu ? -1 : digit(e);
+            if (d >= 0) atomicAdd(&h[d], 1);
+        });
+        cl.sync();
+        int n[PER], sum = 0;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) n[j] = 0;
+        for (int k = 0; k < blocks; ++k) {
+            const int* o = cl.map_shared_rank(h, k) + threadIdx.x * PER;
+#pragma unroll
+            for (int j = 0; j < PER; ++j) n[j] += o[j];
+        }
+#pragma unroll
+        for (int j = 0; j < PER; ++j) sum += n[j];
+        uint32_t total;
+        int r = rank - (int)block_scan_u32<THREADS>((uint32_t)sum, wsum, tot, &total);
+        if (r >= 0 && r < sum) {  // exactly one thread
+            int d = 0;
+#pragma unroll
+            for (int j = 0; j < PER; ++j) {
+                if (r < n[j]) {
+                    d = j;
+                    break;
+                }
+                r -= n[j];
+            }
+            *sd = SplitDigit{(int)threadIdx.x * PER + d, r, n[d]};
+        }
+        __syncthreads();
+        const SplitDigit g = *sd;
+        __syncthreads();
+        rank = g.rank;
+        return g;
+    };
+    v = p = 0;
+    for (int b = 32; b > 0;) {
+        const int w = min(b, SELECT_BITS);
+        const SplitDigit g = step([&](const uint2& e) {
+            return (b < 32 ? e.x >> b : 0u) == v ? (int)((e.x >> (b - w)) & ((1u << w) - 1u)) : -1;
+        });
+        v = (v << w) | (uint32_t)g.digit;
+        b -= w;
+    }
+    for (int b = 32 - __clz(cnt); b > 0;) {
+        const int w = min(b, SELECT_BITS);
+        const SplitDigit g = step([&](const uint2& e) {
+            return e.x == v && (e.y >> b) == p ? (int)((e.y >> (b - w)) & ((1u << w) - 1u)) : -1;
+        });
+        p = (p << w) | (uint32_t)g.digit;
+        b -= w;
+    }
+    const int lane = threadIdx.x & 31;
+    select_each<THREADS>(list, c, blocks, block, [&](const uint2& e) {
+        const bool left = e.y != 0xffffffffu && (e.x < v || (e.x == v && e.y < p));
+        const int tile = left ? (int)(e.y / SPLIT_TILE) : -1;
+        const unsigned same = __match_any_sync(0xffffffffu, tile);
+        if (left && lane == __ffs(same) - 1) atomicAdd(tl + tile, __popc(same));
+    });
+    __threadfence();
+    cl.sync();  // the first block goes on with the counts; nobody's shared memory is read any more
+}
+
+// One 8-bit (or narrower) step of a radix selection: digit(i) of the items that
+// still match (-1: not), rank -> the digit that holds the rank, the rank inside
+// it and the items of that digit.
 template <int THREADS, class F>
 __device__ __forceinline__ SplitDigit split_digit(int n, int rank, int* hist, SplitDigit* out, F digit) {
     for (int i = threadIdx.x; i < 256; i += THREADS) hist[i] = 0;
@@ -1061,57 +1177,59 @@ __global__ void __launch_bounds__(THREADS) split_select_kernel(DevTree t, SplitL
     __shared__ int hist[256];
     __shared__ SplitDigit sd;
     __shared__ uint32_t wsum[THREADS / 32], tot, spos;
-    const int q = blockIdx.x;
+    const int blocks = (int)cooperative_groups::this_cluster().num_blocks(), q = blockIdx.x / blocks;
     if (q >= split_segs(lv, cap)) return;
+    const bool lead = blockIdx.x % blocks == 0;
+    const int c = lv.cand_n[q];
+    if (!lead && c <= SPLIT_CACHE) return;
     const int4 sg = lv.seg[q];
     const int s = sg.x, cnt = sg.y - sg.x, m = cnt / 2, link = sg.z;
     const SplitAxis ax = split_axis(lv.box + 6 * q);
-    const int c = lv.cand_n[q];
     const uint2* list = cand + s;
-    const bool cached = c <= SPLIT_CACHE;
-    if (cached) {
+    int* tl = tile_left + split_tile0(s);  // the tiles' left counts: so far the lower bins'
+    uint32_t v = 0, p = 0;
+    if (c > SPLIT_CACHE) {
+        select_large<THREADS>(list, c, cnt, pick[q].y, tl, reinterpret_cast<int*>(cache), wsum, &tot, &sd, v, p);
+        if (!lead) return;
+    } else {
         for (int i = threadIdx.x; i < c; i += THREADS) cache[i] = list[i];
         __syncthreads();
-    }
-    auto item = [&](int i) { return cached ? cache[i] : list[i]; };
-    // The key of rank n / 2, eight bits at a time.
-    int rank = pick[q].y, same = c;
-    uint32_t v = 0;  // bits found so far
-    for (int b = 32; b > 0; b -= 8) {
-        const SplitDigit r = split_digit<THREADS>(c, rank, hist, &sd, [&](int i) {
-            const uint32_t k = item(i).x;
-            return (b < 32 ? k >> b : 0u) == v ? (int)((k >> (b - 8)) & 255u) : -1;
-        });
-        v = (v << 8) | (uint32_t)r.digit;
-        rank = r.rank;
-        same = r.count;
-    }
-    // Among equal keys the position of that rank.
-    uint32_t p = 0;
-    if (same > 1) {
-        for (int b = 32 - __clz(cnt); b > 0;) {
-            const int w = min(b, 8);
+        // The key of rank n / 2, eight bits at a time.
+        int rank = pick[q].y, same = c;
+        for (int b = 32; b > 0; b -= 8) {
             const SplitDigit r = split_digit<THREADS>(c, rank, hist, &sd, [&](int i) {
-                const uint2 e = item(i);
-                return e.x == v && (e.y >> b) == p ? (int)((e.y >> (b - w)) & ((1u << w) - 1u)) : -1;
+                const uint32_t k = cache[i].x;
+                return (b < 32 ? k >> b : 0u) == v ? (int)((k >> (b - 8)) & 255u) : -1;
             });
-            p = (p << w) | (uint32_t)r.digit;
+            v = (v << 8) | (uint32_t)r.digit;
             rank = r.rank;
-            b -= w;
+            same = r.count;
         }
-    } else {
-        for (int i = threadIdx.x; i < c; i += THREADS)
-            if (item(i).x == v) spos = item(i).y;
+        // Among equal keys the position of that rank.
+        if (same > 1) {
+            for (int b = 32 - __clz(cnt); b > 0;) {
+                const int w = min(b, 8);
+                const SplitDigit r = split_digit<THREADS>(c, rank, hist, &sd, [&](int i) {
+                    const uint2 e = cache[i];
+                    return e.x == v && (e.y >> b) == p ? (int)((e.y >> (b - w)) & ((1u << w) - 1u)) : -1;
+                });
+                p = (p << w) | (uint32_t)r.digit;
+                rank = r.rank;
+                b -= w;
+            }
+        } else {
+            for (int i = threadIdx.x; i < c; i += THREADS)
+                if (cache[i].x == v) spos = cache[i].y;
+            __syncthreads();
+            p = spos;
+        }
+        // the candidates before (v, p)
+        for (int i = threadIdx.x; i < c; i += THREADS) {
+            const uint2 e = cache[i];
+            if (e.x < v || (e.x == v && e.y < p)) atomicAdd(tl + e.y / SPLIT_TILE, 1);
+        }
         __syncthreads();
-        p = spos;
     }
-    // The tiles' left counts: the lower bins', and the candidates before (v, p).
-    int* tl = tile_left + split_tile0(s);
-    for (int i = threadIdx.x; i < c; i += THREADS) {
-        const uint2 e = item(i);
-        if (e.x < v || (e.x == v && e.y < p)) atomicAdd(tl + e.y / SPLIT_TILE, 1);
-    }
-    __syncthreads();
     const int tiles = (cnt + SPLIT_TILE - 1) / SPLIT_TILE;
     uint32_t carry = 0;
     for (int base = 0; base < tiles; base += THREADS) {
@@ -1381,9 +1499,11 @@ void build_subtrees(const DevTree& t, const float4* pts, long long n, const int*
             launch_chain(split_hist_kernel, hblocks, HIST_THREADS, 0, s, src, cur, mh, bs.hist);
             launch_chain(split_pick_kernel, segs, SPLIT_THREADS, 0, s, cur, nx, cap, bs.hist, bs.pick);
             launch_chain(split_classify_kernel, blocks, SPLIT_THREADS, 0, s, src, cur, mt, bs.pick, bs.tile_left, bs.cand);
-            // few segments have many candidates each
+            // Few segments can have many candidates each.
+            unsigned k = 1;
+            while (k < SELECT_CLUSTER && size >= 2 * k * SELECT_SHARE && 2 * k * segs <= 256) k *= 2;
             if (segs <= 64)
-                launch_chain(split_select_kernel<1024>, segs, 1024, 0, s, t, cur, nx, cap, bs.pick, bs.tile_left, bs.cand,
+                launch_chain_if(true, k, split_select_kernel<1024>, k * segs, 1024, 0, s, t, cur, nx, cap, bs.pick, bs.tile_left, bs.cand,
                                                                          bs.thr, bs.kids, bs.small, nsmall, (int)ms,
                                                                          fill);
             else

@@ -35,24 +35,33 @@ inline cudaError_t take_chain_refused() {
     return e;
 }
 template <class... P, class... A>
-inline void launch_chain_if(bool chain, void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s,
-                            A&&... args) {
+inline void launch_chain_if(bool chain, unsigned cluster, void (*kernel)(P...), dim3 grid, unsigned block, size_t smem,
+                            cudaStream_t s, A&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (chain) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = cluster;
+        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        ++n;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = chain ? 1 : 0;
+    cfg.numAttrs = n;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
     if (e != cudaSuccess && chain_refused == cudaSuccess) chain_refused = e;
 }
 template <class... P, class... A>
 inline void launch_chain(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
-    launch_chain_if(true, kernel, grid, block, smem, s, std::forward<A>(args)...);
+    launch_chain_if(true, 1, kernel, grid, block, smem, s, std::forward<A>(args)...);
 }
 
 

@@ -167,14 +167,14 @@ void exclusive_scan_t(const T* in, T* out, long long n, T* total, void* temp, cu
         return;
     }
     if (n <= SCAN_ONE) {
-        launch_chain_if(chain, scan_single_kernel<T>, 1, SCAN_ONE_THREADS, 0, s, in, out, (int)n, total);
+        launch_chain_if(chain, 1, scan_single_kernel<T>, 1, SCAN_ONE_THREADS, 0, s, in, out, (int)n, total);
         return;
     }
     int tiles = (int)((n + SCAN_TILE - 1) / SCAN_TILE);
     T* partial = (T*)temp;
-    launch_chain_if(chain, scan_reduce_kernel<T>, tiles, SCAN_THREADS, 0, s, in, n, partial);
-    launch_chain_if(chain, scan_partials_kernel<T>, 1, 1024, 0, s, partial, tiles, total);
-    launch_chain_if(chain, scan_down_kernel<T>, tiles, SCAN_THREADS, 0, s, in, out, n, partial);
+    launch_chain_if(chain, 1, scan_reduce_kernel<T>, tiles, SCAN_THREADS, 0, s, in, n, partial);
+    launch_chain_if(chain, 1, scan_partials_kernel<T>, 1, 1024, 0, s, partial, tiles, total);
+    launch_chain_if(chain, 1, scan_down_kernel<T>, tiles, SCAN_THREADS, 0, s, in, out, n, partial);
 }
 
 // ---- radix sort --------------------------------------------------------------
@@ -289,9 +289,9 @@ bool radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32
     dim3 grid(tiles, batch);
     for (int p = 0; p < passes; ++p) {
         int shift = 8 * p;
-        launch_chain_if(chain, sort_hist_kernel, grid, SORT_THREADS, 0, s, ki, n, stride, shift, tiles, rounds, hist);
+        launch_chain_if(chain, 1, sort_hist_kernel, grid, SORT_THREADS, 0, s, ki, n, stride, shift, tiles, rounds, hist);
         exclusive_scan(hist, offs, hn, nullptr, stemp, s, chain);
-        launch_chain_if(chain, sort_scatter_kernel, grid, SORT_THREADS, 0, s, ki, vi, ko, vo, n, stride, shift, tiles, rounds, offs);
+        launch_chain_if(chain, 1, sort_scatter_kernel, grid, SORT_THREADS, 0, s, ki, vi, ko, vo, n, stride, shift, tiles, rounds, offs);
         uint32_t* t;
         t = ki; ki = ko; ko = t;
         t = vi; vi = vo; vo = t;
