@@ -410,9 +410,12 @@ __device__ __forceinline__ bool cand_less(float d, int id, float d2, int id2) {
 
 __device__ __forceinline__ void knn_rows_body(const DevTree& t, bool valid, long long qi, float qx, float qy, float qz,
                                               int k, float max_sq, const KnnOut& o, int* __restrict__ slots) {
-    float* gd = o.d2 + qi * k;
-    int* gi = o.id + qi * k;
-    int* gs = slots + qi * k;
+    // (the three parts of a list are arrays of their own: the shifts of an insertion are
+    // bound by the order of their loads and stores; 20k queries, k = 100, on 1M points
+    // 7.6 ms without the qualifiers, 6.3 with)
+    float* __restrict__ gd = o.d2 + qi * k;
+    int* __restrict__ gi = o.id + qi * k;
+    int* __restrict__ gs = slots + qi * k;
     int cnt = 0;
     float worst = FINF;
     int worst_id = 0x7fffffff;
@@ -477,15 +480,37 @@ __device__ __forceinline__ void knn_rows_body(const DevTree& t, bool valid, long
         const bool leafwork = !done && cur < 0;
         if (!__any_sync(0xffffffffu, leafwork)) break;
         if (!leafwork) continue;
+        // Two passes: first the slots that can enter the list are marked, with four
+        // pairs of slots in flight and no branch, so the lanes stay together; then only
+        // those are offered.  (Offering in one pass runs the insertion for every slot
+        // at which any lane has a candidate.)
         const int L = code_leaf(cur);
         const int n = min(__ldg(t.leaf_n + L), LEAF_CAP);
-        for (int j = 0; j < n; ++j) {
-            const float4 p = __ldg(t.pts + (long long)L * LEAF_CAP + j);
-            const uint32_t w = __float_as_uint(p.w);
-            if (w & F_DEL) continue;
+        const float4* lp = t.pts + (long long)L * LEAF_CAP;
+        const f32x2 qxy = pack2(qx, qy);
+        unsigned marks = 0;
+        for (int j0 = 0; j0 < n; j0 += 8) {
+            Quad2 p[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) p[u] = ld_quad2(lp + j0 + 2 * u);  // (slots past the fill stay in the bucket)
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                float z, w;
+                unpack2(p[u >> 1].v[2 * (u & 1) + 1], z, w);
+                const float d = slot_dist(qxy, qz, p[u >> 1].v[2 * (u & 1)], z);
+                const int id = (int)(__float_as_uint(w) & ID_MASK);
+                const bool in = j0 + u < n && !(__float_as_uint(w) & F_DEL) && d <= max_sq &&
+                                cand_less(d, id, worst, worst_id);
+                marks |= (in ? 1u : 0u) << (j0 + u);
+            }
+        }
+        while (marks) {
+            const int j = __ffs(marks) - 1;
+            marks &= marks - 1;
+            const float4 p = __ldg(lp + j);
             const float d = sq_dist(qx, qy, qz, p.x, p.y, p.z);
-            const int id = (int)(w & ID_MASK);
-            if (!(d <= max_sq && cand_less(d, id, worst, worst_id))) continue;
+            const int id = (int)(__float_as_uint(p.w) & ID_MASK);
+            if (!cand_less(d, id, worst, worst_id)) continue;
             int pos = cnt < k ? cnt : k - 1;
             while (pos > 0 && cand_less(d, id, gd[pos - 1], gi[pos - 1])) {
                 gd[pos] = gd[pos - 1];
