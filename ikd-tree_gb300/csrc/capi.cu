@@ -175,13 +175,12 @@ struct Tree {
     int fill = 16;
     int min_size = 2 * LEAF_CAP;
     // Tree levels used to order a kNN batch before the search: -1 (default)
-    // = QBIN_AUTO_BITS for large batches and lists on trees larger than the L2
-    // cache, none otherwise; 0 = never; 1..16 = always (batches of
-    // QBIN_MIN_QUERIES or more).
+    // = knn_auto_bits; 0 = never; 1..16 = always (batches of QBIN_MIN_QUERIES or
+    // more).
     int knn_bin_bits = -1;
-    int bin_bits_for(long long nq, int k) const {
+    int bin_bits_for(long long nq, int k, bool host) const {
         if (knn_bin_bits >= 0) return knn_bin_bits;
-        return nq >= QBIN_AUTO_QUERIES && k >= QBIN_AUTO_K && st->root_slots >= QBIN_AUTO_SLOTS ? QBIN_AUTO_BITS : 0;
+        return knn_auto_bits(nq, k, st->root_slots, host);
     }
     // On Grace-Blackwell the GPU reads and writes pageable host memory through
     // NVLink-C2C with the CPU's page tables (cudaDevAttrPageableMemoryAccess).
@@ -888,7 +887,7 @@ struct Tree {
         const size_t o_cnt = o_xyz + (xyz ? align_up(sizeof(float) * 3 * nk) : 0);
         const size_t o_q = o_cnt + (cnt ? align_up(sizeof(int) * nq) : 0);
         const size_t o_tmp = o_q + align_up(sizeof(float) * nq * stride);
-        const int bits = bin_bits_for(nq, k);
+        const int bits = bin_bits_for(nq, k, true);
         // (a sorted batch's rows would leave one by one)
         const bool direct = this->direct && bits == 0 && knn_apart(q, nq, stride, k, ids, d2, xyz, cnt);
         SearchCtx* c = take_ctx();
@@ -941,11 +940,11 @@ struct Tree {
         size_t nk = (size_t)nq * k;
         if (device_ptrs) {
             small.ensure(knn_temp_bytes(nq, k) + 256, stream);
-            launch_knn(search_tree(), q, stride, nq, k, lim, ids, d2, xyz, cnt, small.p, bin_bits_for(nq, k), stream);
+            launch_knn(search_tree(), q, stride, nq, k, lim, ids, d2, xyz, cnt, small.p, bin_bits_for(nq, k, false), stream);
             CK(cudaGetLastError());
             return;
         }
-        if (direct && k <= KNN_GROUP_MAX && bin_bits_for(nq, k) == 0 && knn_apart(q, nq, stride, k, ids, d2, xyz, cnt)) {
+        if (direct && k <= KNN_GROUP_MAX && bin_bits_for(nq, k, true) == 0 && knn_apart(q, nq, stride, k, ids, d2, xyz, cnt)) {
             // Kernels read the queries and write the results in host memory:
             // each CTA's rows leave as coalesced 16-byte spans.  (A sorted
             // batch's rows would leave one by one, and lists in the output rows
@@ -979,7 +978,7 @@ struct Tree {
         int* dcnt = cnt ? c.take<int>(nq) : nullptr;
         char* temp = c.take<char>(knn_temp_bytes(nq, k));
         CK(cudaMemcpyAsync(dq, q, sizeof(float) * nq * stride, cudaMemcpyHostToDevice, stream));
-        launch_knn(dt, dq, stride, nq, k, lim, dids, dd2, dxyz, dcnt, temp, bin_bits_for(nq, k), stream);
+        launch_knn(dt, dq, stride, nq, k, lim, dids, dd2, dxyz, dcnt, temp, bin_bits_for(nq, k, true), stream);
         CK(cudaMemcpyAsync(ids, dids, sizeof(int) * nk, cudaMemcpyDeviceToHost, stream));
         CK(cudaMemcpyAsync(d2, dd2, sizeof(float) * nk, cudaMemcpyDeviceToHost, stream));
         if (xyz) CK(cudaMemcpyAsync(xyz, dxyz, sizeof(float) * nk * 3, cudaMemcpyDeviceToHost, stream));
@@ -1134,7 +1133,7 @@ struct Tree {
         double* part = reg_sums(nb);
         const RegPose P = reg_pose(pose);
         launch_transform(scan, n, P, w, stream);
-        launch_knn(dt, w, 3, n, k, max_sq_threshold(max_dist), ids, d2, nbr, cnt, temp, bin_bits_for(n, k),
+        launch_knn(dt, w, 3, n, k, max_sq_threshold(max_dist), ids, d2, nbr, cnt, temp, bin_bits_for(n, k, false),
                    stream);
         launch_plane_residual(scan, P, n, k, nbr, cnt, thresh, (float4*)planes, res, valid, part, stream);
         read_status();

@@ -130,17 +130,29 @@ constexpr int KNN_GROUP_MAX = 64;
 constexpr int QBIN_BITS = 16;
 constexpr int QBIN_BINS = 1 << QBIN_BITS;
 constexpr long long QBIN_MIN_QUERIES = 2048;
-// By default a batch is sorted when it and its lists are large and the tree does
-// not fit the L2 cache: neighbouring queries then share what they fetch from
-// HBM.  20M-point slab, 1M queries, unsorted / sorted by 14 levels (us, calls on
-// three trees in turn): k = 32 1676 / 1515, k = 16 1151 / 1067, k = 5 829 / 804,
-// k = 1 445 / 481; 20M uniform points k = 5 974 / 979; 10M points, 500k queries
-// k = 5 484 / 498; 3M points, 250k queries 233 / 243; 1M points, 1M queries
-// 770 / 802.
-constexpr long long QBIN_AUTO_QUERIES = 1 << 19;
-constexpr long long QBIN_AUTO_SLOTS = 12000000;
-constexpr int QBIN_AUTO_K = 8;
-constexpr int QBIN_AUTO_BITS = 14;
+// Whether a batch is sorted by default (by 16 levels).  Sorted neighbours share what
+// they fetch and walk alike, which pays where the search is long against the sort (30 to
+// 60 us per million queries): many queries on a small map, long lists on a map beyond
+// the L2 cache, or very many queries.  With k <= 2 such a batch goes to a thread per
+// query, which issues less than a group when 32 neighbours walk alike.  Device buffers,
+// unsorted / sorted (us), surfaces unless said:
+//   20k points, 1.5M queries: k = 1 426 / 360 (a thread each), k = 2 537 / 470, k = 5
+//   836 / 779, 600k queries: k = 8 455 / 431, k = 32 1886 / 1611;
+//   200k: 1.5M, k = 1 493 / 430, k = 5 890 / 844, uniform 950 / 962;
+//   3M uniform: 1M, k = 1 339 / 378, k = 8 988 / 1030, 5M, k = 8 one per cent apart;
+//   20M slab: 1M, k = 16 1107 / 1064, k = 5 829 / 804, 500k k = 5 on 10M 484 / 498.
+// The lines (slots, queries) lie where surfaces gain more than uniform maps lose; up to
+// 500k queries nothing is sorted.  Host buffers: only the long lists on large maps (a
+// sorted batch's rows come back by copy).
+constexpr int QBIN_AUTO_BITS = 16;
+constexpr long long KNN_THREAD_QUERIES = 900000;
+inline int knn_auto_bits(long long nq, int k, long long slots, bool host) {
+    const bool large_map = k >= 8 && slots >= 12000000 && nq >= 1 << 19;
+    const bool small_map = slots < 300000 && nq >= 1 << 19 && nq * k >= 4500000;
+    const bool threads = k <= 2 && nq >= (slots < 2000000 ? KNN_THREAD_QUERIES : 1 << 21);
+    const bool sort = large_map || (!host && (threads || (k > 2 && (small_map || nq >= 4000000))));
+    return sort ? QBIN_AUTO_BITS : 0;
+}
 size_t knn_temp_bytes(long long nq, int k);
 // Host-pointer kNN calls of at most this many queries (and k <= KNN_GROUP_MAX)
 // run on pooled per-call streams with the tree's lock held shared, so

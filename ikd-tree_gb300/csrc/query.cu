@@ -180,8 +180,9 @@ __global__ void __launch_bounds__(search::RANGE_CTA, 8) range_write_kernel(DevTr
     search::range_warp<MODE, true>(t, w, todo, entries, log, lc, start, start + c, ids, xyz);
 }
 
-// k > 64: a thread per query, the list in its output rows.
-__global__ void __launch_bounds__(KNN_THREADS) knn_rows_kernel(DevTree t, const float* __restrict__ q, int q_stride,
+// A thread per query: k > 64 (K = 0), or k = K and very many sorted queries.
+template <int K>
+__global__ void __launch_bounds__(KNN_THREADS) knn_thread_kernel(DevTree t, const float* __restrict__ q, int q_stride,
                                                                long long nq, int k, float max_sq, search::KnnOut o,
                                                                int* __restrict__ slots, const int* __restrict__ perm) {
     const long long tid = (long long)blockIdx.x * KNN_THREADS + threadIdx.x;
@@ -191,7 +192,7 @@ __global__ void __launch_bounds__(KNN_THREADS) knn_rows_kernel(DevTree t, const 
     const float qx = valid ? q[qi * q_stride + 0] : 0.f;
     const float qy = valid ? q[qi * q_stride + 1] : 0.f;
     const float qz = valid ? q[qi * q_stride + 2] : 0.f;
-    search::knn_rows_body(t, valid, qi, qx, qy, qz, k, max_sq, o, slots);
+    search::knn_thread_body<K>(t, valid, qi, qx, qy, qz, k, max_sq, o, slots);
 }
 
 // ---- query binning -----------------------------------------------------------
@@ -259,8 +260,13 @@ void launch_knn(const DevTree& t, const float* q, int q_stride, long long nq, in
     }
     const search::KnnOut o{out_id, out_d2, out_xyz, out_cnt};
     if (k > KNN_GROUP_MAX) {
-        knn_rows_kernel<<<blocks_for(nq, KNN_THREADS), KNN_THREADS, 0, s>>>(t, q, q_stride, nq, k, max_sq, o, (int*)tp,
-                                                                            perm);
+        knn_thread_kernel<0><<<blocks_for(nq, KNN_THREADS), KNN_THREADS, 0, s>>>(t, q, q_stride, nq, k, max_sq, o,
+                                                                              (int*)tp, perm);
+        return;
+    }
+    if (perm != nullptr && k <= 2 && nq >= KNN_THREAD_QUERIES) {
+        auto kernel = k == 1 ? knn_thread_kernel<1> : knn_thread_kernel<2>;
+        kernel<<<blocks_for(nq, KNN_THREADS), KNN_THREADS, 0, s>>>(t, q, q_stride, nq, k, max_sq, o, nullptr, perm);
         return;
     }
     const bool staged = host_out && perm == nullptr;

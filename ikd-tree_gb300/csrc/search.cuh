@@ -398,18 +398,27 @@ __device__ __forceinline__ void knn_write_rows(const DevTree& t, const KnnLane& 
     if (valid && o.cnt != nullptr && g.sl == 0) o.cnt[row] = cnt;
 }
 
-// ---- kNN, k > 64: a thread per query over the binary records -----------------------
+// ---- kNN, a thread per query over the binary records ---------------------------------
 //
-// The sorted list lives in the query's output rows, with the slot index of each
-// entry in `slots` (k ints per query).  Nearer child first, the farther one
-// stacked with its box distance; leaves are scanned by the warp's threads
-// together, each its own.
+// For k > 64 (K = 0): the sorted list lives in the query's output rows, with the slot
+// index of each entry in `slots` (k ints per query).  For k = K <= 2 and very many
+// sorted queries: in registers (32 neighbours' walks are nearly the same, so a thread
+// each issues less than a group each; see KNN_THREAD_QUERIES).  Nearer child first,
+// the farther one stacked with its box distance; leaves are scanned by the warp's
+// threads together, each its own.
 __device__ __forceinline__ bool cand_less(float d, int id, float d2, int id2) {
     return d < d2 || (d == d2 && id < id2);
 }
 
-__device__ __forceinline__ void knn_rows_body(const DevTree& t, bool valid, long long qi, float qx, float qy, float qz,
-                                              int k, float max_sq, const KnnOut& o, int* __restrict__ slots) {
+template <int K>
+__device__ __forceinline__ void knn_thread_body(const DevTree& t, bool valid, long long qi, float qx, float qy, float qz,
+                                                int k, float max_sq, const KnnOut& o, int* __restrict__ slots) {
+    constexpr int PAIRS = K > 0 ? 2 : 4;  // of slots in flight
+    constexpr int KR = K > 0 ? K : 1;
+    float bd[KR];
+    int bi[KR], bs[KR];
+#pragma unroll
+    for (int m = 0; m < KR; ++m) bd[m] = FINF, bi[m] = 0x7fffffff, bs[m] = -1;
     // (the three parts of a list are arrays of their own: the shifts of an insertion are
     // bound by the order of their loads and stores; 20k queries, k = 100, on 1M points
     // 7.6 ms without the qualifiers, 6.3 with)
@@ -480,7 +489,7 @@ __device__ __forceinline__ void knn_rows_body(const DevTree& t, bool valid, long
         const bool leafwork = !done && cur < 0;
         if (!__any_sync(0xffffffffu, leafwork)) break;
         if (!leafwork) continue;
-        // Two passes: first the slots that can enter the list are marked, with four
+        // Two passes: first the slots that can enter the list are marked, with PAIRS
         // pairs of slots in flight and no branch, so the lanes stay together; then only
         // those are offered.  (Offering in one pass runs the insertion for every slot
         // at which any lane has a candidate.)
@@ -489,12 +498,12 @@ __device__ __forceinline__ void knn_rows_body(const DevTree& t, bool valid, long
         const float4* lp = t.pts + (long long)L * LEAF_CAP;
         const f32x2 qxy = pack2(qx, qy);
         unsigned marks = 0;
-        for (int j0 = 0; j0 < n; j0 += 8) {
-            Quad2 p[4];
+        for (int j0 = 0; j0 < n; j0 += 2 * PAIRS) {
+            Quad2 p[PAIRS];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) p[u] = ld_quad2(lp + j0 + 2 * u);  // (slots past the fill stay in the bucket)
+            for (int u = 0; u < PAIRS; ++u) p[u] = ld_quad2(lp + j0 + 2 * u);  // (slots past the fill stay in the bucket)
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
+            for (int u = 0; u < 2 * PAIRS; ++u) {
                 float z, w;
                 unpack2(p[u >> 1].v[2 * (u & 1) + 1], z, w);
                 const float d = slot_dist(qxy, qz, p[u >> 1].v[2 * (u & 1)], z);
@@ -511,6 +520,21 @@ __device__ __forceinline__ void knn_rows_body(const DevTree& t, bool valid, long
             const float d = sq_dist(qx, qy, qz, p.x, p.y, p.z);
             const int id = (int)(__float_as_uint(p.w) & ID_MASK);
             if (!cand_less(d, id, worst, worst_id)) continue;
+            if constexpr (K > 0) {
+                float cd = d;
+                int ci = id, cs = L * LEAF_CAP + j;
+#pragma unroll
+                for (int m = 0; m < K; ++m) {
+                    const bool sw = cand_less(cd, ci, bd[m], bi[m]);
+                    const float td = bd[m];
+                    const int ti = bi[m], ts = bs[m];
+                    bd[m] = sw ? cd : td, bi[m] = sw ? ci : ti, bs[m] = sw ? cs : ts;
+                    cd = sw ? td : cd, ci = sw ? ti : ci, cs = sw ? ts : cs;
+                }
+                worst = bd[KR - 1];
+                worst_id = bi[KR - 1];
+                continue;
+            }
             int pos = cnt < k ? cnt : k - 1;
             while (pos > 0 && cand_less(d, id, gd[pos - 1], gi[pos - 1])) {
                 gd[pos] = gd[pos - 1];
@@ -530,6 +554,23 @@ __device__ __forceinline__ void knn_rows_body(const DevTree& t, bool valid, long
         pop();
     }
     if (!valid) return;
+    if constexpr (K > 0) {
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            const bool ok = bs[j] >= 0;
+            cnt += ok ? 1 : 0;
+            gi[j] = ok ? bi[j] : -1;
+            gd[j] = bd[j];
+            if (o.xyz != nullptr) {
+                const float4 p = ok ? __ldg(t.pts + bs[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
+                o.xyz[(qi * K + j) * 3 + 0] = p.x;
+                o.xyz[(qi * K + j) * 3 + 1] = p.y;
+                o.xyz[(qi * K + j) * 3 + 2] = p.z;
+            }
+        }
+        if (o.cnt != nullptr) o.cnt[qi] = cnt;
+        return;
+    }
     for (int j = 0; j < k; ++j) {
         const bool ok = j < cnt;
         if (!ok) {

@@ -72,9 +72,10 @@ int ikdg_set_downsample_param(ikdg_tree* t, float box_length);
  * written by (re)builds, 8..32 (default 16); threads cooperating on one kNN
  * query, 1, 2 or 4 (checked, without effect: the searches give every query
  * four lanes); tree levels used to sort a kNN batch into spatially coherent
- * order before the search: -1 (default) sorts by 14 levels where that was
- * measured faster (524,288 queries or more, k >= 8, 12M stored points or
- * more), 0 never sorts, 1..16 sorts every batch of at least 2048 queries.
+ * order before the search: -1 (default) sorts by 16 levels where that was
+ * measured faster (batches of 524,288 queries or more, on small maps, on very
+ * large ones with long lists, or of millions of queries), 0 never sorts, 1..16
+ * sorts every batch of at least 2048 queries.
  * Results depend on none of them. */
 int ikdg_set_leaf_fill(ikdg_tree* t, int fill);
 int ikdg_set_knn_lanes(ikdg_tree* t, int lanes);
