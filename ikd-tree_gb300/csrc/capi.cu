@@ -293,6 +293,7 @@ struct Tree {
         CK(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
         direct = pageable != 0 && std::getenv("IKDG_HOST_STAGING") == nullptr;
         if (const char* e = std::getenv("IKDG_MAX_VISITS")) visit_cap = std::atoi(e);
+        if (const char* e = std::getenv("IKDG_POOL_LIMIT")) pool_limit = std::min(std::atoi(e), pool_limit);
         if (const char* e = std::getenv("IKDG_MAX_LEVELS")) max_levels = std::min(std::atoi(e), MAX_STACK);
         CK(cudaMallocHost(&host_st, sizeof(DevStatus)));
         std::memset(host_st, 0, sizeof(DevStatus));
@@ -349,9 +350,10 @@ struct Tree {
     }
 
     // ---- pools -----------------------------------------------------------------
+    int pool_limit = INT32_MAX / 2;  // nodes or leaves (IKDG_POOL_LIMIT lowers it, for tests)
     void ensure_pools(long long need_nodes, long long need_leaves) {
         int old_n = dt.node_cap, old_l = dt.leaf_cap;
-        if (need_nodes > INT32_MAX / 2 || need_leaves > INT32_MAX / 2) throw CapacityFail{"tree too large"};
+        if (need_nodes > pool_limit || need_leaves > pool_limit) throw CapacityFail{"tree too large"};
         int new_n = old_n, new_l = old_l;
         if (need_nodes > old_n) new_n = (int)std::max<long long>(need_nodes, (long long)old_n * 3 / 2);
         if (need_leaves > old_l) new_l = (int)std::max<long long>(need_leaves, (long long)old_l * 3 / 2);
@@ -420,6 +422,7 @@ struct Tree {
     // The root's position in the top wide record (see common.cuh), and what
     // the searches need to know of the tree's shape.
     int top_pos = 2;
+    long long new_top = -1;  // points of a rebuild of the whole tree that is under way
     void set_top(long long points) {
         const int below = build_levels(std::max<long long>(points, 1), fill) - 1;  // levels below the root
         top_pos = below % 3 == 2 ? 2 : below % 3 == 1 ? 4 : 8;
@@ -544,11 +547,18 @@ struct Tree {
         }
         long long total = st->job_total;
         long long max_job = st->max_job;
-        reserve_build(total, nj);
-        ensure_removed(st->removed_n + st->root_deleted + 1);
-        size_t bytes = align_up(sizeof(float4) * std::max<long long>(total, 1)) +
-                       build_scratch_bytes(std::max<long long>(total, 1), nj) + 4096;
-        bld.ensure(bytes, stream);
+        try {
+            reserve_build(total, nj);
+            ensure_removed(st->removed_n + st->root_deleted + 1);
+            size_t bytes = align_up(sizeof(float4) * std::max<long long>(total, 1)) +
+                           build_scratch_bytes(std::max<long long>(total, 1), nj) + 4096;
+            bld.ensure(bytes, stream);
+        } catch (...) {  // no room: the jobs are dropped, the tree stays as the refit left it
+            launch_job_finish(dt, aux, stream);
+            throw;
+        }
+        if (new_top >= 0) set_top(new_top);  // (from here on the old records are gone)
+        new_top = -1;
         float4* gathered = (float4*)bld.p;
         BuildScratch bs;
         carve_build_scratch((char*)bld.p + align_up(sizeof(float4) * std::max<long long>(total, 1)),
@@ -1252,8 +1262,13 @@ struct Tree {
         if (st->root_code == 0) return;
         reset_counters();
         launch_select_root(dt, aux, stream);
-        set_top((long long)st->root_slots - st->root_deleted);
-        finish_update(nullptr, nullptr, 0, /*refit_first=*/false);
+        new_top = (long long)st->root_slots - st->root_deleted;
+        try {
+            finish_update(nullptr, nullptr, 0, /*refit_first=*/false);
+        } catch (...) {
+            new_top = -1;
+            throw;
+        }
     }
 
     void check_valid(const char* stage, bool at_rest = true) {
