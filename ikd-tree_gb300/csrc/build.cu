@@ -868,8 +868,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_open_kernel(const float4*
     }
 }
 
-// Block-wide bounds of both sides' points into the boxes (nullptr: not wanted).
-// sm: 12 shared words holding reset boxes.
+// A point into a thread's box; the warp's boxes into a shared one (reset before).
 __device__ __forceinline__ void split_grow(uint32_t* b, const float4& p) {
     const uint32_t k[3] = {float_key(p.x), float_key(p.y), float_key(p.z)};
     for (int a = 0; a < 3; ++a) {

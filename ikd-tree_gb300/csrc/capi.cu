@@ -572,7 +572,7 @@ struct Tree {
     }
 
     // After a mutation queued dirty leaves in aux.items: refit, then rebuild
-    // the topmost subtrees that violate the criteria (up to three rounds).
+    // the topmost subtrees that violate the criteria (up to seven rounds).
     void finish_update(const int4* ovf_leaf, const float4* ovf_pts, int ovf_bound, bool refit_first = true) {
         int bound = list_cap;
         if (refit_first) {

@@ -65,7 +65,7 @@ inline void launch_chain(void (*kernel)(P...), dim3 grid, unsigned block, size_t
 }
 
 
-// ---- scan.cu / sort.cu ------------------------------------------------------
+// ---- sort.cu ----------------------------------------------------------------
 // Exclusive prefix sum of n int32 / int64 values; `total` (device, nullable) receives
 // the sum.  `temp` must hold scan_temp_bytes(n) bytes.
 size_t scan_temp_bytes(long long n);

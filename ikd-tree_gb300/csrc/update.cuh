@@ -33,7 +33,8 @@ struct Criteria {
     int fill;       // leaf fill of the builder (height guard)
 };
 
-// Marks / queues leaf L for refit.
+// Appends n points to the buckets they belong to (a full bucket's go to ovf_leaf_pt /
+// ovf_pts) and queues those buckets for the refit.
 void launch_route_append(const DevTree& t, const UpdateAux& a, const float4* pts, long long n, int4* ovf_leaf_pt,
                          float4* ovf_pts, cudaStream_t s);
 // Refit from the codes in a.items[0 .. st->n_items) and record violators;
