@@ -31,8 +31,11 @@ def test_large_boxes_among_many(ikdg_mod, n, m, kind):
         b += 100
     b = b.astype(np.float32)
     gone = np.zeros(n, bool)
+    by_x = np.argsort(pts[:, 0])
+    xs = pts[by_x, 0]
     for x in b:
-        i = np.flatnonzero(~gone)
+        i = by_x[np.searchsorted(xs, x[0]):np.searchsorted(xs, x[3])]
+        i = i[~gone[i]]
         p = pts[i]
         gone[i[((p >= x[:3]) & (p < x[3:])).all(1)]] = True
     assert tree.Delete_Point_Boxes(b) == gone.sum()

@@ -22,8 +22,12 @@ def test_jobs_of_every_size_in_one_call(ikdg_mod, n, big, middle, small):
         boxes += list(np.concatenate([c, c + side], 1))
     b = np.array(boxes, np.float32)
     gone = np.zeros(n, bool)
+    by_x = np.argsort(pts[:, 0])
+    xs = pts[by_x, 0]
     for x in b:
-        gone |= ((pts >= x[:3]) & (pts < x[3:])).all(1)
+        i = by_x[np.searchsorted(xs, x[0]):np.searchsorted(xs, x[3])]
+        p = pts[i]
+        gone[i[((p >= x[:3]) & (p < x[3:])).all(1)]] = True
     assert tree.Delete_Point_Boxes(b) == gone.sum()
     assert tree.validate() == 0 and tree.validnum() == n - gone.sum()
     xyz, ids = tree.flatten(with_ids=True)
