@@ -32,7 +32,7 @@ __device__ __forceinline__ void block_store(float* dst, const float* src, int n)
 // threads' stack columns (`entries` each).  STAGED: the outputs are host memory;
 // the CTA's rows are one span of every array (no permutation), are staged over
 // the stacks once its queries are done and leave as 16-byte stores.
-template <int R, bool STAGED>
+template <int R, bool STAGED, bool EARLY>
 __global__ void __launch_bounds__(KNN_THREADS) knn_group_kernel(DevTree t, const float* __restrict__ q, int q_stride,
                                                                 long long nq, int k, float max_sq, search::KnnOut o,
                                                                 const int* __restrict__ perm, int entries, int per_warp) {
@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(KNN_THREADS) knn_group_kernel(DevTree t, const
     const float qz = valid ? q[qi * q_stride + 2] : 0.f;
     float ld[R];
     int ls[R];
-    search::knn_group<R>(t, g, valid, qx, qy, qz, k, max_sq, reinterpret_cast<int2*>(knn_sm) + threadIdx.x, entries,
+    search::knn_group<R, EARLY>(t, g, valid, qx, qy, qz, k, max_sq, reinterpret_cast<int2*>(knn_sm) + threadIdx.x, entries,
                          per_warp * search::KNN_G / 2, ld, ls);
     if (!STAGED) {
         search::knn_write_rows<R>(t, g, valid, ld, ls, k, qi, o);
@@ -80,6 +80,13 @@ __global__ void __launch_bounds__(KNN_THREADS) knn_group_kernel(DevTree t, const
 // several trees overlap; 15,000 queries 79.7 / 51.5 us.
 constexpr long long KNN_SPREAD_QUERIES = 2048;
 
+// Batches of at most this many queries are bound by the chain of a query and load a
+// bucket's slots beside its fill count; larger ones by issue and occupancy.  3M points, k
+// = 5, us a call alone, after the count / beside it: 1 query 25.8 / 24.7, 2,000 34.6 / 32.3,
+// 15,000 50.6 / 46.0, 30,000 56.5 / 53.4, 45,000 66.5 / 73.9, 80,000 97.9 / 102.5 (k = 32
+// gains up to 80,000, 2 %).
+constexpr long long KNN_EARLY_QUERIES = 32768;
+
 template <int R>
 void knn_group_launch(const DevTree& t, const float* q, int q_stride, long long nq, int k, float max_sq,
                       const search::KnnOut& o, const int* perm, bool staged, cudaStream_t s) {
@@ -88,13 +95,12 @@ void knn_group_launch(const DevTree& t, const float* q, int q_stride, long long 
     const unsigned grid = blocks_for(nq, queries);
     const int entries = search::knn_stack_entries(t.height);
     const size_t stacks = (size_t)KNN_THREADS * entries * sizeof(int2);
-    if (staged) {
-        const size_t rows = (size_t)queries * (5 * k + 1) * sizeof(float);
-        knn_group_kernel<R, true><<<grid, KNN_THREADS, rows > stacks ? rows : stacks, s>>>(t, q, q_stride, nq, k, max_sq,
-                                                                                          o, perm, entries, per_warp);
-    } else {
-        knn_group_kernel<R, false><<<grid, KNN_THREADS, stacks, s>>>(t, q, q_stride, nq, k, max_sq, o, perm, entries, per_warp);
-    }
+    const size_t rows = (size_t)queries * (5 * k + 1) * sizeof(float);
+    const size_t smem = staged && rows > stacks ? rows : stacks;
+    const bool early = nq <= KNN_EARLY_QUERIES;
+    auto kernel = staged ? (early ? knn_group_kernel<R, true, true> : knn_group_kernel<R, true, false>)
+                         : (early ? knn_group_kernel<R, false, true> : knn_group_kernel<R, false, false>);
+    kernel<<<grid, KNN_THREADS, smem, s>>>(t, q, q_stride, nq, k, max_sq, o, perm, entries, per_warp);
 }
 
 // Box (MODE 0) and radius (MODE 1) searches, `per` consecutive queries a warp.

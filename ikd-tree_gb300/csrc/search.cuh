@@ -150,7 +150,9 @@ struct KnnLane {
 // column in shared memory, `entries` entries KNN_CTA apart.  half_lanes: lanes
 // of half the warp's queries.  Leaves the sorted list in ld / ls (slot -1: no
 // entry).
-template <int R>
+// EARLY: a bucket's slots are loaded beside its fill count, not after it, which shortens
+// the chain of a query and costs registers and loads of empty slots (KNN_EARLY_QUERIES).
+template <int R, bool EARLY = false>
 __device__ __forceinline__ void knn_group(const DevTree& t, const KnnLane& g, bool valid, float qx, float qy, float qz,
                                           int k, float max_sq, int2* stk, int entries, int half_lanes, float (&ld)[R],
                                           int (&ls)[R]) {
@@ -215,6 +217,11 @@ __device__ __forceinline__ void knn_group(const DevTree& t, const KnnLane& g, bo
             const int L = act ? code_leaf(cur) : 0;
             const int j0 = half * KNN_LEAF_STEP + S * g.sl;
             const int s0 = L * LEAF_CAP + j0;
+            Quad2 slots[S / 2];
+            if (EARLY && act) {
+#pragma unroll
+                for (int i = 0; i < S / 2; ++i) slots[i] = ld_quad2(t.pts + (long long)s0 + 2 * i);
+            }
             const int n = act ? min(__ldg(t.leaf_n + L), LEAF_CAP) : 0;
             unsigned key[S];
 #pragma unroll
@@ -222,7 +229,7 @@ __device__ __forceinline__ void knn_group(const DevTree& t, const KnnLane& g, bo
             if (act) {
 #pragma unroll
                 for (int i = 0; i < S; i += 2) {
-                    const Quad2 p = ld_quad2(t.pts + (long long)s0 + i);
+                    const Quad2 p = EARLY ? slots[i / 2] : ld_quad2(t.pts + (long long)s0 + i);
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         float z, w;
