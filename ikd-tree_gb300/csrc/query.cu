@@ -74,10 +74,10 @@ __global__ void __launch_bounds__(KNN_THREADS) knn_group_kernel(DevTree t, const
 }
 
 // Batches of at most this many queries get a warp per query (its other groups
-// idle): no query waits for another one's steps.  1M-point map, k = 5, host
-// clock around one call: 1,000 queries 36.3 us a warp each, 46.8 us eight a
-// warp; 4,000 queries 42.9 / 47.6 us, but 14.1 / 12.3 us a call when calls on
-// several trees overlap; 15,000 queries 79.7 / 51.5 us.
+// idle): no query waits for another one's steps.  1M-point map, host clock around
+// one call, a warp each / eight a warp: 1,000 queries k = 5 29.0 / 36.2 us, k = 32 57 / 83;
+// 4,000 queries 34.8 / 39.7 and 90 / 88, but 14.1 / 12.3 (k = 5) a call when calls on
+// several trees overlap; 15,000 queries 71.7 / 41.8.
 constexpr long long KNN_SPREAD_QUERIES = 2048;
 
 // Batches of at most this many queries are bound by the chain of a query and load a

@@ -110,10 +110,10 @@ __device__ __forceinline__ float slot_dist(f32x2 qxy, float qz, f32x2 xy, float 
 // 15 % and 6 % more).
 //
 // 1M-point map, k = 5, kernel time before (a thread per query over the binary
-// records) / now: 1 query 23.6 / 13.7 us, 15k of a LiDAR scan 51 / 24 us, 100k
-// 144 / 96 us (96 / 73 us
+// records) / now: 1 query 23.6 / 13.2 us, 15k of a LiDAR scan 51 / 21 us, 100k
+// 144 / 93 us (96 / 68 us
 // a call when calls on three trees overlap); 20M points, 1M queries, k = 16:
-// 1615 / 1067 us a call.
+// 1595 / 1026 us a call.
 // Bound by instruction issue (the tree is served from L2 and the chain of a
 // query is ~15 loads): a thread per query over the binary records issued less
 // per node but took 27 dependent loads a query, 96 steps a warp (its 32 queries
