@@ -465,8 +465,9 @@ struct Tree {
     void zero_fields(size_t off, size_t bytes) {
         CK(cudaMemsetAsync((char*)st_dev + off, 0, bytes, stream));
     }
-    // Clears the per-call counters.
+    // Clears the per-call counters, and what an earlier call that ended early left behind.
     void reset_counters() {
+        take_chain_refused();
         zero_fields(offsetof(DevStatus, err), offsetof(DevStatus, bad) - offsetof(DevStatus, err));
     }
 

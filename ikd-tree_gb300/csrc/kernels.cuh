@@ -57,7 +57,8 @@ inline void launch_chain_if(bool chain, unsigned cluster, void (*kernel)(P...), 
     cfg.attrs = at;
     cfg.numAttrs = n;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
-    if (e != cudaSuccess && chain_refused == cudaSuccess) chain_refused = e;
+    // (launches outside a chain: left as the thread's last error, as with <<<>>>)
+    if (chain && e != cudaSuccess && chain_refused == cudaSuccess) chain_refused = e;
 }
 template <class... P, class... A>
 inline void launch_chain(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {

@@ -1137,8 +1137,9 @@ __global__ void __launch_bounds__(BD_CTA) box_delete_kernel(DevTree t, UpdateAux
                 break;
             }
             if (limit > 0 && steps == limit) {
-                int base = 0;
-                if (lane == 0) base = atomicAdd(&t.st->n_spill, sp);
+                // (the counter is left alone once the list is full: it must not wrap)
+                int base = spill_cap;
+                if (lane == 0 && __ldcg(&t.st->n_spill) < spill_cap) base = atomicAdd(&t.st->n_spill, sp);
                 base = __shfl_sync(ALL, base, 0);
                 const int k = base < spill_cap ? min(sp, spill_cap - base) : 0;
                 for (int i = lane; i < k; i += 32) spill[base + i] = make_int2(stack[i], (int)bi);
